@@ -199,7 +199,11 @@ template <typename T16> struct PfEpiGate {  // columns (2j, 2j+1) = (w1, w3) col
     }
 };
 
-template <typename T16> struct PfEpiQKV {  // RoPE on q and k; q to a [M, Q] buffer, k and v into the pages
+// RoPE on q and k; q to a [M, Q] buffer, k and v into the pages.  A thread's 32 columns lie inside one head (widths of 64 or
+// 128), so every destination is a run of 64 bytes: 16-byte stores.  (Element by element the epilogue bound the GEMM: 311 us
+// at 1024 x 12288 x 4096 where gate|up, 1.8 times the products, took 300; the 5B model's 1024-token prompt went from 30.5
+// to 25.9 ms, 4096 tokens from 147 to 131 ms, with this and PfEpiAttnOut.)
+template <typename T16> struct PfEpiQKV {
     T16* q;
     T16* q_lo;
     T16* kv_pool;
@@ -217,24 +221,17 @@ template <typename T16> struct PfEpiQKV {  // RoPE on q and k; q to a [M, Q] buf
                 r[2 * j] = v[2 * j] * c.x - v[2 * j + 1] * c.y;
                 r[2 * j + 1] = v[2 * j + 1] * c.x + v[2 * j] * c.y;
             }
-            T16* dst;
             if (col < Q) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) pf_store(q, q_lo, (size_t)row * Q + col + j, r[j]);
+                pf_store_run(q, q_lo, (size_t)row * Q + col, r);
                 return;
-            } else {
-                const int ck = col - Q, head = ck / hd, d = ck % hd;
-                const int page = page_table[pos / page_tokens], off = pos % page_tokens;
-                dst = kv_pool + ((((size_t)page * 2 + 0) * kv_heads + head) * page_tokens + off) * hd + d;
             }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) dst[j] = pf_cast<T16>(r[j]);
+            const int ck = col - Q, head = ck / hd, d = ck % hd;
+            const int page = page_table[pos / page_tokens], off = pos % page_tokens;
+            pf_store_run(kv_pool, (T16*)nullptr, ((((size_t)page * 2 + 0) * kv_heads + head) * page_tokens + off) * hd + d, r);
         } else {
             const int cv = col - Q - KV, head = cv / hd, d = cv % hd;
             const int page = page_table[pos / page_tokens], off = pos % page_tokens;
-            T16* dst = kv_pool + ((((size_t)page * 2 + 1) * kv_heads + head) * page_tokens + off) * hd + d;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) dst[j] = pf_cast<T16>(v[j]);
+            pf_store_run(kv_pool, (T16*)nullptr, ((((size_t)page * 2 + 1) * kv_heads + head) * page_tokens + off) * hd + d, v);
         }
     }
 };
@@ -255,9 +252,7 @@ template <typename T16> struct PfEpiAttnOut {  // head z's output columns of the
     T16* out_lo;
     int ld, hd;
     __device__ void operator()(int z, int row, int col, const float (&v)[32]) const {
-        const size_t at = (size_t)row * ld + z * hd + col;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) pf_store(out, out_lo, at + j, v[j]);
+        pf_store_run(out, out_lo, (size_t)row * ld + z * hd + col, v);
     }
 };
 
