@@ -48,7 +48,7 @@ struct Gemm {
         if (!ok()) return;
         what = name;
         PfGemm p = {};
-        p.M = M; p.N = N; p.K = K; p.b_zdiv = 1; p.page_tokens = m->page_tokens; p.err = &m->st->error;
+        p.M = M; p.N = N; p.K = K; p.err = &m->st->error;
         p.tile_group = tile_group; p.group_rows = group_rows;
         // tiles of 256 columns, of 128 where the wide ones would leave SMs without work
         const int mt = (M + PF_BM - 1) / PF_BM;
@@ -59,7 +59,7 @@ struct Gemm {
         const bool maps = encode_2d(w->encode, &a[0], dt, hi, K, a_rows, (uint64_t)K * 2, PF_BM) && encode_2d(w->encode, &a[1], dt, split ? lo : hi, K, a_rows, (uint64_t)K * 2, PF_BM) &&
                           encode_2d(w->encode, &b, dt, B, K, b_rows, (uint64_t)K * 2, wide ? 256 : 128);
         if (!maps) { e = cudaErrorInvalidValue; return; }
-        e = wide ? pf_launch<256>(m, split, a, b, p, true, 1, epi) : pf_launch<128>(m, split, a, b, p, true, 1, epi);
+        e = wide ? pf_launch<256>(m, split, a, b, p, true, epi) : pf_launch<128>(m, split, a, b, p, true, epi);
     }
 };
 

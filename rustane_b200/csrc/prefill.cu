@@ -34,7 +34,7 @@ struct PrefillCtx {
     SampleGraphKey s_key;
     std::map<int, cudaGraphExec_t> s_graphs;  // captured multi-sample steps by number of occupied attention slices
     uint64_t s_graph_nodes = 0;
-    std::vector<CUtensorMap> w_qkv, w_o, w_13, w_2, k_pages;  // per layer, built once
+    std::vector<CUtensorMap> w_qkv, w_o, w_13, w_2, k_pages, v_pages;  // per layer, built once
     CUtensorMap w_head;
     std::vector<CUtensorMap> sk_qkv, sk_o, sk_13, sk_2;  // the same matrices in 128-row boxes (multi-sample decode)
     CUtensorMap sk_head;
@@ -51,27 +51,17 @@ struct PrefillCtx {
     void *sxn = nullptr, *sgate = nullptr;  // [2][s_cap][...] hi, lo
     DevState* sst = nullptr;
     // workspace (grow-only)
-    size_t rows = 0, key_ld = 0;
+    size_t rows = 0;
     float* x = nullptr;       // [rows][dim] residual stream
     void* xn = nullptr;       // [2][rows][max(dim, q_dim)] normalised input / attention output (hi, lo)
     void* q = nullptr;        // [2][rows][q_dim]
     void* gate = nullptr;     // [2][rows][hidden]
-    float* s = nullptr;       // [heads][rows][key_ld]
-    void* p = nullptr;        // [2][heads][rows][key_ld]
-    void* vt = nullptr;       // [kv_heads * hd][key_ld]
 };
 
-// the K half of one layer's pages as {d, token in page, kv head, k|v, page}; a box is 128 keys of one head
-bool encode_k_pages(PrefillCtx* c, CUtensorMap* map, CUtensorMapDataType dt, const void* base, int hd, int page_tokens, int kv_heads,
-                    int num_pages) {
-    const cuuint64_t dims[5] = {(cuuint64_t)hd, (cuuint64_t)page_tokens, (cuuint64_t)kv_heads, 2, (cuuint64_t)num_pages};
-    const cuuint64_t e = 2;
-    const cuuint64_t strides[4] = {hd * e, (cuuint64_t)page_tokens * hd * e, (cuuint64_t)kv_heads * page_tokens * hd * e,
-                                   (cuuint64_t)2 * kv_heads * page_tokens * hd * e};
-    const cuuint32_t box[5] = {(cuuint32_t)PF_BK, (cuuint32_t)page_tokens, 1, 1, (cuuint32_t)(128 / page_tokens)};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return c->encode(map, dt, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+// one of the two halves (K, V) of a layer's pages as {d, token in page, kv head, page}; a box is 128 keys of one head
+bool encode_pages(PrefillCtx* c, CUtensorMap* map, CUtensorMapDataType dt, const char* pool, int half, int hd, int page_tokens, int kv_heads, int num_pages) {
+    const uint64_t head = (uint64_t)page_tokens * hd * 2, page = 2 * kv_heads * head;
+    return encode_rows_4d(c->encode, map, dt, pool + half * kv_heads * head, hd, page_tokens, kv_heads, num_pages, (uint64_t)hd * 2, head, page);
 }
 
 // the few-rows GEMM: w in 128-row boxes, x = the [NB][K] activation block (hi rows, then lo rows)
@@ -109,10 +99,14 @@ int ensure_weight_maps(cd_model* m, PrefillCtx* c, CUtensorMapDataType dt, CUten
     if (!c->w_qkv.empty()) return CD_OK;
     const cd_config& cf = m->cfg;
     const int D = cf.dim, Q = cf.q_dim, KV = cf.kv_dim, H = cf.hidden;
-    c->w_qkv.resize(cf.nlayers); c->w_o.resize(cf.nlayers); c->w_13.resize(cf.nlayers); c->w_2.resize(cf.nlayers); c->k_pages.resize(cf.nlayers);
+    c->w_qkv.resize(cf.nlayers); c->w_o.resize(cf.nlayers); c->w_13.resize(cf.nlayers); c->w_2.resize(cf.nlayers); c->k_pages.resize(cf.nlayers); c->v_pages.resize(cf.nlayers);
     c->sk_qkv.resize(cf.nlayers); c->sk_o.resize(cf.nlayers); c->sk_13.resize(cf.nlayers); c->sk_2.resize(cf.nlayers);
     bool ok = encode_2d(c->encode, &c->w_head, dt, m->lm_head, D, m->v_loc, (uint64_t)D * 2, 256) &&
               encode_2d(c->encode, &c->sk_head, dt, m->lm_head, D, m->v_loc, (uint64_t)D * 2, 128);
+    auto pages = [&](int l) {
+        return encode_pages(c, &c->k_pages[l], kdt, (const char*)m->layers[l].kv, 0, cf.hd, m->page_tokens, cf.kv_heads, m->num_pages) &&
+               encode_pages(c, &c->v_pages[l], kdt, (const char*)m->layers[l].kv, 1, cf.hd, m->page_tokens, cf.kv_heads, m->num_pages);
+    };
     if (m->opt.weight_dtype == CD_DTYPE_FP8_E4M3) {
         const size_t n_qkv = (size_t)(Q + 2 * KV) * D, n_o = (size_t)D * Q, n_13 = (size_t)2 * H * D, n_2 = (size_t)D * H;
         if (cudaMalloc(&c->f8_qkv, n_qkv * 2) != cudaSuccess || cudaMalloc(&c->f8_o, n_o * 2) != cudaSuccess ||
@@ -125,7 +119,7 @@ int ensure_weight_maps(cd_model* m, PrefillCtx* c, CUtensorMapDataType dt, CUten
             ok = ok && encode_2d(c->encode, &c->w_o[l], dt, c->f8_o, Q, D, (uint64_t)Q * 2, 256);
             ok = ok && encode_2d(c->encode, &c->w_13[l], dt, c->f8_13, D, 2 * H, (uint64_t)D * 2, 256);
             ok = ok && encode_2d(c->encode, &c->w_2[l], dt, c->f8_2, H, D, (uint64_t)H * 2, 256);
-            ok = ok && encode_k_pages(c, &c->k_pages[l], kdt, m->layers[l].kv, cf.hd, m->page_tokens, cf.kv_heads, m->num_pages);
+            ok = ok && pages(l);
         }
         if (!ok) { c->w_qkv.clear(); return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for a weight matrix"); }
         return CD_OK;
@@ -140,7 +134,7 @@ int ensure_weight_maps(cd_model* m, PrefillCtx* c, CUtensorMapDataType dt, CUten
         ok = ok && encode_2d(c->encode, &c->w_o[l], dt, L.wo, Q, D, (uint64_t)Q * 2, 256);
         ok = ok && encode_2d(c->encode, &c->w_13[l], dt, L.w13, D, 2 * H, (uint64_t)D * 2, 256);
         ok = ok && encode_2d(c->encode, &c->w_2[l], dt, L.w2, H, D, (uint64_t)H * 2, 256);
-        ok = ok && encode_k_pages(c, &c->k_pages[l], kdt, L.kv, cf.hd, m->page_tokens, cf.kv_heads, m->num_pages);
+        ok = ok && pages(l);
     }
     if (!ok) { c->w_qkv.clear(); return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for a weight matrix"); }
     return CD_OK;
@@ -177,41 +171,38 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
     const CUtensorMapDataType dt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const CUtensorMapDataType kdt = kbf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const int D = cf.dim, Q = cf.q_dim, KV = cf.kv_dim, H = cf.hidden, hd = cf.hd;
-    const int pos0 = (int)m->len, M = (int)n, nkeys = pos0 + M;
+    const int pos0 = (int)m->len, M = (int)n;
     auto cuda_fail = [&](const char* what, cudaError_t e) { return fail(m, CD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)); };
 
     int rc = ensure_weight_maps(m, c, dt, kdt);
     if (rc) return rc;
     // ---- workspace
-    const size_t rows = round_up(n, PF_BM), key_ld = round_up((size_t)nkeys, 128);
-    if (rows > c->rows || key_ld > c->key_ld) {
-        for (void* ptr : {(void*)c->x, c->xn, c->q, c->gate, (void*)c->s, c->p, c->vt}) if (ptr) cudaFree(ptr);
-        c->x = nullptr; c->xn = c->q = c->gate = c->p = c->vt = nullptr; c->s = nullptr;
-        const size_t r = std::max(rows, c->rows), k = std::max(key_ld, c->key_ld);
-        c->rows = c->key_ld = 0;
+    const size_t rows = round_up(n, PF_BM);
+    if (rows > c->rows) {
+        for (void* ptr : {(void*)c->x, c->xn, c->q, c->gate}) if (ptr) cudaFree(ptr);
+        c->x = nullptr; c->xn = c->q = c->gate = nullptr;
+        const size_t r = rows;
+        c->rows = 0;
         struct { void** ptr; size_t bytes; } want[] = {
-            {(void**)&c->x, r * D * 4}, {&c->xn, 2 * r * (size_t)std::max(D, Q) * 2}, {&c->q, 2 * r * (size_t)Q * 2}, {&c->gate, 2 * r * (size_t)H * 2},
-            {(void**)&c->s, (size_t)cf.heads * r * k * 4}, {&c->p, 2 * (size_t)cf.heads * r * k * 2}, {&c->vt, (size_t)cf.kv_heads * hd * k * 2}};
+            {(void**)&c->x, r * D * 4}, {&c->xn, 2 * r * (size_t)std::max(D, Q) * 2}, {&c->q, 2 * r * (size_t)Q * 2}, {&c->gate, 2 * r * (size_t)H * 2}};
         for (auto& w : want) {
             cudaError_t e = cudaMalloc(w.ptr, w.bytes);
             if (e == cudaSuccess) e = cudaMemsetAsync(*w.ptr, 0, w.bytes, m->stream);
             if (e != cudaSuccess) return cuda_fail("prefill workspace", e);
         }
-        c->rows = r; c->key_ld = k;
+        c->rows = r;
     }
-    const size_t R = c->rows, KL = c->key_ld, plane = R * KL;
+    const size_t R = c->rows;
     // hi matrices first, lo matrices (split mode) in the second half of each buffer
-    T16* xn = (T16*)c->xn; KT* qb = (KT*)c->q; T16* gate = (T16*)c->gate; KT* pm = (KT*)c->p; KT* vt = (KT*)c->vt;
+    T16* xn = (T16*)c->xn; KT* qb = (KT*)c->q; T16* gate = (T16*)c->gate;
     T16* xn_lo = split ? xn + R * (size_t)std::max(D, Q) : nullptr;
     KT* q_lo = split ? qb + R * (size_t)Q : nullptr;
     T16* gate_lo = split ? gate + R * (size_t)H : nullptr;
-    KT* p_lo = split ? pm + (size_t)cf.heads * plane : nullptr;
-    CUtensorMap a_xn[2], a_attn[2], a_gate[2], a_q[2], a_p[2], b_vt;
-    bool ok = encode_2d(c->encode, &b_vt, kdt, c->vt, KL, (uint64_t)cf.kv_heads * hd, (uint64_t)KL * 2, (uint32_t)hd);
+    CUtensorMap a_xn[2], a_attn[2], a_gate[2], a_q[2];
+    bool ok = true;
     for (int h = 0; h < (split ? 2 : 1) && ok; ++h) {
         ok = encode_2d(c->encode, &a_xn[h], dt, h ? xn_lo : xn, D, R, (uint64_t)D * 2, PF_BM) && encode_2d(c->encode, &a_attn[h], dt, h ? xn_lo : xn, Q, R, (uint64_t)Q * 2, PF_BM) &&
-             encode_2d(c->encode, &a_gate[h], dt, h ? gate_lo : gate, H, R, (uint64_t)H * 2, PF_BM) && encode_2d(c->encode, &a_q[h], kdt, h ? q_lo : qb, Q, R, (uint64_t)Q * 2, PF_BM) &&
-             encode_2d(c->encode, &a_p[h], kdt, h ? p_lo : pm, KL, (uint64_t)cf.heads * R, (uint64_t)KL * 2, PF_BM);
+             encode_2d(c->encode, &a_gate[h], dt, h ? gate_lo : gate, H, R, (uint64_t)H * 2, PF_BM) && encode_2d(c->encode, &a_q[h], kdt, h ? q_lo : qb, Q, R, (uint64_t)Q * 2, PF_BM);
     }
     if (!ok) return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for an activation buffer");
 
@@ -235,8 +226,8 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
         return cudaGetLastError();
     };
     PfGemm g = {};
-    g.b_zdiv = 1; g.page_tokens = m->page_tokens; g.pos0 = pos0; g.err = &m->st->error;
-    const float scale = 1.0f / std::sqrt((float)hd);
+    g.err = &m->st->error;
+    const PfAttn attn{M, pos0, 0, 1, cf.gqa_ratio, m->page_tokens, split ? 1 : 0, (float)(1.4426950408889634 / std::sqrt((double)hd)), nullptr, &m->st->error};
     const bool fp8 = m->opt.weight_dtype == CD_DTYPE_FP8_E4M3;
     auto quantised = [&](PfGemm& p, const void* rows, int K) {  // the GEMM's output columns take the FP8 row scales
         if (!fp8) return;
@@ -258,31 +249,19 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
             PfGemm p = g; p.M = M; p.N = Q + 2 * KV; p.K = D;
             quantised(p, L.wqkv, D);
             PfEpiQKV<KT> epi{qb, q_lo, (KT*)L.kv, m->page_table, m->rope, Q, KV, hd, cf.kv_heads, m->page_tokens, pos0};
-            PF_TRY("qkv gemm", (pf_launch<256>(m, split, a_xn, c->w_qkv[l], p, bf16, 1, epi)));
+            PF_TRY("qkv gemm", (pf_launch<256>(m, split, a_xn, c->w_qkv[l], p, bf16, epi)));
         }
-        pf_transpose_v_kernel<KT><<<dim3((unsigned)(KL / 64), cf.kv_heads), 256, 0, m->stream>>>((const KT*)L.kv, m->page_table, vt, nkeys, (int)KL,
-                                                                                                 cf.kv_heads, hd, m->page_tokens);
-        m->launches++;
-        {   // scores = q k^T per head over the cached keys (tiles above the diagonal skipped)
-            PfGemm p = g; p.M = M; p.N = nkeys; p.K = hd; p.a_col_z = hd; p.b_zdiv = cf.gqa_ratio; p.b_paged = 1; p.causal = 1;
-            PF_TRY("score gemm", (pf_launch<128>(m, split, a_q, c->k_pages[l], p, kbf16, cf.heads, PfEpiScores{c->s, plane, (int)KL})));
-        }
-        pf_softmax_kernel<KT><<<dim3(M, cf.heads), 256, 0, m->stream>>>(c->s, pm, p_lo, plane, (int)KL, pos0, scale);
-        m->launches++;
-        {   // attention output = P V per head (the K loop stops at the diagonal)
-            PfGemm p = g; p.M = M; p.N = hd; p.K = nkeys; p.a_row_z = (int)R; p.b_row_z = hd; p.b_zdiv = cf.gqa_ratio; p.causal = 2;
-            PfEpiAttnOut<T16> epi{xn, xn_lo, Q, hd};
-            if (hd == 128) PF_TRY("pv gemm", (pf_launch<128>(m, split, a_p, b_vt, p, kbf16, cf.heads, epi)));
-            else PF_TRY("pv gemm", (pf_launch<64>(m, split, a_p, b_vt, p, kbf16, cf.heads, epi)));
-        }
+        const PaOut<T16> attn_out{xn, xn_lo, Q, hd};
+        if (hd == 128) PF_TRY("attention", (pa_launch<KT, 128, 128, false>(m, a_q, split, c->k_pages[l], c->v_pages[l], attn, cf.heads, attn_out)));
+        else PF_TRY("attention", (pa_launch<KT, 64, 64, false>(m, a_q, split, c->k_pages[l], c->v_pages[l], attn, cf.heads, attn_out)));
         {   // x2 = x + alpha * (attn Wo)
             PfGemm p = g; p.M = M; p.N = D; p.K = Q;
             quantised(p, L.wo, Q);
             if (tpar) {
-                PF_TRY("wo gemm", (pf_launch<256>(m, split, a_attn, c->w_o[l], p, bf16, 1, PfEpiPartial{tp_buf(), D})));
+                PF_TRY("wo gemm", (pf_launch<256>(m, split, a_attn, c->w_o[l], p, bf16, PfEpiPartial{tp_buf(), D})));
                 PF_TRY("wo all-reduce", tp_allreduce());
             } else {
-                PF_TRY("wo gemm", (pf_launch<256>(m, split, a_attn, c->w_o[l], p, bf16, 1, PfEpiResidual{c->x, D, m->alpha})));
+                PF_TRY("wo gemm", (pf_launch<256>(m, split, a_attn, c->w_o[l], p, bf16, PfEpiResidual{c->x, D, m->alpha})));
             }
         }
         pf_rmsnorm_kernel<T16><<<M, 256, 0, m->stream>>>(c->x, L.gamma2, xn, xn_lo, D);
@@ -290,16 +269,16 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
         {   // gate = act(x2n W1) * (x2n W3)
             PfGemm p = g; p.M = M; p.N = 2 * H; p.K = D;
             quantised(p, L.w13, D);
-            PF_TRY("w13 gemm", (pf_launch<256>(m, split, a_xn, c->w_13[l], p, bf16, 1, PfEpiGate<T16>{gate, gate_lo, H, m->opt.activation})));
+            PF_TRY("w13 gemm", (pf_launch<256>(m, split, a_xn, c->w_13[l], p, bf16, PfEpiGate<T16>{gate, gate_lo, H, m->opt.activation})));
         }
         {   // x = x2 + alpha * (gate W2^T)
             PfGemm p = g; p.M = M; p.N = D; p.K = H;
             quantised(p, L.w2, H);
             if (tpar) {
-                PF_TRY("w2 gemm", (pf_launch<256>(m, split, a_gate, c->w_2[l], p, bf16, 1, PfEpiPartial{tp_buf(), D})));
+                PF_TRY("w2 gemm", (pf_launch<256>(m, split, a_gate, c->w_2[l], p, bf16, PfEpiPartial{tp_buf(), D})));
                 PF_TRY("w2 all-reduce", tp_allreduce());
             } else {
-                PF_TRY("w2 gemm", (pf_launch<256>(m, split, a_gate, c->w_2[l], p, bf16, 1, PfEpiResidual{c->x, D, m->alpha})));
+                PF_TRY("w2 gemm", (pf_launch<256>(m, split, a_gate, c->w_2[l], p, bf16, PfEpiResidual{c->x, D, m->alpha})));
             }
         }
     }
@@ -542,7 +521,7 @@ void prefill_release(cd_model* m) {
     PrefillCtx* c = (PrefillCtx*)m->prefill_ctx;
     if (!c) return;
     for (auto& kv : c->s_graphs) cudaGraphExecDestroy(kv.second);
-    for (void* ptr : {(void*)c->x, c->xn, c->q, c->gate, (void*)c->s, c->p, c->vt, (void*)c->s_arena, c->f8_qkv, c->f8_o, c->f8_13, c->f8_2}) if (ptr) cudaFree(ptr);
+    for (void* ptr : {(void*)c->x, c->xn, c->q, c->gate, (void*)c->s_arena, c->f8_qkv, c->f8_o, c->f8_13, c->f8_2}) if (ptr) cudaFree(ptr);
     delete c;
     m->prefill_ctx = nullptr;
 }

@@ -1,8 +1,7 @@
 // Batched prefill for sm_100a: every linear of the prompt pass is one tensor-core GEMM
 //   C[M tokens, N features] = A[M, K] (activations, 16-bit) * B[N, K]^T (weights as stored for the GEMVs)
 // issued with tcgen05.mma, accumulators in tensor memory, operands staged by TMA.
-// The same kernel also computes the attention of the prompt as two batched GEMMs per
-// layer (scores = Q K^T over the paged cache, output = P V) with a row softmax between.
+// The attention of the prompt between them is pf_attn_kernel (pf_attn.cuh).
 // Math follows the naive forward (full_model.rs:336-437, layer.rs:1287-1431) restricted to
 // the prompt positions; K and V land in the decode layout (pages).  There is no batched
 // prompt pass in the reference's Metal decoder: it feeds prompt tokens one at a time
@@ -18,7 +17,7 @@
 //
 // Further down: pf_skinny_kernel, the same machinery with the operands swapped for at most 16
 // activation rows (several samples decoding together), its epilogues, and the small kernels
-// around both (embedding rows, RMSNorm to hi + lo 16-bit operands, softmax, V transpose).
+// around both (embedding rows, RMSNorm to hi + lo 16-bit operands).
 #pragma once
 #include <cuda.h>
 
@@ -39,15 +38,7 @@ template <int BN, bool SPLIT> struct PfTile {
 };
 
 struct PfGemm {
-    int M, N, K;        // one problem per blockIdx.z
-    int a_col_z;        // A column offset per z (a head's slice of q; 0 otherwise)
-    int a_row_z;        // A row offset per z (a head's plane of P)
-    int b_row_z;        // B row offset per z / b_zdiv (a kv head's rows of V^T)
-    int b_zdiv;         // query heads per kv head
-    int b_paged;        // 1: B is the K half of the paged cache through a 5-D map {d, token, kv head, k|v, page}
-    int page_tokens;
-    int causal;         // 1: tiles wholly above the diagonal are skipped; 2: the K loop stops at the diagonal
-    int pos0;           // tokens already cached before this prompt chunk
+    int M, N, K;
     int* err;
     // FP8 linears: B holds the e4m3 values widened to 16 bits; output column n is multiplied by the
     // row scale stored behind row n of the quantised matrix (Wfmt<Fp8Row>), nullptr otherwise
@@ -63,10 +54,6 @@ struct PfGemm {
 __device__ inline void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-__device__ inline void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
 __device__ inline void tmem_alloc(uint32_t slot_smem, uint32_t ncols) {  // whole warp
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
@@ -236,26 +223,6 @@ template <typename T16> struct PfEpiQKV {
     }
 };
 
-struct PfEpiScores {  // raw q.k into the fp32 score planes [heads][rows][ld]
-    float* s;
-    size_t plane;
-    int ld;
-    __device__ void operator()(int z, int row, int col, const float (&v)[32]) const {
-        float4* p = reinterpret_cast<float4*>(s + (size_t)z * plane + (size_t)row * ld + col);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) p[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-    }
-};
-
-template <typename T16> struct PfEpiAttnOut {  // head z's output columns of the [M, Q] attention buffer
-    T16* out;
-    T16* out_lo;
-    int ld, hd;
-    __device__ void operator()(int z, int row, int col, const float (&v)[32]) const {
-        pf_store_run(out, out_lo, (size_t)row * ld + z * hd + col, v);
-    }
-};
-
 // ------------------------------------------------------------------ the GEMM
 template <int BN, bool SPLIT, class Epi>
 __global__ void __launch_bounds__(PF_THREADS, 1)
@@ -265,17 +232,14 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     constexpr uint32_t B_OFF = (SPLIT ? 2 : 1) * TL::A_BYTES;  // stage = A hi | A lo (SPLIT) | B
     constexpr int NST = TL::NST;
     extern __shared__ unsigned char pf_raw[];
-    const int m0 = blockIdx.y * PF_BM, n0 = blockIdx.x * BN, z = blockIdx.z;
-    if (p.causal == 1 && n0 > p.pos0 + m0 + PF_BM - 1) return;  // every key of this tile lies after every query of it
+    const int m0 = blockIdx.y * PF_BM, n0 = blockIdx.x * BN;
     int b_row0 = n0;
     if (p.tile_group != nullptr) {
         const int g = p.tile_group[blockIdx.y];
         if (g < 0) return;
         b_row0 += g * p.group_rows;
     }
-    int kmax = p.K;
-    if (p.causal == 2) kmax = min(kmax, p.pos0 + m0 + PF_BM);    // P is zero beyond the diagonal
-    const int nkb = (kmax + PF_BK - 1) / PF_BK;
+    const int nkb = (p.K + PF_BK - 1) / PF_BK;
 
     const uint32_t tiles = (smem_addr(pf_raw) + 1023u) & ~1023u;
     const uint32_t bars = tiles + NST * TL::STAGE;
@@ -300,7 +264,6 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 
     if (warp == 0) {
         if (lane == 0) {  // ---- TMA producer
-            const int zb = z / p.b_zdiv;
             for (int kb = 0; kb < nkb; ++kb) {
                 const int s = kb % NST;
                 if (kb >= NST && !mbar_wait(empty0 + 8u * s, ((kb / NST) - 1) & 1)) {
@@ -310,10 +273,9 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
                 }
                 const uint32_t a_dst = tiles + s * TL::STAGE, b_dst = a_dst + B_OFF;
                 mbar_arrive_expect_tx(full0 + 8u * s, TL::STAGE);
-                tma_load_2d(a_dst, &tma_a, z * p.a_col_z + kb * PF_BK, z * p.a_row_z + m0, full0 + 8u * s);
-                if (SPLIT) tma_load_2d(a_dst + TL::A_BYTES, &tma_a_lo, z * p.a_col_z + kb * PF_BK, z * p.a_row_z + m0, full0 + 8u * s);
-                if (p.b_paged) tma_load_5d(b_dst, &tma_b, kb * PF_BK, 0, zb, 0, n0 / p.page_tokens, full0 + 8u * s);
-                else tma_load_2d(b_dst, &tma_b, kb * PF_BK, zb * p.b_row_z + b_row0, full0 + 8u * s);
+                tma_load_2d(a_dst, &tma_a, kb * PF_BK, m0, full0 + 8u * s);
+                if (SPLIT) tma_load_2d(a_dst + TL::A_BYTES, &tma_a_lo, kb * PF_BK, m0, full0 + 8u * s);
+                tma_load_2d(b_dst, &tma_b, kb * PF_BK, b_row0, full0 + 8u * s);
             }
         }
     } else if (warp == 1) {
@@ -360,7 +322,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
                     for (int i = 0; i < 32; ++i)
                         v[i] *= *reinterpret_cast<const float*>(p.qrows + (size_t)(n0 + c * 32 + i) * p.qstride + p.qscale_off);
                 }
-                if (row < p.M && n0 + c * 32 < p.N) epi(z, row, n0 + c * 32, v);
+                if (row < p.M && n0 + c * 32 < p.N) epi(0, row, n0 + c * 32, v);
             }
         }
     }
@@ -634,50 +596,6 @@ __global__ void __launch_bounds__(1024) pf_reduce_rmsnorm_kernel(float* __restri
     }
     const float inv = 1.0f / sqrtf(block_sum(ss, red) * (1.0f / (float)D) + RMS_EPS);
     for (int i = threadIdx.x; i < D; i += blockDim.x) pf_store(out, out_lo, (size_t)blockIdx.x * D + i, row[i] * inv * gamma[i]);
-}
-
-// V of the first ntok cached positions, transposed per kv head: vt[head][d][tok] (ld = ntok rounded up)
-template <typename T16>
-__global__ void __launch_bounds__(256) pf_transpose_v_kernel(const T16* __restrict__ kv_pool, const int* __restrict__ page_table, T16* __restrict__ vt,
-                                                             int ntok, int ld, int kv_heads, int hd, int page_tokens) {
-    __shared__ T16 tile[64][130];
-    const int t0 = blockIdx.x * 64, head = blockIdx.y;
-    for (int j = threadIdx.x; j < 64 * hd; j += blockDim.x) {
-        const int t = j / hd, d = j % hd, tok = t0 + t;
-        T16 val = pf_cast<T16>(0.0f);
-        if (tok < ntok) {
-            const int page = page_table[tok / page_tokens], off = tok % page_tokens;
-            val = kv_pool[((((size_t)page * 2 + 1) * kv_heads + head) * page_tokens + off) * hd + d];
-        }
-        tile[t][d] = val;
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < 64 * hd; j += blockDim.x) {
-        const int d = j / 64, t = j % 64;
-        if (t0 + t < ld) vt[((size_t)head * hd + d) * ld + t0 + t] = tile[t][d];
-    }
-}
-
-// Causal softmax of one query row of one head: p = exp(s * scale - max) / sum over keys
-// 0 .. pos0 + row (sdpa_fwd.rs:36-46, :325-354), written as 16-bit; the rest of the row up
-// to where the P V product stops reading (the end of the row's 128-row tile) is zeroed.
-template <typename T16>
-__global__ void __launch_bounds__(256) pf_softmax_kernel(const float* __restrict__ s, T16* __restrict__ pmat, T16* __restrict__ pmat_lo, size_t plane,
-                                                         int ld, int pos0, float scale) {
-    __shared__ float red[32];
-    const int row = blockIdx.x, z = blockIdx.y;
-    const float* srow = s + (size_t)z * plane + (size_t)row * ld;
-    const size_t prow = (size_t)z * plane + (size_t)row * ld;
-    const int valid = pos0 + row + 1;
-    const int upto = min(ld, pos0 + (row / PF_BM + 1) * PF_BM);
-    float mx = -INFINITY;
-    for (int i = threadIdx.x; i < valid; i += blockDim.x) mx = fmaxf(mx, srow[i] * scale);
-    mx = block_max(mx, red);
-    float sum = 0.0f;
-    for (int i = threadIdx.x; i < valid; i += blockDim.x) sum += expf(srow[i] * scale - mx);
-    sum = block_sum(sum, red);
-    const float inv = 1.0f / sum;
-    for (int i = threadIdx.x; i < upto; i += blockDim.x) pf_store(pmat, pmat_lo, prow + i, i < valid ? expf(srow[i] * scale - mx) * inv : 0.0f);
 }
 
 // ---------------------------------------------------------------------- tensor parallel: all-reduce of a [rows, dim] partial product

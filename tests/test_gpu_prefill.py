@@ -134,3 +134,21 @@ def test_logits_at_chosen_places_of_a_prompt(R, oracle, dtype):
     assert float(np.abs(gm.prefill_logits(prompt[11:16], [4]) - ref[15]).max()) < (1e-4 if dtype == "f32" else SPLIT_TOL)
     with pytest.raises(R.CudaDecodeError):
         gm.prefill_logits(prompt[:3], [3])
+
+
+@pytest.mark.parametrize("hd,kv_heads,page", [(64, 1, 32), (128, 4, 64), (128, 2, 128)])
+@pytest.mark.parametrize("cached,n", [(0, 8), (0, 127), (0, 128), (0, 129), (0, 257), (100, 156), (130, 255)])
+def test_attention_at_the_edges_of_its_tiles(R, oracle, hd, kv_heads, page, cached, n):
+    """Prompt lengths around 128 keys and 256 query rows, with and without cached tokens ahead of the chunk, over grouped heads
+    and page sizes.  Whatever the cache holds behind the last key (NaN here) must not reach the logits."""
+    dims = (256, 320, 4, hd, 512, 2, 300)
+    oc, om, gm = _models(R, oracle, dims, "bf16", dict(kv_heads=kv_heads, page_tokens=page))
+    nan = np.full(oc.kv_heads * hd * oc.seq, np.nan, np.float32)
+    for l in range(oc.nlayers):
+        gm.seed_layer_cache_from_channel_first(l, oc.seq, nan, nan)
+    prompt = oracle.synth_prompt(9, oc.vocab, cached + n)
+    _, ref = _oracle_prefill(oracle, om, prompt)
+    gm.set_len(0)
+    if cached:
+        gm.prefill(prompt[:cached], want_logits=False)
+    assert float(np.abs(gm.prefill(prompt[cached:]) - ref).max()) < SPLIT_TOL
