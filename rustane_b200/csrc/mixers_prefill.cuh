@@ -264,6 +264,31 @@ __global__ void __launch_bounds__(128) attn_window_kernel(const __grid_constant_
             for (int c = a.H * a.vdim; c < p.out_ld; ++c) pf_store(out_hi, out_lo, (size_t)(r0 + r) * p.out_ld + c, 0.0f);
 }
 
+// The same attention through pf_attn_kernel: what becomes of a query row's output there.  (m, l: the row's reference in log2
+// units and the sum of its probabilities relative to it.)
+template <typename AT> struct PaWindowOut {
+    AttnWindow w;
+    AT *hi, *lo;
+    __device__ float factor(int z, int row, float m, float l) const {
+        const int h = z / w.a.maps;
+        float f = 1.0f / l;
+        if (w.sink != nullptr) {
+            const float s = w.sink[h] * 1.4426950408889634f, M = fmaxf(m, s), e = exp2f(m - M);
+            f = e / (l * e + exp2f(s - M));
+        }
+        return w.a.gate == 1 ? f * sigmoid(w.proj[(size_t)row * w.proj_ld + w.gate_off + h]) : f;
+    }
+    __device__ void operator()(int z, int row, int col, const float (&v)[32]) const {
+        if (w.raw != nullptr) {
+            float4* p = reinterpret_cast<float4*>(w.raw + ((size_t)row * w.a.H * w.a.maps + z) * w.a.vdim + col);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) p[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        } else {
+            pf_store_run(hi, lo, (size_t)row * w.out_ld + z * w.a.vdim + col, v);
+        }
+    }
+};
+
 // per token: the second map's output subtracted from the first's, each head divided by its root mean square, times the
 // constant factor and the gate of every element; one warp per head
 template <typename AT>

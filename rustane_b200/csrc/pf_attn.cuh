@@ -282,9 +282,9 @@ pf_attn_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant_
             const bool inner = key0 + PA_KEYS - 1 <= first_pos && (p.window <= 0 || key0 > first_pos + 127 - p.window);
             float mx = -INFINITY;
             if (BIAS) {
-                const float base = slope * (float)(pos - key0);
+                const float d0 = (float)(pos - key0);
 #pragma unroll
-                for (int i = 0; i < 128; ++i) s[i] = fmaf(s[i], p.scale_log2, fmaf(slope, (float)i, -base));
+                for (int i = 0; i < 128; ++i) s[i] = fmaf(-slope, d0 - (float)i, s[i] * p.scale_log2);
             }
             if (!inner) {
                 const int hi = pos - key0, lo = p.window > 0 ? hi - p.window : -1;  // visible: lo < i <= hi

@@ -86,6 +86,20 @@ def test_portions_of_a_prompt_do_not_change_its_logits(R, made, name, portions):
     assert M.error(all_logits(m, ids, list(portions)), ref) < TOL["bf16"]
 
 
+@pytest.mark.parametrize("dim,vdim,window", [(128, 128, 150), (64, 64, None), (64, 128, 300)])
+def test_heads_on_tensor_memory(R, tmp_path, dim, vdim, window):
+    """Head widths the prompt's tcgen05 attention takes, over several of its tiles: windows that end inside, at and before a
+    tile, portions that start inside one."""
+    cfg = M.config(96, 120, [(M.attn(4, 2, dim, vdim, window, dim ** -0.5, 0.3, 32), M.memory(1, 8, 16, 9.0), M.dense(64))])
+    W = M.weights(cfg, 6)
+    ids = np.random.default_rng(6).integers(0, 120, 430)
+    m = R.Model.from_pretrained(folder(tmp_path, cfg, W), max_tokens=512, page_tokens=32)
+    rounded = D.forward(cfg, M.f64(W), ids, cache=np.float16)
+    for portions in ([430], [70, 300, 60]):
+        m.set_len(0)
+        assert M.error(all_logits(m, ids, portions), rounded) < KEPT
+
+
 def test_long_prompts_are_processed_in_pieces(R, made, monkeypatch):
     cfg, _, path, ids, ref = made("ODD")
     monkeypatch.setenv("CD_PREFILL_ROWS", "70")
