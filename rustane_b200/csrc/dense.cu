@@ -43,18 +43,22 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     constexpr int RH = NH == 1 ? 4 : NH == 2 ? 2 : 1;
     const cd_config& c = m->cfg;
     auto kern = decode_mega_kernel<WT, KT, ND, RD, NH, RH, TPAR>;
-    const int grid = m->sm_count;
+    // every CTA owns rows of every matrix: what tells a CTA that another one is done with a vector is that one's next rows
+    const int grid = TPAR ? m->sm_count : std::min({m->sm_count, c.dim, c.hidden, (c.q_dim + 2 * c.kv_dim) / 2});
     const size_t es = sizeof(WT);
-    const size_t stage_cap = (std::max((size_t)RD * c.dim * es, (size_t)RH * c.hidden * es) + 127) / 128 * 128;
+    const size_t stage_cap = (std::max((size_t)RD * std::max(c.dim, c.q_dim) * es, (size_t)RH * c.hidden * es) + 127) / 128 * 128;
     int max_rows = 0;
     for (int n : {c.q_dim + 2 * c.kv_dim, c.dim, 2 * c.hidden, want_logits ? m->v_loc : 0}) max_rows = std::max(max_rows, n / grid + 2);
-    const int xs_dim = m->tp_world > 1 ? std::max(c.q_dim, c.dim) : c.q_dim;
-    const size_t fixed = ((size_t)max_rows * (GEMV_CONSUMERS / 32) + 32 * MEGA_GROUPS + mega_attn_smem_floats(xs_dim)) * sizeof(float) + 32 +
-                         (size_t)((m->pages_per_seq + 3) & ~3) * 4 + 2 * 16 * 8 + 128;
+    const int xs_dim = TPAR ? std::max(c.q_dim, c.dim) : std::max({c.q_dim, c.dim, c.hidden});
+    const int rows_cap = (max_rows + 3) & ~3;
+    size_t off = 0;
+    auto carve = [&](size_t bytes) { const size_t o = off; off += (bytes + 15) / 16 * 16; return o; };
+    const size_t xs_off = carve((size_t)xs_dim * 4), partial_off = carve((size_t)rows_cap * (GEMV_CONSUMERS / 32) * 4), resid_off = carve((size_t)2 * rows_cap * 4),
+                 pt_off = carve((size_t)m->pages_per_seq * 4), layers_off = carve((size_t)c.nlayers * sizeof(MegaLayer)), bars_off = carve(2 * 16 * 8);
     const size_t budget = (size_t)m->ring_kb * 1024;
-    if (fixed + 2 * stage_cap > budget) return cudaErrorInvalidConfiguration;
-    const int nstages = (int)std::min<size_t>(16, (budget - fixed) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
-    const size_t smem = (size_t)nstages * stage_cap + fixed;
+    if (sizeof(MegaShared) + off + 2 * stage_cap > budget) return cudaErrorInvalidConfiguration;
+    const int nstages = (int)std::min<size_t>(16, (budget - sizeof(MegaShared) - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
+    const size_t ring = (size_t)nstages * stage_cap, smem = ring + off;
     // attention tiles: the largest power-of-two run of cached positions that stays inside a page and fits a stage
     int tile = 64;
     while (tile > 1 && (tile > m->page_tokens || m->page_tokens % tile || (size_t)tile * c.hd * sizeof(KT) > stage_cap)) tile >>= 1;
@@ -68,6 +72,10 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     p.layers = (const MegaLayer*)m->mega_layers;
     p.embed = m->embed; p.lm_head = m->lm_head; p.gamma_final = m->gamma_final;
     p.x_a = m->x_a; p.x_b = m->x_b; p.q = m->q; p.gate = m->gate; p.logits = m->logits; p.norm_final = m->norm_final;
+    {
+        unsigned long long* t = (unsigned long long*)m->mega_tagged;
+        p.tx_a = t; p.tx_b = p.tx_a + c.dim; p.tq = p.tx_b + c.dim; p.tkv = p.tq + c.q_dim; p.tgate = p.tkv + 2 * c.kv_dim; p.tparts = p.tgate + c.hidden;
+    }
     p.part_acc = m->part_acc; p.part_ml = m->part_ml; p.grid_counter = m->grid_counter;
     p.st = m->st; p.page_table = m->page_table; p.rope = m->rope;
     p.dim = c.dim; p.hidden = c.hidden; p.heads = c.heads; p.kv_heads = c.kv_heads; p.hd = c.hd; p.nlayers = c.nlayers;
@@ -79,8 +87,9 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     p.wait_ns = m->wait_ns;
     p.tp = m->tp;  // world <= 1 on one GPU
     p.tp.wait_ns = m->wait_ns;
-    p.xs_dim = xs_dim;
-    p.nstages = nstages; p.stage_cap = (uint32_t)stage_cap; p.rows_cap = max_rows; p.input_embed = input_embed; p.want_logits = want_logits;
+    p.off_xs = ring + xs_off; p.off_partial = ring + partial_off; p.off_resid = ring + resid_off; p.off_pt = ring + pt_off; p.off_layers = ring + layers_off;
+    p.off_bars = ring + bars_off;
+    p.nstages = nstages; p.stage_cap = (uint32_t)stage_cap; p.rows_cap = rows_cap; p.input_embed = input_embed; p.want_logits = want_logits;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(grid);
     lc.blockDim = dim3(MEGA_THREADS);
@@ -101,10 +110,13 @@ cudaError_t launch_mega_tp(cd_model* m, int input_embed, int want_logits) {
     switch (m->mega_nd * 10 + m->mega_nh) {
         case 11: return launch_mega_t<WT, KT, 1, 1, TPAR>(m, input_embed, want_logits);
         case 12: return launch_mega_t<WT, KT, 1, 2, TPAR>(m, input_embed, want_logits);
+        case 14: if constexpr (!TPAR) return launch_mega_t<WT, KT, 1, 4, TPAR>(m, input_embed, want_logits); else break;
         case 24: return launch_mega_t<WT, KT, 2, 4, TPAR>(m, input_embed, want_logits);
         case 26: return launch_mega_t<WT, KT, 2, 6, TPAR>(m, input_embed, want_logits);
-        default: return cudaErrorInvalidConfiguration;
+        case 28: if constexpr (!TPAR) return launch_mega_t<WT, KT, 2, 8, TPAR>(m, input_embed, want_logits); else break;
+        default: break;
     }
+    return cudaErrorInvalidConfiguration;
 }
 template <typename WT, typename KT>
 cudaError_t launch_mega(cd_model* m, int input_embed, int want_logits) {
@@ -239,7 +251,8 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
     spec.rope_dim = c.hd;
     spec.attn_parts = MEGA_MAX_PARTS;  // CTAs of the persistent kernel that share a head
     const size_t ml_bytes = align_up((size_t)c.nlayers * sizeof(MegaLayer), 256);
-    spec.family_ws_bytes = ml_bytes + (size_t)2 * (10 * c.nlayers + 2) * 8;
+    const size_t tagged_at = align_up(ml_bytes + (size_t)2 * (10 * c.nlayers + 2) * 8, 256);
+    spec.family_ws_bytes = tagged_at + ((size_t)2 * c.dim + c.q_dim + 2 * c.kv_dim + c.hidden + (size_t)c.heads * MEGA_CPH_CAP * (c.hd + 2)) * 8;
     cd_model* m = nullptr;
     if ((rc = model_alloc(cfg, opts, untied, spec, &m))) return rc;
     auto bail = [&](int code) { cd_model_destroy(m); return code; };
@@ -270,6 +283,7 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
     }
     {   // per-layer pointer table and tiling of the persistent kernel
         m->mega_layers = m->family_ws;
+        m->mega_tagged = m->family_ws + tagged_at;
         if (opts.test_flags & 4) m->mega_trace = (unsigned long long*)(m->family_ws + ml_bytes);  // test_flags bit 2: phase stamps of the persistent kernel
         std::vector<MegaLayer> ml(c.nlayers);
         for (int l = 0; l < c.nlayers; ++l) {
@@ -279,10 +293,11 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
         CKB(cudaMemcpyAsync(m->mega_layers, ml.data(), ml.size() * sizeof(MegaLayer), cudaMemcpyHostToDevice, m->stream));
         CKB(cudaStreamSynchronize(m->stream));
         const int epc = dt == CD_DTYPE_F32 ? 4 : 8;
-        const int nd = (c.dim / epc + 255) / 256, nh = (c.hidden / epc + 255) / 256;
+        const int nd = (std::max(c.dim, c.q_dim) / epc + 255) / 256, nh = (c.hidden / epc + 255) / 256, g = c.gqa_ratio;
         // (c is this rank's shard under tensor parallelism: hidden and q_dim shrink, dim does not)
-        const bool combo = (nd == 1 && (nh == 1 || nh == 2)) || (nd == 2 && nh >= 3 && nh <= 6);
-        if (combo && c.q_dim <= c.dim && c.gqa_ratio <= MEGA_MAX_GQA) { m->mega_nd = nd; m->mega_nh = nh == 3 ? 4 : nh == 5 ? 6 : nh; }
+        const bool combo = tpw > 1 ? ((nd == 1 && (nh == 1 || nh == 2)) || (nd == 2 && nh >= 3 && nh <= 6)) && c.q_dim <= c.dim && g <= 2
+                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= 8)) && (g == 1 || g == 2 || g == 4 || g == MEGA_MAX_GQA);
+        if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
         // tensor parallel: measured on the 5B model, the persistent kernel wins at 2 ranks (601 against 569 tokens/s) and
         // loses at 8 (841 against 896), where a layer's data are 8 us and its fixed per-phase times dominate either way
         const bool mega_ok = !is_quant(dt) && (tpw == 1 || (tpw == 2 && dt != CD_DTYPE_F32));

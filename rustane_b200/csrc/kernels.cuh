@@ -31,20 +31,21 @@ struct EpiResidual {  // residual_add, lib.rs:1491-1502 / w2_proj beta=1, :1189-
     __device__ void operator()(int unit, const float (&y)[1]) const { out[unit] = __ldcg(res + unit) + alpha * y[0]; }
 };
 
-struct EpiGate {  // silu_gate, lib.rs:1504-1513; rows (2j, 2j+1) hold w1 and w3 column j
+__device__ inline float gate_value(float y0, float y1, int act) {  // silu_gate, lib.rs:1504-1513
+    float a;
+    if (act == 1) {  // LeakyReLU^2 (layer.rs:826-830)
+        const float l = fmaxf(y0, 0.5f * y0);
+        a = l * l;
+    } else {
+        const float sig = 1.0f / (1.0f + expf(-y0));
+        a = y0 * sig;
+    }
+    return a * y1;
+}
+struct EpiGate {  // rows (2j, 2j+1) hold w1 and w3 column j
     float* gate;
     int act;
-    __device__ void operator()(int unit, const float (&y)[2]) const {
-        float a;
-        if (act == 1) {  // LeakyReLU^2 (layer.rs:826-830)
-            const float l = fmaxf(y[0], 0.5f * y[0]);
-            a = l * l;
-        } else {
-            const float sig = 1.0f / (1.0f + expf(-y[0]));
-            a = y[0] * sig;
-        }
-        gate[unit] = a * y[1];
-    }
+    __device__ void operator()(int unit, const float (&y)[2]) const { gate[unit] = gate_value(y[0], y[1], act); }
 };
 
 // rope_inplace + append_kv (lib.rs:1392-1424) on the fused [q | k | v] rows.

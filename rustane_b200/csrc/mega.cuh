@@ -51,7 +51,7 @@ struct MegaLayer {
 
 constexpr int MEGA_MAX_PARTS = 64;  // partial attention results per head the buffers hold
 constexpr int MEGA_CPH_CAP = 8;     // CTAs that share a kv head: every CTA merges that many partials per head before Wo
-constexpr int MEGA_MAX_GQA = 2;     // q heads per kv head the attention phase keeps in registers
+constexpr int MEGA_MAX_GQA = 8;     // q heads per kv head: 1, 2, 4 or 8 (a warp team works on one or two of them)
 
 struct MegaParams {
     const MegaLayer* layers;  // device array [nlayers]
@@ -77,7 +77,13 @@ struct MegaParams {
     unsigned long long wait_ns; // bound of a grid-barrier wait
     unsigned long long* trace;  // optional [2][1 + 10 * nlayers + 1] globaltimer stamps of CTA 0 and the last CTA
     TpLink tp;                  // tensor parallel (world > 1): the dimensions above are this rank's shard
-    int xs_dim;                 // floats of the CTA's vector scratch: q_dim, and dim when inputs are gathered from the ranks' inboxes
+    // byte offsets in dynamic shared memory, behind the ring: widest input vector, [rows_cap][8] partial sums, [2][rows_cap] residual
+    // entries, page table, [nlayers] layer table, barriers.  (Offsets as kernel parameters and the rest of the CTA's scratch as
+    // static shared memory cost no registers; with a pointer each the GEMV loops spilled, and at 544 threads a CTA's spills
+    // do not fit the L1 that the ring leaves.)
+    uint32_t off_xs, off_partial, off_resid, off_pt, off_layers, off_bars;
+    // one GPU: the vectors between phases as tagged words (tag_store); tparts: [heads][MEGA_CPH_CAP][hd + 2], max and sum last
+    unsigned long long *tx_a, *tx_b, *tq, *tkv, *tgate, *tparts;
 };
 
 // Wo / W2 epilogue: x_out = res + alpha y on one GPU; tensor parallel, the rank's partial y goes to every rank's
@@ -103,14 +109,38 @@ constexpr int MEGA_CONSUMERS = MEGA_GROUPS * GEMV_CONSUMERS;
 constexpr int MEGA_THREADS = MEGA_CONSUMERS + 32;  // + the producer's warp (one working thread)
 constexpr int MEGA_TEAMS = MEGA_CONSUMERS / 128;
 constexpr int MEGA_TEAM_SMEM = 128 * 8 + 64;  // floats per team: lane-group accumulators, then (max, sum) pairs
-// floats of shared memory the attention phase needs: the teams' scratch (which the merged attention vector
-// of the following phase reuses), then the teams' partials
-__host__ __device__ inline size_t mega_attn_scratch_floats(int q_dim) {
-    return (size_t)MEGA_TEAMS * MEGA_TEAM_SMEM > (size_t)q_dim ? (size_t)MEGA_TEAMS * MEGA_TEAM_SMEM : (size_t)q_dim;
+// ---- who computes which part of the attention
+// A kv head belongs to `cph` consecutive CTAs (as many as fit, at most one per tile and at most
+// MEGA_CPH_CAP); CTA j of them takes tiles [j * ntiles / cph, (j + 1) * ntiles / cph) and
+// produces partial j of every q head of that kv head.  With more kv heads than CTAs each CTA
+// walks heads blockIdx.x, blockIdx.x + gridDim.x, ... on its own (cph = 1).
+struct AttnPlan {
+    int cph;          // CTAs (= partials) per kv head
+    int first, step;  // this CTA's kv heads: first, first + step, ... (first < 0: none)
+    int part;         // this CTA's partial index within its head
+    int t0, t1;       // its tiles
+};
+struct MegaShared {
+    float accs[MEGA_TEAMS][MEGA_TEAM_SMEM];  // attention: lane-group accumulators, then (max, sum) pairs
+    float tparts[MEGA_TEAMS][2][128 + 2];    // per team and q head: weighted V, max, sum
+    float q[MEGA_MAX_GQA * 128];             // q of the kv head's q heads
+    uint4 row[2 * 128 / 4];                  // this position's K and V row as cached
+    float2 rope[64];                         // (cos, sin) of this position
+    float red[64];
+    AttnPlan plan;
+    int2 rows[4];                            // this CTA's rows of q|k|v, the residual stream, gate|up, head
+    size_t kv_at;                            // this position's K row of kv head 0 in a layer's pages (elements)
+    int abort;
+};
+__device__ inline MegaShared& mega_shared() {
+    __shared__ MegaShared sh;
+    return sh;
 }
-__host__ __device__ inline size_t mega_attn_smem_floats(int q_dim) {
-    return mega_attn_scratch_floats(q_dim) + (size_t)MEGA_TEAMS * MEGA_MAX_GQA * (128 + 2);
+__device__ inline unsigned char* mega_dyn() {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    return smraw;
 }
+__device__ inline bool mega_aborted() { return *const_cast<const volatile int*>(&mega_shared().abort) != 0; }
 
 __device__ inline void mega_bar() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 __device__ inline void group_bar(int grp) { asm volatile("bar.sync %0, 256;" ::"r"(4 + grp) : "memory"); }
@@ -160,16 +190,6 @@ __device__ inline void cta_rows(int N, int unit, int& r0, int& r1) {
     r1 = (int)((long long)(blockIdx.x + 1) * nunits / gridDim.x) * unit;
 }
 
-// ---- who computes which part of the attention
-// A kv head belongs to `cph` consecutive CTAs (as many as fit, at most one per tile and at most
-// MEGA_MAX_PARTS); CTA j of them takes tiles [j * ntiles / cph, (j + 1) * ntiles / cph) and
-// produces partial j of every q head of that kv head.  With more kv heads than CTAs each CTA
-// walks heads blockIdx.x, blockIdx.x + gridDim.x, ... on its own (cph = 1).
-struct AttnPlan {
-    int cph;          // CTAs (= partials) per kv head
-    int first, step;  // this CTA's kv heads: first, first + step, ... (first < 0: none)
-    int part;         // this CTA's partial index within its head
-};
 __device__ inline AttnPlan attn_plan(int kv_heads, int ntiles) {
     AttnPlan a;
     const int G = gridDim.x, c = blockIdx.x;
@@ -184,11 +204,9 @@ __device__ inline AttnPlan attn_plan(int kv_heads, int ntiles) {
         a.step = G;
         a.part = 0;
     }
+    a.t0 = (int)((long long)a.part * ntiles / a.cph);
+    a.t1 = (int)((long long)(a.part + 1) * ntiles / a.cph);
     return a;
-}
-__device__ inline void attn_tiles(const AttnPlan& a, int ntiles, int& t0, int& t1) {
-    t0 = (int)((long long)a.part * ntiles / a.cph);
-    t1 = (int)((long long)(a.part + 1) * ntiles / a.cph);
 }
 
 // ---- the token's stream: everything this CTA reads from HBM for one token, stage by stage, in the
@@ -211,8 +229,7 @@ __device__ inline bool walk_attention(const MegaParams& p, const char* kv, const
     const int T = p.tile_tokens, ntiles = (attn_len + T - 1) / T;
     const AttnPlan plan = attn_plan(p.kv_heads, ntiles);
     if (plan.first < 0) return true;
-    int t0, t1;
-    attn_tiles(plan, ntiles, t0, t1);
+    const int t0 = plan.t0, t1 = plan.t1;
     const size_t head_bytes = (size_t)p.page_tokens * p.hd * kes, page_bytes = (size_t)2 * p.kv_heads * head_bytes;
     const uint32_t bytes = (uint32_t)T * p.hd * kes;
     // (one thread walks this: its dependent integer arithmetic is part of the pace of the phase, so page and offset
@@ -249,7 +266,7 @@ __device__ inline bool walk_token_stream(const MegaParams& p, const int* pt, int
 // in_reduce), gathered from this rank's inbox into shared memory (xg), every thread a few float4 positions; both
 // consumer groups then take their slices from there, CTA 0 keeps the vector in x_out.  Out of line: one copy for
 // all phases, and none of it in the instruction stream of a single-GPU token.
-__device__ __noinline__ void gather_input(const TpLink& tin, int K, float* xg, int* err, int* abort_flag) {
+__device__ __noinline__ void gather_input(const TpLink& tin, int K, float* xg, int* err) {
     const unsigned int seq = __ldcg(&tin.st->ar_base) + (unsigned int)tin.in_reduce;
     float* base = reinterpret_cast<float*>(tin.peers[tin.rank]);
     const float* inbox = base + (size_t)(seq % 3u) * tin.world * tin.dim;
@@ -262,7 +279,7 @@ __device__ __noinline__ void gather_input(const TpLink& tin, int K, float* xg, i
         float4 a;  // summed in fixed rank order: identical on every rank
         if (!tp_gather4(inbox, tin.world, tin.dim, (size_t)q4 * 4, a, tin.st, tin.wait_ns)) {
             atomicCAS(err, 0, DEV_ERR_TP_WAIT);
-            *abort_flag = 1;
+            mega_shared().abort = 1;
         }
         const float4 r4 = __ldcg(reinterpret_cast<const float4*>(tin.res + (size_t)q4 * 4));
         const float4 v = make_float4(r4.x + tin.alpha * a.x, r4.y + tin.alpha * a.y, r4.z + tin.alpha * a.z, r4.w + tin.alpha * a.w);
@@ -296,89 +313,17 @@ __device__ __noinline__ void stage_first_input(const MegaParams& p, float* xs) {
     mega_bar();
 }
 
-// ---- consumer side: one GEMV phase.  The input vector comes from `x` (fp32, L2-only loads), from
-// `x_smem` (this CTA's shared memory) or, when `embed_row` is given, from a row of the embedding
-// table in storage form.
-template <typename WT, int NITER, int R, int UNIT, bool NORM, class Epi>
-__device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_smem, const WT* embed_row, float* x_copy, const float* gamma,
-                                    float* norm_out, int N, int K, float* partial, float* red, int* err, int* abort_flag,
-                                    const Epi& epi) {
+// ---- consumer side of one GEMV phase: this CTA's rows [r0, r1) out of the ring times the input slices xr each thread holds
+// (chunks tid, tid + 256, ... of the vector, the same in both groups), then the epilogue on its units
+template <typename WT, int NITER, int R, int UNIT, class Epi>
+__device__ inline bool stream_rows(Ring& ring, const float (&xr)[NITER][Elem<WT>::EPC], int r0, int r1, int K, const MegaParams& p, const Epi& epi) {
+    float* partial = reinterpret_cast<float*>(mega_dyn() + p.off_partial);
     constexpr int EPC = Elem<WT>::EPC;
     constexpr int NW = GEMV_CONSUMERS / 32;
     const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255, lane = tid & 31, warp = tid >> 5;
     const int nchunks = K / EPC;
     const uint32_t row_bytes = (uint32_t)K * sizeof(WT);
-    int r0, r1;
-    cta_rows(N, UNIT, r0, r1);
     const int ngroups = (r1 - r0 + R - 1) / R;
-    red += grp * 32;
-
-    float xr[NITER][EPC];
-    float gm[NORM ? NITER : 1][NORM ? EPC : 1];  // gamma, requested together with x: one memory latency for both
-    if (NORM) {
-#pragma unroll
-        for (int i = 0; i < NITER; ++i) {
-            const int c = tid + i * GEMV_CONSUMERS;
-#pragma unroll
-            for (int e = 0; e < EPC; e += 4) {
-                const float4 g = c < nchunks ? *reinterpret_cast<const float4*>(gamma + (size_t)c * EPC + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-                gm[NORM ? i : 0][NORM ? e : 0] = g.x; gm[NORM ? i : 0][NORM ? e + 1 : 0] = g.y;
-                gm[NORM ? i : 0][NORM ? e + 2 : 0] = g.z; gm[NORM ? i : 0][NORM ? e + 3 : 0] = g.w;
-            }
-        }
-    }
-    float ss = 0.0f;
-#pragma unroll
-    for (int i = 0; i < NITER; ++i) {
-        const int c = tid + i * GEMV_CONSUMERS;
-        if (embed_row != nullptr) {
-            if (c < nchunks) {
-                const uint4 w = ldg_stream(reinterpret_cast<const char*>(embed_row) + (size_t)c * 16);
-                Elem<WT>::unpack(w, xr[i]);
-                if (x_copy != nullptr && blockIdx.x == 0 && grp == 0) {
-#pragma unroll
-                    for (int e = 0; e < EPC; e += 4)
-                        *reinterpret_cast<float4*>(x_copy + (size_t)c * EPC + e) = make_float4(xr[i][e], xr[i][e + 1], xr[i][e + 2], xr[i][e + 3]);
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < EPC; ++e) xr[i][e] = 0.0f;
-            }
-#pragma unroll
-            for (int e = 0; e < EPC; ++e) ss += xr[i][e] * xr[i][e];
-        } else {
-#pragma unroll
-            for (int e = 0; e < EPC; e += 4) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (c < nchunks) {
-                    if (x_smem != nullptr) v = *reinterpret_cast<const float4*>(x_smem + (size_t)c * EPC + e);
-                    else v = __ldcg(reinterpret_cast<const float4*>(x + (size_t)c * EPC + e));
-                }
-                xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            }
-        }
-    }
-    if (NORM) {
-        const float tot = group_sum(ss, red, grp);
-        const float inv = 1.0f / sqrtf(tot * (1.0f / (float)K) + RMS_EPS);
-#pragma unroll
-        for (int i = 0; i < NITER; ++i) {
-            const int c = tid + i * GEMV_CONSUMERS;
-            if (c < nchunks) {
-#pragma unroll
-                for (int e = 0; e < EPC; e += 4) {
-                    xr[i][e] = xr[i][e] * inv * gm[NORM ? i : 0][NORM ? e : 0];
-                    xr[i][e + 1] = xr[i][e + 1] * inv * gm[NORM ? i : 0][NORM ? e + 1 : 0];
-                    xr[i][e + 2] = xr[i][e + 2] * inv * gm[NORM ? i : 0][NORM ? e + 2 : 0];
-                    xr[i][e + 3] = xr[i][e + 3] * inv * gm[NORM ? i : 0][NORM ? e + 3 : 0];
-                    if (norm_out != nullptr && blockIdx.x == 0 && grp == 0)
-                        *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) =
-                            make_float4(xr[i][e], xr[i][e + 1], xr[i][e + 2], xr[i][e + 3]);
-                }
-            }
-        }
-    }
 
     // Ring slots are owned by groups for the whole GEMV phase: group = (global stage number) & 1,
     // and the ring has an even number of slots, so the successive uses of one slot are all
@@ -389,8 +334,8 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
         const int rg = ring.g + g;
         const int s = rg % ring.nstages;
         if (!mbar_wait(ring.full0 + 8u * s, (rg / ring.nstages) & 1)) {
-            atomicCAS(err, 0, DEV_ERR_FULL_WAIT);
-            *abort_flag = 1;  // every consumer still meets at the barrier below, then all leave together
+            atomicCAS(&p.st->error, 0, DEV_ERR_FULL_WAIT);
+            mega_shared().abort = 1;  // every consumer still meets at the barrier below, then all leave together
             break;
         }
         const uint32_t base = ring.base + (uint32_t)s * ring.stage_cap;
@@ -424,8 +369,9 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
     }
     ring.g += ngroups;
     mega_bar();
-    if (*reinterpret_cast<volatile int*>(abort_flag) != 0) return false;
+    if (mega_aborted()) return false;
     const int u0 = r0 / UNIT, nu = (r1 - r0) / UNIT;
+#pragma unroll 1
     for (int u = threadIdx.x; u < nu; u += MEGA_CONSUMERS) {
         float y[UNIT];
 #pragma unroll
@@ -440,11 +386,252 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
     return true;
 }
 
+// ---- one GEMV phase of the tensor-parallel form.  The input vector comes from `x` (fp32, L2-only loads), from
+// `x_smem` (this CTA's shared memory).
+template <typename WT, int NITER, int R, int UNIT, bool NORM, class Epi>
+__device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_smem, const float* gamma, float* norm_out, int N, int K,
+                                    const MegaParams& p, const Epi& epi) {
+    constexpr int EPC = Elem<WT>::EPC;
+    const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255;
+    const int nchunks = K / EPC;
+    float* red = mega_shared().red + grp * 32;
+    int r0, r1;
+    cta_rows(N, UNIT, r0, r1);
+
+    float xr[NITER][EPC];
+    float gm[NORM ? NITER : 1][NORM ? EPC : 1];  // gamma, requested together with x: one memory latency for both
+    if (NORM) {
+#pragma unroll
+        for (int i = 0; i < NITER; ++i) {
+            const int c = tid + i * GEMV_CONSUMERS;
+#pragma unroll
+            for (int e = 0; e < EPC; e += 4) {
+                const float4 g = c < nchunks ? *reinterpret_cast<const float4*>(gamma + (size_t)c * EPC + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                gm[NORM ? i : 0][NORM ? e : 0] = g.x; gm[NORM ? i : 0][NORM ? e + 1 : 0] = g.y;
+                gm[NORM ? i : 0][NORM ? e + 2 : 0] = g.z; gm[NORM ? i : 0][NORM ? e + 3 : 0] = g.w;
+            }
+        }
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NITER; ++i) {
+        const int c = tid + i * GEMV_CONSUMERS;
+#pragma unroll
+        for (int e = 0; e < EPC; e += 4) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < nchunks) {
+                if (x_smem != nullptr) v = *reinterpret_cast<const float4*>(x_smem + (size_t)c * EPC + e);
+                else v = __ldcg(reinterpret_cast<const float4*>(x + (size_t)c * EPC + e));
+            }
+            xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
+            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        }
+    }
+    if (NORM) {
+        const float tot = group_sum(ss, red, grp);
+        const float inv = 1.0f / sqrtf(tot * (1.0f / (float)K) + RMS_EPS);
+#pragma unroll
+        for (int i = 0; i < NITER; ++i) {
+            const int c = tid + i * GEMV_CONSUMERS;
+            if (c < nchunks) {
+#pragma unroll
+                for (int e = 0; e < EPC; e += 4) {
+                    xr[i][e] = xr[i][e] * inv * gm[NORM ? i : 0][NORM ? e : 0];
+                    xr[i][e + 1] = xr[i][e + 1] * inv * gm[NORM ? i : 0][NORM ? e + 1 : 0];
+                    xr[i][e + 2] = xr[i][e + 2] * inv * gm[NORM ? i : 0][NORM ? e + 2 : 0];
+                    xr[i][e + 3] = xr[i][e + 3] * inv * gm[NORM ? i : 0][NORM ? e + 3 : 0];
+                    if (norm_out != nullptr && blockIdx.x == 0 && grp == 0)
+                        *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) =
+                            make_float4(xr[i][e], xr[i][e + 1], xr[i][e + 2], xr[i][e + 3]);
+                }
+            }
+        }
+    }
+    return stream_rows<WT, NITER, R, UNIT>(ring, xr, r0, r1, K, p, epi);
+}
+
+// ---- one GPU: vectors between phases travel as tagged words.  A word is a 64-bit pair (value, tag), written by one
+// relaxed store and read by relaxed loads, so a reader knows from the word itself that it holds this layer's value: no
+// fence, no counter, no barrier, and the poll that sees the last word already has the data in registers.  A buffer is
+// written once per layer; its readers of layer l are done before any CTA can write layer l + 1, because every CTA owns
+// rows of every matrix and a CTA's rows of the next phase are stored only after it has read its whole input.
+__device__ inline void tag_store(unsigned long long* p, float v, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)tag << 32 | __float_as_uint(v)) : "memory");
+}
+__device__ inline void tag_load2(const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ inline float tag_value(unsigned long long w) { return __uint_as_float((uint32_t)w); }
+
+// Polls the pairs of words at src[0 .. N - 1] until all carry `tag`.  False when the time is up or another CTA has
+// already failed (the CTA's abort flag is raised then).
+template <int N>
+__device__ inline bool tag_poll(const unsigned long long* const (&src)[N], uint32_t tag, unsigned long long (&w)[N][2], const MegaParams& p) {
+    unsigned long long t0 = 0;
+#pragma unroll 1
+    for (int i = 1;; ++i) {
+#pragma unroll
+        for (int b = 0; b < N; ++b) tag_load2(src[b], w[b][0], w[b][1]);
+        bool all = true;
+#pragma unroll
+        for (int b = 0; b < N; ++b) all = all && (uint32_t)(w[b][0] >> 32) == tag && (uint32_t)(w[b][1] >> 32) == tag;
+        if (all) return true;
+        if ((i & 63) == 0) {
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > p.wait_ns || dev_failed(p.st) || mega_aborted()) break;
+        }
+    }
+    atomicCAS(&p.st->error, 0, 3);
+    mega_shared().abort = 1;
+    return false;
+}
+
+// Where an input vector goes: times gamma (when given) into xs, and its entries at this CTA's rows of the residual stream
+// as they are into resid (when given; two arrays take turns, since the epilogue of the phase before may still read the other).
+struct InputTo {
+    float *xs, *resid;
+    const float* gamma;
+    int2 rows;  // this CTA's rows of the residual stream
+    __device__ float2 scale(int i) const { return gamma != nullptr ? *reinterpret_cast<const float2*>(gamma + i) : make_float2(1.0f, 1.0f); }
+    __device__ void put(int i, float2 v, float2 g) const {
+        *reinterpret_cast<float2*>(xs + i) = make_float2(v.x * g.x, v.y * g.y);
+        if (resid != nullptr) {
+            if (i >= rows.x && i < rows.y) resid[i - rows.x] = v.x;
+            if (i + 1 >= rows.x && i + 1 < rows.y) resid[i + 1 - rows.x] = v.y;
+        }
+    }
+};
+// A whole vector from its tagged words; returns this thread's share of the sum of squares.
+__device__ inline float gather_tagged(const unsigned long long* src, uint32_t tag, int K, const InputTo& to, const MegaParams& p) {
+    constexpr int B = 4;
+    const int n = K / 2;
+    float ss = 0.0f;
+#pragma unroll 1
+    for (int c0 = threadIdx.x; c0 < n; c0 += MEGA_CONSUMERS * B) {
+        const unsigned long long* at[B];
+        unsigned long long w[B][2];
+        float2 g[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int c = c0 + b * MEGA_CONSUMERS < n ? c0 + b * MEGA_CONSUMERS : c0;
+            at[b] = src + 2 * c;
+            g[b] = to.scale(2 * c);  // ahead of the polls: its latency passes while the input arrives
+        }
+        if (!tag_poll<B>(at, tag, w, p)) break;
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            if (c0 + b * MEGA_CONSUMERS < n) {
+                const float2 v = make_float2(tag_value(w[b][0]), tag_value(w[b][1]));
+                to.put(2 * (c0 + b * MEGA_CONSUMERS), v, g[b]);
+                ss = fmaf(v.x, v.x, fmaf(v.y, v.y, ss));
+            }
+    }
+    return ss;
+}
+// the first layer's: the embedding row of the current token, or x_a as the host left it
+template <typename WT> __device__ inline float gather_first(const MegaParams& p, const InputTo& to) {
+    const WT* row = reinterpret_cast<const WT*>(p.embed) + (p.input_embed ? (size_t)checked_token(__ldcg(&p.st->token), p.embed_rows, &p.st->error) * p.dim : 0);
+    float ss = 0.0f;
+#pragma unroll 1
+    for (int i = 2 * threadIdx.x; i < p.dim; i += 2 * MEGA_CONSUMERS) {
+        const float2 v = p.input_embed ? make_float2(Elem<WT>::to_f32(row[i]), Elem<WT>::to_f32(row[i + 1])) : __ldcg(reinterpret_cast<const float2*>(p.x_a + i));
+        to.put(i, v, to.scale(i));
+        ss = fmaf(v.x, v.x, fmaf(v.y, v.y, ss));
+    }
+    return ss;
+}
+
+// One GEMV phase: the input vector (in() fills xs and returns the thread's share of the sum of squares) into registers,
+// under NORM over its root mean square, then this CTA's rows.
+template <typename WT, int NITER, int R, int UNIT, bool NORM, class In, class Epi, class Tick>
+__device__ inline bool tagged_gemv(Ring& ring, const MegaParams& p, const In& in, float* norm_out, const int2& rows, int K, const Epi& epi, const Tick& input_is_in) {
+    const float* xs = reinterpret_cast<const float*>(mega_dyn() + p.off_xs);
+    float* red = mega_shared().red;
+    constexpr int EPC = Elem<WT>::EPC;
+    const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255;
+    const int nchunks = K / EPC;
+    const float ss = NORM ? warp_sum(in()) : in();
+    if (NORM && (threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    mega_bar();
+    input_is_in();
+    float inv = 1.0f;
+    if (NORM) {
+        float tot = 0.0f;
+#pragma unroll
+        for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) tot += red[i];
+        inv = 1.0f / sqrtf(tot * (1.0f / (float)K) + RMS_EPS);
+    }
+    float xr[NITER][EPC];
+#pragma unroll
+    for (int i = 0; i < NITER; ++i) {
+        const int c = tid + i * GEMV_CONSUMERS;
+#pragma unroll
+        for (int e = 0; e < EPC; e += 4) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < nchunks) v = *reinterpret_cast<const float4*>(xs + (size_t)c * EPC + e);
+            if (NORM) {
+                v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+                if (norm_out != nullptr && blockIdx.x == 0 && grp == 0 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
+            }
+            xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
+        }
+    }
+    return stream_rows<WT, NITER, R, UNIT>(ring, xr, rows.x, rows.y, K, p, epi);
+}
+
+// epilogues of the tagged phases (arithmetic of EpiQKV, EpiGate, EpiResidual)
+template <typename KT> struct TagQKV {
+    const MegaParams& p;
+    KT* kv;
+    uint32_t tag;
+    __device__ void operator()(int unit, const float (&y)[2]) const {
+        const MegaShared& sh = mega_shared();
+        const int r = unit * 2, d = r & (p.hd - 1);  // (hd is 64 or 128)
+        float e = y[0], o = y[1];
+        if (r < p.q_dim + p.kv_dim) {
+            const float2 cs = sh.rope[d >> 1];
+            e = y[0] * cs.x - y[1] * cs.y;
+            o = y[1] * cs.x + y[0] * cs.y;
+        }
+        if (r < p.q_dim) {
+            tag_store(p.tq + r, e, tag);
+            tag_store(p.tq + r + 1, o, tag);
+            return;
+        }
+        // tkv: this position's K then V as cached (rounded), for the CTAs that attend to it in this layer
+        const int rk = r - p.q_dim, v = rk >= p.kv_dim, head = (v ? rk - p.kv_dim : rk) >> (p.hd == 128 ? 7 : 6);
+        const KT ek = Elem<KT>::from_f32(e), ok = Elem<KT>::from_f32(o);
+        tag_store(p.tkv + rk, Elem<KT>::to_f32(ek), tag);
+        tag_store(p.tkv + rk + 1, Elem<KT>::to_f32(ok), tag);
+        KT* dst = kv + sh.kv_at + (size_t)(v * p.kv_heads + head) * p.page_tokens * p.hd + d;
+        dst[0] = ek;
+        dst[1] = ok;
+    }
+};
+struct TagGate {
+    const MegaParams& p;
+    uint32_t tag;
+    __device__ void operator()(int unit, const float (&y)[2]) const { tag_store(p.tgate + unit, gate_value(y[0], y[1], p.activation), tag); }
+};
+struct TagResidual {
+    const float* resid;       // this CTA's entries, from its first row on
+    float alpha;
+    unsigned long long* out;
+    float* plain;             // also as plain floats (the last layer's result), or null
+    uint32_t tag;
+    __device__ void operator()(int unit, const float (&y)[1]) const {
+        const float v = resid[unit - mega_shared().rows[1].x] + alpha * y[0];
+        tag_store(out + unit, v, tag);
+        if (plain != nullptr) plain[unit] = v;
+    }
+};
+
 // ---- grid barrier for the consumer threads of all CTAs (arrival k of this launch).  One thread
 // per CTA adds to a monotonic counter with release semantics (a reduction, not an atomic with a
 // result: no round trip) and polls it with acquire loads until all CTAs of this arrival are in;
 // the wait is bounded by time.
-__device__ inline bool grid_barrier(unsigned long long* counter, unsigned long long target, unsigned long long wait_ns, int* err, int* abort_flag) {
+__device__ inline bool grid_barrier(unsigned long long* counter, unsigned long long target, unsigned long long wait_ns, int* err) {
     mega_bar();  // every consumer's global writes of the phase are issued
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(counter), "l"(1ull) : "memory");
@@ -462,22 +649,49 @@ __device__ inline bool grid_barrier(unsigned long long* counter, unsigned long l
         }
         if (!ok) {
             atomicCAS(err, 0, 3);
-            *abort_flag = 1;
+            mega_shared().abort = 1;
         }
     }
     mega_bar();
-    return *reinterpret_cast<volatile int*>(abort_flag) == 0;
+    return !mega_aborted();
+}
+
+// q of the kv head's q heads and, where the CTA holds the newest tile, this position's K and V row (as cached) from the
+// tagged words into shared memory: every lane group needs the same values.
+template <typename KT>
+__device__ inline bool attention_inputs(const MegaParams& p, int h, bool newest, uint32_t tag) {
+    MegaShared& sh = mega_shared();
+    const int nq = p.gqa * p.hd / 2, t = threadIdx.x;  // pairs of q, at most one per thread
+    const bool want_q = t < nq, want_row = newest && t < p.hd;  // pair t of the row: K's pairs, then V's
+    if (want_q || want_row) {
+        const unsigned long long* const q = p.tq + (size_t)h * p.gqa * p.hd + 2 * t;
+        const unsigned long long* const row = p.tkv + h * p.hd + (t < p.hd / 2 ? 2 * t : p.kv_dim + 2 * t - p.hd);
+        const unsigned long long* const at[2] = {want_q ? q : row, want_row ? row : q};
+        unsigned long long w[2][2];
+        if (tag_poll<2>(at, tag, w, p)) {
+            if (want_q) *reinterpret_cast<float2*>(sh.q + 2 * t) = make_float2(tag_value(w[0][0]), tag_value(w[0][1]));
+            if (want_row) {
+                KT* kv = reinterpret_cast<KT*>(sh.row);
+                kv[2 * t] = Elem<KT>::from_f32(tag_value(w[1][0]));
+                kv[2 * t + 1] = Elem<KT>::from_f32(tag_value(w[1][1]));
+            }
+        }
+    }
+    mega_bar();
+    return !mega_aborted();
 }
 
 // ---- attention phase (sdpa_causal, lib.rs:1426-1489, for the tiles of this CTA).  All sixteen warps
-// work on every tile: team k (four warps) takes positions [k T / 4, (k + 1) T / 4) of it; LPT lanes hold one
-// cached position's row as 16-byte chunks, 128 / LPT positions side by side, UNR deep, with a running
-// (max, sum, weighted V) per lane group and q head.  A warp copies its rows of a tile to registers,
-// releases the two ring slots (every warp arrives once on each) and computes while the next tile lands;
-// nothing but the ring's barriers orders the warps until the merge at the end.
-template <typename KT, int GQA>
-__device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const void* kv_pool, float* attn_smem, int* abort_flag, const int* pt,
-                                       int attn_len, int* err) {
+// work on every tile, in four teams of four warps.  A team takes GQ of the kv head's q heads; with more than that
+// (grouped queries) the teams divide the q heads first, and the teams of the same q heads divide a tile's positions:
+// 4 q heads: 2 x 2 teams, 8 q heads: 4 x 1.  LPT lanes hold one cached position's row as 16-byte chunks, 128 / LPT
+// positions side by side, UNR deep, with a running (max, sum, weighted V) per lane group and q head.  A warp copies its
+// rows of a tile to registers, releases the two ring slots (every warp arrives once on each) and computes while the next
+// tile lands; nothing but the ring's barriers orders the warps until the merge at the end.
+// TAG: q and the new position's row arrive, and the CTA's partials leave, as tagged words.
+template <typename KT, int GQ, bool TAG, class Tick>
+__device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const void* kv_pool, int attn_len, uint32_t tag, const Tick& input_is_in) {
+    MegaShared& sh = mega_shared();
     constexpr int EPC = Elem<KT>::EPC;
     constexpr int UNR = 2;
     constexpr float NEG = -3.402823466e+38f;
@@ -485,44 +699,48 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
     const int HD = p.hd, LPT = HD / EPC, NG = 128 / LPT;
     const int g = tt / LPT, l = tt % LPT;
     const int T = p.tile_tokens, ntiles = (attn_len + T - 1) / T, pos = attn_len - 1;
-    constexpr int gqa = GQA;  // q heads per kv head: a template parameter so that one head's state costs no registers when there is one
-    const AttnPlan plan = attn_plan(p.kv_heads, ntiles);
+    const int gqa = p.gqa, qgroups = gqa / GQ;  // (GQ is a template parameter so that one head's state costs no registers when there is one)
+    const int qg = team % qgroups, slice = team / qgroups, nslices = MEGA_TEAMS / qgroups;
     const uint32_t row_bytes = (uint32_t)HD * sizeof(KT);
     const size_t head_stride = (size_t)p.page_tokens * HD, page_stride = (size_t)2 * p.kv_heads * head_stride;
     const KT* pool = reinterpret_cast<const KT*>(kv_pool);
-    float* accs = attn_smem + team * MEGA_TEAM_SMEM;  // [NG][HD] lane-group accumulators of this team
-    float* gm = accs + 128 * 8;                        // [NG] max, then [NG] sum
+    float* accs = sh.accs[team];  // [NG][HD] lane-group accumulators of this team
+    float* gm = accs + 128 * 8;    // [NG] max, then [NG] sum
     float* gl = gm + 32;
-    // per team and q head: (acc[HD], max, sum) for the merge across teams
-    float* tparts = attn_smem + mega_attn_scratch_floats(p.xs_dim);  // [MEGA_TEAMS][MEGA_MAX_GQA][128 + 2]
     bool ok = true;
+    const AttnPlan plan = sh.plan;
     if (plan.first >= 0) {
-        int t0, t1;
-        attn_tiles(plan, ntiles, t0, t1);
+        const int t0 = plan.t0, t1 = plan.t1;
         const int ncta_tiles = t1 - t0;
         for (int h = plan.first; h < p.kv_heads && ok; h += plan.step) {
-            float qf[GQA][EPC], acc[GQA][EPC], m[GQA], lsum[GQA];
+            if constexpr (TAG) {
+                if (!attention_inputs<KT>(p, h, t1 == ntiles, tag)) { ok = false; break; }
+                if (h == plan.first) input_is_in();
+            }
+            float qf[GQ][EPC], acc[GQ][EPC], m[GQ], lsum[GQ];
 #pragma unroll
-            for (int qi = 0; qi < GQA; ++qi) {
+            for (int qi = 0; qi < GQ; ++qi) {
                 m[qi] = NEG;
                 lsum[qi] = 0.0f;
 #pragma unroll
                 for (int e = 0; e < EPC; ++e) acc[qi][e] = 0.0f;
+                const int hq = qg * GQ + qi;
 #pragma unroll
                 for (int e = 0; e < EPC; e += 4) {
-                    const float4 v = __ldcg(reinterpret_cast<const float4*>(p.q + (size_t)(h * gqa + qi) * HD + l * EPC + e));
+                    const float4 v = TAG ? *reinterpret_cast<const float4*>(sh.q + hq * HD + l * EPC + e)
+                                         : __ldcg(reinterpret_cast<const float4*>(p.q + (size_t)(h * gqa + hq) * HD + l * EPC + e));
                     qf[qi][e] = v.x; qf[qi][e + 1] = v.y; qf[qi][e + 2] = v.z; qf[qi][e + 3] = v.w;
                 }
             }
-            const int TQ = max(1, T / MEGA_TEAMS);  // positions of a tile per team
+            const int TQ = max(1, T / nslices);  // positions of a tile per team
             for (int idx = 0; idx < ncta_tiles; ++idx) {
                 if (!ok) break;  // this warp only: the others learn it from the abort flag behind the barrier below
                 const int tile = t0 + idx;
                 const int sk = ring.g + 2 * idx, sv = sk + 1;
                 const int slot_k = sk % ring.nstages, slot_v = sv % ring.nstages;
                 if (!mbar_wait(ring.full0 + 8u * slot_k, (sk / ring.nstages) & 1) || !mbar_wait(ring.full0 + 8u * slot_v, (sv / ring.nstages) & 1)) {
-                    atomicCAS(err, 0, DEV_ERR_FULL_WAIT);
-                    *abort_flag = 1;
+                    atomicCAS(&p.st->error, 0, DEV_ERR_FULL_WAIT);
+                    sh.abort = 1;
                     ok = false;
                     break;
                 }
@@ -532,16 +750,22 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                     bool live[UNR];
 #pragma unroll
                     for (int u = 0; u < UNR; ++u) {
-                        const int tq = tb + g + u * NG, ti = team * TQ + tq, tok = tile * T + ti;
+                        const int tq = tb + g + u * NG, ti = slice * TQ + tq, tok = tile * T + ti;
                         kw[u] = make_uint4(0, 0, 0, 0);
                         vw[u] = make_uint4(0, 0, 0, 0);
                         live[u] = tq < TQ && ti < T && tok < attn_len;
                         if (live[u]) {
                             if (tok == pos) {  // this token's own row was written after the tile was requested: read it from global memory
-                                const int page = pt[tok / p.page_tokens], off = tok % p.page_tokens;
-                                const KT* kp = pool + (size_t)page * page_stride + (size_t)h * head_stride + (size_t)off * HD + l * EPC;
-                                kw[u] = ldg_stream_coherent(kp);
-                                vw[u] = ldg_stream_coherent(kp + (size_t)p.kv_heads * head_stride);
+                                if constexpr (TAG) {
+                                    kw[u] = sh.row[l];
+                                    vw[u] = sh.row[LPT + l];
+                                } else {
+                                    const int* pt = reinterpret_cast<const int*>(mega_dyn() + p.off_pt);
+                                    const int page = pt[tok / p.page_tokens], off = tok % p.page_tokens;
+                                    const KT* kp = pool + (size_t)page * page_stride + (size_t)h * head_stride + (size_t)off * HD + l * EPC;
+                                    kw[u] = ldg_stream_coherent(kp);
+                                    vw[u] = ldg_stream_coherent(kp + (size_t)p.kv_heads * head_stride);
+                                }
                             } else {
                                 kw[u] = lds128(kbase + (uint32_t)ti * row_bytes + (uint32_t)l * 16u);
                                 vw[u] = lds128(vbase + (uint32_t)ti * row_bytes + (uint32_t)l * 16u);
@@ -556,7 +780,7 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                         }
                     }
 #pragma unroll
-                    for (int qi = 0; qi < GQA; ++qi) {
+                    for (int qi = 0; qi < GQ; ++qi) {
                         float sc[UNR];
                         float mnew = m[qi];
 #pragma unroll
@@ -592,17 +816,17 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                 }
             }
             mega_bar();  // every warp is through its tiles (or has given up)
-            if (*reinterpret_cast<volatile int*>(abort_flag) != 0) ok = false;
+            if (mega_aborted()) ok = false;
             ring.g += 2 * ncta_tiles;
             if (!ok) break;
             // ---- merge: lane groups of a team, then the teams; team 0 stores this CTA's partial of every q head
 #pragma unroll
-            for (int qi = 0; qi < GQA; ++qi) {  // unrolled: a run-time index would put the per-head state in local memory
+            for (int qi = 0; qi < GQ; ++qi) {  // unrolled: a run-time index would put the per-head state in local memory
 #pragma unroll
                 for (int e = 0; e < EPC; ++e) accs[g * HD + l * EPC + e] = acc[qi][e];
                 if (l == 0) { gm[g] = m[qi]; gl[g] = lsum[qi]; }
                 team_bar(team);
-                float* mine = tparts + ((size_t)team * MEGA_MAX_GQA + qi) * (128 + 2);
+                float* mine = sh.tparts[team][qi];
                 if (tt < HD) {
                     float M = NEG;
                     for (int gg = 0; gg < NG; ++gg) M = fmaxf(M, gm[gg]);
@@ -620,25 +844,29 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                 team_bar(team);
             }
             mega_bar();
-            if (team == 0) {
-                for (int qi = 0; qi < gqa; ++qi) {
-                    if (tt < HD) {
-                        float M = NEG;
-#pragma unroll
-                        for (int k = 0; k < MEGA_TEAMS; ++k) {
-                            const float* tp = tparts + ((size_t)k * MEGA_MAX_GQA + qi) * (128 + 2);
-                            if (tp[129] > 0.0f) M = fmaxf(M, tp[128]);
+            for (int qi = team; qi < gqa; qi += MEGA_TEAMS) {  // team k merges the slices of q heads k, k + 4, ...
+                if (tt < HD) {
+                    const float* first = sh.tparts[qi / GQ][qi % GQ];  // slice k: team k * qgroups + qi / GQ
+                    const size_t step = (size_t)qgroups * 2 * (128 + 2);
+                    float M = NEG;
+                    for (int k = 0; k < nslices; ++k) {
+                        const float* tp = first + k * step;
+                        if (tp[129] > 0.0f) M = fmaxf(M, tp[128]);
+                    }
+                    float L = 0.0f, a = 0.0f;
+                    for (int k = 0; k < nslices; ++k) {
+                        const float* tp = first + k * step;
+                        if (tp[129] > 0.0f) {
+                            const float wgt = expf(tp[128] - M);
+                            L += tp[129] * wgt;
+                            a += tp[tt] * wgt;
                         }
-                        float L = 0.0f, a = 0.0f;
-#pragma unroll
-                        for (int k = 0; k < MEGA_TEAMS; ++k) {
-                            const float* tp = tparts + ((size_t)k * MEGA_MAX_GQA + qi) * (128 + 2);
-                            if (tp[129] > 0.0f) {
-                                const float wgt = expf(tp[128] - M);
-                                L += tp[129] * wgt;
-                                a += tp[tt] * wgt;
-                            }
-                        }
+                    }
+                    if constexpr (TAG) {
+                        unsigned long long* o = p.tparts + ((size_t)(h * gqa + qi) * MEGA_CPH_CAP + plan.part) * (HD + 2);
+                        tag_store(o + tt, a, tag);
+                        if (tt < 2) tag_store(o + HD + tt, tt ? L : M, tag);
+                    } else {
                         const size_t slot = (size_t)(h * gqa + qi) * MEGA_MAX_PARTS + plan.part;
                         p.part_acc[slot * HD + tt] = a;
                         if (tt == 0) {
@@ -651,15 +879,14 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
             mega_bar();  // the teams' partials are free for the next head
         }
     }
-    return ok && *reinterpret_cast<volatile int*>(abort_flag) == 0;
+    return ok && !mega_aborted();
 }
 
 // ---- after the barrier behind the attention phase: every CTA merges the partials of every head
 // (fixed order) into the attention vector, in its own shared memory
-__device__ inline void merge_attention(const MegaParams& p, float* xs, int attn_len) {
+__device__ inline void merge_attention(const MegaParams& p, float* xs) {
     constexpr float NEG = -3.402823466e+38f;
-    const int HD = p.hd, T = p.tile_tokens, ntiles = (attn_len + T - 1) / T;
-    const int cph = attn_plan(p.kv_heads, ntiles).cph;
+    const int HD = p.hd, cph = mega_shared().plan.cph;
     for (int c = threadIdx.x; c < p.q_dim / 4; c += MEGA_CONSUMERS) {  // four consecutive dimensions of one head
         const int hq = (c * 4) / HD, d = (c * 4) % HD;
         const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + (size_t)hq * MEGA_MAX_PARTS;
@@ -685,28 +912,66 @@ __device__ inline void merge_attention(const MegaParams& p, float* xs, int attn_
     mega_bar();
 }
 
+// the same from tagged partials, as the input of the Wo phase
+__device__ inline float gather_merged(const MegaParams& p, uint32_t tag) {
+    constexpr float NEG = -3.402823466e+38f;
+    constexpr int B = 4;  // partials in flight
+    float* xs = reinterpret_cast<float*>(mega_dyn() + p.off_xs);
+    const int HD = p.hd, cph = mega_shared().plan.cph;
+#pragma unroll 1
+    for (int c = threadIdx.x; c < p.q_dim / 4; c += MEGA_CONSUMERS) {
+        const int hq = (c * 4) / HD, d = (c * 4) % HD;
+        const unsigned long long* base = p.tparts + (size_t)hq * MEGA_CPH_CAP * (HD + 2);
+        float M = NEG, L = 0.0f;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int k0 = 0; k0 < cph; k0 += B) {
+            const unsigned long long* at[3 * B];
+            unsigned long long w[3 * B][2];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const unsigned long long* part = base + (k0 + k < cph ? k0 + k : k0) * (HD + 2);
+                at[3 * k] = part + d;
+                at[3 * k + 1] = part + d + 2;
+                at[3 * k + 2] = part + HD;
+            }
+            if (!tag_poll<3 * B>(at, tag, w, p)) break;
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const float m1 = tag_value(w[3 * k + 2][0]), l1 = tag_value(w[3 * k + 2][1]);
+                if (k0 + k < cph && l1 > 0.0f) {
+                    const float Mn = fmaxf(M, m1);
+                    const float corr = expf(M - Mn), wgt = expf(m1 - Mn);
+                    L = L * corr + l1 * wgt;
+                    o.x = o.x * corr + tag_value(w[3 * k][0]) * wgt; o.y = o.y * corr + tag_value(w[3 * k][1]) * wgt;
+                    o.z = o.z * corr + tag_value(w[3 * k + 1][0]) * wgt; o.w = o.w * corr + tag_value(w[3 * k + 1][1]) * wgt;
+                    M = Mn;
+                }
+            }
+        }
+        const float inv = L > 0.0f ? 1.0f / L : 0.0f;
+        *reinterpret_cast<float4*>(xs + (size_t)c * 4) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    }
+    return 0.0f;
+}
+
 // TPAR: the tensor-parallel form (a kernel of its own, so that none of it weighs on the single-GPU token)
 template <typename WT, typename KT, int ND, int RD, int NH, int RH, bool TPAR>
-__global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const MegaParams p) {
+__global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaParams p) {
     constexpr int NW = GEMV_CONSUMERS / 32;
-    extern __shared__ __align__(128) unsigned char smraw[];
-    float* partial = reinterpret_cast<float*>(smraw + (size_t)p.nstages * p.stage_cap);  // [rows_cap][NW]
-    float* red = partial + (size_t)p.rows_cap * NW;                                       // 32 per group
-    float* attn_smem = red + 32 * MEGA_GROUPS;                                            // see mega_attn_smem_floats
-    float* xs = attn_smem;                                                                // [xs_dim] merged attention vector / gathered input, over the teams' scratch
-    int* flags = reinterpret_cast<int*>(attn_smem + mega_attn_smem_floats(p.xs_dim));      // [4] abort
-    int* pt_s = flags + 8;                                                                // page table copy
-    uint64_t* bars = reinterpret_cast<uint64_t*>(pt_s + ((p.npages + 3) & ~3));
+    MegaShared& sh = mega_shared();
+    float* const xs = reinterpret_cast<float*>(mega_dyn() + p.off_xs);
+    int* const pt_s = reinterpret_cast<int*>(mega_dyn() + p.off_pt);
+    MegaLayer* const layers_s = reinterpret_cast<MegaLayer*>(mega_dyn() + p.off_layers);
     Ring ring;
-    ring.base = smem_addr(smraw);
-    ring.full0 = smem_addr(bars);
+    ring.base = smem_addr(mega_dyn());
+    ring.full0 = ring.base + p.off_bars;
     ring.empty0 = ring.full0 + 8u * p.nstages;
     ring.stage_cap = p.stage_cap;
     ring.nstages = p.nstages;
     ring.g = 0;
-    int* err = &p.st->error;
+    int* const err = &p.st->error;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const uint32_t rb_d = (uint32_t)p.dim * sizeof(WT), rb_h = (uint32_t)p.hidden * sizeof(WT);
 
     if (tid == 0) {
         for (int s = 0; s < p.nstages; ++s) {
@@ -714,11 +979,24 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const Mega
             mbar_init(ring.empty0 + 8u * s, 2 * NW);  // the GEMV group's eight warps twice, or all sixteen warps of the attention phase
         }
         mbar_fence_init();
-        for (int i = 0; i < 8; ++i) flags[i] = 0;
+        sh.abort = 0;
     }
-    for (int i = tid; i < p.npages; i += MEGA_THREADS) pt_s[i] = p.page_table[i];
-    __syncthreads();
     const int attn_len = __ldcg(&p.st->pos) + 1;  // written by the previous token's last kernel
+    for (int i = tid; i < p.npages; i += MEGA_THREADS) pt_s[i] = p.page_table[i];
+    for (int i = tid; i < p.nlayers * (int)(sizeof(MegaLayer) / 8); i += MEGA_THREADS)
+        reinterpret_cast<unsigned long long*>(layers_s)[i] = reinterpret_cast<const unsigned long long*>(p.layers)[i];
+    if (tid < 4) {
+        int r0, r1;
+        cta_rows(tid == 0 ? p.q_dim + 2 * p.kv_dim : tid == 1 ? p.dim : tid == 2 ? 2 * p.hidden : p.vocab, tid == 0 || tid == 2 ? 2 : 1, r0, r1);
+        sh.rows[tid] = make_int2(r0, r1);
+    }
+    if (tid == 32) sh.plan = attn_plan(p.kv_heads, (attn_len + p.tile_tokens - 1) / p.tile_tokens);
+    if (tid == 64) {
+        const int page = p.page_table[(attn_len - 1) / p.page_tokens], off = (attn_len - 1) % p.page_tokens;
+        sh.kv_at = ((size_t)page * 2 * p.kv_heads * p.page_tokens + off) * p.hd;
+    }
+    if (tid < p.hd / 2) sh.rope[tid] = p.rope[(size_t)(attn_len - 1) * (p.hd / 2) + tid];
+    __syncthreads();
 
     if (warp == MEGA_CONSUMERS / 32) {  // ---- producer: fills the ring, stage after stage, as slots come free
         if ((tid & 31) == 0) {
@@ -731,37 +1009,24 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const Mega
             const unsigned long long producer_budget = p.wait_ns + 2000000000ull;
             auto put = [&](const char* src, uint32_t bytes, bool is_kv) {
                 // (a consumer that gave up raises the CTA's abort flag: the slot will not come free, and that is no error of its own)
-                if (turns > 0 && !mbar_wait_or_abort(empty, (turns - 1) & 1u, flags + 4, producer_budget)) {
-                    if (*reinterpret_cast<volatile int*>(flags + 4) == 0) atomicCAS(err, 0, DEV_ERR_EMPTY_WAIT);
+                if (turns > 0 && !mbar_wait_or_abort(empty, (turns - 1) & 1u, &sh.abort, producer_budget)) {
+                    if (!mega_aborted()) atomicCAS(err, 0, DEV_ERR_EMPTY_WAIT);
                     return false;
                 }
                 mbar_arrive_expect_tx(full, bytes);
-                if (is_kv) bulk_g2s_stream(dst, src, bytes, full, kv_policy);  // cached positions are read again by the next token: no evict-first
-                else bulk_g2s_stream(dst, src, bytes, full, policy);
+                // (cached positions are read again by the next token: no evict-first)
+                bulk_g2s_stream(dst, src, bytes, full, is_kv ? kv_policy : policy);
                 ring.g += 1;
                 if (++slot == ring.nstages) { slot = 0; turns += 1; dst = ring.base; full = ring.full0; empty = ring.empty0; }
                 else { dst += ring.stage_cap; full += 8u; empty += 8u; }
                 return true;
             };
-            walk_token_stream<RD, RH>(p, pt_s, attn_len, rb_d, (uint32_t)p.q_dim * (uint32_t)sizeof(WT), rb_h, (uint32_t)sizeof(KT), put);
+            walk_token_stream<RD, RH>(p, pt_s, attn_len, (uint32_t)p.dim * (uint32_t)sizeof(WT), (uint32_t)p.q_dim * (uint32_t)sizeof(WT),
+                                      (uint32_t)p.hidden * (uint32_t)sizeof(WT), (uint32_t)sizeof(KT), put);
         }
         return;
     }
     // ---- consumers
-    const unsigned long long nbar = (TPAR ? 3ull : 5ull) * (unsigned long long)p.nlayers;
-    const unsigned long long epoch = __ldcg(&p.st->epoch);  // launches completed so far; stable until the last barrier
-    unsigned long long arrivals = epoch * nbar;  // barriers completed by earlier launches
-    auto barrier = [&]() {
-        arrivals += 1;
-        return grid_barrier(p.grid_counter, arrivals * gridDim.x, p.wait_ns, err, flags + 4);
-    };
-    // behind a phase whose output travels through the ranks' inboxes the consumer's poll is the synchronisation: the CTA
-    // only has to be done with its own shared memory
-    auto exchange = [&]() {
-        if constexpr (!TPAR) return barrier();
-        mega_bar();
-        return *reinterpret_cast<volatile int*>(flags + 4) == 0;
-    };
     unsigned long long* tr = nullptr;
     if (p.trace != nullptr && tid == 0 && (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1))
         tr = p.trace + (blockIdx.x == 0 ? 0 : 1) * (size_t)(10 * p.nlayers + 2);
@@ -769,77 +1034,97 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const Mega
         if (tr != nullptr) *tr++ = global_ns();
     };
     stamp();
-    const WT* embed_row = nullptr;
-    if (!TPAR && p.input_embed) embed_row = reinterpret_cast<const WT*>(p.embed) + (size_t)checked_token(__ldcg(&p.st->token), p.embed_rows, err) * p.dim;
-    TpLink tin = p.tp;  // tensor parallel: the all-reduced input of a phase, x = res + alpha * sum
-    tin.alpha = p.alpha;
     bool ok = true;
-    for (int l = 0; l < p.nlayers && ok; ++l) {
-        const MegaLayer L = p.layers[l];
-        EpiQKV<KT> eq{p.q, reinterpret_cast<KT*>(L.kv), p.page_table, p.st, p.rope, p.q_dim, p.kv_dim, p.hd, p.kv_heads, p.page_tokens};
-        if constexpr (TPAR) {
+    if constexpr (!TPAR) {
+        // layer l's words carry tag0 + l (st->epoch, launches completed so far, is stable until CTA 0 has finished its last phase)
+        const uint32_t tag0 = (uint32_t)__ldcg(&p.st->epoch) * (uint32_t)p.nlayers + 1u;
+        float* const resid = reinterpret_cast<float*>(mega_dyn() + p.off_resid);
+        float* const resid_b = resid + p.rows_cap;
+        auto gather = [&](const unsigned long long* src, uint32_t tag, int K, const float* gamma, float* res) {
+            return gather_tagged(src, tag, K, InputTo{xs, res, gamma, sh.rows[1]}, p);
+        };
+        for (int l = 0; l < p.nlayers && ok; ++l) {
+            const MegaLayer& L = layers_s[l];
+            const uint32_t tag = tag0 + (uint32_t)l;
+            ok = tagged_gemv<WT, ND, RD, 2, true>(
+                ring, p, [&]() { return l == 0 ? gather_first<WT>(p, InputTo{xs, resid, L.gamma1, sh.rows[1]}) : gather(p.tx_a, tag - 1u, p.dim, L.gamma1, resid); }, nullptr,
+                sh.rows[0], p.dim, TagQKV<KT>{p, reinterpret_cast<KT*>(L.kv), tag}, stamp);
+            stamp();
+            if (!ok) break;
+            ok = p.gqa == 1 ? attention_phase<KT, 1, true>(ring, p, L.kv, attn_len, tag, stamp) : attention_phase<KT, 2, true>(ring, p, L.kv, attn_len, tag, stamp);
+            stamp();
+            if (!ok) break;
+            ok = tagged_gemv<WT, ND, RD, 1, false>(ring, p, [&]() { return gather_merged(p, tag); }, nullptr, sh.rows[1], p.q_dim,
+                                                   TagResidual{resid, p.alpha, p.tx_b, nullptr, tag}, stamp);
+            stamp();
+            if (!ok) break;
+            ok = tagged_gemv<WT, ND, RD, 2, true>(ring, p, [&]() { return gather(p.tx_b, tag, p.dim, L.gamma2, resid_b); }, nullptr, sh.rows[2], p.dim, TagGate{p, tag}, stamp);
+            stamp();
+            if (!ok) break;
+            ok = tagged_gemv<WT, NH, RH, 1, false>(ring, p, [&]() { return gather(p.tgate, tag, p.hidden, nullptr, nullptr); }, nullptr, sh.rows[1], p.hidden,
+                                                   TagResidual{resid_b, p.alpha, p.tx_a, l + 1 == p.nlayers ? p.x_a : nullptr, tag}, stamp);
+            stamp();
+        }
+        if (ok && p.want_logits)
+            ok = tagged_gemv<WT, ND, RD, 1, true>(ring, p, [&]() { return gather(p.tx_a, tag0 + (uint32_t)p.nlayers - 1u, p.dim, p.gamma_final, nullptr); }, p.norm_final,
+                                                  sh.rows[3], p.dim, EpiStore{p.logits}, []() {});
+        stamp();
+        // (also after a failure: the next launch must not take this one's words for its own)
+        if (tid == 0 && blockIdx.x == 0) p.st->epoch += 1;
+    } else {
+        const unsigned long long epoch = __ldcg(&p.st->epoch);
+        unsigned long long arrivals = epoch * 3ull * (unsigned long long)p.nlayers;  // barriers completed by earlier launches
+        auto barrier = [&]() {
+            arrivals += 1;
+            return grid_barrier(p.grid_counter, arrivals * gridDim.x, p.wait_ns, err);
+        };
+        // behind a phase whose output travels through the ranks' inboxes the consumer's poll is the synchronisation: the CTA
+        // only has to be done with its own shared memory
+        auto exchange = [&]() {
+            mega_bar();
+            return !mega_aborted();
+        };
+        TpLink tin = p.tp;  // the all-reduced input of a phase, x = res + alpha * sum
+        tin.alpha = p.alpha;
+        for (int l = 0; l < p.nlayers && ok; ++l) {
+            const MegaLayer L = layers_s[l];
+            EpiQKV<KT> eq{p.q, reinterpret_cast<KT*>(L.kv), p.page_table, p.st, p.rope, p.q_dim, p.kv_dim, p.hd, p.kv_heads, p.page_tokens};
             // layers after the first: x = x2 + alpha * sum(W2 partials of the layer before), kept in x_a
             if (l == 0) stage_first_input<WT>(p, xs);
-            else { tin.in_reduce = 2 * l; tin.res = p.x_b; tin.x_out = p.x_a; gather_input(tin, p.dim, xs, err, flags + 4); }
-            ok = consume_gemv<WT, ND, RD, 2, true>(ring, nullptr, xs, nullptr, nullptr, L.gamma1, nullptr, p.q_dim + 2 * p.kv_dim, p.dim, partial,
-                                                   red, err, flags + 4, eq);
-        } else {
-            ok = consume_gemv<WT, ND, RD, 2, true>(ring, p.x_a, nullptr, l == 0 ? embed_row : nullptr, p.x_a, L.gamma1, nullptr,
-                                                   p.q_dim + 2 * p.kv_dim, p.dim, partial, red, err, flags + 4, eq);
-        }
-        stamp();
-        if (!ok || !(ok = barrier())) break;
-        stamp();
-        ok = p.gqa == 1 ? attention_phase<KT, 1>(ring, p, L.kv, attn_smem, flags + 4, pt_s, attn_len, err)
-                        : attention_phase<KT, 2>(ring, p, L.kv, attn_smem, flags + 4, pt_s, attn_len, err);
-        stamp();
-        if (!ok || !(ok = barrier())) break;
-        stamp();
-        merge_attention(p, xs, attn_len);
-        if constexpr (TPAR)
-            ok = consume_gemv<WT, ND, RD, 1, false>(ring, nullptr, xs, nullptr, nullptr, nullptr, nullptr, p.dim, p.q_dim, partial, red, err,
-                                                    flags + 4, EpiPushPartial{&p.tp, 2 * l + 1});
-        else
-            ok = consume_gemv<WT, ND, RD, 1, false>(ring, nullptr, xs, nullptr, nullptr, nullptr, nullptr, p.dim, p.q_dim, partial, red, err,
-                                                    flags + 4, EpiResidual{p.x_a, p.x_b, p.alpha});
-        stamp();
-        if (!ok || !(ok = exchange())) break;
-        stamp();
-        if constexpr (TPAR) {  // x2 = x + alpha * sum(Wo partials), kept in x_b
+            else { tin.in_reduce = 2 * l; tin.res = p.x_b; tin.x_out = p.x_a; gather_input(tin, p.dim, xs, err); }
+            ok = consume_gemv<WT, ND, RD, 2, true>(ring, nullptr, xs, L.gamma1, nullptr, p.q_dim + 2 * p.kv_dim, p.dim, p, eq);
+            stamp();
+            if (!ok || !(ok = barrier())) break;
+            stamp();
+            ok = p.gqa == 1 ? attention_phase<KT, 1, false>(ring, p, L.kv, attn_len, 0u, stamp) : attention_phase<KT, 2, false>(ring, p, L.kv, attn_len, 0u, stamp);
+            stamp();
+            if (!ok || !(ok = barrier())) break;
+            stamp();
+            merge_attention(p, xs);
+            ok = consume_gemv<WT, ND, RD, 1, false>(ring, nullptr, xs, nullptr, nullptr, p.dim, p.q_dim, p, EpiPushPartial{&p.tp, 2 * l + 1});
+            stamp();
+            if (!ok || !(ok = exchange())) break;
+            stamp();
+            // x2 = x + alpha * sum(Wo partials), kept in x_b
             tin.in_reduce = 2 * l + 1; tin.res = p.x_a; tin.x_out = p.x_b;
-            gather_input(tin, p.dim, xs, err, flags + 4);
-            ok = consume_gemv<WT, ND, RD, 2, true>(ring, nullptr, xs, nullptr, nullptr, L.gamma2, nullptr, 2 * p.hidden, p.dim, partial, red, err,
-                                                   flags + 4, EpiGate{p.gate, p.activation});
-        } else {
-            ok = consume_gemv<WT, ND, RD, 2, true>(ring, p.x_b, nullptr, nullptr, nullptr, L.gamma2, nullptr, 2 * p.hidden, p.dim, partial, red, err,
-                                                   flags + 4, EpiGate{p.gate, p.activation});
+            gather_input(tin, p.dim, xs, err);
+            ok = consume_gemv<WT, ND, RD, 2, true>(ring, nullptr, xs, L.gamma2, nullptr, 2 * p.hidden, p.dim, p, EpiGate{p.gate, p.activation});
+            stamp();
+            if (!ok || !(ok = barrier())) break;
+            stamp();
+            ok = consume_gemv<WT, NH, RH, 1, false>(ring, p.gate, nullptr, nullptr, nullptr, p.dim, p.hidden, p, EpiPushPartial{&p.tp, 2 * l + 2});
+            stamp();
+            if (!ok || !(ok = exchange())) break;
+            stamp();
         }
-        stamp();
-        if (!ok || !(ok = barrier())) break;
-        stamp();
-        if constexpr (TPAR)
-            ok = consume_gemv<WT, NH, RH, 1, false>(ring, p.gate, nullptr, nullptr, nullptr, nullptr, nullptr, p.dim, p.hidden, partial, red, err,
-                                                    flags + 4, EpiPushPartial{&p.tp, 2 * l + 2});
-        else
-            ok = consume_gemv<WT, NH, RH, 1, false>(ring, p.gate, nullptr, nullptr, nullptr, nullptr, nullptr, p.dim, p.hidden, partial, red, err,
-                                                    flags + 4, EpiResidual{p.x_b, p.x_a, p.alpha});
-        stamp();
-        if (!ok || !(ok = exchange())) break;
-        stamp();
-    }
-    if (ok && p.want_logits) {
-        if constexpr (TPAR) {
+        if (ok && p.want_logits) {
             tin.in_reduce = 2 * p.nlayers; tin.res = p.x_b; tin.x_out = p.x_a;
-            gather_input(tin, p.dim, xs, err, flags + 4);
-            ok = consume_gemv<WT, ND, RD, 1, true>(ring, nullptr, xs, nullptr, nullptr, p.gamma_final, p.norm_final, p.vocab, p.dim, partial, red,
-                                                   err, flags + 4, EpiStore{p.logits});
-        } else {
-            ok = consume_gemv<WT, ND, RD, 1, true>(ring, p.x_a, nullptr, nullptr, nullptr, p.gamma_final, p.norm_final, p.vocab, p.dim, partial, red,
-                                                   err, flags + 4, EpiStore{p.logits});
+            gather_input(tin, p.dim, xs, err);
+            ok = consume_gemv<WT, ND, RD, 1, true>(ring, nullptr, xs, p.gamma_final, p.norm_final, p.vocab, p.dim, p, EpiStore{p.logits});
         }
+        stamp();
+        if (ok && tid == 0 && blockIdx.x == 0) p.st->epoch = epoch + 1;  // every CTA read it before its first barrier
     }
-    stamp();
-    if (ok && tid == 0 && blockIdx.x == 0) p.st->epoch = epoch + 1;  // every CTA read it before its first barrier
     if (!ok) {
         // leave only once copies that may still be in flight towards this CTA have landed: a copy lands within
         // microseconds, and a slot nobody filled never completes, so the wait for each is short

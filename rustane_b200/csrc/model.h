@@ -140,6 +140,7 @@ struct cd_model {
     bool mega = false;       // one persistent kernel per token
     int mega_nd = 0, mega_nh = 0;  // GEMV tiling of the K = dim and K = hidden phases; 0 = shape not supported
     void* mega_layers = nullptr;   // device array of cd::MegaLayer
+    void* mega_tagged = nullptr;   // its vectors between phases (64-bit words), zeroed when the model is made
     unsigned long long* grid_counter = nullptr;
     unsigned long long* mega_trace = nullptr;  // per-phase timestamps of the persistent kernel
     int prefetch_kb = 192;  // head of the next kernel's weight stream pulled into L2 by each CTA (0 = off)
