@@ -296,7 +296,7 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
         const int nd = (std::max(c.dim, c.q_dim) / epc + 255) / 256, nh = (c.hidden / epc + 255) / 256, g = c.gqa_ratio;
         // (c is this rank's shard under tensor parallelism: hidden and q_dim shrink, dim does not)
         const bool combo = tpw > 1 ? ((nd == 1 && (nh == 1 || nh == 2)) || (nd == 2 && nh >= 3 && nh <= 6)) && c.q_dim <= c.dim && g <= 2
-                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= 8)) && (g == 1 || g == 2 || g == 4 || g == MEGA_MAX_GQA);
+                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= 8)) && (g == 1 || g == 2);  // 4 and 8: the attention phase takes 15 us where the chain's kernel takes 10
         if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
         // tensor parallel: measured on the 5B model, the persistent kernel wins at 2 ranks (601 against 569 tokens/s) and
         // loses at 8 (841 against 896), where a layer's data are 8 us and its fixed per-phase times dominate either way

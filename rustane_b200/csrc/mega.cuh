@@ -128,7 +128,7 @@ struct MegaShared {
     float2 rope[64];                         // (cos, sin) of this position
     float red[64];
     AttnPlan plan;
-    int2 rows[4];                            // this CTA's rows of q|k|v, the residual stream, gate|up, head
+    int2 rows[5];                            // this CTA's rows of q|k|v, the residual stream, gate|up; [4] the head
     size_t kv_at;                            // this position's K row of kv head 0 in a layer's pages (elements)
     int abort;
 };
@@ -210,55 +210,55 @@ __device__ inline AttnPlan attn_plan(int kv_heads, int ntiles) {
 }
 
 // ---- the token's stream: everything this CTA reads from HBM for one token, stage by stage, in the
-// order the consumers use it.  f(src, bytes, is_kv) is called once per ring stage; false stops the walk.
-template <int R, class F>
-__device__ inline bool walk_rows(const void* W, uint32_t row_bytes, int N, int unit, F& f) {
-    int r0, r1;
-    cta_rows(N, unit, r0, r1);
-    const char* Wb = reinterpret_cast<const char*>(W) + (size_t)r0 * row_bytes;
-    const int ngroups = (r1 - r0 + R - 1) / R;
-    for (int g = 0; g < ngroups; ++g) {
-        const int rows = min(R, (r1 - r0) - g * R);
-        if (!f(Wb + (size_t)g * R * row_bytes, (uint32_t)rows * row_bytes, false)) return false;
-    }
-    return true;
-}
-// the K and V tiles of this CTA's attention work, one stage each, K before V
-template <class F>
-__device__ inline bool walk_attention(const MegaParams& p, const char* kv, const int* pt, int attn_len, uint32_t kes, F& f) {
-    const int T = p.tile_tokens, ntiles = (attn_len + T - 1) / T;
-    const AttnPlan plan = attn_plan(p.kv_heads, ntiles);
-    if (plan.first < 0) return true;
-    const int t0 = plan.t0, t1 = plan.t1;
-    const size_t head_bytes = (size_t)p.page_tokens * p.hd * kes, page_bytes = (size_t)2 * p.kv_heads * head_bytes;
-    const uint32_t bytes = (uint32_t)T * p.hd * kes;
-    // (one thread walks this: its dependent integer arithmetic is part of the pace of the phase, so page and offset
-    // advance by increments instead of a division per tile)
-    const int tpp = p.page_tokens / T;  // tiles per page
-    const size_t v_off = (size_t)p.kv_heads * head_bytes;
-    for (int h = plan.first; h < p.kv_heads; h += plan.step) {
-        int pg = t0 / tpp, sub = t0 % tpp;
-        const char* hb = kv + (size_t)h * head_bytes;
-        for (int t = t0; t < t1; ++t) {
-            const char* k = hb + (size_t)pt[pg] * page_bytes + (size_t)sub * bytes;
-            if (!f(k, bytes, true) || !f(k + v_off, bytes, true)) return false;
-            if (++sub == tpp) { sub = 0; ++pg; }
+// order the consumers use it: its rows of q|k|v, the K and V tiles of its attention work (one stage each, K before V),
+// its rows of Wo, W1|W3 and W2, layer after layer, then of the LM head.  f(src, bytes, is_kv) is called once per ring
+// stage; false stops the walk.  (One call of f: its wait loop inlined per segment was a quarter of the kernel's code.)
+template <int RD, int RH, class F>
+__device__ inline bool walk_token_stream(const MegaParams& p, const MegaLayer* layers, const int* pt, uint32_t rb_d, uint32_t rb_q, uint32_t rb_h, uint32_t kes, F& f) {
+    const MegaShared& sh = mega_shared();
+    const AttnPlan plan = sh.plan;
+    const int T = p.tile_tokens, tpp = p.page_tokens / T;  // tiles per page
+    const size_t head_bytes = (size_t)p.page_tokens * p.hd * kes, page_bytes = (size_t)2 * p.kv_heads * head_bytes, v_off = (size_t)p.kv_heads * head_bytes;
+    const uint32_t tile_bytes = (uint32_t)T * p.hd * kes;
+    for (int l = 0; l <= p.nlayers; ++l) {
+        if (l == p.nlayers && !p.want_logits) break;
+        const MegaLayer& L = layers[min(l, p.nlayers - 1)];
+        for (int seg = 0; seg < (l < p.nlayers ? 5 : 1); ++seg) {
+            const bool kv = l < p.nlayers && seg == 1;
+            const char* base = nullptr;
+            uint32_t step = tile_bytes, left = 0;  // bytes per stage, bytes of the whole segment
+            int n, h = plan.first, pg = 0, sub = 0, t = plan.t0;
+            if (kv) {
+                n = 2 * (h < 0 ? 0 : (plan.t1 - plan.t0) * ((p.kv_heads - h + plan.step - 1) / plan.step));
+                pg = t / tpp; sub = t % tpp;
+            } else {
+                const bool head = l == p.nlayers;
+                const int2 r = sh.rows[head ? 4 : seg == 0 ? 0 : seg == 3 ? 2 : 1];
+                const uint32_t rb = head || seg == 0 || seg == 3 ? rb_d : seg == 2 ? rb_q : rb_h;
+                const int R = !head && seg == 4 ? RH : RD;
+                base = reinterpret_cast<const char*>(head ? p.lm_head : seg == 0 ? L.wqkv : seg == 2 ? L.wo : seg == 3 ? L.w13 : L.w2) + (size_t)r.x * rb;
+                n = (r.y - r.x + R - 1) / R;
+                step = (uint32_t)R * rb;
+                left = (uint32_t)(r.y - r.x) * rb;
+            }
+            for (int i = 0; i < n; ++i) {
+                const char* src = base;
+                uint32_t bytes = step;
+                if (kv) {  // page and offset advance by increments instead of a division per tile
+                    src = reinterpret_cast<const char*>(L.kv) + (size_t)h * head_bytes + (size_t)pt[pg] * page_bytes + (size_t)sub * tile_bytes + ((i & 1) ? v_off : 0);
+                    if (i & 1) {
+                        if (++sub == tpp) { sub = 0; ++pg; }
+                        if (++t == plan.t1) { h += plan.step; t = plan.t0; pg = t / tpp; sub = t % tpp; }
+                    }
+                } else {
+                    bytes = min(step, left);
+                    base += step;
+                    left -= bytes;
+                }
+                if (!f(src, bytes, kv)) return false;
+            }
         }
     }
-    return true;
-}
-template <int RD, int RH, class F>
-__device__ inline bool walk_token_stream(const MegaParams& p, const int* pt, int attn_len, uint32_t rb_d, uint32_t rb_q, uint32_t rb_h, uint32_t kes, F& f) {
-    for (int l = 0; l < p.nlayers; ++l) {
-        const MegaLayer& L = p.layers[l];
-        if (!(walk_rows<RD>(L.wqkv, rb_d, p.q_dim + 2 * p.kv_dim, 2, f) &&
-              walk_attention(p, reinterpret_cast<const char*>(L.kv), pt, attn_len, kes, f) &&
-              walk_rows<RD>(L.wo, rb_q, p.dim, 1, f) &&
-              walk_rows<RD>(L.w13, rb_d, 2 * p.hidden, 2, f) &&
-              walk_rows<RH>(L.w2, rb_h, p.dim, 1, f)))
-            return false;
-    }
-    if (p.want_logits) return walk_rows<RD>(p.lm_head, rb_d, p.vocab, 1, f);
     return true;
 }
 
@@ -314,9 +314,9 @@ __device__ __noinline__ void stage_first_input(const MegaParams& p, float* xs) {
 }
 
 // ---- consumer side of one GEMV phase: this CTA's rows [r0, r1) out of the ring times the input slices xr each thread holds
-// (chunks tid, tid + 256, ... of the vector, the same in both groups), then the epilogue on its units
-template <typename WT, int NITER, int R, int UNIT, class Epi>
-__device__ inline bool stream_rows(Ring& ring, const float (&xr)[NITER][Elem<WT>::EPC], int r0, int r1, int K, const MegaParams& p, const Epi& epi) {
+// (chunks tid, tid + 256, ... of the vector, the same in both groups), a partial sum per row and warp of a group
+template <typename WT, int NITER, int R>
+__device__ inline void stream_partials(Ring& ring, const float (&xr)[NITER][Elem<WT>::EPC], int r0, int r1, int K, const MegaParams& p) {
     float* partial = reinterpret_cast<float*>(mega_dyn() + p.off_partial);
     constexpr int EPC = Elem<WT>::EPC;
     constexpr int NW = GEMV_CONSUMERS / 32;
@@ -368,22 +368,13 @@ __device__ inline bool stream_rows(Ring& ring, const float (&xr)[NITER][Elem<WT>
         if ((lane & (32 / R - 1)) == 0 && row < r1 - r0) partial[row * NW + warp] = tot;
     }
     ring.g += ngroups;
-    mega_bar();
-    if (mega_aborted()) return false;
-    const int u0 = r0 / UNIT, nu = (r1 - r0) / UNIT;
-#pragma unroll 1
-    for (int u = threadIdx.x; u < nu; u += MEGA_CONSUMERS) {
-        float y[UNIT];
+}
+// row r of the phase: the sums of its group's warps
+__device__ inline float row_sum(const float* partial, int r) {
+    float t = 0.0f;
 #pragma unroll
-        for (int k = 0; k < UNIT; ++k) {
-            float sacc = 0.0f;
-#pragma unroll
-            for (int wi = 0; wi < NW; ++wi) sacc += partial[(u * UNIT + k) * NW + wi];
-            y[k] = sacc;
-        }
-        epi(u0 + u, y);
-    }
-    return true;
+    for (int w = 0; w < GEMV_CONSUMERS / 32; ++w) t += partial[r * (GEMV_CONSUMERS / 32) + w];
+    return t;
 }
 
 // ---- one GEMV phase of the tensor-parallel form.  The input vector comes from `x` (fp32, L2-only loads), from
@@ -447,7 +438,19 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
             }
         }
     }
-    return stream_rows<WT, NITER, R, UNIT>(ring, xr, r0, r1, K, p, epi);
+    stream_partials<WT, NITER, R>(ring, xr, r0, r1, K, p);
+    mega_bar();
+    if (mega_aborted()) return false;
+    const float* partial = reinterpret_cast<const float*>(mega_dyn() + p.off_partial);
+    const int u0 = r0 / UNIT, nu = (r1 - r0) / UNIT;
+#pragma unroll 1
+    for (int u = threadIdx.x; u < nu; u += MEGA_CONSUMERS) {
+        float y[UNIT];
+#pragma unroll
+        for (int k = 0; k < UNIT; ++k) y[k] = row_sum(partial, u * UNIT + k);
+        epi(u0 + u, y);
+    }
+    return true;
 }
 
 // ---- one GPU: vectors between phases travel as tagged words.  A word is a 64-bit pair (value, tag), written by one
@@ -455,6 +458,8 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
 // fence, no counter, no barrier, and the poll that sees the last word already has the data in registers.  A buffer is
 // written once per layer; its readers of layer l are done before any CTA can write layer l + 1, because every CTA owns
 // rows of every matrix and a CTA's rows of the next phase are stored only after it has read its whole input.
+// (Against a grid barrier per phase - release reduction, acquire polls, then the loads: 2.8-3.0 us and the loads - a token of
+// the 5B model takes 2.12 instead of 2.25 ms, of a 0.6B model of 24 layers 0.74 instead of 0.91 ms.)
 __device__ inline void tag_store(unsigned long long* p, float v, uint32_t tag) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)tag << 32 | __float_as_uint(v)) : "memory");
 }
@@ -542,26 +547,16 @@ template <typename WT> __device__ inline float gather_first(const MegaParams& p,
     return ss;
 }
 
-// One GEMV phase: the input vector (in() fills xs and returns the thread's share of the sum of squares) into registers,
-// under NORM over its root mean square, then this CTA's rows.
-template <typename WT, int NITER, int R, int UNIT, bool NORM, class In, class Epi, class Tick>
-__device__ inline bool tagged_gemv(Ring& ring, const MegaParams& p, const In& in, float* norm_out, const int2& rows, int K, const Epi& epi, const Tick& input_is_in) {
-    const float* xs = reinterpret_cast<const float*>(mega_dyn() + p.off_xs);
-    float* red = mega_shared().red;
+// The phases of one GPU share their code: a layer's instructions run once per layer and CTA, and five inlined copies of
+// the GEMV waited for the instruction cache (about 0.5 us at the start of every phase of a small model).
+enum { PH_QKV = 0, PH_WO = 1, PH_W13 = 2, PH_W2 = 3, PH_HEAD = 4 };
+
+// the rows of a phase: input slices out of xs, times inv (1 / root mean square, or 1)
+template <typename WT, int NITER, int R>
+__device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, float* norm_out, const int2& rows, int K) {
     constexpr int EPC = Elem<WT>::EPC;
-    const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255;
-    const int nchunks = K / EPC;
-    const float ss = NORM ? warp_sum(in()) : in();
-    if (NORM && (threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    mega_bar();
-    input_is_in();
-    float inv = 1.0f;
-    if (NORM) {
-        float tot = 0.0f;
-#pragma unroll
-        for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) tot += red[i];
-        inv = 1.0f / sqrtf(tot * (1.0f / (float)K) + RMS_EPS);
-    }
+    const float* xs = reinterpret_cast<const float*>(mega_dyn() + p.off_xs);
+    const int tid = threadIdx.x & 255, nchunks = K / EPC;
     float xr[NITER][EPC];
 #pragma unroll
     for (int i = 0; i < NITER; ++i) {
@@ -570,62 +565,66 @@ __device__ inline bool tagged_gemv(Ring& ring, const MegaParams& p, const In& in
         for (int e = 0; e < EPC; e += 4) {
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (c < nchunks) v = *reinterpret_cast<const float4*>(xs + (size_t)c * EPC + e);
-            if (NORM) {
-                v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
-                if (norm_out != nullptr && blockIdx.x == 0 && grp == 0 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
-            }
+            v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+            if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x < 256 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
             xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
         }
     }
-    return stream_rows<WT, NITER, R, UNIT>(ring, xr, rows.x, rows.y, K, p, epi);
+    stream_partials<WT, NITER, R>(ring, xr, rows.x, rows.y, K, p);
 }
 
-// epilogues of the tagged phases (arithmetic of EpiQKV, EpiGate, EpiResidual)
-template <typename KT> struct TagQKV {
-    const MegaParams& p;
-    KT* kv;
-    uint32_t tag;
-    __device__ void operator()(int unit, const float (&y)[2]) const {
-        const MegaShared& sh = mega_shared();
-        const int r = unit * 2, d = r & (p.hd - 1);  // (hd is 64 or 128)
-        float e = y[0], o = y[1];
-        if (r < p.q_dim + p.kv_dim) {
-            const float2 cs = sh.rope[d >> 1];
-            e = y[0] * cs.x - y[1] * cs.y;
-            o = y[1] * cs.x + y[0] * cs.y;
+// the epilogue of a phase on this CTA's rows (arithmetic of EpiQKV, EpiGate, EpiResidual, EpiStore)
+template <typename KT>
+__device__ inline void tagged_epilogue(const MegaParams& p, int ph, bool last_layer, void* kv, uint32_t tag) {
+    const MegaShared& sh = mega_shared();
+    const float* partial = reinterpret_cast<const float*>(mega_dyn() + p.off_partial);
+    const float* resid = reinterpret_cast<const float*>(mega_dyn() + p.off_resid);
+    const int2 rows = sh.rows[ph == PH_W2 ? PH_WO : ph];
+    if (ph == PH_QKV || ph == PH_W13) {  // pairs of rows
+#pragma unroll 1
+        for (int j = 2 * threadIdx.x; j < rows.y - rows.x; j += 2 * MEGA_CONSUMERS) {
+            const int r = rows.x + j;
+            float e = row_sum(partial, j), o = row_sum(partial, j + 1);
+            if (ph == PH_W13) {
+                tag_store(p.tgate + (r >> 1), gate_value(e, o, p.activation), tag);
+                continue;
+            }
+            const int d = r & (p.hd - 1);  // (hd is 64 or 128)
+            if (r < p.q_dim + p.kv_dim) {
+                const float2 cs = sh.rope[d >> 1];
+                const float a = e * cs.x - o * cs.y, b = o * cs.x + e * cs.y;
+                e = a;
+                o = b;
+            }
+            unsigned long long* dst = p.tq + r;
+            if (r >= p.q_dim) {  // tkv: this position's K then V as cached (rounded), for the CTAs that attend to it in this layer
+                const int rk = r - p.q_dim, v = rk >= p.kv_dim, head = (v ? rk - p.kv_dim : rk) >> (p.hd == 128 ? 7 : 6);
+                const KT ek = Elem<KT>::from_f32(e), ok = Elem<KT>::from_f32(o);
+                KT* page = reinterpret_cast<KT*>(kv) + sh.kv_at + (size_t)(v * p.kv_heads + head) * p.page_tokens * p.hd + d;
+                page[0] = ek;
+                page[1] = ok;
+                e = Elem<KT>::to_f32(ek);
+                o = Elem<KT>::to_f32(ok);
+                dst = p.tkv + rk;
+            }
+            tag_store(dst, e, tag);
+            tag_store(dst + 1, o, tag);
         }
-        if (r < p.q_dim) {
-            tag_store(p.tq + r, e, tag);
-            tag_store(p.tq + r + 1, o, tag);
-            return;
+    } else {
+#pragma unroll 1
+        for (int j = threadIdx.x; j < rows.y - rows.x; j += MEGA_CONSUMERS) {
+            const int r = rows.x + j;
+            const float y = row_sum(partial, j);
+            if (ph == PH_HEAD) {
+                p.logits[r] = y;
+            } else {
+                const float v = resid[(ph == PH_W2 ? p.rows_cap : 0) + j] + p.alpha * y;
+                tag_store((ph == PH_W2 ? p.tx_a : p.tx_b) + r, v, tag);
+                if (ph == PH_W2 && last_layer) p.x_a[r] = v;
+            }
         }
-        // tkv: this position's K then V as cached (rounded), for the CTAs that attend to it in this layer
-        const int rk = r - p.q_dim, v = rk >= p.kv_dim, head = (v ? rk - p.kv_dim : rk) >> (p.hd == 128 ? 7 : 6);
-        const KT ek = Elem<KT>::from_f32(e), ok = Elem<KT>::from_f32(o);
-        tag_store(p.tkv + rk, Elem<KT>::to_f32(ek), tag);
-        tag_store(p.tkv + rk + 1, Elem<KT>::to_f32(ok), tag);
-        KT* dst = kv + sh.kv_at + (size_t)(v * p.kv_heads + head) * p.page_tokens * p.hd + d;
-        dst[0] = ek;
-        dst[1] = ok;
     }
-};
-struct TagGate {
-    const MegaParams& p;
-    uint32_t tag;
-    __device__ void operator()(int unit, const float (&y)[2]) const { tag_store(p.tgate + unit, gate_value(y[0], y[1], p.activation), tag); }
-};
-struct TagResidual {
-    const float* resid;       // this CTA's entries, from its first row on
-    float alpha;
-    unsigned long long* out;
-    float* plain;             // also as plain floats (the last layer's result), or null
-    uint32_t tag;
-    __device__ void operator()(int unit, const float (&y)[1]) const {
-        const float v = resid[unit - mega_shared().rows[1].x] + alpha * y[0];
-        tag_store(out + unit, v, tag);
-        if (plain != nullptr) plain[unit] = v;
-    }
-};
+}
 
 // ---- grid barrier for the consumer threads of all CTAs (arrival k of this launch).  One thread
 // per CTA adds to a monotonic counter with release semantics (a reduction, not an atomic with a
@@ -988,7 +987,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
     if (tid < 4) {
         int r0, r1;
         cta_rows(tid == 0 ? p.q_dim + 2 * p.kv_dim : tid == 1 ? p.dim : tid == 2 ? 2 * p.hidden : p.vocab, tid == 0 || tid == 2 ? 2 : 1, r0, r1);
-        sh.rows[tid] = make_int2(r0, r1);
+        sh.rows[tid == 3 ? PH_HEAD : tid] = make_int2(r0, r1);
     }
     if (tid == 32) sh.plan = attn_plan(p.kv_heads, (attn_len + p.tile_tokens - 1) / p.tile_tokens);
     if (tid == 64) {
@@ -1021,7 +1020,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
                 else { dst += ring.stage_cap; full += 8u; empty += 8u; }
                 return true;
             };
-            walk_token_stream<RD, RH>(p, pt_s, attn_len, (uint32_t)p.dim * (uint32_t)sizeof(WT), (uint32_t)p.q_dim * (uint32_t)sizeof(WT),
+            walk_token_stream<RD, RH>(p, layers_s, pt_s, (uint32_t)p.dim * (uint32_t)sizeof(WT), (uint32_t)p.q_dim * (uint32_t)sizeof(WT),
                                       (uint32_t)p.hidden * (uint32_t)sizeof(WT), (uint32_t)sizeof(KT), put);
         }
         return;
@@ -1039,35 +1038,42 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
         // layer l's words carry tag0 + l (st->epoch, launches completed so far, is stable until CTA 0 has finished its last phase)
         const uint32_t tag0 = (uint32_t)__ldcg(&p.st->epoch) * (uint32_t)p.nlayers + 1u;
         float* const resid = reinterpret_cast<float*>(mega_dyn() + p.off_resid);
-        float* const resid_b = resid + p.rows_cap;
-        auto gather = [&](const unsigned long long* src, uint32_t tag, int K, const float* gamma, float* res) {
-            return gather_tagged(src, tag, K, InputTo{xs, res, gamma, sh.rows[1]}, p);
-        };
-        for (int l = 0; l < p.nlayers && ok; ++l) {
-            const MegaLayer& L = layers_s[l];
+        const int phases = 4 * p.nlayers + (p.want_logits ? 1 : 0);
+        for (int step = 0; step < phases; ++step) {
+            const int l = step >> 2, ph = l < p.nlayers ? step & 3 : PH_HEAD;
+            const MegaLayer& L = layers_s[min(l, p.nlayers - 1)];
             const uint32_t tag = tag0 + (uint32_t)l;
-            ok = tagged_gemv<WT, ND, RD, 2, true>(
-                ring, p, [&]() { return l == 0 ? gather_first<WT>(p, InputTo{xs, resid, L.gamma1, sh.rows[1]}) : gather(p.tx_a, tag - 1u, p.dim, L.gamma1, resid); }, nullptr,
-                sh.rows[0], p.dim, TagQKV<KT>{p, reinterpret_cast<KT*>(L.kv), tag}, stamp);
+            float ss;
+            if (ph == PH_WO) {
+                ok = p.gqa == 1 ? attention_phase<KT, 1, true>(ring, p, L.kv, attn_len, tag, stamp) : attention_phase<KT, 2, true>(ring, p, L.kv, attn_len, tag, stamp);
+                stamp();
+                if (!ok) break;
+                ss = gather_merged(p, tag);
+            } else {
+                const InputTo to{xs, ph == PH_QKV ? resid : ph == PH_W13 ? resid + p.rows_cap : nullptr,
+                                 ph == PH_QKV ? L.gamma1 : ph == PH_W13 ? L.gamma2 : ph == PH_HEAD ? p.gamma_final : nullptr, sh.rows[PH_WO]};
+                if (step == 0) ss = gather_first<WT>(p, to);
+                else ss = gather_tagged(ph == PH_W13 ? p.tx_b : ph == PH_W2 ? p.tgate : p.tx_a, ph == PH_W13 || ph == PH_W2 ? tag : tag - 1u, ph == PH_W2 ? p.hidden : p.dim, to, p);
+            }
+            const bool norm = ph != PH_WO && ph != PH_W2;
+            ss = warp_sum(ss);
+            if ((tid & 31) == 0) sh.red[warp] = ss;
+            mega_bar();
             stamp();
-            if (!ok) break;
-            ok = p.gqa == 1 ? attention_phase<KT, 1, true>(ring, p, L.kv, attn_len, tag, stamp) : attention_phase<KT, 2, true>(ring, p, L.kv, attn_len, tag, stamp);
-            stamp();
-            if (!ok) break;
-            ok = tagged_gemv<WT, ND, RD, 1, false>(ring, p, [&]() { return gather_merged(p, tag); }, nullptr, sh.rows[1], p.q_dim,
-                                                   TagResidual{resid, p.alpha, p.tx_b, nullptr, tag}, stamp);
-            stamp();
-            if (!ok) break;
-            ok = tagged_gemv<WT, ND, RD, 2, true>(ring, p, [&]() { return gather(p.tx_b, tag, p.dim, L.gamma2, resid_b); }, nullptr, sh.rows[2], p.dim, TagGate{p, tag}, stamp);
-            stamp();
-            if (!ok) break;
-            ok = tagged_gemv<WT, NH, RH, 1, false>(ring, p, [&]() { return gather(p.tgate, tag, p.hidden, nullptr, nullptr); }, nullptr, sh.rows[1], p.hidden,
-                                                   TagResidual{resid_b, p.alpha, p.tx_a, l + 1 == p.nlayers ? p.x_a : nullptr, tag}, stamp);
-            stamp();
+            float inv = 1.0f;
+            if (norm) {
+                float tot = 0.0f;
+#pragma unroll
+                for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) tot += sh.red[i];
+                inv = 1.0f / sqrtf(tot * (1.0f / (float)p.dim) + RMS_EPS);
+            }
+            if (ph == PH_W2) tagged_rows<WT, NH, RH>(ring, p, inv, nullptr, sh.rows[PH_WO], p.hidden);
+            else tagged_rows<WT, ND, RD>(ring, p, inv, ph == PH_HEAD ? p.norm_final : nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
+            mega_bar();
+            if (mega_aborted()) { ok = false; break; }
+            tagged_epilogue<KT>(p, ph, l + 1 == p.nlayers, L.kv, tag);
+            if (ph != PH_HEAD) stamp();
         }
-        if (ok && p.want_logits)
-            ok = tagged_gemv<WT, ND, RD, 1, true>(ring, p, [&]() { return gather(p.tx_a, tag0 + (uint32_t)p.nlayers - 1u, p.dim, p.gamma_final, nullptr); }, p.norm_final,
-                                                  sh.rows[3], p.dim, EpiStore{p.logits}, []() {});
         stamp();
         // (also after a failure: the next launch must not take this one's words for its own)
         if (tid == 0 && blockIdx.x == 0) p.st->epoch += 1;
