@@ -37,16 +37,18 @@ cudaError_t launch_attn(cd_model* m, const cd_layer_dev& L) {
 }
 
 // ------------------------------------------------------------------ persistent kernel launch
-template <typename WT, typename KT, int ND, int NH, bool TPAR>
+template <typename WT, typename LT, typename KT, int ND, int NH, bool TPAR>
 cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
-    constexpr int RD = ND == 1 ? 4 : ND == 2 ? 2 : 1;
-    constexpr int RH = NH == 1 ? 4 : NH == 2 ? 2 : 1;
+    constexpr bool Q = Wfmt<LT>::QUANT;
+    constexpr int RD = ND == 1 ? 4 : ND == 2 || Q ? 2 : 1;
+    constexpr int RH = NH == 1 ? 4 : NH == 2 || Q ? 2 : 1;
+    constexpr int NO = Q ? 2 * ND : ND;  // an FP8 chunk is twice as many elements as one of the head's
+    constexpr int RO = Q ? (NO == 2 ? 2 : 1) : RD;
     const cd_config& c = m->cfg;
-    auto kern = decode_mega_kernel<WT, KT, ND, RD, NH, RH, TPAR>;
+    auto kern = decode_mega_kernel<WT, LT, KT, ND, RD, NH, RH, NO, RO, TPAR>;
     // every CTA owns rows of every matrix: what tells a CTA that another one is done with a vector is that one's next rows
     const int grid = TPAR ? m->sm_count : std::min({m->sm_count, c.dim, c.hidden, (c.q_dim + 2 * c.kv_dim) / 2});
-    const size_t es = sizeof(WT);
-    const size_t stage_cap = (std::max((size_t)RD * std::max(c.dim, c.q_dim) * es, (size_t)RH * c.hidden * es) + 127) / 128 * 128;
+    const size_t stage_cap = (std::max({(size_t)RD * Wfmt<LT>::row_stride(std::max(c.dim, c.q_dim)), (size_t)RH * Wfmt<LT>::row_stride(c.hidden), (size_t)RO * c.dim * sizeof(WT)}) + 127) / 128 * 128;
     int max_rows = 0;
     for (int n : {c.q_dim + 2 * c.kv_dim, c.dim, 2 * c.hidden, want_logits ? m->v_loc : 0}) max_rows = std::max(max_rows, n / grid + 2);
     const int xs_dim = TPAR ? std::max(c.q_dim, c.dim) : std::max({c.q_dim, c.dim, c.hidden});
@@ -105,25 +107,26 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     return e;
 }
 
-template <typename WT, typename KT, bool TPAR>
+template <typename WT, typename LT, typename KT, bool TPAR>
 cudaError_t launch_mega_tp(cd_model* m, int input_embed, int want_logits) {
     switch (m->mega_nd * 10 + m->mega_nh) {
-        case 11: return launch_mega_t<WT, KT, 1, 1, TPAR>(m, input_embed, want_logits);
-        case 12: return launch_mega_t<WT, KT, 1, 2, TPAR>(m, input_embed, want_logits);
-        case 14: if constexpr (!TPAR) return launch_mega_t<WT, KT, 1, 4, TPAR>(m, input_embed, want_logits); else break;
-        case 24: return launch_mega_t<WT, KT, 2, 4, TPAR>(m, input_embed, want_logits);
-        case 26: return launch_mega_t<WT, KT, 2, 6, TPAR>(m, input_embed, want_logits);
-        case 28: if constexpr (!TPAR) return launch_mega_t<WT, KT, 2, 8, TPAR>(m, input_embed, want_logits); else break;
+        case 11: return launch_mega_t<WT, LT, KT, 1, 1, TPAR>(m, input_embed, want_logits);
+        case 12: return launch_mega_t<WT, LT, KT, 1, 2, TPAR>(m, input_embed, want_logits);
+        case 14: if constexpr (!TPAR) return launch_mega_t<WT, LT, KT, 1, 4, TPAR>(m, input_embed, want_logits); else break;
+        case 13: if constexpr (Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 1, 3, TPAR>(m, input_embed, want_logits); else break;
+        case 24: return launch_mega_t<WT, LT, KT, 2, 4, TPAR>(m, input_embed, want_logits);
+        case 26: if constexpr (!Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 6, TPAR>(m, input_embed, want_logits); else break;
+        case 28: if constexpr (!TPAR && !Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 8, TPAR>(m, input_embed, want_logits); else break;
         default: break;
     }
     return cudaErrorInvalidConfiguration;
 }
-template <typename WT, typename KT>
+template <typename WT, typename LT, typename KT>
 cudaError_t launch_mega(cd_model* m, int input_embed, int want_logits) {
-    if constexpr (!std::is_same<WT, float>::value) {  // the tensor-parallel form exists for the 16-bit storage types
-        if (m->tp_world > 1) return launch_mega_tp<WT, KT, true>(m, input_embed, want_logits);
+    if constexpr (!std::is_same<WT, float>::value && !Wfmt<LT>::QUANT) {  // the tensor-parallel form exists for the 16-bit storage types
+        if (m->tp_world > 1) return launch_mega_tp<WT, LT, KT, true>(m, input_embed, want_logits);
     }
-    return launch_mega_tp<WT, KT, false>(m, input_embed, want_logits);
+    return launch_mega_tp<WT, LT, KT, false>(m, input_embed, want_logits);
 }
 
 // One token through the whole model; everything is enqueued on m->stream.
@@ -138,9 +141,10 @@ cudaError_t enqueue_step_t(cd_model* m, const cd_step& p) {
         next_prompt_kernel<<<1, 1, 0, m->stream>>>(m->st, m->prompt_dev);
         count_launch(m);
     }
-    const bool use_mega = std::is_same<WT, LT>::value && m->mega && m->mega_nd > 0 && !m->profiling;
+    constexpr bool has_mega = !std::is_same<LT, Int4G32>::value;
+    const bool use_mega = has_mega && m->mega && m->mega_nd > 0 && !m->profiling;
     if (use_mega) {
-        if constexpr (std::is_same<WT, LT>::value) TRY((launch_mega<WT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0)));
+        if constexpr (has_mega) TRY((launch_mega<WT, LT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0)));
     } else if (p.input >= 1) {
         embed_kernel<WT><<<std::max(1, c.dim / 256), 256, 0, m->stream>>>((const WT*)m->embed, m->st, m->x_a, c.dim, m->full_cfg.vocab);
         count_launch(m);
@@ -292,15 +296,15 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
         }
         CKB(cudaMemcpyAsync(m->mega_layers, ml.data(), ml.size() * sizeof(MegaLayer), cudaMemcpyHostToDevice, m->stream));
         CKB(cudaStreamSynchronize(m->stream));
-        const int epc = dt == CD_DTYPE_F32 ? 4 : 8;
+        const int epc = dt == CD_DTYPE_F32 ? 4 : dt == CD_DTYPE_FP8_E4M3 ? 16 : 8;
         const int nd = (std::max(c.dim, c.q_dim) / epc + 255) / 256, nh = (c.hidden / epc + 255) / 256, g = c.gqa_ratio;
         // (c is this rank's shard under tensor parallelism: hidden and q_dim shrink, dim does not)
         const bool combo = tpw > 1 ? ((nd == 1 && (nh == 1 || nh == 2)) || (nd == 2 && nh >= 3 && nh <= 6)) && c.q_dim <= c.dim && g <= 2
-                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= 8)) && (g == 1 || g == 2);  // 4 and 8: the attention phase takes 15 us where the chain's kernel takes 10
-        if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
+                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= (dt == CD_DTYPE_FP8_E4M3 ? 4 : 8))) && (g == 1 || g == 2);  // 4 and 8: the attention phase takes 15 us where the chain's kernel takes 10
+        if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 && dt != CD_DTYPE_FP8_E4M3 ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
         // tensor parallel: measured on the 5B model, the persistent kernel wins at 2 ranks (601 against 569 tokens/s) and
         // loses at 8 (841 against 896), where a layer's data are 8 us and its fixed per-phase times dominate either way
-        const bool mega_ok = !is_quant(dt) && (tpw == 1 || (tpw == 2 && dt != CD_DTYPE_F32));
+        const bool mega_ok = dt != CD_DTYPE_INT4_G32 && (tpw == 1 || (tpw == 2 && dt != CD_DTYPE_F32 && !is_quant(dt)));
         // one persistent kernel per token wherever its tiling covers the shape; test_flags bit 1 keeps one kernel per operator
         m->mega = (opts.test_flags & 2) == 0 && mega_ok && m->mega_nd > 0;
     }

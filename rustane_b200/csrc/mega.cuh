@@ -213,8 +213,8 @@ __device__ inline AttnPlan attn_plan(int kv_heads, int ntiles) {
 // order the consumers use it: its rows of q|k|v, the K and V tiles of its attention work (one stage each, K before V),
 // its rows of Wo, W1|W3 and W2, layer after layer, then of the LM head.  f(src, bytes, is_kv) is called once per ring
 // stage; false stops the walk.  (One call of f: its wait loop inlined per segment was a quarter of the kernel's code.)
-template <int RD, int RH, class F>
-__device__ inline bool walk_token_stream(const MegaParams& p, const MegaLayer* layers, const int* pt, uint32_t rb_d, uint32_t rb_q, uint32_t rb_h, uint32_t kes, F& f) {
+template <int RD, int RH, int RO, class F>
+__device__ inline bool walk_token_stream(const MegaParams& p, const MegaLayer* layers, const int* pt, uint32_t rb_d, uint32_t rb_q, uint32_t rb_h, uint32_t rb_o, uint32_t kes, F& f) {
     const MegaShared& sh = mega_shared();
     const AttnPlan plan = sh.plan;
     const int T = p.tile_tokens, tpp = p.page_tokens / T;  // tiles per page
@@ -234,8 +234,8 @@ __device__ inline bool walk_token_stream(const MegaParams& p, const MegaLayer* l
             } else {
                 const bool head = l == p.nlayers;
                 const int2 r = sh.rows[head ? 4 : seg == 0 ? 0 : seg == 3 ? 2 : 1];
-                const uint32_t rb = head || seg == 0 || seg == 3 ? rb_d : seg == 2 ? rb_q : rb_h;
-                const int R = !head && seg == 4 ? RH : RD;
+                const uint32_t rb = head ? rb_o : seg == 0 || seg == 3 ? rb_d : seg == 2 ? rb_q : rb_h;
+                const int R = head ? RO : seg == 4 ? RH : RD;
                 base = reinterpret_cast<const char*>(head ? p.lm_head : seg == 0 ? L.wqkv : seg == 2 ? L.wo : seg == 3 ? L.w13 : L.w2) + (size_t)r.x * rb;
                 n = (r.y - r.x + R - 1) / R;
                 step = (uint32_t)R * rb;
@@ -313,16 +313,94 @@ __device__ __noinline__ void stage_first_input(const MegaParams& p, float* xs) {
     mega_bar();
 }
 
-// ---- consumer side of one GEMV phase: this CTA's rows [r0, r1) out of the ring times the input slices xr each thread holds
-// (chunks tid, tid + 256, ... of the vector, the same in both groups), a partial sum per row and warp of a group
-template <typename WT, int NITER, int R>
-__device__ inline void stream_partials(Ring& ring, const float (&xr)[NITER][Elem<WT>::EPC], int r0, int r1, int K, const MegaParams& p) {
+// ---- the input slice a thread holds (chunks tid, tid + 256, ... of the vector, the same in both groups), and the rows of
+// a stage times it
+template <typename LT, int NITER> struct Slices {
+    static constexpr int EPC = Wfmt<LT>::EPC;
+    float x[NITER][EPC];
+    __device__ void set(int i, int e, float4 v) { x[i][e] = v.x; x[i][e + 1] = v.y; x[i][e + 2] = v.z; x[i][e + 3] = v.w; }
+    // load(j, i): chunk i of row j; all of them are in registers when release() hands the stage back
+    template <int R, class Load, class Release> __device__ void rows(const Load& load, const Release& release, float (&acc)[R]) const {
+        uint4 w[R][NITER];
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+#pragma unroll
+            for (int i = 0; i < NITER; ++i) w[j][i] = load(j, i);
+        release();
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            float a = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NITER; ++i) a = Wfmt<LT>::dot(w[j][i], 0u, x[i], a);
+            acc[j] = a;
+        }
+    }
+};
+__device__ inline void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// FP8 rows: the bytes widen to fp16 pairs exactly, and mma.m16n8k16 does what an fp32 FMA per weight did (with its
+// conversions two instructions per weight: the decoder was bound by issue slots, not by HBM).  Chunks stay where they are:
+// lane (g, t) = lane / 4, lane % 4 puts its own weights of two rows into rows g and g + 8 of A and its own inputs into
+// column g of B, so the diagonal elements (g, g) and (g + 8, g) are the sums over the four lanes of quad g; the others are
+// not used.  The inputs are fp16 pairs hi + lo, rounded to nearest, of x times a power of two that brings the largest of
+// the vector to 2^14: 2^-24 of x, as fp32, or of what is 2^-24 of the largest.  Products are exact, sums fp32.
+// (5B model, one token: 1.60 ms, 1.85 ms with fp32 FMAs in a kernel per operator; error against 64 bits 3.6e-4 both.)
+template <int NITER> struct Slices<Fp8Row, NITER> {
+    static constexpr int EPC = 16;
+    uint32_t hi[NITER][8], lo[NITER][8];
+    __device__ void set(int i, int e, float4 v) {
+        pair(hi[i][e / 2], lo[i][e / 2], v.x, v.y);
+        pair(hi[i][e / 2 + 1], lo[i][e / 2 + 1], v.z, v.w);
+    }
+    __device__ static void pair(uint32_t& h, uint32_t& l, float a, float b) {
+        const __half2 p = __floats2half2_rn(a, b);
+        const float2 f = __half22float2(p);
+        const __half2 q = __floats2half2_rn(isfinite(f.x) ? a - f.x : 0.0f, isfinite(f.y) ? b - f.y : 0.0f);
+        h = *reinterpret_cast<const uint32_t*>(&p);
+        l = *reinterpret_cast<const uint32_t*>(&q);
+    }
+    __device__ static uint32_t widen(uint32_t two) {
+        const __half2 h(__nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)two, __NV_E4M3));
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+    // (two chunks at a time: the inputs take the registers that holding a whole stage would need)
+    template <int R, class Load, class Release> __device__ void rows(const Load& load, const Release& release, float (&acc)[R]) const {
+        static_assert(R % 2 == 0, "rows come in pairs");
+        const int lane = threadIdx.x & 31, g = lane >> 2;
+#pragma unroll
+        for (int j = 0; j < R; j += 2) {
+            float dh[4] = {0.f, 0.f, 0.f, 0.f}, dl[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < NITER; ++i) {
+                const uint4 w0 = load(j, i), w1 = load(j + 1, i);
+                const uint32_t u[4] = {w0.x, w0.y, w0.z, w0.w}, v[4] = {w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t a0 = widen(u[k] & 0xffffu), a1 = widen(v[k] & 0xffffu), a2 = widen(u[k] >> 16), a3 = widen(v[k] >> 16);
+                    mma_f16(dh, a0, a1, a2, a3, hi[i][2 * k], hi[i][2 * k + 1]);
+                    mma_f16(dl, a0, a1, a2, a3, lo[i][2 * k], lo[i][2 * k + 1]);
+                }
+            }
+            const bool diagonal = (lane & 3) == (g >> 1), odd = g & 1;
+            acc[j] = diagonal ? (odd ? dh[1] + dl[1] : dh[0] + dl[0]) : 0.0f;
+            acc[j + 1] = diagonal ? (odd ? dh[3] + dl[3] : dh[2] + dl[2]) : 0.0f;
+        }
+        release();
+    }
+};
+
+// ---- consumer side of one GEMV phase: this CTA's rows [r0, r1) out of the ring times the input slices, times `unscale`; a
+// partial sum per row and warp of a group
+template <typename LT, int NITER, int R>
+__device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, float unscale, int r0, int r1, int K, const MegaParams& p) {
+    using F = Wfmt<LT>;
     float* partial = reinterpret_cast<float*>(mega_dyn() + p.off_partial);
-    constexpr int EPC = Elem<WT>::EPC;
     constexpr int NW = GEMV_CONSUMERS / 32;
     const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255, lane = tid & 31, warp = tid >> 5;
-    const int nchunks = K / EPC;
-    const uint32_t row_bytes = (uint32_t)K * sizeof(WT);
+    const int nchunks = K / F::EPC;
+    const uint32_t row_bytes = F::row_stride(K);
     const int ngroups = (r1 - r0 + R - 1) / R;
 
     // Ring slots are owned by groups for the whole GEMV phase: group = (global stage number) & 1,
@@ -339,28 +417,26 @@ __device__ inline void stream_partials(Ring& ring, const float (&xr)[NITER][Elem
             break;
         }
         const uint32_t base = ring.base + (uint32_t)s * ring.stage_cap;
-        uint4 w[R][NITER];
-#pragma unroll
-        for (int j = 0; j < R; ++j)
-#pragma unroll
-            for (int i = 0; i < NITER; ++i) {
-                const int c = tid + i * GEMV_CONSUMERS;
-                w[j][i] = (c < nchunks) ? lds128(base + (uint32_t)j * row_bytes + (uint32_t)c * 16u) : make_uint4(0, 0, 0, 0);
-            }
-        __syncwarp();
-        if (lane == 0) mbar_arrive_n(ring.empty0 + 8u * s, 2);  // a stage expects 16 arrivals: eight warps of one group, twice each
-        float acc[R];
+        float scale[R];
 #pragma unroll
         for (int j = 0; j < R; ++j) {
-            float a = 0.0f;
+            scale[j] = 1.0f;
+            if (F::ROW_SCALE) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(scale[j]) : "r"(base + (uint32_t)j * row_bytes + F::scale_off(K)) : "memory");
+        }
+        float acc[R];
+        x.template rows<R>(
+            [&](int j, int i) {
+                const int c = tid + i * GEMV_CONSUMERS;
+                return c < nchunks ? lds128(base + (uint32_t)j * row_bytes + (uint32_t)c * 16u) : make_uint4(0, 0, 0, 0);
+            },
+            [&]() {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(ring.empty0 + 8u * s, 2);  // a stage expects 16 arrivals: eight warps of one group, twice each
+            },
+            acc);
+        if (F::ROW_SCALE) {
 #pragma unroll
-            for (int i = 0; i < NITER; ++i) {
-                float f[EPC];
-                Elem<WT>::unpack(w[j][i], f);
-#pragma unroll
-                for (int e = 0; e < EPC; ++e) a = fmaf(f[e], xr[i][e], a);
-            }
-            acc[j] = a;
+            for (int j = 0; j < R; ++j) acc[j] *= scale[j] * unscale;
         }
         int rr;
         const float tot = warp_reduce_rows<R>(acc, lane, rr);
@@ -389,7 +465,8 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
     int r0, r1;
     cta_rows(N, UNIT, r0, r1);
 
-    float xr[NITER][EPC];
+    Slices<WT, NITER> slices;
+    float(&xr)[NITER][EPC] = slices.x;
     float gm[NORM ? NITER : 1][NORM ? EPC : 1];  // gamma, requested together with x: one memory latency for both
     if (NORM) {
 #pragma unroll
@@ -438,7 +515,7 @@ __device__ inline bool consume_gemv(Ring& ring, const float* x, const float* x_s
             }
         }
     }
-    stream_partials<WT, NITER, R>(ring, xr, r0, r1, K, p);
+    stream_partials<WT, NITER, R>(ring, slices, 1.0f, r0, r1, K, p);
     mega_bar();
     if (mega_aborted()) return false;
     const float* partial = reinterpret_cast<const float*>(mega_dyn() + p.off_partial);
@@ -507,11 +584,11 @@ struct InputTo {
         }
     }
 };
-// A whole vector from its tagged words; returns this thread's share of the sum of squares.
-__device__ inline float gather_tagged(const unsigned long long* src, uint32_t tag, int K, const InputTo& to, const MegaParams& p) {
+// A whole vector from its tagged words; returns this thread's share of the sum of squares, and the largest magnitude it put.
+__device__ inline float2 gather_tagged(const unsigned long long* src, uint32_t tag, int K, const InputTo& to, const MegaParams& p) {
     constexpr int B = 4;
     const int n = K / 2;
-    float ss = 0.0f;
+    float ss = 0.0f, mx = 0.0f;
 #pragma unroll 1
     for (int c0 = threadIdx.x; c0 < n; c0 += MEGA_CONSUMERS * B) {
         const unsigned long long* at[B];
@@ -530,34 +607,37 @@ __device__ inline float gather_tagged(const unsigned long long* src, uint32_t ta
                 const float2 v = make_float2(tag_value(w[b][0]), tag_value(w[b][1]));
                 to.put(2 * (c0 + b * MEGA_CONSUMERS), v, g[b]);
                 ss = fmaf(v.x, v.x, fmaf(v.y, v.y, ss));
+                mx = fmaxf(mx, fmaxf(fabsf(v.x * g[b].x), fabsf(v.y * g[b].y)));
             }
     }
-    return ss;
+    return make_float2(ss, mx);
 }
 // the first layer's: the embedding row of the current token, or x_a as the host left it
-template <typename WT> __device__ inline float gather_first(const MegaParams& p, const InputTo& to) {
+template <typename WT> __device__ inline float2 gather_first(const MegaParams& p, const InputTo& to) {
     const WT* row = reinterpret_cast<const WT*>(p.embed) + (p.input_embed ? (size_t)checked_token(__ldcg(&p.st->token), p.embed_rows, &p.st->error) * p.dim : 0);
-    float ss = 0.0f;
+    float ss = 0.0f, mx = 0.0f;
 #pragma unroll 1
     for (int i = 2 * threadIdx.x; i < p.dim; i += 2 * MEGA_CONSUMERS) {
         const float2 v = p.input_embed ? make_float2(Elem<WT>::to_f32(row[i]), Elem<WT>::to_f32(row[i + 1])) : __ldcg(reinterpret_cast<const float2*>(p.x_a + i));
-        to.put(i, v, to.scale(i));
+        const float2 g = to.scale(i);
+        to.put(i, v, g);
         ss = fmaf(v.x, v.x, fmaf(v.y, v.y, ss));
+        mx = fmaxf(mx, fmaxf(fabsf(v.x * g.x), fabsf(v.y * g.y)));
     }
-    return ss;
+    return make_float2(ss, mx);
 }
 
 // The phases of one GPU share their code: a layer's instructions run once per layer and CTA, and five inlined copies of
 // the GEMV waited for the instruction cache (about 0.5 us at the start of every phase of a small model).
 enum { PH_QKV = 0, PH_WO = 1, PH_W13 = 2, PH_W2 = 3, PH_HEAD = 4 };
 
-// the rows of a phase: input slices out of xs, times inv (1 / root mean square, or 1)
-template <typename WT, int NITER, int R>
-__device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, float* norm_out, const int2& rows, int K) {
-    constexpr int EPC = Elem<WT>::EPC;
+// the rows of a phase: input slices out of xs, times inv (1 / root mean square, or 1); the rows' results times unscale
+template <typename LT, int NITER, int R>
+__device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, float unscale, float* norm_out, const int2& rows, int K) {
+    constexpr int EPC = Wfmt<LT>::EPC;
     const float* xs = reinterpret_cast<const float*>(mega_dyn() + p.off_xs);
     const int tid = threadIdx.x & 255, nchunks = K / EPC;
-    float xr[NITER][EPC];
+    Slices<LT, NITER> x;
 #pragma unroll
     for (int i = 0; i < NITER; ++i) {
         const int c = tid + i * GEMV_CONSUMERS;
@@ -567,10 +647,10 @@ __device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, f
             if (c < nchunks) v = *reinterpret_cast<const float4*>(xs + (size_t)c * EPC + e);
             v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
             if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x < 256 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
-            xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
+            x.set(i, e, v);
         }
     }
-    stream_partials<WT, NITER, R>(ring, xr, rows.x, rows.y, K, p);
+    stream_partials<LT, NITER, R>(ring, x, unscale, rows.x, rows.y, K, p);
 }
 
 // the epilogue of a phase on this CTA's rows (arithmetic of EpiQKV, EpiGate, EpiResidual, EpiStore)
@@ -912,9 +992,10 @@ __device__ inline void merge_attention(const MegaParams& p, float* xs) {
 }
 
 // the same from tagged partials, as the input of the Wo phase
-__device__ inline float gather_merged(const MegaParams& p, uint32_t tag) {
+__device__ inline float2 gather_merged(const MegaParams& p, uint32_t tag) {
     constexpr float NEG = -3.402823466e+38f;
     constexpr int B = 4;  // partials in flight
+    float mx = 0.0f;
     float* xs = reinterpret_cast<float*>(mega_dyn() + p.off_xs);
     const int HD = p.hd, cph = mega_shared().plan.cph;
 #pragma unroll 1
@@ -949,13 +1030,17 @@ __device__ inline float gather_merged(const MegaParams& p, uint32_t tag) {
             }
         }
         const float inv = L > 0.0f ? 1.0f / L : 0.0f;
-        *reinterpret_cast<float4*>(xs + (size_t)c * 4) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+        o = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+        *reinterpret_cast<float4*>(xs + (size_t)c * 4) = o;
+        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(o.x), fabsf(o.y))), fmaxf(fabsf(o.z), fabsf(o.w)));
     }
-    return 0.0f;
+    return make_float2(0.0f, mx);
 }
 
 // TPAR: the tensor-parallel form (a kernel of its own, so that none of it weighs on the single-GPU token)
-template <typename WT, typename KT, int ND, int RD, int NH, int RH, bool TPAR>
+// WT: storage of the embedding and the LM head, LT: row format of the linears, KT: of the cache; N, R: chunks a thread takes of
+// a row and rows of a stage, at K = dim or q_dim (D), K = hidden (H), and the head's (O)
+template <typename WT, typename LT, typename KT, int ND, int RD, int NH, int RH, int NO, int RO, bool TPAR>
 __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaParams p) {
     constexpr int NW = GEMV_CONSUMERS / 32;
     MegaShared& sh = mega_shared();
@@ -1020,8 +1105,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
                 else { dst += ring.stage_cap; full += 8u; empty += 8u; }
                 return true;
             };
-            walk_token_stream<RD, RH>(p, layers_s, pt_s, (uint32_t)p.dim * (uint32_t)sizeof(WT), (uint32_t)p.q_dim * (uint32_t)sizeof(WT),
-                                      (uint32_t)p.hidden * (uint32_t)sizeof(WT), (uint32_t)sizeof(KT), put);
+            walk_token_stream<RD, RH, RO>(p, layers_s, pt_s, Wfmt<LT>::row_stride(p.dim), Wfmt<LT>::row_stride(p.q_dim), Wfmt<LT>::row_stride(p.hidden),
+                                          (uint32_t)p.dim * (uint32_t)sizeof(WT), (uint32_t)sizeof(KT), put);
         }
         return;
     }
@@ -1043,21 +1128,22 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
             const int l = step >> 2, ph = l < p.nlayers ? step & 3 : PH_HEAD;
             const MegaLayer& L = layers_s[min(l, p.nlayers - 1)];
             const uint32_t tag = tag0 + (uint32_t)l;
-            float ss;
+            float2 in;  // sum of squares, largest magnitude
             if (ph == PH_WO) {
                 ok = p.gqa == 1 ? attention_phase<KT, 1, true>(ring, p, L.kv, attn_len, tag, stamp) : attention_phase<KT, 2, true>(ring, p, L.kv, attn_len, tag, stamp);
                 stamp();
                 if (!ok) break;
-                ss = gather_merged(p, tag);
+                in = gather_merged(p, tag);
             } else {
                 const InputTo to{xs, ph == PH_QKV ? resid : ph == PH_W13 ? resid + p.rows_cap : nullptr,
                                  ph == PH_QKV ? L.gamma1 : ph == PH_W13 ? L.gamma2 : ph == PH_HEAD ? p.gamma_final : nullptr, sh.rows[PH_WO]};
-                if (step == 0) ss = gather_first<WT>(p, to);
-                else ss = gather_tagged(ph == PH_W13 ? p.tx_b : ph == PH_W2 ? p.tgate : p.tx_a, ph == PH_W13 || ph == PH_W2 ? tag : tag - 1u, ph == PH_W2 ? p.hidden : p.dim, to, p);
+                if (step == 0) in = gather_first<WT>(p, to);
+                else in = gather_tagged(ph == PH_W13 ? p.tx_b : ph == PH_W2 ? p.tgate : p.tx_a, ph == PH_W13 || ph == PH_W2 ? tag : tag - 1u, ph == PH_W2 ? p.hidden : p.dim, to, p);
             }
             const bool norm = ph != PH_WO && ph != PH_W2;
-            ss = warp_sum(ss);
-            if ((tid & 31) == 0) sh.red[warp] = ss;
+            in.x = warp_sum(in.x);
+            if (Wfmt<LT>::QUANT) in.y = warp_max(in.y);
+            if ((tid & 31) == 0) { sh.red[warp] = in.x; sh.red[32 + warp] = in.y; }
             mega_bar();
             stamp();
             float inv = 1.0f;
@@ -1067,8 +1153,22 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
                 for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) tot += sh.red[i];
                 inv = 1.0f / sqrtf(tot * (1.0f / (float)p.dim) + RMS_EPS);
             }
-            if (ph == PH_W2) tagged_rows<WT, NH, RH>(ring, p, inv, nullptr, sh.rows[PH_WO], p.hidden);
-            else tagged_rows<WT, ND, RD>(ring, p, inv, ph == PH_HEAD ? p.norm_final : nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
+            if constexpr (Wfmt<LT>::QUANT) {
+                float mx = 0.0f, unscale = 1.0f;
+                if (ph != PH_HEAD) {  // the power of two that brings the largest input to [2^14, 2^15)
+#pragma unroll
+                    for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) mx = fmaxf(mx, sh.red[32 + i]);
+                    const int e = (int)(__float_as_uint(mx * inv) >> 23), f = e == 255 ? 127 : min(253, max(1, 268 - e));
+                    inv *= __uint_as_float((uint32_t)f << 23);
+                    unscale = __uint_as_float((uint32_t)(254 - f) << 23);
+                }
+                if (ph == PH_HEAD) tagged_rows<WT, NO, RO>(ring, p, inv, 1.0f, p.norm_final, sh.rows[ph], p.dim);
+                else if (ph == PH_W2) tagged_rows<LT, NH, RH>(ring, p, inv, unscale, nullptr, sh.rows[PH_WO], p.hidden);
+                else tagged_rows<LT, ND, RD>(ring, p, inv, unscale, nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
+            } else {
+                if (ph == PH_W2) tagged_rows<LT, NH, RH>(ring, p, inv, 1.0f, nullptr, sh.rows[PH_WO], p.hidden);
+                else tagged_rows<LT, ND, RD>(ring, p, inv, 1.0f, ph == PH_HEAD ? p.norm_final : nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
+            }
             mega_bar();
             if (mega_aborted()) { ok = false; break; }
             tagged_epilogue<KT>(p, ph, l + 1 == p.nlayers, L.kv, tag);
