@@ -37,7 +37,7 @@ cudaError_t launch_attn(cd_model* m, const cd_layer_dev& L) {
 }
 
 // ------------------------------------------------------------------ persistent kernel launch
-template <typename WT, typename LT, typename KT, int ND, int NH, bool TPAR>
+template <typename WT, typename LT, typename KT, int ND, int NH, bool TPAR, bool GROUPED>
 cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     constexpr bool Q = Wfmt<LT>::QUANT;
     constexpr int RD = ND == 1 ? 4 : ND == 2 || Q ? 2 : 1;
@@ -45,7 +45,7 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     constexpr int NO = Q ? 2 * ND : ND;  // an FP8 chunk is twice as many elements as one of the head's
     constexpr int RO = Q ? (NO == 2 ? 2 : 1) : RD;
     const cd_config& c = m->cfg;
-    auto kern = decode_mega_kernel<WT, LT, KT, ND, RD, NH, RH, NO, RO, TPAR>;
+    auto kern = decode_mega_kernel<WT, LT, KT, ND, RD, NH, RH, NO, RO, TPAR, GROUPED>;
     // every CTA owns rows of every matrix: what tells a CTA that another one is done with a vector is that one's next rows
     const int grid = TPAR ? m->sm_count : std::min({m->sm_count, c.dim, c.hidden, (c.q_dim + 2 * c.kv_dim) / 2});
     const size_t stage_cap = (std::max({(size_t)RD * Wfmt<LT>::row_stride(std::max(c.dim, c.q_dim)), (size_t)RH * Wfmt<LT>::row_stride(c.hidden), (size_t)RO * c.dim * sizeof(WT)}) + 127) / 128 * 128;
@@ -107,16 +107,16 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     return e;
 }
 
-template <typename WT, typename LT, typename KT, bool TPAR>
+template <typename WT, typename LT, typename KT, bool TPAR, bool GROUPED>
 cudaError_t launch_mega_tp(cd_model* m, int input_embed, int want_logits) {
     switch (m->mega_nd * 10 + m->mega_nh) {
-        case 11: return launch_mega_t<WT, LT, KT, 1, 1, TPAR>(m, input_embed, want_logits);
-        case 12: return launch_mega_t<WT, LT, KT, 1, 2, TPAR>(m, input_embed, want_logits);
-        case 14: if constexpr (!TPAR) return launch_mega_t<WT, LT, KT, 1, 4, TPAR>(m, input_embed, want_logits); else break;
-        case 13: if constexpr (Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 1, 3, TPAR>(m, input_embed, want_logits); else break;
-        case 24: return launch_mega_t<WT, LT, KT, 2, 4, TPAR>(m, input_embed, want_logits);
-        case 26: if constexpr (!Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 6, TPAR>(m, input_embed, want_logits); else break;
-        case 28: if constexpr (!TPAR && !Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 8, TPAR>(m, input_embed, want_logits); else break;
+        case 11: return launch_mega_t<WT, LT, KT, 1, 1, TPAR, GROUPED>(m, input_embed, want_logits);
+        case 12: return launch_mega_t<WT, LT, KT, 1, 2, TPAR, GROUPED>(m, input_embed, want_logits);
+        case 14: if constexpr (!TPAR) return launch_mega_t<WT, LT, KT, 1, 4, TPAR, GROUPED>(m, input_embed, want_logits); else break;
+        case 13: if constexpr (Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 1, 3, TPAR, GROUPED>(m, input_embed, want_logits); else break;
+        case 24: return launch_mega_t<WT, LT, KT, 2, 4, TPAR, GROUPED>(m, input_embed, want_logits);
+        case 26: if constexpr (!Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 6, TPAR, GROUPED>(m, input_embed, want_logits); else break;
+        case 28: if constexpr (!TPAR && !Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 8, TPAR, GROUPED>(m, input_embed, want_logits); else break;
         default: break;
     }
     return cudaErrorInvalidConfiguration;
@@ -124,9 +124,12 @@ cudaError_t launch_mega_tp(cd_model* m, int input_embed, int want_logits) {
 template <typename WT, typename LT, typename KT>
 cudaError_t launch_mega(cd_model* m, int input_embed, int want_logits) {
     if constexpr (!std::is_same<WT, float>::value && !Wfmt<LT>::QUANT) {  // the tensor-parallel form exists for the 16-bit storage types
-        if (m->tp_world > 1) return launch_mega_tp<WT, LT, KT, true>(m, input_embed, want_logits);
+        if (m->tp_world > 1) return launch_mega_tp<WT, LT, KT, true, false>(m, input_embed, want_logits);
     }
-    return launch_mega_tp<WT, LT, KT, false>(m, input_embed, want_logits);
+    if constexpr (std::is_same<KT, __half>::value) {
+        if (m->cfg.gqa_ratio > 2) return launch_mega_tp<WT, LT, KT, false, true>(m, input_embed, want_logits);
+    }
+    return launch_mega_tp<WT, LT, KT, false, false>(m, input_embed, want_logits);
 }
 
 // One token through the whole model; everything is enqueued on m->stream.
@@ -300,7 +303,7 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
         const int nd = (std::max(c.dim, c.q_dim) / epc + 255) / 256, nh = (c.hidden / epc + 255) / 256, g = c.gqa_ratio;
         // (c is this rank's shard under tensor parallelism: hidden and q_dim shrink, dim does not)
         const bool combo = tpw > 1 ? ((nd == 1 && (nh == 1 || nh == 2)) || (nd == 2 && nh >= 3 && nh <= 6)) && c.q_dim <= c.dim && g <= 2
-                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= (dt == CD_DTYPE_FP8_E4M3 ? 4 : 8))) && (g == 1 || g == 2);  // 4 and 8: the attention phase takes 15 us where the chain's kernel takes 10
+                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= (dt == CD_DTYPE_FP8_E4M3 ? 4 : 8))) && (g == 1 || g == 2 || ((g == 4 || g == MEGA_MAX_GQA) && m->kv_dtype == CD_DTYPE_F16));
         if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 && dt != CD_DTYPE_FP8_E4M3 ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
         // tensor parallel: measured on the 5B model, the persistent kernel wins at 2 ranks (601 against 569 tokens/s) and
         // loses at 8 (841 against 896), where a layer's data are 8 us and its fixed per-phase times dominate either way

@@ -2,15 +2,15 @@
 //
 // The multi-kernel path pays a fixed 4-6 us at each of its 5 x nlayers kernel boundaries
 // (drain, launch, ring refill) during which HBM idles.  Here one cooperative grid of one
-// CTA per SM walks the whole token.  Its producer thread streams, layer after layer and
+// CTA per SM walks the whole token.  Its producers stream, layer after layer and
 // through one shared-memory ring of 1-D bulk copies, everything this CTA will read from
 // HBM in the order it will need it: its rows of the q|k|v matrix, the K/V tiles of the
 // cached positions its attention work covers, its rows of Wo, W1|W3 and W2 - and never
 // stops at an operator boundary, because none of that depends on this token's activations
 // (the one K/V row that does, the current position's, is read straight from global memory
-// by the consumers instead).  Sixteen consumer warps run the operators in order and meet
-// the other CTAs at a grid barrier wherever the next operator needs a whole activation
-// vector (five times per layer).  While consumers sit in a barrier the ring keeps filling,
+// by the consumers instead).  Sixteen consumer warps run the operators in order; a vector
+// that the next operator needs whole (five times per layer) reaches every CTA as tagged words,
+// which it polls for (tag_store below).  While consumers wait for them the ring keeps filling,
 // so HBM stays busy; afterwards they drain shared memory several times faster than HBM can
 // refill it and catch up.
 //
@@ -39,6 +39,8 @@
 // wait runs out.  No reference counterpart (the reference encodes 15 dispatches per layer,
 // lib.rs:513-634).
 #pragma once
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace cd {
@@ -106,7 +108,10 @@ struct EpiPushPartial {  // Wo / W2 under tensor parallelism: the rank's partial
 // what lets them catch up after every barrier.
 constexpr int MEGA_GROUPS = 2;
 constexpr int MEGA_CONSUMERS = MEGA_GROUPS * GEMV_CONSUMERS;
-constexpr int MEGA_THREADS = MEGA_CONSUMERS + 32;  // + the producer's warp (one working thread)
+// + the producers, one working thread each: one alone took 0.3 us per stage (its wait, its copy, the walk), 54 GB/s per SM at
+// 16 KB stages and less at smaller ones.  Twenty warps take no more registers than seventeen.
+constexpr int MEGA_PRODUCERS = 4;
+constexpr int MEGA_THREADS = MEGA_CONSUMERS + 32 * MEGA_PRODUCERS;
 constexpr int MEGA_TEAMS = MEGA_CONSUMERS / 128;
 constexpr int MEGA_TEAM_SMEM = 128 * 8 + 64;  // floats per team: lane-group accumulators, then (max, sum) pairs
 // ---- who computes which part of the attention
@@ -180,7 +185,13 @@ __device__ inline void mbar_arrive_n(uint32_t bar, uint32_t n) {
 struct Ring {
     uint32_t base, full0, empty0, stage_cap;
     int nstages;
-    int g;  // stages used so far (producer and consumers count the same sequence)
+    // the next stage's slot and the parity of its turn, kept by increments: a division per stage was a third of the
+    // consumers' latency per stage (producer and consumers count the same sequence)
+    int slot;
+    uint32_t turn;
+    __device__ void advance(int n) {
+        for (slot += n; slot >= nstages; slot -= nstages) turn ^= 1u;
+    }
 };
 
 // rows [r0, r1) of an [N, K] matrix owned by this CTA
@@ -408,10 +419,12 @@ __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, f
     // consumed, in order, by the same group.  (A parity wait can only tell adjacent phases of
     // an mbarrier apart; a group that skipped another group's use of a slot could mistake
     // an old phase for the one it wants.)
-    for (int g = (grp - ring.g) & 1; g < ngroups; g += MEGA_GROUPS) {
-        const int rg = ring.g + g;
-        const int s = rg % ring.nstages;
-        if (!mbar_wait(ring.full0 + 8u * s, (rg / ring.nstages) & 1)) {
+    const int g0 = (grp - ring.slot) & 1;
+    Ring at = ring;
+    at.advance(g0);
+    for (int g = g0; g < ngroups; g += MEGA_GROUPS, at.advance(MEGA_GROUPS)) {
+        const int s = at.slot;
+        if (!mbar_wait(ring.full0 + 8u * s, at.turn)) {
             atomicCAS(&p.st->error, 0, DEV_ERR_FULL_WAIT);
             mega_shared().abort = 1;  // every consumer still meets at the barrier below, then all leave together
             break;
@@ -443,7 +456,7 @@ __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, f
         const int row = g * R + rr;
         if ((lane & (32 / R - 1)) == 0 && row < r1 - r0) partial[row * NW + warp] = tot;
     }
-    ring.g += ngroups;
+    ring.advance(ngroups);
 }
 // row r of the phase: the sums of its group's warps
 __device__ inline float row_sum(const float* partial, int r) {
@@ -742,13 +755,18 @@ __device__ inline bool attention_inputs(const MegaParams& p, int h, bool newest,
     MegaShared& sh = mega_shared();
     const int nq = p.gqa * p.hd / 2, t = threadIdx.x;  // pairs of q, at most one per thread
     const bool want_q = t < nq, want_row = newest && t < p.hd;  // pair t of the row: K's pairs, then V's
+    float mx = 0.0f;
     if (want_q || want_row) {
         const unsigned long long* const q = p.tq + (size_t)h * p.gqa * p.hd + 2 * t;
         const unsigned long long* const row = p.tkv + h * p.hd + (t < p.hd / 2 ? 2 * t : p.kv_dim + 2 * t - p.hd);
         const unsigned long long* const at[2] = {want_q ? q : row, want_row ? row : q};
         unsigned long long w[2][2];
         if (tag_poll<2>(at, tag, w, p)) {
-            if (want_q) *reinterpret_cast<float2*>(sh.q + 2 * t) = make_float2(tag_value(w[0][0]), tag_value(w[0][1]));
+            if (want_q) {
+                const float2 v = make_float2(tag_value(w[0][0]), tag_value(w[0][1]));
+                *reinterpret_cast<float2*>(sh.q + 2 * t) = v;
+                mx = fmaxf(fabsf(v.x), fabsf(v.y));
+            }
             if (want_row) {
                 KT* kv = reinterpret_cast<KT*>(sh.row);
                 kv[2 * t] = Elem<KT>::from_f32(tag_value(w[1][0]));
@@ -756,8 +774,208 @@ __device__ inline bool attention_inputs(const MegaParams& p, int h, bool newest,
             }
         }
     }
+    if (p.gqa > 2) {  // the largest magnitude per warp
+        mx = warp_max(mx);
+        if ((t & 31) == 0) sh.red[t >> 5] = mx;
+    }
     mega_bar();
     return !mega_aborted();
+}
+
+// ---- attention phase with 4 or 8 q heads per kv head and an fp16 cache.  Scores are a product with M = heads: rows 0-7 of
+// mma.m16n8k16 hold the heads' q rounded to fp16 (times a power of two that brings the largest to 2^14), rows 8-15 the
+// remainders, so one instruction gives both parts of eight positions' scores and no shuffle sums them up (the general
+// phase below spends 40 instructions per position and head on that: 15.6 us per layer of a 1B model at 2000 positions, 9.1 us
+// here; a token of it 0.88 ms, 0.91 ms with a kernel per operator).  A warp takes eight positions of a tile; its probabilities go through 128
+// bytes of shared memory to lanes that hold 16 bytes of a V row each, for four heads.  Warps 0-7 and 8-15 take alternate
+// tiles (4 heads), or heads 0-3 and 4-7 of every tile (8 heads).  q and the newest row arrive, partials leave as tagged words.
+template <class Tick>
+__device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int attn_len, uint32_t tag, const Tick& input_is_in) {
+    constexpr float NEG = -3.402823466e+38f;
+    constexpr int NH = 4;  // heads a warp accumulates
+    MegaShared& sh = mega_shared();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp >> 3, g = lane >> 2, t = lane & 3;
+    const int HD = p.hd, T = p.tile_tokens, ntiles = (attn_len + T - 1) / T, pos = attn_len - 1, CH = HD / 8;  // CH: 16-byte chunks of a row
+    const bool by_head = p.gqa > NH;
+    const int h0 = by_head ? NH * set : 0;  // this warp's heads among the kv head's
+    const uint32_t row_bytes = (uint32_t)HD * 2u;
+    float* probs_all = &sh.tparts[0][0][0];
+    float* probs = probs_all + warp * 8 * NH;  // [8 positions][NH]
+    const AttnPlan plan = sh.plan;
+    bool ok = true;
+    if (plan.first < 0) return !mega_aborted();
+    for (int h = plan.first; h < p.kv_heads && ok; h += plan.step) {
+        if (!attention_inputs<__half>(p, h, plan.t1 == ntiles, tag)) { ok = false; break; }
+        if (h == plan.first) input_is_in();
+        float mx = 0.0f;
+#pragma unroll
+        for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) mx = fmaxf(mx, sh.red[i]);
+        const int e = (int)(__float_as_uint(mx) >> 23), f = e == 255 ? 127 : min(253, max(1, 268 - e));
+        const float up = __uint_as_float((uint32_t)f << 23), down = __uint_as_float((uint32_t)(254 - f) << 23) * p.attn_scale;
+        // step s = 2 j + b: elements 4 b .. 4 b + 3 of chunk 4 j + t
+        uint32_t qa[8][4];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const int d = (4 * (s >> 1) + t) * 8 + 4 * (s & 1);
+            const bool live = g < p.gqa && d < HD;
+            const float4 v = live ? *reinterpret_cast<const float4*>(sh.q + g * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            Slices<Fp8Row, 1>::pair(qa[s][0], qa[s][1], v.x * up, v.y * up);
+            Slices<Fp8Row, 1>::pair(qa[s][2], qa[s][3], v.z * up, v.w * up);
+        }
+        float acc[NH][8], m = NEG, lsum = 0.0f;  // m, lsum: of head h0 + g (lsum of this lane's positions), meaningful for g < NH
+#pragma unroll
+        for (int q = 0; q < NH; ++q)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[q][i] = 0.0f;
+        const int ncta_tiles = plan.t1 - plan.t0;
+        Ring at = ring;
+        for (int idx = 0; idx < ncta_tiles; ++idx) {
+            const int tile = plan.t0 + idx;
+            const int slot_k = at.slot;
+            const uint32_t turn_k = at.turn;
+            at.advance(1);
+            const int slot_v = at.slot;
+            const uint32_t turn_v = at.turn;
+            at.advance(1);
+            if (!mbar_wait(ring.full0 + 8u * slot_k, turn_k) || !mbar_wait(ring.full0 + 8u * slot_v, turn_v)) {
+                atomicCAS(&p.st->error, 0, DEV_ERR_FULL_WAIT);
+                sh.abort = 1;
+                ok = false;
+                break;
+            }
+            const int w0 = (warp & 7) * 8;  // first position of this warp in the tile
+            if ((by_head || (idx & 1) == set) && w0 < T && tile * T + w0 < attn_len) {  // (uniform in the warp)
+                const uint32_t kbase = ring.base + (uint32_t)slot_k * ring.stage_cap, vbase = ring.base + (uint32_t)slot_v * ring.stage_cap;
+                float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+                const int kpos = tile * T + w0 + g;
+                const bool klive = w0 + g < T && kpos < attn_len;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (4 * j < CH) {
+                        const int ch = 4 * j + t;
+                        uint4 k = make_uint4(0, 0, 0, 0);
+                        if (klive) k = kpos == pos ? sh.row[ch] : lds128(kbase + (uint32_t)(w0 + g) * row_bytes + (uint32_t)ch * 16u);
+                        mma_f16(c, qa[2 * j][0], qa[2 * j][1], qa[2 * j][2], qa[2 * j][3], k.x, k.y);
+                        mma_f16(c2, qa[2 * j + 1][0], qa[2 * j + 1][1], qa[2 * j + 1][2], qa[2 * j + 1][3], k.z, k.w);
+                    }
+                }
+                // scores of head g at positions 2 t and 2 t + 1; this warp's heads move to g = 0 .. NH - 1
+                float s0 = ((c[0] + c2[0]) + (c[2] + c2[2])) * down, s1 = ((c[1] + c2[1]) + (c[3] + c2[3])) * down;
+                if (by_head) {
+                    s0 = __shfl_sync(0xffffffffu, s0, ((g + h0) & 7) * 4 + t);
+                    s1 = __shfl_sync(0xffffffffu, s1, ((g + h0) & 7) * 4 + t);
+                }
+                const int p0 = w0 + 2 * t;
+                if (p0 >= T || tile * T + p0 >= attn_len) s0 = NEG;
+                if (p0 + 1 >= T || tile * T + p0 + 1 >= attn_len) s1 = NEG;
+                float top = fmaxf(s0, s1);
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+                const float mnew = fmaxf(m, top), corr = expf(m - mnew);
+                const float e0 = s0 > NEG ? expf(s0 - mnew) : 0.0f, e1 = s1 > NEG ? expf(s1 - mnew) : 0.0f;
+                lsum = lsum * corr + e0 + e1;
+                m = mnew;
+                __syncwarp();
+                if (g < NH) {
+                    probs[(2 * t) * NH + g] = e0;
+                    probs[(2 * t + 1) * NH + g] = e1;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < NH; ++q) {
+                    const float cq = __shfl_sync(0xffffffffu, corr, 4 * q);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[q][i] *= cq;
+                }
+                const int ch = lane & (CH - 1), side = 32 / CH;  // positions side by side
+#pragma unroll 2
+                for (int r = lane / CH; r < 8; r += side) {
+                    const int vpos = tile * T + w0 + r;
+                    uint4 v = make_uint4(0, 0, 0, 0);
+                    if (w0 + r < T && vpos < attn_len) v = vpos == pos ? sh.row[CH + ch] : lds128(vbase + (uint32_t)(w0 + r) * row_bytes + (uint32_t)ch * 16u);
+                    const float4 pr = *reinterpret_cast<const float4*>(probs + r * NH);
+                    float x[8];
+                    Elem<__half>::unpack(v, x);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        acc[0][i] = fmaf(pr.x, x[i], acc[0][i]);
+                        acc[1][i] = fmaf(pr.y, x[i], acc[1][i]);
+                        acc[2][i] = fmaf(pr.z, x[i], acc[2][i]);
+                        acc[3][i] = fmaf(pr.w, x[i], acc[3][i]);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(ring.empty0 + 8u * slot_k);
+                mbar_arrive(ring.empty0 + 8u * slot_v);
+            }
+        }
+        // ---- merge: the warps' maxima, then every warp's sums relative to the CTA's, added in two halves of eight warps
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
+        float* ls = probs_all + 16 * 8 * NH;  // [16 warps][NH] sums of the probabilities, then their maxima
+    float* mxs = ls + 16 * NH;
+        if (t == 0 && g < NH) mxs[warp * NH + g] = m;
+        mega_bar();
+        if (mega_aborted()) ok = false;
+        ring.advance(2 * ncta_tiles);
+        if (!ok) break;
+        const int first = by_head ? 8 * set : 0, last = by_head ? first + 8 : 16;  // warps with the same heads
+        float M = NEG;
+        if (g < NH)
+            for (int w = first; w < last; ++w) M = fmaxf(M, mxs[w * NH + g]);
+        const float wgt = m > NEG ? expf(m - M) : 0.0f;
+        lsum *= wgt;
+        // slots: [8][NH][128] weighted V
+        float* slots = &sh.accs[0][0];
+#pragma unroll
+        for (int q = 0; q < NH; ++q) {
+            const float wq = __shfl_sync(0xffffffffu, wgt, 4 * q);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float v = acc[q][i] * wq;
+                v += __shfl_xor_sync(0xffffffffu, v, 16);
+                if (CH == 8) v += __shfl_xor_sync(0xffffffffu, v, 8);
+                acc[q][i] = v;
+            }
+        }
+        if (t == 0 && g < NH) ls[warp * NH + g] = lsum;
+        const bool second = by_head ? (warp & 4) != 0 : set != 0;           // which half of the warps writes first
+        float* mine = slots + (by_head ? set * 4 + (warp & 3) : warp & 7) * NH * 128;
+        if (second && lane < CH)
+#pragma unroll
+            for (int q = 0; q < NH; ++q)
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(mine + q * 128 + lane * 8 + i) = make_float4(acc[q][i], acc[q][i + 1], acc[q][i + 2], acc[q][i + 3]);
+        mega_bar();
+        if (!second && lane < CH)
+#pragma unroll
+            for (int q = 0; q < NH; ++q)
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                    float4* at = reinterpret_cast<float4*>(mine + q * 128 + lane * 8 + i);
+                    const float4 o = *at;
+                    *at = make_float4(acc[q][i] + o.x, acc[q][i + 1] + o.y, acc[q][i + 2] + o.z, acc[q][i + 3] + o.w);
+                }
+        mega_bar();
+        for (int i = threadIdx.x; i < p.gqa * HD; i += MEGA_CONSUMERS) {
+            const int q = i / HD, d = i & (HD - 1);
+            const int s0 = by_head ? 4 * (q / NH) : 0, s1 = by_head ? s0 + 4 : 8, wa = by_head ? 8 * (q / NH) : 0, wb = by_head ? wa + 8 : 16;
+            float a = 0.0f;
+            for (int s = s0; s < s1; ++s) a += slots[(s * NH + q % NH) * 128 + d];
+            unsigned long long* o = p.tparts + ((size_t)(h * p.gqa + q) * MEGA_CPH_CAP + plan.part) * (HD + 2);
+            tag_store(o + d, a, tag);
+            if (d < 2) {
+                float r = NEG;
+                if (d == 0) for (int w = wa; w < wb; ++w) r = fmaxf(r, mxs[w * NH + q % NH]);
+                else { r = 0.0f; for (int w = wa; w < wb; ++w) r += ls[w * NH + q % NH]; }
+                tag_store(o + HD + d, r, tag);
+            }
+        }
+        mega_bar();  // the slots are free for the next head
+    }
+    return ok && !mega_aborted();
 }
 
 // ---- attention phase (sdpa_causal, lib.rs:1426-1489, for the tiles of this CTA).  All sixteen warps
@@ -812,12 +1030,17 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                 }
             }
             const int TQ = max(1, T / nslices);  // positions of a tile per team
+            Ring at = ring;
             for (int idx = 0; idx < ncta_tiles; ++idx) {
                 if (!ok) break;  // this warp only: the others learn it from the abort flag behind the barrier below
                 const int tile = t0 + idx;
-                const int sk = ring.g + 2 * idx, sv = sk + 1;
-                const int slot_k = sk % ring.nstages, slot_v = sv % ring.nstages;
-                if (!mbar_wait(ring.full0 + 8u * slot_k, (sk / ring.nstages) & 1) || !mbar_wait(ring.full0 + 8u * slot_v, (sv / ring.nstages) & 1)) {
+                const int slot_k = at.slot;
+                const uint32_t turn_k = at.turn;
+                at.advance(1);
+                const int slot_v = at.slot;
+                const uint32_t turn_v = at.turn;
+                at.advance(1);
+                if (!mbar_wait(ring.full0 + 8u * slot_k, turn_k) || !mbar_wait(ring.full0 + 8u * slot_v, turn_v)) {
                     atomicCAS(&p.st->error, 0, DEV_ERR_FULL_WAIT);
                     sh.abort = 1;
                     ok = false;
@@ -896,7 +1119,7 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
             }
             mega_bar();  // every warp is through its tiles (or has given up)
             if (mega_aborted()) ok = false;
-            ring.g += 2 * ncta_tiles;
+            ring.advance(2 * ncta_tiles);
             if (!ok) break;
             // ---- merge: lane groups of a team, then the teams; team 0 stores this CTA's partial of every q head
 #pragma unroll
@@ -1039,8 +1262,9 @@ __device__ inline float2 gather_merged(const MegaParams& p, uint32_t tag) {
 
 // TPAR: the tensor-parallel form (a kernel of its own, so that none of it weighs on the single-GPU token)
 // WT: storage of the embedding and the LM head, LT: row format of the linears, KT: of the cache; N, R: chunks a thread takes of
-// a row and rows of a stage, at K = dim or q_dim (D), K = hidden (H), and the head's (O)
-template <typename WT, typename LT, typename KT, int ND, int RD, int NH, int RH, int NO, int RO, bool TPAR>
+// a row and rows of a stage, at K = dim or q_dim (D), K = hidden (H), and the head's (O); GROUPED: more than two q
+// heads per kv head (kernels of their own, like TPAR)
+template <typename WT, typename LT, typename KT, int ND, int RD, int NH, int RH, int NO, int RO, bool TPAR, bool GROUPED>
 __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaParams p) {
     constexpr int NW = GEMV_CONSUMERS / 32;
     MegaShared& sh = mega_shared();
@@ -1053,7 +1277,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
     ring.empty0 = ring.full0 + 8u * p.nstages;
     ring.stage_cap = p.stage_cap;
     ring.nstages = p.nstages;
-    ring.g = 0;
+    ring.slot = 0;
+    ring.turn = 0;
     int* const err = &p.st->error;
     const int tid = threadIdx.x, warp = tid >> 5;
 
@@ -1082,27 +1307,33 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
     if (tid < p.hd / 2) sh.rope[tid] = p.rope[(size_t)(attn_len - 1) * (p.hd / 2) + tid];
     __syncthreads();
 
-    if (warp == MEGA_CONSUMERS / 32) {  // ---- producer: fills the ring, stage after stage, as slots come free
+    if (warp >= MEGA_CONSUMERS / 32) {  // ---- producers: fill the ring, stage after stage, as slots come free; each every fourth stage
         if ((tid & 31) == 0) {
             const uint64_t policy = l2_evict_first_policy();
             uint64_t kv_policy;
             asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(kv_policy));
-            int slot = 0;        // ring.g % nstages and ring.g / nstages, kept by increments (no division per stage)
-            uint32_t turns = 0;
-            uint32_t dst = ring.base, full = ring.full0, empty = ring.empty0;
+            const int mine = warp - MEGA_CONSUMERS / 32;
+            // A slot's successive stages may belong to different producers.  A parity wait tells adjacent turns apart: a producer
+            // that is done with its stage n - np knows the stages up to n - np - nstages read, and so, with np <= nstages, the
+            // slot's turn before last.
+            const int np = min(MEGA_PRODUCERS, ring.nstages);  // 2 or 4 (nstages is even)
+            if (mine >= np) return;
+            int n = 0;
+            uint32_t first = 1;  // the ring's first turn: every slot is free
             const unsigned long long producer_budget = p.wait_ns + 2000000000ull;
             auto put = [&](const char* src, uint32_t bytes, bool is_kv) {
-                // (a consumer that gave up raises the CTA's abort flag: the slot will not come free, and that is no error of its own)
-                if (turns > 0 && !mbar_wait_or_abort(empty, (turns - 1) & 1u, &sh.abort, producer_budget)) {
-                    if (!mega_aborted()) atomicCAS(err, 0, DEV_ERR_EMPTY_WAIT);
-                    return false;
+                if ((n++ & (np - 1)) == mine) {
+                    const uint32_t full = ring.full0 + 8u * ring.slot, empty = ring.empty0 + 8u * ring.slot;
+                    // (a consumer that gave up raises the CTA's abort flag: the slot will not come free, and that is no error of its own)
+                    if (!first && !mbar_wait_or_abort(empty, ring.turn ^ 1u, &sh.abort, producer_budget)) {
+                        if (!mega_aborted()) atomicCAS(err, 0, DEV_ERR_EMPTY_WAIT);
+                        return false;
+                    }
+                    mbar_arrive_expect_tx(full, bytes);
+                    // (cached positions are read again by the next token: no evict-first)
+                    bulk_g2s_stream(ring.base + (uint32_t)ring.slot * ring.stage_cap, src, bytes, full, is_kv ? kv_policy : policy);
                 }
-                mbar_arrive_expect_tx(full, bytes);
-                // (cached positions are read again by the next token: no evict-first)
-                bulk_g2s_stream(dst, src, bytes, full, is_kv ? kv_policy : policy);
-                ring.g += 1;
-                if (++slot == ring.nstages) { slot = 0; turns += 1; dst = ring.base; full = ring.full0; empty = ring.empty0; }
-                else { dst += ring.stage_cap; full += 8u; empty += 8u; }
+                if (++ring.slot == ring.nstages) { ring.slot = 0; ring.turn ^= 1u; first = 0; }
                 return true;
             };
             walk_token_stream<RD, RH, RO>(p, layers_s, pt_s, Wfmt<LT>::row_stride(p.dim), Wfmt<LT>::row_stride(p.q_dim), Wfmt<LT>::row_stride(p.hidden),
@@ -1130,7 +1361,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
             const uint32_t tag = tag0 + (uint32_t)l;
             float2 in;  // sum of squares, largest magnitude
             if (ph == PH_WO) {
-                ok = p.gqa == 1 ? attention_phase<KT, 1, true>(ring, p, L.kv, attn_len, tag, stamp) : attention_phase<KT, 2, true>(ring, p, L.kv, attn_len, tag, stamp);
+                if constexpr (GROUPED) ok = attention_grouped(ring, p, attn_len, tag, stamp);
+                else ok = p.gqa == 1 ? attention_phase<KT, 1, true>(ring, p, L.kv, attn_len, tag, stamp) : attention_phase<KT, 2, true>(ring, p, L.kv, attn_len, tag, stamp);
                 stamp();
                 if (!ok) break;
                 in = gather_merged(p, tag);
@@ -1234,7 +1466,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
     if (!ok) {
         // leave only once copies that may still be in flight towards this CTA have landed: a copy lands within
         // microseconds, and a slot nobody filled never completes, so the wait for each is short
-        for (int s = 0; s < p.nstages; ++s) mbar_wait_or_abort(ring.full0 + 8u * s, (ring.g / ring.nstages) & 1, nullptr, 200000ull);
+        for (int s = 0; s < p.nstages; ++s) mbar_wait_or_abort(ring.full0 + 8u * s, ring.turn, nullptr, 200000ull);
     }
 }
 

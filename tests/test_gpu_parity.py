@@ -432,3 +432,29 @@ def test_logits_without_a_finite_maximum_never_become_an_address(R, oracle, mega
     gm.set_len(0)
     good = R.Model.new(gpu_cfg(R, oc), layers, dict(head, gamma_final=np.ones(oc.dim, dtype=np.float32)), dtype="bf16", mega=mega)
     assert all(0 <= t < oc.vocab for t in good.decode_steps_greedy(1, 6).tolist())
+
+GROUPED_CASES = [
+    # dims (dim, hidden, heads, hd, seq, layers, vocab), kv heads, type, page tokens, cached positions
+    ((2048, 4128, 16, 128, 2304, 2, 3000), 4, "bf16", 64, 2001),  # four q heads per kv head, several tiles per CTA
+    ((1024, 2080, 8, 128, 1024, 2, 3000), 1, "f16", 64, 700),     # eight q heads per kv head
+    ((1024, 2080, 16, 64, 512, 2, 3000), 4, "bf16", 16, 77),      # head width 64, 16-token tiles
+    ((512, 1056, 8, 64, 512, 2, 3000), 1, "f16", 8, 130),         # tiles of one warp
+    ((512, 1056, 4, 128, 64, 2, 3000), 1, "bf16", 64, 1),         # the first positions
+]
+
+
+@pytest.mark.parametrize("dims,kv_heads,dtype,page,cached", GROUPED_CASES)
+def test_grouped_queries_on_the_persistent_kernel(R, dims, kv_heads, dtype, page, cached):
+    """Four and eight q heads per kv head: scores on the tensor cores (q as fp16 hi + lo pairs) against the kernel per operator.
+    Inputs differ by 2^-24 relative, sums by their order; a cache entry may round to its neighbour: 2e-4 of the logits."""
+    dim, hidden, heads, hd, seq, layers, vocab = dims
+    cfg = R.Config(dim, hidden, heads, hd, seq, layers, vocab, kv_heads=kv_heads)
+    a, b = (R.Model.synthetic(cfg, 7, dtype=dtype, page_tokens=page, mega=mega) for mega in (True, False))
+    prompt = np.random.default_rng(1).integers(0, vocab, cached).astype(np.uint32)
+    for m in (a, b):
+        m.prefill(prompt, want_logits=False)
+    before = a.kernel_launches()
+    for tok in (5, 9, 77):
+        x, y = a.decode_token_logits_from_id(tok), b.decode_token_logits_from_id(tok)
+        assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
+    assert a.kernel_launches() - before == 6  # the persistent kernel and the position's advance
