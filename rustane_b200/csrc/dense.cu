@@ -6,7 +6,7 @@
 #include <type_traits>
 
 #include "step.cuh"
-#include "mega.cuh"
+#include "mega_launch.h"
 
 using namespace cd;
 
@@ -36,102 +36,6 @@ cudaError_t launch_attn(cd_model* m, const cd_layer_dev& L) {
     return m->cfg.hd == 128 ? launch_attn_hd<KT, 128>(m, L) : launch_attn_hd<KT, 64>(m, L);
 }
 
-// ------------------------------------------------------------------ persistent kernel launch
-template <typename WT, typename LT, typename KT, int ND, int NH, bool TPAR, bool GROUPED>
-cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
-    constexpr bool Q = Wfmt<LT>::QUANT;
-    constexpr int RD = ND == 1 ? 4 : ND == 2 || Q ? 2 : 1;
-    constexpr int RH = NH == 1 ? 4 : NH == 2 || Q ? 2 : 1;
-    constexpr int NO = Q ? 2 * ND : ND;  // an FP8 chunk is twice as many elements as one of the head's
-    constexpr int RO = Q ? (NO == 2 ? 2 : 1) : RD;
-    const cd_config& c = m->cfg;
-    auto kern = decode_mega_kernel<WT, LT, KT, ND, RD, NH, RH, NO, RO, TPAR, GROUPED>;
-    // every CTA owns rows of every matrix: what tells a CTA that another one is done with a vector is that one's next rows
-    const int grid = TPAR ? m->sm_count : std::min({m->sm_count, c.dim, c.hidden, (c.q_dim + 2 * c.kv_dim) / 2});
-    const size_t stage_cap = (std::max({(size_t)RD * Wfmt<LT>::row_stride(std::max(c.dim, c.q_dim)), (size_t)RH * Wfmt<LT>::row_stride(c.hidden), (size_t)RO * c.dim * sizeof(WT)}) + 127) / 128 * 128;
-    int max_rows = 0;
-    for (int n : {c.q_dim + 2 * c.kv_dim, c.dim, 2 * c.hidden, want_logits ? m->v_loc : 0}) max_rows = std::max(max_rows, n / grid + 2);
-    const int xs_dim = TPAR ? std::max(c.q_dim, c.dim) : std::max({c.q_dim, c.dim, c.hidden});
-    const int rows_cap = (max_rows + 3) & ~3;
-    size_t off = 0;
-    auto carve = [&](size_t bytes) { const size_t o = off; off += (bytes + 15) / 16 * 16; return o; };
-    const size_t xs_off = carve((size_t)xs_dim * 4), partial_off = carve((size_t)rows_cap * (GEMV_CONSUMERS / 32) * 4), resid_off = carve((size_t)2 * rows_cap * 4),
-                 pt_off = carve((size_t)m->pages_per_seq * 4), layers_off = carve((size_t)c.nlayers * sizeof(MegaLayer)), bars_off = carve(2 * 16 * 8);
-    const size_t budget = (size_t)m->ring_kb * 1024;
-    if (sizeof(MegaShared) + off + 2 * stage_cap > budget) return cudaErrorInvalidConfiguration;
-    const int nstages = (int)std::min<size_t>(16, (budget - sizeof(MegaShared) - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
-    const size_t ring = (size_t)nstages * stage_cap, smem = ring + off;
-    // attention tiles: the largest power-of-two run of cached positions that stays inside a page and fits a stage
-    int tile = 64;
-    while (tile > 1 && (tile > m->page_tokens || m->page_tokens % tile || (size_t)tile * c.hd * sizeof(KT) > stage_cap)) tile >>= 1;
-    static size_t smem_set = 0;
-    if (smem > smem_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        smem_set = smem;
-    }
-    MegaParams p;
-    p.layers = (const MegaLayer*)m->mega_layers;
-    p.embed = m->embed; p.lm_head = m->lm_head; p.gamma_final = m->gamma_final;
-    p.x_a = m->x_a; p.x_b = m->x_b; p.q = m->q; p.gate = m->gate; p.logits = m->logits; p.norm_final = m->norm_final;
-    {
-        unsigned long long* t = (unsigned long long*)m->mega_tagged;
-        p.tx_a = t; p.tx_b = p.tx_a + c.dim; p.tq = p.tx_b + c.dim; p.tkv = p.tq + c.q_dim; p.tgate = p.tkv + 2 * c.kv_dim; p.tparts = p.tgate + c.hidden;
-    }
-    p.part_acc = m->part_acc; p.part_ml = m->part_ml; p.grid_counter = m->grid_counter;
-    p.st = m->st; p.page_table = m->page_table; p.rope = m->rope;
-    p.dim = c.dim; p.hidden = c.hidden; p.heads = c.heads; p.kv_heads = c.kv_heads; p.hd = c.hd; p.nlayers = c.nlayers;
-    p.vocab = m->v_loc; p.embed_rows = m->full_cfg.vocab; p.q_dim = c.q_dim; p.kv_dim = c.kv_dim; p.gqa = c.gqa_ratio; p.page_tokens = m->page_tokens;
-    p.activation = m->opt.activation; p.alpha = m->alpha; p.attn_scale = 1.0f / std::sqrt((float)c.hd);
-    p.trace = m->mega_trace;
-    p.npages = m->pages_per_seq;
-    p.tile_tokens = tile;
-    p.wait_ns = m->wait_ns;
-    p.tp = m->tp;  // world <= 1 on one GPU
-    p.tp.wait_ns = m->wait_ns;
-    p.off_xs = ring + xs_off; p.off_partial = ring + partial_off; p.off_resid = ring + resid_off; p.off_pt = ring + pt_off; p.off_layers = ring + layers_off;
-    p.off_bars = ring + bars_off;
-    p.nstages = nstages; p.stage_cap = (uint32_t)stage_cap; p.rows_cap = rows_cap; p.input_embed = input_embed; p.want_logits = want_logits;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(grid);
-    lc.blockDim = dim3(MEGA_THREADS);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = m->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident: they meet at grid barriers
-    at[0].val.cooperative = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&lc, kern, p);
-    count_launch(m);
-    return e;
-}
-
-template <typename WT, typename LT, typename KT, bool TPAR, bool GROUPED>
-cudaError_t launch_mega_tp(cd_model* m, int input_embed, int want_logits) {
-    switch (m->mega_nd * 10 + m->mega_nh) {
-        case 11: return launch_mega_t<WT, LT, KT, 1, 1, TPAR, GROUPED>(m, input_embed, want_logits);
-        case 12: return launch_mega_t<WT, LT, KT, 1, 2, TPAR, GROUPED>(m, input_embed, want_logits);
-        case 14: if constexpr (!TPAR) return launch_mega_t<WT, LT, KT, 1, 4, TPAR, GROUPED>(m, input_embed, want_logits); else break;
-        case 13: if constexpr (Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 1, 3, TPAR, GROUPED>(m, input_embed, want_logits); else break;
-        case 24: return launch_mega_t<WT, LT, KT, 2, 4, TPAR, GROUPED>(m, input_embed, want_logits);
-        case 26: if constexpr (!Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 6, TPAR, GROUPED>(m, input_embed, want_logits); else break;
-        case 28: if constexpr (!TPAR && !Wfmt<LT>::QUANT) return launch_mega_t<WT, LT, KT, 2, 8, TPAR, GROUPED>(m, input_embed, want_logits); else break;
-        default: break;
-    }
-    return cudaErrorInvalidConfiguration;
-}
-template <typename WT, typename LT, typename KT>
-cudaError_t launch_mega(cd_model* m, int input_embed, int want_logits) {
-    if constexpr (!std::is_same<WT, float>::value && !Wfmt<LT>::QUANT) {  // the tensor-parallel form exists for the 16-bit storage types
-        if (m->tp_world > 1) return launch_mega_tp<WT, LT, KT, true, false>(m, input_embed, want_logits);
-    }
-    if constexpr (std::is_same<KT, __half>::value) {
-        if (m->cfg.gqa_ratio > 2) return launch_mega_tp<WT, LT, KT, false, true>(m, input_embed, want_logits);
-    }
-    return launch_mega_tp<WT, LT, KT, false, false>(m, input_embed, want_logits);
-}
-
 // One token through the whole model; everything is enqueued on m->stream.
 // WT: storage of the embedding and the LM head; LT: row format of the linears; KT: storage of the KV cache.
 template <typename WT, typename LT, typename KT>
@@ -145,10 +49,15 @@ cudaError_t enqueue_step_t(cd_model* m, const cd_step& p) {
         count_launch(m);
     }
     constexpr bool has_mega = !std::is_same<LT, Int4G32>::value;
-    const bool use_mega = has_mega && m->mega && m->mega_nd > 0 && !m->profiling;
-    if (use_mega) {
-        if constexpr (has_mega) TRY((launch_mega<WT, LT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0)));
-    } else if (p.input >= 1) {
+    bool use_mega = has_mega && m->mega && m->mega_nd > 0 && !m->profiling;
+    if constexpr (has_mega) {
+        if (use_mega) {
+            e = launch_mega<WT, LT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0);
+            if (e == cudaErrorNotSupported) m->mega = use_mega = false;  // its buffers do not fit this model's shared memory: nothing was launched
+            else if (e != cudaSuccess) return e;
+        }
+    }
+    if (!use_mega && p.input >= 1) {
         embed_kernel<WT><<<std::max(1, c.dim / 256), 256, 0, m->stream>>>((const WT*)m->embed, m->st, m->x_a, c.dim, m->full_cfg.vocab);
         count_launch(m);
         TRY(cudaGetLastError());

@@ -90,7 +90,7 @@ struct MegaParams {
 
 // Wo / W2 epilogue: x_out = res + alpha y on one GPU; tensor parallel, the rank's partial y goes to every rank's
 // inbox instead (EpiPush) and the phase that consumes it adds the residual.
-__device__ __noinline__ void push_partial(const TpLink& tp, int ar_out, int unit, float y) {
+static __device__ __noinline__ void push_partial(const TpLink& tp, int ar_out, int unit, float y) {
     const unsigned int seq = __ldcg(&tp.st->ar_base) + (unsigned int)ar_out;
     const size_t at = ((size_t)(seq % 3u) * tp.world + tp.rank) * tp.dim + unit;
     const float v = tp_sanitize(y);
@@ -277,7 +277,7 @@ __device__ inline bool walk_token_stream(const MegaParams& p, const MegaLayer* l
 // in_reduce), gathered from this rank's inbox into shared memory (xg), every thread a few float4 positions; both
 // consumer groups then take their slices from there, CTA 0 keeps the vector in x_out.  Out of line: one copy for
 // all phases, and none of it in the instruction stream of a single-GPU token.
-__device__ __noinline__ void gather_input(const TpLink& tin, int K, float* xg, int* err) {
+static __device__ __noinline__ void gather_input(const TpLink& tin, int K, float* xg, int* err) {
     const unsigned int seq = __ldcg(&tin.st->ar_base) + (unsigned int)tin.in_reduce;
     float* base = reinterpret_cast<float*>(tin.peers[tin.rank]);
     const float* inbox = base + (size_t)(seq % 3u) * tin.world * tin.dim;

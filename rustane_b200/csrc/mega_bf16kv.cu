@@ -1,0 +1,5 @@
+#include "mega_launch.cuh"
+
+namespace cd {
+template cudaError_t launch_mega<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(cd_model*, int, int);
+}  // namespace cd
