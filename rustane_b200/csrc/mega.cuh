@@ -7,24 +7,22 @@
 // HBM in the order it will need it: its rows of the q|k|v matrix, the K/V tiles of the
 // cached positions its attention work covers, its rows of Wo, W1|W3 and W2 - and never
 // stops at an operator boundary, because none of that depends on this token's activations
-// (the one K/V row that does, the current position's, is read straight from global memory
-// by the consumers instead).  Sixteen consumer warps run the operators in order; a vector
+// (the one K/V row that does, the current position's, reaches the consumers as tagged words).  Sixteen consumer warps run the operators in order; a vector
 // that the next operator needs whole (five times per layer) reaches every CTA as tagged words,
 // which it polls for (tag_store below).  While consumers wait for them the ring keeps filling,
-// so HBM stays busy; afterwards they drain shared memory several times faster than HBM can
-// refill it and catch up.
+// so HBM stays busy.
 //
 // Phases of a layer (same arithmetic and epilogues as the stand-alone kernels):
-//   1 RMSNorm + q|k|v GEMV + RoPE + KV append                                        | barrier
+//   1 RMSNorm + q|k|v GEMV + RoPE + KV append
 //   2 attention: every kv head belongs to a few CTAs, each of which takes a contiguous
 //     run of tiles of cached positions out of the ring (already resident: they were
-//     requested while phase 1 ran), keeps a running softmax per team of four warps,
-//     merges its teams in shared memory and stores ONE partial (max, sum, weighted V)
-//     per q head                                                                      | barrier
+//     requested while phase 1 ran), keeps a running softmax per warp or team of
+//     warps, merges them in shared memory and stores ONE partial (max, sum, weighted V)
+//     per q head
 //   3 every CTA merges the few partials of every head (fixed order: deterministic, no
-//     atomics, nobody waits for a "last arriver"), then Wo GEMV + scaled residual       | barrier
-//   4 RMSNorm + W1|W3 GEMV + gate                                                     | barrier
-//   5 W2 GEMV + scaled residual                                                       | barrier
+//     atomics, nobody waits for a "last arriver"), then Wo GEMV + scaled residual
+//   4 RMSNorm + W1|W3 GEMV + gate
+//   5 W2 GEMV + scaled residual
 // then the final RMSNorm + LM head into the logits buffer; the per-block head reductions
 // and samplers run as the small kernels they already are.
 //
@@ -32,7 +30,7 @@
 // its LM-head rows).  The Wo and W2 phases push their partial vectors into every rank's inbox from the
 // epilogue, and the phase that follows takes its input from the inbox - it polls (bounded by time) until
 // all ranks' words are there and adds them in rank order - so the exchange needs no grid barrier of its
-// own: barriers 3 and 5 become CTA-local, three grid barriers per layer remain.
+// own: behind Wo and W2 a CTA-local barrier is enough, three grid barriers per layer remain.
 //
 // Every wait (mbarrier, grid barrier) is bounded: on expiry the CTA records an error in
 // DevState::error, stops working and leaves, and so does every other CTA when its own
