@@ -400,8 +400,8 @@ template <int NITER> struct Slices<Fp8Row, NITER> {
     }
 };
 
-// ---- consumer side of one GEMV phase: this CTA's rows [r0, r1) out of the ring times the input slices, times `unscale`; a
-// partial sum per row and warp of a group
+// ---- consumer side of one GEMV phase: this CTA's rows [r0, r1) out of the ring times the input slices, times `unscale` (a power
+// of two, applied behind the row's scale: their product may be subnormal); a partial sum per row and warp of a group
 template <typename LT, int NITER, int R>
 __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, float unscale, int r0, int r1, int K, const MegaParams& p) {
     using F = Wfmt<LT>;
@@ -447,7 +447,7 @@ __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, f
             acc);
         if (F::ROW_SCALE) {
 #pragma unroll
-            for (int j = 0; j < R; ++j) acc[j] *= scale[j] * unscale;
+            for (int j = 0; j < R; ++j) acc[j] = acc[j] * scale[j] * unscale;
         }
         int rr;
         const float tot = warp_reduce_rows<R>(acc, lane, rr);
@@ -642,9 +642,10 @@ template <typename WT> __device__ inline float2 gather_first(const MegaParams& p
 // the GEMV waited for the instruction cache (about 0.5 us at the start of every phase of a small model).
 enum { PH_QKV = 0, PH_WO = 1, PH_W13 = 2, PH_W2 = 3, PH_HEAD = 4 };
 
-// the rows of a phase: input slices out of xs, times inv (1 / root mean square, or 1); the rows' results times unscale
+// the rows of a phase: input slices out of xs, times inv (1 / root mean square, or 1), then times the power of two `up` of quantised
+// rows (one after the other: their product overflows where the vector is zero or tiny); the rows' results times unscale
 template <typename LT, int NITER, int R>
-__device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, float unscale, float* norm_out, const int2& rows, int K) {
+__device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, float up, float unscale, float* norm_out, const int2& rows, int K) {
     constexpr int EPC = Wfmt<LT>::EPC;
     const float* xs = reinterpret_cast<const float*>(mega_dyn() + p.off_xs);
     const int tid = threadIdx.x & 255, nchunks = K / EPC;
@@ -658,6 +659,7 @@ __device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, f
             if (c < nchunks) v = *reinterpret_cast<const float4*>(xs + (size_t)c * EPC + e);
             v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
             if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x < 256 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
+            if (Wfmt<LT>::QUANT) { v.x *= up; v.y *= up; v.z *= up; v.w *= up; }
             x.set(i, e, v);
         }
     }
@@ -1384,20 +1386,20 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
                 inv = 1.0f / sqrtf(tot * (1.0f / (float)p.dim) + RMS_EPS);
             }
             if constexpr (Wfmt<LT>::QUANT) {
-                float mx = 0.0f, unscale = 1.0f;
+                float mx = 0.0f, up = 1.0f, unscale = 1.0f;
                 if (ph != PH_HEAD) {  // the power of two that brings the largest input to [2^14, 2^15)
 #pragma unroll
                     for (int i = 0; i < MEGA_CONSUMERS / 32; ++i) mx = fmaxf(mx, sh.red[32 + i]);
                     const int e = (int)(__float_as_uint(mx * inv) >> 23), f = e == 255 ? 127 : min(253, max(1, 268 - e));
-                    inv *= __uint_as_float((uint32_t)f << 23);
+                    up = __uint_as_float((uint32_t)f << 23);
                     unscale = __uint_as_float((uint32_t)(254 - f) << 23);
                 }
-                if (ph == PH_HEAD) tagged_rows<WT, NO, RO>(ring, p, inv, 1.0f, p.norm_final, sh.rows[ph], p.dim);
-                else if (ph == PH_W2) tagged_rows<LT, NH, RH>(ring, p, inv, unscale, nullptr, sh.rows[PH_WO], p.hidden);
-                else tagged_rows<LT, ND, RD>(ring, p, inv, unscale, nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
+                if (ph == PH_HEAD) tagged_rows<WT, NO, RO>(ring, p, inv, 1.0f, 1.0f, p.norm_final, sh.rows[ph], p.dim);
+                else if (ph == PH_W2) tagged_rows<LT, NH, RH>(ring, p, inv, up, unscale, nullptr, sh.rows[PH_WO], p.hidden);
+                else tagged_rows<LT, ND, RD>(ring, p, inv, up, unscale, nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
             } else {
-                if (ph == PH_W2) tagged_rows<LT, NH, RH>(ring, p, inv, 1.0f, nullptr, sh.rows[PH_WO], p.hidden);
-                else tagged_rows<LT, ND, RD>(ring, p, inv, 1.0f, ph == PH_HEAD ? p.norm_final : nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
+                if (ph == PH_W2) tagged_rows<LT, NH, RH>(ring, p, inv, 1.0f, 1.0f, nullptr, sh.rows[PH_WO], p.hidden);
+                else tagged_rows<LT, ND, RD>(ring, p, inv, 1.0f, 1.0f, ph == PH_HEAD ? p.norm_final : nullptr, sh.rows[ph], ph == PH_WO ? p.q_dim : p.dim);
             }
             mega_bar();
             if (mega_aborted()) { ok = false; break; }

@@ -167,3 +167,25 @@ def test_fp8_persistent_kernel_matches_the_kernel_per_operator(R, dim, hidden, h
         x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
         assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
     assert a.kernel_launches() - before == 10  # the persistent kernel and the position's advance
+
+
+@pytest.mark.parametrize("value", [0.0, 1e-36, 1e-20])
+@pytest.mark.parametrize("zero_gamma", [False, True])
+def test_fp8_zero_and_tiny_inputs(R, value, zero_gamma):
+    """A token whose embedding row is zero or tiny (padding rows of checkpoints), a zero hidden vector, a norm with a zero gamma:
+    the scale that brings an input to fp16's range must not overflow, and nothing may reach the cache that disturbs later tokens."""
+    cfg, rng = R.Config(256, 640, 2, 128, 64, 2, 320), np.random.default_rng(4)
+    shapes = dict(wq=(256, 256), wk=(256, 256), wv=(256, 256), wo=(256, 256), w1=(256, 640), w3=(256, 640), w2=(256, 640))
+    layers = [dict({n: rng.normal(0, 0.05, s).astype(np.float32) for n, s in shapes.items()}, gamma1=np.ones(256), gamma2=np.ones(256)) for _ in range(2)]
+    if zero_gamma:
+        layers[1]["gamma1"] = np.zeros(256)
+    embed = rng.normal(0, 0.05, (320, 256)).astype(np.float32)
+    embed[5] = value
+    a, b = (R.Model.new(cfg, layers, dict(gamma_final=np.ones(256), embed=embed), dtype="fp8", mega=mega) for mega in (True, False))
+    for t in (5, 7, 5, 9, 300):
+        x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
+        assert np.isfinite(y).all() and np.abs(x - y).max() <= 2e-4 * np.abs(y).max(), t
+    x, y = a.decode_token(np.full(256, value)), b.decode_token(np.full(256, value))
+    assert np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
+    x, y = a.decode_token_logits_from_id(11), b.decode_token_logits_from_id(11)
+    assert np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
