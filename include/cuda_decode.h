@@ -310,8 +310,8 @@ int cd_decode_steps_samples(cd_model* m, const uint32_t* first_tokens, size_t ns
 int cd_profile_decode_step(cd_model* m, uint32_t token, float* ms_by_class, uint32_t* launches_by_class,
                            size_t nclasses);
 /* Measurement aid for the one-kernel-per-token path: globaltimer stamps (ns) taken by the
- * first and the last CTA when a phase's input is in and when the phase ends (tensor parallel: at the barriers) of the most
- * recent token; a CTA without attention work skips that phase's first stamp; only with test_flags bit 2.  Layout: 2 x (1 + 10*nlayers + 1). */
+ * first and the last CTA at the start, when each phase's input is in and when the phase ends (tensor parallel: at the barriers),
+ * and at the end of the most recent token that took that path; only with test_flags bit 2.  Layout: 2 x (1 + 10*nlayers + 1). */
 int cd_debug_phase_trace(cd_model* m, unsigned long long* out, size_t cap, size_t* n);
 /* device time of the last cd_decode_steps_* / cd_prefill call, from CUDA events */
 int cd_last_device_ms(const cd_model* m, float* ms);

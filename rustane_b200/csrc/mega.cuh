@@ -75,7 +75,7 @@ struct MegaParams {
     int npages;                 // page-table entries of the sequence
     int tile_tokens;            // cached positions per attention tile (divides page_tokens; a K tile fits one ring stage)
     unsigned long long wait_ns; // bound of a grid-barrier wait
-    unsigned long long* trace;  // optional [2][1 + 10 * nlayers + 1] globaltimer stamps of CTA 0 and the last CTA
+    unsigned long long* trace;  // optional [2][1 + 10 * nlayers + 1] globaltimer stamps of CTA 0 and the last CTA: start, two per phase of a layer, end
     TpLink tp;                  // tensor parallel (world > 1): the dimensions above are this rank's shard
     // byte offsets in dynamic shared memory, behind the ring: widest input vector, [rows_cap][8] partial sums, [2][rows_cap] residual
     // entries, page table, [nlayers] layer table, barriers.  (Offsets as kernel parameters and the rest of the CTA's scratch as
@@ -803,7 +803,7 @@ __device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int at
     float* probs = probs_all + warp * 8 * NH;  // [8 positions][NH]
     const AttnPlan plan = sh.plan;
     bool ok = true;
-    if (plan.first < 0) return !mega_aborted();
+    if (plan.first < 0) { input_is_in(); return !mega_aborted(); }
     for (int h = plan.first; h < p.kv_heads && ok; h += plan.step) {
         if (!attention_inputs<__half>(p, h, plan.t1 == ntiles, tag)) { ok = false; break; }
         if (h == plan.first) input_is_in();
@@ -1180,6 +1180,8 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
             }
             mega_bar();  // the teams' partials are free for the next head
         }
+    } else if constexpr (TAG) {
+        input_is_in();
     }
     return ok && !mega_aborted();
 }
@@ -1377,7 +1379,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
             if (Wfmt<LT>::QUANT) in.y = warp_max(in.y);
             if ((tid & 31) == 0) { sh.red[warp] = in.x; sh.red[32 + warp] = in.y; }
             mega_bar();
-            stamp();
+            if (ph != PH_HEAD) stamp();
             float inv = 1.0f;
             if (norm) {
                 float tot = 0.0f;

@@ -6,6 +6,8 @@ difference orders of magnitude smaller, and tighter bounds are asserted where th
 top-k values 1e-4, block max 1e-4, block sum 1e-3, materialised block 1e-4
 (tests/auto_kv_decode.rs:136-215).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -458,3 +460,22 @@ def test_grouped_queries_on_the_persistent_kernel(R, dims, kv_heads, dtype, page
         x, y = a.decode_token_logits_from_id(tok), b.decode_token_logits_from_id(tok)
         assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
     assert a.kernel_launches() - before == 6  # the persistent kernel and the position's advance
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(37, 37, 64), (2, 2, 128), (8, 2, 64)])
+@pytest.mark.parametrize("logits", [True, False])
+def test_phase_stamps_of_the_persistent_kernel_fill_their_rows(R, heads, kv_heads, hd, logits):
+    """Start, two stamps per phase of a layer, end: of the first and the last CTA, whether the last one has attention work
+    (37 kv heads of four CTAs each) or not.  A stamp too many would land on the other row, or behind the buffer."""
+    cfg = R.Config(512, 640, heads, hd, 512, 3, 1500, kv_heads=kv_heads)
+    m = R.Model.synthetic(cfg, 7, dtype="bf16", trace=True, mega=True)
+    m.prefill(np.arange(300, dtype=np.uint32), want_logits=False)
+    m.decode_token_logits_from_id(5) if logits else m.decode_token_from_id(5)
+    n = 10 * cfg.nlayers + 2
+    out, count = np.zeros(2 * n, dtype=np.uint64), ctypes.c_size_t()
+    from rustane_b200 import _ffi
+    assert _ffi.lib.cd_debug_phase_trace(m._h, out.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), out.size, ctypes.byref(count)) == 0
+    assert count.value == 2 * n
+    rows = out.reshape(2, n).astype(np.int64)
+    assert (rows > 0).all() and (np.diff(rows, axis=1) >= 0).all()
+    assert abs(int(rows[0, 0]) - int(rows[1, 0])) < 1_000_000  # both of the same token
