@@ -21,7 +21,7 @@ struct DevState {
     int32_t error;       // first device-side error code (0 = none)
     int32_t block_idx;   // last block chosen by the full-vocab sampler
     int32_t cursor;      // next prompt token to feed during prefill
-    unsigned long long epoch;  // persistent-kernel launches completed (grid-barrier bookkeeping)
+    unsigned long long epoch;  // persistent-kernel launches completed, tensor parallel (grid-barrier bookkeeping)
     uint32_t ar_base;    // tensor-parallel all-reduces issued by the tokens completed so far (same on every rank)
     uint32_t cand_seq;   // tensor-parallel head exchanges issued so far
 };

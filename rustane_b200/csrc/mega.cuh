@@ -60,7 +60,7 @@ struct MegaParams {
     const float* gamma_final;
     float *x_a, *x_b, *q, *gate, *logits, *norm_final;
     float *part_acc, *part_ml;         // [heads][MEGA_MAX_PARTS][hd], [heads][MEGA_MAX_PARTS][2]
-    unsigned long long* grid_counter;  // monotonic arrival counter of the grid barrier
+    unsigned long long* grid_counter;  // monotonic: arrivals at the grid barrier (tensor parallel), CTAs started (one GPU)
     DevState* st;
     const int* page_table;
     const float2* rope;
@@ -133,6 +133,7 @@ struct MegaShared {
     AttnPlan plan;
     int2 rows[5];                            // this CTA's rows of q|k|v, the residual stream, gate|up; [4] the head
     size_t kv_at;                            // this position's K row of kv head 0 in a layer's pages (elements)
+    unsigned long long launch;               // one GPU: launches of this model ahead of this one
     int abort;
 };
 __device__ inline MegaShared& mega_shared() {
@@ -1306,6 +1307,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
         const int page = p.page_table[(attn_len - 1) / p.page_tokens], off = (attn_len - 1) % p.page_tokens;
         sh.kv_at = ((size_t)page * 2 * p.kv_heads * p.page_tokens + off) * p.hd;
     }
+    // every CTA of a launch adds one, however it ends, and the next launch starts behind the last of them
+    if (!TPAR && tid == 96) sh.launch = atomicAdd(p.grid_counter, 1ull) / gridDim.x;
     if (tid < p.hd / 2) sh.rope[tid] = p.rope[(size_t)(attn_len - 1) * (p.hd / 2) + tid];
     __syncthreads();
 
@@ -1353,8 +1356,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
     stamp();
     bool ok = true;
     if constexpr (!TPAR) {
-        // layer l's words carry tag0 + l (st->epoch, launches completed so far, is stable until CTA 0 has finished its last phase)
-        const uint32_t tag0 = (uint32_t)__ldcg(&p.st->epoch) * (uint32_t)p.nlayers + 1u;
+        // layer l's words carry tag0 + l: no two launches share a tag, whether the earlier one got through or not
+        const uint32_t tag0 = (uint32_t)sh.launch * (uint32_t)p.nlayers + 1u;
         float* const resid = reinterpret_cast<float*>(mega_dyn() + p.off_resid);
         const int phases = 4 * p.nlayers + (p.want_logits ? 1 : 0);
         for (int step = 0; step < phases; ++step) {
@@ -1409,8 +1412,6 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
             if (ph != PH_HEAD) stamp();
         }
         stamp();
-        // (also after a failure: the next launch must not take this one's words for its own)
-        if (tid == 0 && blockIdx.x == 0) p.st->epoch += 1;
     } else {
         const unsigned long long epoch = __ldcg(&p.st->epoch);
         unsigned long long arrivals = epoch * 3ull * (unsigned long long)p.nlayers;  // barriers completed by earlier launches
