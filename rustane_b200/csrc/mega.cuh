@@ -70,6 +70,7 @@ struct MegaParams {
     int nstages;
     uint32_t stage_cap;   // bytes per ring stage
     int rows_cap;         // rows a CTA may own in any phase
+    int resid_cap;        // of them, rows of the residual stream
     int input_embed;      // 1: x = embed[st->token]; 0: x already in x_a
     int want_logits;
     int npages;                 // page-table entries of the sequence
@@ -77,7 +78,7 @@ struct MegaParams {
     unsigned long long wait_ns; // bound of a grid-barrier wait
     unsigned long long* trace;  // optional [2][1 + 10 * nlayers + 1] globaltimer stamps of CTA 0 and the last CTA: start, two per phase of a layer, end
     TpLink tp;                  // tensor parallel (world > 1): the dimensions above are this rank's shard
-    // byte offsets in dynamic shared memory, behind the ring: widest input vector, [rows_cap][8] partial sums, [2][rows_cap] residual
+    // byte offsets in dynamic shared memory, behind the ring: widest input vector, [rows_cap][8] partial sums, [2][resid_cap] residual
     // entries, page table, [nlayers] layer table, barriers.  (Offsets as kernel parameters and the rest of the CTA's scratch as
     // static shared memory cost no registers; with a pointer each the GEMV loops spilled, and at 544 threads a CTA's spills
     // do not fit the L1 that the ring leaves.)
@@ -712,7 +713,7 @@ __device__ inline void tagged_epilogue(const MegaParams& p, int ph, bool last_la
             if (ph == PH_HEAD) {
                 p.logits[r] = y;
             } else {
-                const float v = resid[(ph == PH_W2 ? p.rows_cap : 0) + j] + p.alpha * y;
+                const float v = resid[(ph == PH_W2 ? p.resid_cap : 0) + j] + p.alpha * y;
                 tag_store((ph == PH_W2 ? p.tx_a : p.tx_b) + r, v, tag);
                 if (ph == PH_W2 && last_layer) p.x_a[r] = v;
             }
@@ -1372,7 +1373,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_mega_kernel(const __gr
                 if (!ok) break;
                 in = gather_merged(p, tag);
             } else {
-                const InputTo to{xs, ph == PH_QKV ? resid : ph == PH_W13 ? resid + p.rows_cap : nullptr,
+                const InputTo to{xs, ph == PH_QKV ? resid : ph == PH_W13 ? resid + p.resid_cap : nullptr,
                                  ph == PH_QKV ? L.gamma1 : ph == PH_W13 ? L.gamma2 : ph == PH_HEAD ? p.gamma_final : nullptr, sh.rows[PH_WO]};
                 if (step == 0) in = gather_first<WT>(p, to);
                 else in = gather_tagged(ph == PH_W13 ? p.tx_b : ph == PH_W2 ? p.tgate : p.tx_a, ph == PH_W13 || ph == PH_W2 ? tag : tag - 1u, ph == PH_W2 ? p.hidden : p.dim, to, p);

@@ -27,10 +27,11 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     int max_rows = 0;
     for (int n : {c.q_dim + 2 * c.kv_dim, c.dim, 2 * c.hidden, want_logits ? m->v_loc : 0}) max_rows = std::max(max_rows, n / grid + 2);
     const int xs_dim = TPAR ? std::max(c.q_dim, c.dim) : std::max({c.q_dim, c.dim, c.hidden});
-    const int rows_cap = (max_rows + 3) & ~3;
+    // (the residual entries are the CTA's rows of Wo and W2, not of the LM head: with 128 k rows of it those are 866 a CTA)
+    const int rows_cap = (max_rows + 3) & ~3, resid_cap = (c.dim / grid + 2 + 3) & ~3;
     size_t off = 0;
     auto carve = [&](size_t bytes) { const size_t o = off; off += (bytes + 15) / 16 * 16; return o; };
-    const size_t xs_off = carve((size_t)xs_dim * 4), partial_off = carve((size_t)rows_cap * (GEMV_CONSUMERS / 32) * 4), resid_off = carve((size_t)2 * rows_cap * 4),
+    const size_t xs_off = carve((size_t)xs_dim * 4), partial_off = carve((size_t)rows_cap * (GEMV_CONSUMERS / 32) * 4), resid_off = carve((size_t)2 * resid_cap * 4),
                  pt_off = carve((size_t)m->pages_per_seq * 4), layers_off = carve((size_t)c.nlayers * sizeof(MegaLayer)), bars_off = carve(2 * 16 * 8);
     const size_t budget = (size_t)m->ring_kb * 1024;
     if (sizeof(MegaShared) + off + 2 * stage_cap > budget) return cudaErrorNotSupported;
@@ -66,7 +67,7 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     p.tp.wait_ns = m->wait_ns;
     p.off_xs = ring + xs_off; p.off_partial = ring + partial_off; p.off_resid = ring + resid_off; p.off_pt = ring + pt_off; p.off_layers = ring + layers_off;
     p.off_bars = ring + bars_off;
-    p.nstages = nstages; p.stage_cap = (uint32_t)stage_cap; p.rows_cap = rows_cap; p.input_embed = input_embed; p.want_logits = want_logits;
+    p.nstages = nstages; p.stage_cap = (uint32_t)stage_cap; p.rows_cap = rows_cap; p.resid_cap = resid_cap; p.input_embed = input_embed; p.want_logits = want_logits;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(grid);
     lc.blockDim = dim3(MEGA_THREADS);

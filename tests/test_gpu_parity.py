@@ -479,3 +479,19 @@ def test_phase_stamps_of_the_persistent_kernel_fill_their_rows(R, heads, kv_head
     rows = out.reshape(2, n).astype(np.int64)
     assert (rows > 0).all() and (np.diff(rows, axis=1) >= 0).all()
     assert abs(int(rows[0, 0]) - int(rows[1, 0])) < 1_000_000  # both of the same token
+
+
+@pytest.mark.parametrize("ring_kb,launches", [(70, 2), (60, None), (0, 2)])
+def test_a_large_vocabulary_leaves_the_ring_its_shared_memory(R, ring_kb, launches):
+    """A CTA of the persistent kernel keeps its rows' partial sums (here 888 rows of the LM head) and the residual entries of its
+    few rows of the stream beside the ring.  70 KB hold both with two stages; 60 KB do not, and the token runs a kernel per
+    operator.  Same logits every way (sums in another order, a cache entry may round to its neighbour: 2e-4)."""
+    cfg = R.Config(256, 640, 2, 128, 64, 2, 131072)
+    m = R.Model.synthetic(cfg, 7, dtype="bf16", ring_kb=ring_kb, mega=True, use_graph=True)
+    ref = R.Model.synthetic(cfg, 7, dtype="bf16", mega=False)
+    for t in (5, 131071, 9):
+        before = m.kernel_launches()
+        x, y = m.decode_token_logits_from_id(t), ref.decode_token_logits_from_id(t)
+        n = m.kernel_launches() - before
+        assert n == launches if launches else n > 2
+        assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
