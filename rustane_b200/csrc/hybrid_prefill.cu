@@ -64,16 +64,18 @@ struct Gemm {
 };
 
 // pf_attn_kernel takes query and key rows of 64 or 128 entries, value rows of 64 or 128, tiles of 128 keys made of whole
-// pages (or pages of whole tiles), and a positive scale (its running maximum is taken before scaling); gates per element and
-// padded widths stay with attn_window_kernel.  Per layer of a 16-head model with windows of 1024 at 1500 tokens: 183 us there.
+// pages (or pages of whole tiles), and a positive scale (its running maximum is taken before scaling); padded widths stay with
+// attn_window_kernel.  (A gate per element is none of either kernel's work: diff_rows_kernel applies it.)  Per layer of a 16-head model with windows of 1024 at 1500 tokens: 183 us there.
 bool on_tensor_memory(const AttnDims& a) {
     const bool widths = (a.kp == 64 && a.vp == 64) || (a.kp == 64 && a.vp == 128) || (a.kp == 128 && a.vp == 128);
     const bool pages = a.page_tokens <= PA_KEYS ? PA_KEYS % a.page_tokens == 0 : a.page_tokens % PA_KEYS == 0;
     return widths && a.dim == a.kp && a.vdim == a.vp && pages && a.scale > 0.0f;
 }
 
+// Queries and probabilities are hi + lo pairs whatever the mode of the prompt pass, as in attn_window_kernel (without the pairs
+// the "fast" mode's logits moved by 1e-3 of the largest more than its rounding of the linears' inputs does).
 template <typename KT>
-cudaError_t launch_attn_tm(cd_model* m, EncodeTiledFn encode, const AttnWindow& p, size_t q_rows, bool split, const KT* q_hi, const KT* q_lo, const KT* pool, size_t pages,
+cudaError_t launch_attn_tm(cd_model* m, EncodeTiledFn encode, const AttnWindow& p, size_t q_rows, const KT* q_hi, const KT* q_lo, const KT* pool, size_t pages,
                            __nv_bfloat16* hi, __nv_bfloat16* lo) {
     const AttnDims& a = p.a;
     const CUtensorMapDataType dt = std::is_same<KT, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -83,14 +85,14 @@ cudaError_t launch_attn_tm(cd_model* m, EncodeTiledFn encode, const AttnWindow& 
                     encode_rows_4d(encode, &k, dt, pool, a.kr(), a.page_tokens, a.G, pages, (uint64_t)a.kr() * 2, (uint64_t)a.page_tokens * a.kr() * 2, page) &&
                     encode_rows_4d(encode, &v, dt, pool + a.v_at(0, 0, 0), a.vp, a.page_tokens, a.G, pages, (uint64_t)a.vp * 2, (uint64_t)a.page_tokens * a.vp * 2, page);
     if (!ok) return cudaErrorInvalidValue;
-    const PfAttn pa{p.rows, p.pos0, a.window, a.maps, a.H / a.G, a.page_tokens, split ? 1 : 0, a.scale * 1.4426950408889634f, p.slopes, &m->st->error};
+    const PfAttn pa{p.rows, p.pos0, a.window, a.maps, a.H / a.G, a.page_tokens, 1, a.scale * 1.4426950408889634f, p.slopes, &m->st->error};
     const PaWindowOut<__nv_bfloat16> out{p, hi, lo};
     const int nz = a.H * a.maps;
     if (p.slopes != nullptr)
-        return a.kp == 128 ? pa_launch<KT, 128, 128, true>(m, q, split, k, v, pa, nz, out)
-               : a.vp == 128 ? pa_launch<KT, 64, 128, true>(m, q, split, k, v, pa, nz, out) : pa_launch<KT, 64, 64, true>(m, q, split, k, v, pa, nz, out);
-    return a.kp == 128 ? pa_launch<KT, 128, 128, false>(m, q, split, k, v, pa, nz, out)
-           : a.vp == 128 ? pa_launch<KT, 64, 128, false>(m, q, split, k, v, pa, nz, out) : pa_launch<KT, 64, 64, false>(m, q, split, k, v, pa, nz, out);
+        return a.kp == 128 ? pa_launch<KT, 128, 128, true>(m, q, true, k, v, pa, nz, out)
+               : a.vp == 128 ? pa_launch<KT, 64, 128, true>(m, q, true, k, v, pa, nz, out) : pa_launch<KT, 64, 64, true>(m, q, true, k, v, pa, nz, out);
+    return a.kp == 128 ? pa_launch<KT, 128, 128, false>(m, q, true, k, v, pa, nz, out)
+           : a.vp == 128 ? pa_launch<KT, 64, 128, false>(m, q, true, k, v, pa, nz, out) : pa_launch<KT, 64, 64, false>(m, q, true, k, v, pa, nz, out);
 }
 
 template <typename KT>
@@ -230,7 +232,7 @@ int run_piece(cd_model* m, HybridPrefill* w, float* x, const uint32_t* ids, int 
             const bool two = L.ad.maps == 2;
             const AttnWindow aw{L.ad, L.slopes, L.sink, w->proj, proj_ld, pl.lg, m->page_table, rows, pos0, L.kl, two ? w->raw : nullptr};
             if (gemm.ok()) {
-                gemm.e = on_tensor_memory(L.ad) ? launch_attn_tm<KT>(m, w->encode, aw, R, split, q, q_lo, pool, (size_t)m->num_pages, attn, attn_lo)
+                gemm.e = on_tensor_memory(L.ad) ? launch_attn_tm<KT>(m, w->encode, aw, R, q, q_lo, pool, (size_t)m->num_pages, attn, attn_lo)
                                                 : launch_attn_window<KT>(m, aw, q, q_lo, pool, attn, attn_lo);
                 gemm.what = "attention";
             }

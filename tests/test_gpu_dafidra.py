@@ -100,6 +100,27 @@ def test_heads_on_tensor_memory(R, tmp_path, dim, vdim, window):
         assert M.error(all_logits(m, ids, portions), rounded) < KEPT
 
 
+@pytest.mark.parametrize("mode", ["", "fast"])
+@pytest.mark.parametrize("dim,vdim,window", [(128, 128, 150), (64, 64, None), (64, 128, 300)])
+def test_tensor_memory_heads_agree_with_the_window_kernel(R, tmp_path, monkeypatch, dim, vdim, window, mode):
+    """Pages of 32, 128 and 256 tokens go through the tcgen05 attention, pages of 96 through the windowed kernel.  Both keep
+    queries and probabilities as 16-bit pairs in every mode of the prompt pass, so most rows of a one-layer model differ by the
+    order of fp32 sums only (the "fast" mode rounds the rows that follow to bf16: an element near a tie may go the other way)."""
+    monkeypatch.setenv("CD_PREFILL", mode)
+    cfg = M.config(96, 120, [(M.attn(4, 2, dim, vdim, window, dim ** -0.5, 0.3, 32), M.memory(1, 8, 16, 9.0), M.dense(64))])
+    path = folder(tmp_path, cfg, M.weights(cfg, 6))
+    ids = np.random.default_rng(6).integers(0, 120, 430)
+    got = {}
+    for page in (96, 32, 128, 256):
+        m = R.Model.from_pretrained(path, max_tokens=512, page_tokens=page)
+        got[page] = all_logits(m, ids, [70, 300, 60])
+        m.close()
+    for page in (32, 128, 256):
+        rows = np.abs(got[page] - got[96]).max(1) / np.abs(got[96]).max(1)
+        print(mode, dim, vdim, page, "median %.2e, largest %.2e" % (np.median(rows), rows.max()))
+        assert np.median(rows) < 2e-5 and rows.max() < KEPT
+
+
 def test_long_prompts_are_processed_in_pieces(R, made, monkeypatch):
     cfg, _, path, ids, ref = made("ODD")
     monkeypatch.setenv("CD_PREFILL_ROWS", "70")
