@@ -49,7 +49,7 @@ cudaError_t enqueue_step_t(cd_model* m, const cd_step& p) {
         count_launch(m);
     }
     constexpr bool has_mega = !std::is_same<LT, Int4G32>::value;
-    bool use_mega = has_mega && m->mega && m->mega_nd > 0 && !m->profiling;
+    bool use_mega = has_mega && p.one_kernel && m->mega;
     if constexpr (has_mega) {
         if (use_mega) {
             e = launch_mega<WT, LT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0);
@@ -137,6 +137,27 @@ static int validate(const cd_config& c, int dtype) {
     return CD_OK;
 }
 
+// The positions up to which a token is faster as one persistent kernel than as a kernel per operator.  It saves the boundaries
+// between operators (1 us a layer of small models, 5 to 20 us of large ones) but gives a kv head to at most MEGA_CPH_CAP CTAs,
+// which walk their tiles of it one after the other: 0.5 us a tile, 1 to 1.2 with 2 or 4 q heads per kv head, 1.9 with 8.  The kernel
+// per operator spreads q heads times up to 32 slices.  Over 270 shapes (dim 512 to 4096; f32, 16 bits, FP8; 1 to 8 q heads per
+// kv head; 40 to 3500 positions) the tiles at which the two meet grow with the bytes of a layer's weights, as below; the choice
+// is within 0.2 % of the better form in the mean.  Us a token of 8 layers, persistent and per operator: dim 1024 in bf16, 8 q heads
+// on one kv head, 64 positions 200 and 219, 1000 positions 256 and 222 (limit 492); dim 2048, 16 on 4, 1000 positions 279 and 317
+// (limit 5600).  Grouped heads of small layers: 0.90 to 1.05 of the other's speed at any length.
+static size_t persistent_positions(const cd_model* m, size_t layer_bytes) {
+    struct Line { double tiles, per_mb, none_below_mb; };
+    const cd_config& c = m->cfg;
+    const Line line = c.gqa_ratio == 1 ? Line{1.0, 0.4, 0.0} : c.gqa_ratio == 2 ? Line{1.5, 0.1, 12.0} : c.gqa_ratio == 4 ? Line{2.0, 0.1, 8.0} : Line{0.5, 0.06, 12.0};
+    const double mb = layer_bytes / 1e6;
+    if (mb < line.none_below_mb) return 0;
+    const int dt = m->opt.weight_dtype;
+    const size_t head_row = (size_t)c.dim * (dt == CD_DTYPE_F32 ? 4 : 2), cached_row = (size_t)c.hd * (m->kv_dtype == CD_DTYPE_F32 ? 4 : 2);
+    const size_t stage = mega_stage_bytes(m->mega_nd, m->mega_nh, is_quant(dt), lin_row_bytes(dt, std::max(c.dim, c.q_dim)), lin_row_bytes(dt, c.hidden), head_row);
+    const double ctas_per_head = c.kv_heads <= m->sm_count ? std::min(m->sm_count / c.kv_heads, MEGA_CPH_CAP) : 1.0 / ((c.kv_heads + m->sm_count - 1) / m->sm_count);
+    return (size_t)((line.tiles + line.per_mb * mb) * mega_tile_tokens(m->page_tokens, cached_row, stage) * ctas_per_head);
+}
+
 int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_model** out) {
     *out = nullptr;
     cd_options opts;
@@ -217,8 +238,11 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
         // tensor parallel: measured on the 5B model, the persistent kernel wins at 2 ranks (601 against 569 tokens/s) and
         // loses at 8 (841 against 896), where a layer's data are 8 us and its fixed per-phase times dominate either way
         const bool mega_ok = dt != CD_DTYPE_INT4_G32 && (tpw == 1 || (tpw == 2 && dt != CD_DTYPE_F32 && !is_quant(dt)));
-        // one persistent kernel per token wherever its tiling covers the shape; test_flags bit 1 keeps one kernel per operator
+        // one persistent kernel per token where its tiling covers the shape; test_flags bit 1 keeps one kernel per operator, bit 4
+        // takes the persistent one whatever the length
         m->mega = (opts.test_flags & 2) == 0 && mega_ok && m->mega_nd > 0;
+        const size_t layer_bytes = (Q + 2 * KV) * lin_row_bytes(dt, c.dim) + D * lin_row_bytes(dt, c.q_dim) + 2 * H * lin_row_bytes(dt, c.dim) + D * lin_row_bytes(dt, c.hidden);
+        if (m->mega) m->mega_len = tpw > 1 || (opts.test_flags & 16) ? SIZE_MAX : persistent_positions(m, layer_bytes);
     }
 #undef CKB
     *out = m;

@@ -15,15 +15,13 @@ using namespace cd;
 template <typename WT, typename LT, typename KT, int ND, int NH, bool TPAR, bool GROUPED>
 cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     constexpr bool Q = Wfmt<LT>::QUANT;
-    constexpr int RD = ND == 1 ? 4 : ND == 2 || Q ? 2 : 1;
-    constexpr int RH = NH == 1 ? 4 : NH == 2 || Q ? 2 : 1;
+    constexpr int RD = mega_stage_rows(ND, Q), RH = mega_stage_rows(NH, Q), RO = mega_head_rows(ND, Q);
     constexpr int NO = Q ? 2 * ND : ND;  // an FP8 chunk is twice as many elements as one of the head's
-    constexpr int RO = Q ? (NO == 2 ? 2 : 1) : RD;
     const cd_config& c = m->cfg;
     auto kern = decode_mega_kernel<WT, LT, KT, ND, RD, NH, RH, NO, RO, TPAR, GROUPED>;
     // every CTA owns rows of every matrix: what tells a CTA that another one is done with a vector is that one's next rows
     const int grid = TPAR ? m->sm_count : std::min({m->sm_count, c.dim, c.hidden, (c.q_dim + 2 * c.kv_dim) / 2});
-    const size_t stage_cap = (std::max({(size_t)RD * Wfmt<LT>::row_stride(std::max(c.dim, c.q_dim)), (size_t)RH * Wfmt<LT>::row_stride(c.hidden), (size_t)RO * c.dim * sizeof(WT)}) + 127) / 128 * 128;
+    const size_t stage_cap = mega_stage_bytes(ND, NH, Q, Wfmt<LT>::row_stride(std::max(c.dim, c.q_dim)), Wfmt<LT>::row_stride(c.hidden), (size_t)c.dim * sizeof(WT));
     int max_rows = 0;
     for (int n : {c.q_dim + 2 * c.kv_dim, c.dim, 2 * c.hidden, want_logits ? m->v_loc : 0}) max_rows = std::max(max_rows, n / grid + 2);
     const int xs_dim = TPAR ? std::max(c.q_dim, c.dim) : std::max({c.q_dim, c.dim, c.hidden});
@@ -37,9 +35,6 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     if (sizeof(MegaShared) + off + 2 * stage_cap > budget) return cudaErrorNotSupported;
     const int nstages = (int)std::min<size_t>(16, (budget - sizeof(MegaShared) - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
     const size_t ring = (size_t)nstages * stage_cap, smem = ring + off;
-    // attention tiles: the largest power-of-two run of cached positions that stays inside a page and fits a stage
-    int tile = 64;
-    while (tile > 1 && (tile > m->page_tokens || m->page_tokens % tile || (size_t)tile * c.hd * sizeof(KT) > stage_cap)) tile >>= 1;
     static size_t smem_set = 0;
     if (smem > smem_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -61,7 +56,7 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     p.activation = m->opt.activation; p.alpha = m->alpha; p.attn_scale = 1.0f / std::sqrt((float)c.hd);
     p.trace = m->mega_trace;
     p.npages = m->pages_per_seq;
-    p.tile_tokens = tile;
+    p.tile_tokens = mega_tile_tokens(m->page_tokens, (size_t)c.hd * sizeof(KT), stage_cap);
     p.wait_ns = m->wait_ns;
     p.tp = m->tp;  // world <= 1 on one GPU
     p.tp.wait_ns = m->wait_ns;

@@ -45,15 +45,16 @@ __global__ void softcap_copy_kernel(const float* __restrict__ in, float* __restr
 
 cudaError_t enqueue_step(cd_model* m, const cd_step& p) { return m->family->enqueue_step(m, p); }
 
-// Run one step: directly, or by replaying the captured graph of the same shape.
-int run_step(cd_model* m, const cd_step& p) {
+// Run one step for the token behind `pos` cached ones: directly, or by replaying the captured graph of the same shape.
+int run_step(cd_model* m, cd_step p, size_t pos) {
+    p.one_kernel = m->mega && pos < m->mega_len;
     m->state_len = SIZE_MAX;  // until the call has succeeded (advance)
     if (!m->opt.use_graph) {
         cudaError_t e = enqueue_step(m, p);
         if (e != cudaSuccess) return fail(m, CD_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
         return CD_OK;
     }
-    const cd_graph_key key{p.head, p.k, p.input, p.t, p.inv_t, p.softcap};
+    const cd_graph_key key{p.head, p.k, p.input, p.t, p.inv_t, p.softcap, p.one_kernel};
     auto it = m->graphs.find(key);
     if (it == m->graphs.end()) {
         const uint64_t before = m->launches;
@@ -417,7 +418,7 @@ int cd_decode_token(cd_model* m, const float* x_in, float* x_out) {
     CK(m, cudaMemcpyAsync(m->x_a, x_in, (size_t)m->full_cfg.dim * 4, cudaMemcpyHostToDevice, m->stream));
     if ((rc = set_state(m, 0))) return rc;
     cd_step p{0, HEAD_NONE};
-    if ((rc = run_step(m, p))) return rc;
+    if ((rc = run_step(m, p, m->len))) return rc;
     CK(m, cudaMemcpyAsync(x_out, m->x_a, (size_t)m->full_cfg.dim * 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaMemcpyAsync(&m->h_in[2], &m->st->error, 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaStreamSynchronize(m->stream));
@@ -434,7 +435,7 @@ int cd_decode_token_from_id(cd_model* m, uint32_t token, float* x_out) {
     if ((rc = check_token(m, token))) return rc;
     if ((rc = set_state(m, token))) return rc;
     cd_step p{1, HEAD_NONE};
-    if ((rc = run_step(m, p))) return rc;
+    if ((rc = run_step(m, p, m->len))) return rc;
     CK(m, cudaMemcpyAsync(x_out, m->x_a, (size_t)m->full_cfg.dim * 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaMemcpyAsync(&m->h_in[2], &m->st->error, 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaStreamSynchronize(m->stream));
@@ -447,7 +448,7 @@ static int argmax_common(cd_model* m, int input, uint32_t token, uint32_t* out) 
     int rc = set_state(m, token);
     if (rc) return rc;
     cd_step p{input, HEAD_ARGMAX};
-    if ((rc = run_step(m, p))) return rc;
+    if ((rc = run_step(m, p, m->len))) return rc;
     CK(m, cudaMemcpyAsync(m->h_ring, m->out_token, 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaMemcpyAsync(&m->h_in[2], &m->st->error, 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaStreamSynchronize(m->stream));
@@ -489,7 +490,7 @@ int cd_decode_token_topk_from_id(cd_model* m, uint32_t token, size_t top_k, floa
     if ((rc = set_state(m, token))) return rc;
     cd_step p{1, HEAD_TOPK};
     p.k = (int)top_k;
-    if ((rc = run_step(m, p))) return rc;
+    if ((rc = run_step(m, p, m->len))) return rc;
     if (m->tp_world > 1) {
         for (int r = 0; r < m->tp_world; ++r) {  // rank r's row of the gathered candidates holds its blocks, k entries each
             const int nb_r = std::min(m->tp_nb, nblk_all - r * m->tp_nb);
@@ -522,7 +523,7 @@ int cd_decode_token_block_stats_from_id(cd_model* m, uint32_t token, float inv_t
     cd_step p{1, HEAD_STATS};
     p.inv_t = inv_temperature;
     p.softcap = softcap;
-    if ((rc = run_step(m, p))) return rc;
+    if ((rc = run_step(m, p, m->len))) return rc;
     CK(m, cudaMemcpyAsync(out_maxes, m->maxes, (size_t)m->nblocks * 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaMemcpyAsync(out_sums, m->sums, (size_t)m->nblocks * 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaMemcpyAsync(&m->h_in[2], &m->st->error, 4, cudaMemcpyDeviceToHost, m->stream));
@@ -578,7 +579,7 @@ int cd_decode_token_logits_from_id(cd_model* m, uint32_t token, float softcap, f
     if ((rc = check_token(m, token))) return rc;
     if ((rc = set_state(m, token))) return rc;
     cd_step p{1, HEAD_LOGITS};
-    if ((rc = run_step(m, p))) return rc;
+    if ((rc = run_step(m, p, m->len))) return rc;
     if ((rc = fetch_logits(m, softcap, out_logits))) return rc;
     advance(m, 1);
     return CD_OK;
@@ -630,7 +631,7 @@ static int prefill_impl(cd_model* m, const uint32_t* ids, size_t n, const size_t
     for (size_t i = 0; i < n; ++i) {
         const size_t* w = std::find(want, want + nwant, i);
         cd_step p{2, w != want + nwant ? HEAD_LOGITS : HEAD_NONE};
-        if ((rc = run_step(m, p))) return rc;
+        if ((rc = run_step(m, p, m->len + i))) return rc;
         if (i + 1 == n) CK(m, cudaEventRecord(m->ev1, m->stream));
         for (; w != want + nwant; w = std::find(w + 1, want + nwant, i))
             if ((rc = fetch_logits(m, softcap, out + (size_t)(w - want) * V))) return rc;
@@ -663,7 +664,7 @@ static int decode_loop(cd_model* m, uint32_t first, size_t nsteps, cd_step p, ui
     CK(m, cudaGetLastError());
     CK(m, cudaEventRecord(m->ev0, m->stream));
     for (size_t i = 0; i < nsteps; ++i)
-        if ((rc = run_step(m, p))) return rc;
+        if ((rc = run_step(m, p, m->len + i))) return rc;
     CK(m, cudaEventRecord(m->ev1, m->stream));
     CK(m, cudaMemcpyAsync(m->h_ring, m->out_ring, nsteps * 4, cudaMemcpyDeviceToHost, m->stream));
     CK(m, cudaMemcpyAsync(m->h_state, m->st, sizeof(DevState), cudaMemcpyDeviceToHost, m->stream));

@@ -30,6 +30,7 @@ struct cd_step {
     int head;   // cd_head_mode
     int k = 0;
     float t = 0.f, softcap = 0.f, inv_t = 1.f;
+    bool one_kernel = false;  // the whole token as one persistent kernel (run_step sets it by the token's position)
 };
 
 // A model family: how its layers are stepped and what it keeps per sequence besides the shared cache.  The token loop,
@@ -53,13 +54,15 @@ struct cd_family {
 struct cd_graph_key {
     int mode, k, input;
     float t, inv_t, softcap;
+    bool one_kernel;
     bool operator<(const cd_graph_key& o) const {
         if (mode != o.mode) return mode < o.mode;
         if (k != o.k) return k < o.k;
         if (input != o.input) return input < o.input;
         if (t != o.t) return t < o.t;
         if (inv_t != o.inv_t) return inv_t < o.inv_t;
-        return softcap < o.softcap;
+        if (softcap != o.softcap) return softcap < o.softcap;
+        return one_kernel < o.one_kernel;
     }
 };
 
@@ -137,7 +140,8 @@ struct cd_model {
     int kv_dtype = 0;    // CD_DTYPE_F32 / F16 / BF16: storage of the KV cache (cd_options.kv_dtype resolved)
     unsigned long long wait_ns = 2000000000ull;  // bound of a device-side wait on a peer GPU
     // persistent one-kernel-per-token path (mega.cuh)
-    bool mega = false;       // one persistent kernel per token
+    bool mega = false;       // one persistent kernel per token ...
+    size_t mega_len = 0;     // ... that sees at most so many positions, itself included
     int mega_nd = 0, mega_nh = 0;  // GEMV tiling of the K = dim and K = hidden phases; 0 = shape not supported
     void* mega_layers = nullptr;   // device array of cd::MegaLayer
     void* mega_tagged = nullptr;   // its vectors between phases (64-bit words), zeroed when the model is made

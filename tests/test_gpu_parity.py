@@ -495,3 +495,38 @@ def test_a_large_vocabulary_leaves_the_ring_its_shared_memory(R, ring_kb, launch
         n = m.kernel_launches() - before
         assert n == launches if launches else n > 2
         assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_form_of_a_token_by_its_position(R, use_graph):
+    """Eight q heads on one kv head: a few CTAs walk the cache in the persistent kernel, so tokens behind a long enough context run
+    a kernel per operator.  Both forms in one sequence, either way across the line, give what one kernel per operator gives (sums
+    in another order, a cache entry may round to its neighbour: 2e-4 of the logits); mega=True keeps the one kernel."""
+    cfg = R.Config(1024, 3072, 8, 128, 1024, 2, 3000, kv_heads=1)
+    make = lambda mega: R.Model.synthetic(cfg, 7, dtype="bf16", mega=mega, use_graph=use_graph)
+    auto, always, never = make(None), make(True), make(False)
+    prompt = np.random.default_rng(1).integers(0, 3000, 470).astype(np.uint32)
+    for m in (auto, always, never):
+        m.prefill(prompt, want_logits=False)
+
+    def step(m, tok):
+        before = m.kernel_launches()
+        x = m.decode_token_logits_from_id(tok)
+        return x, m.kernel_launches() - before
+
+    one = []
+    for tok in range(60):
+        (x, n), (y, k), (z, _) = step(auto, tok), step(always, tok), step(never, tok)
+        assert k == 2 and max(np.abs(x - z).max(), np.abs(y - z).max()) < 2e-4 * np.abs(z).max()
+        one.append(n == 2)
+    assert one[0] and not one[-1] and one == sorted(one, reverse=True)  # short ones as one kernel, long ones not
+    line = 470 + sum(one)
+    for m in (auto, never):
+        m.set_len(line - 3)
+    assert [step(auto, t)[1] == 2 for t in range(6)] == [True] * 3 + [False] * 3
+    auto.set_len(line - 8)
+    before = auto.kernel_launches()
+    ids = auto.decode_steps_greedy(5, 16)
+    assert auto.kernel_launches() - before == 1 + 8 * 2 + 8 * (5 * cfg.nlayers + 3)
+    never.set_len(line - 8)
+    assert np.array_equal(ids, never.decode_steps_greedy(5, 16))
