@@ -31,8 +31,13 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     auto carve = [&](size_t bytes) { const size_t o = off; off += (bytes + 15) / 16 * 16; return o; };
     const size_t xs_off = carve((size_t)xs_dim * 4), partial_off = carve((size_t)rows_cap * (GEMV_CONSUMERS / 32) * 4), resid_off = carve((size_t)2 * resid_cap * 4),
                  pt_off = carve((size_t)m->pages_per_seq * 4), layers_off = carve((size_t)c.nlayers * sizeof(MegaLayer)), bars_off = carve(2 * 16 * 8);
-    const size_t budget = (size_t)m->ring_kb * 1024;
-    if (sizeof(MegaShared) + off + 2 * stage_cap > budget) return cudaErrorNotSupported;
+    // One GPU: all that a CTA can have (with 220 KB, as the kernels per operator use, hidden 11968 to 12288 had four stages, not six;
+    // 6 layers of 3648 x 11968, 40 positions, 493 and 458 us).  But eight chunks of W2's rows a thread spill 280 to 360 bytes of
+    // registers a thread, which the L1 holds as long as shared memory takes no more than 196 KB (60 KB of L1, 28 KB behind that): 5
+    // layers of dim 4096, 1000 positions, here and per operator: hidden 13312 (195 KB) 520 and 562 us, 13824 (202 KB) 574 and 567 us.
+    const size_t budget = (size_t)(TPAR || m->opt.test_ring_kb > 0 ? m->ring_kb : NH == 8 ? 195 : 227) * 1024;
+    // (a ring of two stages loses to the kernels per operator: FP8, 5 layers of 4096 x 16384, 200 positions, 541 and 424 us)
+    if (sizeof(MegaShared) + off + (TPAR ? 2 : 4) * stage_cap > budget) return cudaErrorNotSupported;
     const int nstages = (int)std::min<size_t>(16, (budget - sizeof(MegaShared) - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
     const size_t ring = (size_t)nstages * stage_cap, smem = ring + off;
     static size_t smem_set = 0;

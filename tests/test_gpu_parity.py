@@ -481,10 +481,10 @@ def test_phase_stamps_of_the_persistent_kernel_fill_their_rows(R, heads, kv_head
     assert abs(int(rows[0, 0]) - int(rows[1, 0])) < 1_000_000  # both of the same token
 
 
-@pytest.mark.parametrize("ring_kb,launches", [(70, 2), (60, None), (0, 2)])
+@pytest.mark.parametrize("ring_kb,launches", [(80, 2), (70, None), (0, 2)])
 def test_a_large_vocabulary_leaves_the_ring_its_shared_memory(R, ring_kb, launches):
     """A CTA of the persistent kernel keeps its rows' partial sums (here 888 rows of the LM head) and the residual entries of its
-    few rows of the stream beside the ring.  70 KB hold both with two stages; 60 KB do not, and the token runs a kernel per
+    few rows of the stream beside the ring.  80 KB hold both with four stages; 70 KB do not, and the token runs a kernel per
     operator.  Same logits every way (sums in another order, a cache entry may round to its neighbour: 2e-4)."""
     cfg = R.Config(256, 640, 2, 128, 64, 2, 131072)
     m = R.Model.synthetic(cfg, 7, dtype="bf16", ring_kb=ring_kb, mega=True, use_graph=True)
@@ -530,3 +530,15 @@ def test_form_of_a_token_by_its_position(R, use_graph):
     assert auto.kernel_launches() - before == 1 + 8 * 2 + 8 * (5 * cfg.nlayers + 3)
     never.set_len(line - 8)
     assert np.array_equal(ids, never.decode_steps_greedy(5, 16))
+
+
+@pytest.mark.parametrize("hidden", [12544, 13312, 13824, 16384])
+def test_widest_rows_of_the_persistent_kernel(R, hidden):
+    """Seven and eight chunks a thread of W2's rows: as one kernel where four ring stages fit beside the L1 that its spilled registers need, else per operator."""
+    cfg = R.Config(2176, hidden, 17, 128, 64, 2, 1500)
+    a, b = (R.Model.synthetic(cfg, 3, dtype="bf16", mega=mega) for mega in (None, False))
+    before = a.kernel_launches()
+    for t in (7, 1499, 3):
+        x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
+        assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
+    assert (a.kernel_launches() - before == 6) == (hidden < 13800)

@@ -189,3 +189,16 @@ def test_fp8_zero_and_tiny_inputs(R, value, zero_gamma):
     assert np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
     x, y = a.decode_token_logits_from_id(11), b.decode_token_logits_from_id(11)
     assert np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("dim,hidden,vocab", [(1024, 4112, 1500), (512, 12304, 1500), (512, 16384, 1500), (4224, 15360, 1500), (512, 16384, 60000)])
+def test_fp8_chunks_per_thread(R, dim, hidden, vocab):
+    """The tilings of FP8 rows that the shapes above leave out: two, and four chunks a thread of W2's rows (all live at 16384).
+    Beside the sums of 60000 rows of the LM head a ring of four such stages does not fit: a kernel per operator."""
+    cfg = R.Config(dim, hidden, dim // 128, 128, 64, 2, vocab)
+    a, b = R.Model.synthetic(cfg, 3, dtype="fp8", mega=True), R.Model.synthetic(cfg, 3, dtype="fp8", mega=False)
+    before = a.kernel_launches()
+    for t in (7, 1499, 3):
+        x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
+        assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
+    assert (a.kernel_launches() - before == 6) == (vocab < 60000)
