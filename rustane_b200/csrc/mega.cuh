@@ -51,7 +51,7 @@ struct MegaLayer {
 
 constexpr int MEGA_MAX_PARTS = 64;  // partial attention results per head the buffers hold
 constexpr int MEGA_CPH_CAP = 8;     // CTAs that share a kv head: every CTA merges that many partials per head before Wo
-constexpr int MEGA_MAX_GQA = 8;     // q heads per kv head: 1, 2, 4 or 8 (a warp team works on one or two of them)
+constexpr int MEGA_MAX_GQA = 8;     // q heads per kv head: 1 or 2 (attention_phase), 4 or 8 (attention_grouped)
 
 struct MegaParams {
     const MegaLayer* layers;  // device array [nlayers]
@@ -80,7 +80,7 @@ struct MegaParams {
     TpLink tp;                  // tensor parallel (world > 1): the dimensions above are this rank's shard
     // byte offsets in dynamic shared memory, behind the ring: widest input vector, [rows_cap][8] partial sums, [2][resid_cap] residual
     // entries, page table, [nlayers] layer table, barriers.  (Offsets as kernel parameters and the rest of the CTA's scratch as
-    // static shared memory cost no registers; with a pointer each the GEMV loops spilled, and at 544 threads a CTA's spills
+    // static shared memory cost no registers; with a pointer each the GEMV loops spilled, and at 640 threads a CTA's spills
     // do not fit the L1 that the ring leaves.)
     uint32_t off_xs, off_partial, off_resid, off_pt, off_layers, off_bars;
     // one GPU: the vectors between phases as tagged words (tag_store); tparts: [heads][MEGA_CPH_CAP][hd + 2], max and sum last
@@ -356,8 +356,9 @@ __device__ inline void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t
 // lane (g, t) = lane / 4, lane % 4 puts its own weights of two rows into rows g and g + 8 of A and its own inputs into
 // column g of B, so the diagonal elements (g, g) and (g + 8, g) are the sums over the four lanes of quad g; the others are
 // not used.  The inputs are fp16 pairs hi + lo, rounded to nearest, of x times a power of two that brings the largest of
-// the vector to 2^14: 2^-24 of x, as fp32, or of what is 2^-24 of the largest.  Products are exact, sums fp32.
-// (5B model, one token: 1.60 ms, 1.85 ms with fp32 FMAs in a kernel per operator; error against 64 bits 3.6e-4 both.)
+// the vector to 2^14: off by at most 2^-23 of x (three of four fp32 values are exact), or by 2^-39 of the largest where that is
+// more.  Products are exact, sums fp32.  (5B model, one token: 1.60 ms, 1.85 ms with fp32 FMAs in a kernel per operator; error
+// against 64 bits 3.6e-4 both: the cache's rounding.)
 template <int NITER> struct Slices<Fp8Row, NITER> {
     static constexpr int EPC = 16;
     uint32_t hi[NITER][8], lo[NITER][8];
@@ -786,7 +787,7 @@ __device__ inline bool attention_inputs(const MegaParams& p, int h, bool newest,
 
 // ---- attention phase with 4 or 8 q heads per kv head and an fp16 cache.  Scores are a product with M = heads: rows 0-7 of
 // mma.m16n8k16 hold the heads' q rounded to fp16 (times a power of two that brings the largest to 2^14), rows 8-15 the
-// remainders, so one instruction gives both parts of eight positions' scores and no shuffle sums them up (the general
+// remainders (together within 2^-23 of q, as above), so one instruction gives both parts of eight positions' scores and no shuffle sums them up (the general
 // phase below spends 40 instructions per position and head on that: 15.6 us per layer of a 1B model at 2000 positions, 9.1 us
 // here; a token of it 0.88 ms, 0.91 ms with a kernel per operator).  A warp takes eight positions of a tile; its probabilities go through 128
 // bytes of shared memory to lanes that hold 16 bytes of a V row each, for four heads.  Warps 0-7 and 8-15 take alternate
@@ -917,7 +918,7 @@ __device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int at
         lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
         lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
         float* ls = probs_all + 16 * 8 * NH;  // [16 warps][NH] sums of the probabilities, then their maxima
-    float* mxs = ls + 16 * NH;
+        float* mxs = ls + 16 * NH;
         if (t == 0 && g < NH) mxs[warp * NH + g] = m;
         mega_bar();
         if (mega_aborted()) ok = false;
@@ -981,9 +982,8 @@ __device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int at
 }
 
 // ---- attention phase (sdpa_causal, lib.rs:1426-1489, for the tiles of this CTA).  All sixteen warps
-// work on every tile, in four teams of four warps.  A team takes GQ of the kv head's q heads; with more than that
-// (grouped queries) the teams divide the q heads first, and the teams of the same q heads divide a tile's positions:
-// 4 q heads: 2 x 2 teams, 8 q heads: 4 x 1.  LPT lanes hold one cached position's row as 16-byte chunks, 128 / LPT
+// work on every tile, in four teams of four warps that divide its positions; GQ is the number of q heads per kv head (a
+// template parameter, so that one head's state costs no registers when there is one).  LPT lanes hold one cached position's row as 16-byte chunks, 128 / LPT
 // positions side by side, UNR deep, with a running (max, sum, weighted V) per lane group and q head.  A warp copies its
 // rows of a tile to registers, releases the two ring slots (every warp arrives once on each) and computes while the next
 // tile lands; nothing but the ring's barriers orders the warps until the merge at the end.
@@ -998,8 +998,6 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
     const int HD = p.hd, LPT = HD / EPC, NG = 128 / LPT;
     const int g = tt / LPT, l = tt % LPT;
     const int T = p.tile_tokens, ntiles = (attn_len + T - 1) / T, pos = attn_len - 1;
-    const int gqa = p.gqa, qgroups = gqa / GQ;  // (GQ is a template parameter so that one head's state costs no registers when there is one)
-    const int qg = team % qgroups, slice = team / qgroups, nslices = MEGA_TEAMS / qgroups;
     const uint32_t row_bytes = (uint32_t)HD * sizeof(KT);
     const size_t head_stride = (size_t)p.page_tokens * HD, page_stride = (size_t)2 * p.kv_heads * head_stride;
     const KT* pool = reinterpret_cast<const KT*>(kv_pool);
@@ -1023,15 +1021,14 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                 lsum[qi] = 0.0f;
 #pragma unroll
                 for (int e = 0; e < EPC; ++e) acc[qi][e] = 0.0f;
-                const int hq = qg * GQ + qi;
 #pragma unroll
                 for (int e = 0; e < EPC; e += 4) {
-                    const float4 v = TAG ? *reinterpret_cast<const float4*>(sh.q + hq * HD + l * EPC + e)
-                                         : __ldcg(reinterpret_cast<const float4*>(p.q + (size_t)(h * gqa + hq) * HD + l * EPC + e));
+                    const float4 v = TAG ? *reinterpret_cast<const float4*>(sh.q + qi * HD + l * EPC + e)
+                                         : __ldcg(reinterpret_cast<const float4*>(p.q + (size_t)(h * GQ + qi) * HD + l * EPC + e));
                     qf[qi][e] = v.x; qf[qi][e + 1] = v.y; qf[qi][e + 2] = v.z; qf[qi][e + 3] = v.w;
                 }
             }
-            const int TQ = max(1, T / nslices);  // positions of a tile per team
+            const int TQ = max(1, T / MEGA_TEAMS);  // positions of a tile per team
             Ring at = ring;
             for (int idx = 0; idx < ncta_tiles; ++idx) {
                 if (!ok) break;  // this warp only: the others learn it from the abort flag behind the barrier below
@@ -1054,7 +1051,7 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                     bool live[UNR];
 #pragma unroll
                     for (int u = 0; u < UNR; ++u) {
-                        const int tq = tb + g + u * NG, ti = slice * TQ + tq, tok = tile * T + ti;
+                        const int tq = tb + g + u * NG, ti = team * TQ + tq, tok = tile * T + ti;
                         kw[u] = make_uint4(0, 0, 0, 0);
                         vw[u] = make_uint4(0, 0, 0, 0);
                         live[u] = tq < TQ && ti < T && tok < attn_len;
@@ -1148,35 +1145,31 @@ __device__ inline bool attention_phase(Ring& ring, const MegaParams& p, const vo
                 team_bar(team);
             }
             mega_bar();
-            for (int qi = team; qi < gqa; qi += MEGA_TEAMS) {  // team k merges the slices of q heads k, k + 4, ...
-                if (tt < HD) {
-                    const float* first = sh.tparts[qi / GQ][qi % GQ];  // slice k: team k * qgroups + qi / GQ
-                    const size_t step = (size_t)qgroups * 2 * (128 + 2);
-                    float M = NEG;
-                    for (int k = 0; k < nslices; ++k) {
-                        const float* tp = first + k * step;
-                        if (tp[129] > 0.0f) M = fmaxf(M, tp[128]);
+            if (team < GQ && tt < HD) {  // team k merges the teams' results of q head k
+                float M = NEG;
+                for (int k = 0; k < MEGA_TEAMS; ++k) {
+                    const float* tp = sh.tparts[k][team];
+                    if (tp[129] > 0.0f) M = fmaxf(M, tp[128]);
+                }
+                float L = 0.0f, a = 0.0f;
+                for (int k = 0; k < MEGA_TEAMS; ++k) {
+                    const float* tp = sh.tparts[k][team];
+                    if (tp[129] > 0.0f) {
+                        const float wgt = expf(tp[128] - M);
+                        L += tp[129] * wgt;
+                        a += tp[tt] * wgt;
                     }
-                    float L = 0.0f, a = 0.0f;
-                    for (int k = 0; k < nslices; ++k) {
-                        const float* tp = first + k * step;
-                        if (tp[129] > 0.0f) {
-                            const float wgt = expf(tp[128] - M);
-                            L += tp[129] * wgt;
-                            a += tp[tt] * wgt;
-                        }
-                    }
-                    if constexpr (TAG) {
-                        unsigned long long* o = p.tparts + ((size_t)(h * gqa + qi) * MEGA_CPH_CAP + plan.part) * (HD + 2);
-                        tag_store(o + tt, a, tag);
-                        if (tt < 2) tag_store(o + HD + tt, tt ? L : M, tag);
-                    } else {
-                        const size_t slot = (size_t)(h * gqa + qi) * MEGA_MAX_PARTS + plan.part;
-                        p.part_acc[slot * HD + tt] = a;
-                        if (tt == 0) {
-                            p.part_ml[slot * 2 + 0] = M;
-                            p.part_ml[slot * 2 + 1] = L;
-                        }
+                }
+                if constexpr (TAG) {
+                    unsigned long long* o = p.tparts + ((size_t)(h * GQ + team) * MEGA_CPH_CAP + plan.part) * (HD + 2);
+                    tag_store(o + tt, a, tag);
+                    if (tt < 2) tag_store(o + HD + tt, tt ? L : M, tag);
+                } else {
+                    const size_t slot = (size_t)(h * GQ + team) * MEGA_MAX_PARTS + plan.part;
+                    p.part_acc[slot * HD + tt] = a;
+                    if (tt == 0) {
+                        p.part_ml[slot * 2 + 0] = M;
+                        p.part_ml[slot * 2 + 1] = L;
                     }
                 }
             }

@@ -32,7 +32,7 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     const size_t xs_off = carve((size_t)xs_dim * 4), partial_off = carve((size_t)rows_cap * (GEMV_CONSUMERS / 32) * 4), resid_off = carve((size_t)2 * resid_cap * 4),
                  pt_off = carve((size_t)m->pages_per_seq * 4), layers_off = carve((size_t)c.nlayers * sizeof(MegaLayer)), bars_off = carve(2 * 16 * 8);
     // One GPU: all that a CTA can have (with 220 KB, as the kernels per operator use, hidden 11968 to 12288 had four stages, not six;
-    // 6 layers of 3648 x 11968, 40 positions, 493 and 458 us).  But eight chunks of W2's rows a thread spill 280 to 360 bytes of
+    // 6 layers of 3648 x 11968, 40 positions, 493 and 458 us).  But eight chunks of W2's rows a thread spill 200 to 360 bytes of
     // registers a thread, which the L1 holds as long as shared memory takes no more than 196 KB (60 KB of L1, 28 KB behind that): 5
     // layers of dim 4096, 1000 positions, here and per operator: hidden 13312 (195 KB) 520 and 562 us, 13824 (202 KB) 574 and 567 us.
     const size_t budget = (size_t)(TPAR || m->opt.test_ring_kb > 0 ? m->ring_kb : NH == 8 ? 195 : 227) * 1024;
@@ -74,7 +74,7 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     lc.dynamicSmemBytes = smem;
     lc.stream = m->stream;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident: they meet at grid barriers
+    at[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident: they wait for one another
     at[0].val.cooperative = 1;
     lc.attrs = at;
     lc.numAttrs = 1;

@@ -362,7 +362,7 @@ template <typename KT> struct PfEpiExpand {
     KT* expanded;
     AttnDims x;
     int nope;
-    __device__ void operator()(int, int row, int col, const float (&v)[32]) const {
+    __device__ void operator()(int row, int col, const float (&v)[32]) const {
         const int keys = x.H * nope;
         int h = col < keys ? col / nope : (col - keys) / x.vdim, d = col < keys ? col % nope : (col - keys) % x.vdim;
         bool key = col < keys;
@@ -398,7 +398,7 @@ template <typename AT, typename WT> struct PfEpiTokenGate {
     const WT* table;      // the layer's first column
     int table_ld, dim;
     const uint32_t* ids;
-    __device__ void operator()(int, int row, int col, const float (&v)[32]) const {
+    __device__ void operator()(int row, int col, const float (&v)[32]) const {
         const WT* e = table + (size_t)ids[row] * table_ld;
         float g[32];
         const bool run = col + 32 <= dim && table_ld % 8 == 0 && (reinterpret_cast<size_t>(table) & 15) == 0;

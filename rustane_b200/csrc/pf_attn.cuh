@@ -1,6 +1,8 @@
 // Attention of a prompt in one kernel (tcgen05): scores, causal / windowed softmax and the product with V never leave the
 // chip.  No batched counterpart in the reference (its decoder feeds prompt tokens one at a time, inference.rs:650-670); the
-// math is sdpa_fwd.rs:36-46, :325-354 restricted to the visible keys.
+// math is sdpa_fwd.rs:36-46, :325-354 restricted to the visible keys.  The method is FlashAttention (Dao et al. 2022) in the form
+// published for this architecture (FlashAttention-4): tiles of keys with a running softmax, two query tiles in turns, a reference
+// that is seldom raised.
 //
 // One CTA = 256 query rows of one head, as two tiles of 128 that take turns: while one tile's softmax runs on its four
 // warps, the tensor cores work on the other one.  Warps 0-3 / 4-7: softmax of tile 0 / 1, a query row per thread.

@@ -107,7 +107,7 @@ struct PfEpiPartial {  // the product y, raw (tensor parallel: this rank's parti
     float* y;
     int ld;
     int silu_cols = 0;  // the first columns go through silu
-    __device__ void operator()(int, int row, int col, const float (&v)[32]) const {
+    __device__ void operator()(int row, int col, const float (&v)[32]) const {
         float4* p = reinterpret_cast<float4*>(y + (size_t)row * ld + col);
         if (col < silu_cols) {
 #pragma unroll
@@ -123,7 +123,7 @@ struct PfEpiResidual {  // x += alpha * y on the fp32 residual stream
     float* x;
     int ld;
     float alpha;
-    __device__ void operator()(int, int row, int col, const float (&v)[32]) const {
+    __device__ void operator()(int row, int col, const float (&v)[32]) const {
         float4* p = reinterpret_cast<float4*>(x + (size_t)row * ld + col);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -162,7 +162,7 @@ template <typename T16> struct PfEpiGate {  // columns (2j, 2j+1) = (w1, w3) col
     T16* gate;
     T16* gate_lo;
     int ld, act;
-    __device__ void operator()(int, int row, int col, const float (&v)[32]) const {
+    __device__ void operator()(int row, int col, const float (&v)[32]) const {
         const size_t at = (size_t)row * ld + (col >> 1);
         float g[16];
 #pragma unroll
@@ -189,7 +189,7 @@ template <typename T16> struct PfEpiGate {  // columns (2j, 2j+1) = (w1, w3) col
 // RoPE on q and k; q to a [M, Q] buffer, k and v into the pages.  A thread's 32 columns lie inside one head (widths of 64 or
 // 128), so every destination is a run of 64 bytes: 16-byte stores.  (Element by element the epilogue bound the GEMM: 311 us
 // at 1024 x 12288 x 4096 where gate|up, 1.8 times the products, took 300; the 5B model's 1024-token prompt went from 30.5
-// to 25.9 ms, 4096 tokens from 147 to 131 ms, with this and PfEpiAttnOut.)
+// to 25.9 ms, 4096 tokens from 147 to 131 ms, with this and the same for the attention's output.)
 template <typename T16> struct PfEpiQKV {
     T16* q;
     T16* q_lo;
@@ -197,7 +197,7 @@ template <typename T16> struct PfEpiQKV {
     const int* page_table;
     const float2* rope;
     int Q, KV, hd, kv_heads, page_tokens, pos0;
-    __device__ void operator()(int, int row, int col, const float (&v)[32]) const {
+    __device__ void operator()(int row, int col, const float (&v)[32]) const {
         const int pos = pos0 + row;
         if (col < Q + KV) {
             float r[32];
@@ -322,7 +322,7 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
                     for (int i = 0; i < 32; ++i)
                         v[i] *= *reinterpret_cast<const float*>(p.qrows + (size_t)(n0 + c * 32 + i) * p.qstride + p.qscale_off);
                 }
-                if (row < p.M && n0 + c * 32 < p.N) epi(0, row, n0 + c * 32, v);
+                if (row < p.M && n0 + c * 32 < p.N) epi(row, n0 + c * 32, v);
             }
         }
     }

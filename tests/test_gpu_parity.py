@@ -448,7 +448,7 @@ GROUPED_CASES = [
 @pytest.mark.parametrize("dims,kv_heads,dtype,page,cached", GROUPED_CASES)
 def test_grouped_queries_on_the_persistent_kernel(R, dims, kv_heads, dtype, page, cached):
     """Four and eight q heads per kv head: scores on the tensor cores (q as fp16 hi + lo pairs) against the kernel per operator.
-    Inputs differ by 2^-24 relative, sums by their order; a cache entry may round to its neighbour: 2e-4 of the logits."""
+    Inputs differ by at most 2^-23 relative, sums by their order; a cache entry may round to its neighbour: 2e-4 of the logits."""
     dim, hidden, heads, hd, seq, layers, vocab = dims
     cfg = R.Config(dim, hidden, heads, hd, seq, layers, vocab, kv_heads=kv_heads)
     a, b = (R.Model.synthetic(cfg, 7, dtype=dtype, page_tokens=page, mega=mega) for mega in (True, False))

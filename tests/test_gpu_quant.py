@@ -158,7 +158,7 @@ def test_stored_quantised_checkpoint_loads_bit_identically(R, tmp_path, dtype):
 @pytest.mark.parametrize("dim,hidden,heads,hd,seq", [(256, 640, 4, 64, 64), (1024, 2832, 8, 128, 256), (512, 8208, 4, 128, 64), (4096 + 128, 8192, 33, 128, 64)])
 def test_fp8_persistent_kernel_matches_the_kernel_per_operator(R, dim, hidden, heads, hd, seq):
     """FP8 rows through the tensor cores (fp16 weights, inputs as hi + lo pairs, fp32 sums) against the same rows through fp32
-    FMAs: one to four chunks per thread, a ragged last chunk, rows that end inside a stage.  Inputs differ by 2^-24 relative and
+    FMAs: one to four chunks per thread, a ragged last chunk, rows that end inside a stage.  Inputs differ by at most 2^-23 relative and
     sums by their order: a few 1e-6 of logits of order one over two layers; an fp16 cache entry may round to its neighbour."""
     cfg = R.Config(dim, hidden, heads, hd, seq, 2, 1500)
     a, b = R.Model.synthetic(cfg, 3, dtype="fp8"), R.Model.synthetic(cfg, 3, dtype="fp8", mega=False)
