@@ -35,10 +35,15 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     // 6 layers of 3648 x 11968, 40 positions, 493 and 458 us).  But eight chunks of W2's rows a thread spill 200 to 360 bytes of
     // registers a thread, which the L1 holds as long as shared memory takes no more than 196 KB (60 KB of L1, 28 KB behind that): 5
     // layers of dim 4096, 1000 positions, here and per operator: hidden 13312 (195 KB) 520 and 562 us, 13824 (202 KB) 574 and 567 us.
-    const size_t budget = (size_t)(TPAR || m->opt.test_ring_kb > 0 ? m->ring_kb : NH == 8 ? 195 : 227) * 1024;
+    const size_t budget = TPAR || m->opt.test_ring_kb > 0 ? (size_t)m->ring_kb * 1024 : NH == 8 ? (size_t)195 * 1024 : m->smem_per_block;
+    // (MegaShared as the compiler laid it out: with sizeof in its place a ring that just fits asked for 96 bytes too many)
+    static const size_t fixed = [&] {
+        cudaFuncAttributes fa;
+        return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? (size_t)fa.sharedSizeBytes : sizeof(MegaShared) + 1024;
+    }();
     // (a ring of two stages loses to the kernels per operator: FP8, 5 layers of 4096 x 16384, 200 positions, 541 and 424 us)
-    if (sizeof(MegaShared) + off + (TPAR ? 2 : 4) * stage_cap > budget) return cudaErrorNotSupported;
-    const int nstages = (int)std::min<size_t>(16, (budget - sizeof(MegaShared) - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
+    if (fixed + off + (TPAR ? 2 : 4) * stage_cap > budget) return cudaErrorNotSupported;
+    const int nstages = (int)std::min<size_t>(16, (budget - fixed - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
     const size_t ring = (size_t)nstages * stage_cap, smem = ring + off;
     static size_t smem_set = 0;
     if (smem > smem_set) {

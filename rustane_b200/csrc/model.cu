@@ -180,6 +180,7 @@ int model_alloc(const cd_config* cfg, const cd_options& opts, int untied, const 
     cudaDeviceProp prop;
     CKB(cudaGetDeviceProperties(&prop, m->device));
     m->sm_count = prop.multiProcessorCount;
+    m->smem_per_block = prop.sharedMemPerBlockOptin;
     CKB(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     CKB(cudaEventCreate(&m->ev0));
     CKB(cudaEventCreate(&m->ev1));

@@ -135,6 +135,7 @@ struct cd_model {
     int untied = 0;
     int device = 0;
     int sm_count = 0;
+    size_t smem_per_block = 0;  // shared memory a block can have at most, static and dynamic
     int page_tokens = 64, pages_per_seq = 0, num_pages = 0, nsplit = 1;
     bool pdl = true;     // programmatic dependent launch between the kernels of a token
     int kv_dtype = 0;    // CD_DTYPE_F32 / F16 / BF16: storage of the KV cache (cd_options.kv_dtype resolved)

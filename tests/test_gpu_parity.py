@@ -542,3 +542,16 @@ def test_widest_rows_of_the_persistent_kernel(R, hidden):
         x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
         assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
     assert (a.kernel_launches() - before == 6) == (hidden < 13800)
+
+
+@pytest.mark.parametrize("dims,kv_heads,dtype", [((576, 1536, 8, 64, 4096, 13, 10303), 1, "bf16"), ((1664, 3328, 26, 64, 4096, 20, 300), 13, "fp8"),
+                                                 ((2624, 6208, 41, 64, 4096, 16, 2778), 41, "fp8")])
+def test_a_ring_that_just_fits(R, dims, kv_heads, dtype):
+    """Shapes whose stages, beside the other buffers, come within 100 bytes of the shared memory a block can have."""
+    cfg = R.Config(*dims, kv_heads=kv_heads)
+    a, b = (R.Model.synthetic(cfg, 3, dtype=dtype, mega=mega, use_graph=True) for mega in (True, False))
+    before = a.kernel_launches()
+    for t in (7, 299, 3):
+        x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
+        assert np.abs(x - y).max() < 1e-3 * np.abs(y).max()  # (up to 20 layers of caches that may round to the neighbour)
+    assert a.kernel_launches() - before == 6
