@@ -28,6 +28,7 @@
 namespace cd {
 
 constexpr int PA_KEYS = 128, PA_ROWS = 256, PA_THREADS = 384, PA_RING = 3;
+constexpr int PA_REGS = 256 * 216 + 128 * 72;  // registers of the split: what a block has to hold at launch
 enum { DEV_ERR_PA_WAIT = 11 };
 
 struct PfAttn {

@@ -80,7 +80,10 @@ cudaError_t pa_launch(cd_model* m, const CUtensorMap (&q)[2], bool split, const 
     constexpr size_t smem = PaSmem<KD, VD>::BYTES;
     static bool attr_set = false;  // per instantiation
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncAttributes fa;
+        cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+        if (e == cudaSuccess && fa.numRegs * PA_THREADS < PA_REGS) e = cudaErrorInvalidConfiguration;  // the warpgroups' split would wait for registers that the block does not have
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
