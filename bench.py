@@ -31,8 +31,8 @@ MODEL = dict(dim=4096, hidden=11008, heads=32, hd=128, seq=4096, nlayers=26, voc
 SEED, PROMPT_LEN, DECODE_TOKENS = 2, 1024, 512
 METRIC, UNIT = "decode_tokens_per_s", "tokens/s"
 # DRAM bytes moved per algorithmic byte by one launch of the persistent token kernel, from the ncu capture on the
-# 3-layer profile case (profiles/decode_mega_5b_profile_case.md): 1.5367 GB of DRAM traffic for 1.5271 GB algorithmic
-MEGA_TRAFFIC_RATIO = 1.006
+# 3-layer profile case (profiles/decode_mega_5b_profile_case.md): 1.5340 GB of DRAM traffic for 1.5271 GB algorithmic
+MEGA_TRAFFIC_RATIO = 1.0045
 WORKLOAD = ("config 3: 5B rustane LM bf16 (V32000 D4096 L26 32x128 H11008 seq4096), synthetic N(0,0.02) seed 2, "
             "1024-token random prompt, batch-1 greedy, 512 decode tokens per step")
 
