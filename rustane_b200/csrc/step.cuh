@@ -70,11 +70,13 @@ cudaError_t gemv_go(cd_model* m, const WT* W, const float* x, const float* gamma
             // never less than half an SM's shared memory: two of these CTAs (of consecutive kernels, under programmatic
             // dependent launch) on one SM measured 16 % slower per token and, rarely, gave run-to-run different logits
             const size_t smem = std::max((size_t)nstages * stage_bytes + fixed, (size_t)116 * 1024);
-            static size_t smem_set = 0;  // per instantiation
-            if (smem > smem_set) {
-                cudaError_t e = cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// (the same value from every family: each keeps a flag of its own for kernels they share, and the attribute is what was
+            // set last; ring_kb is at most 220)
+            static bool attr_set = false;  // per instantiation
+            if (!attr_set) {
+                cudaError_t e = cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
                 if (e != cudaSuccess) return e;
-                smem_set = smem;
+                attr_set = true;
             }
             cudaLaunchConfig_t lc = {};
             lc.gridDim = dim3(grid);
