@@ -44,22 +44,13 @@ struct Gemm {
     // C[M][N] = A[M][K] (head and, under split, remainder) * B[rows][K]^T through `epi`
     template <class Epi>
     void operator()(const char* name, const __nv_bfloat16* hi, const __nv_bfloat16* lo, const void* B, int M, int N, int K, size_t b_rows, const Epi& epi,
-                    const int* tile_group = nullptr, int group_rows = 0, size_t a_rows = 0) {
+                    const int* tile_group = nullptr, int group_rows = 0) {
         if (!ok()) return;
         what = name;
         PfGemm p = {};
         p.M = M; p.N = N; p.K = K; p.err = &m->st->error;
         p.tile_group = tile_group; p.group_rows = group_rows;
-        // tiles of 256 columns, of 128 where the wide ones would leave SMs without work
-        const int mt = (M + PF_BM - 1) / PF_BM;
-        const bool wide = (long)mt * ((N + 255) / 256) >= m->sm_count;
-        CUtensorMap a[2], b;
-        const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-        if (!a_rows) a_rows = (size_t)mt * PF_BM;
-        const bool maps = encode_2d(w->encode, &a[0], dt, hi, K, a_rows, (uint64_t)K * 2, PF_BM) && encode_2d(w->encode, &a[1], dt, split ? lo : hi, K, a_rows, (uint64_t)K * 2, PF_BM) &&
-                          encode_2d(w->encode, &b, dt, B, K, b_rows, (uint64_t)K * 2, wide ? 256 : 128);
-        if (!maps) { e = cudaErrorInvalidValue; return; }
-        e = wide ? pf_launch<256>(m, split, a, b, p, true, epi) : pf_launch<128>(m, split, a, b, p, true, epi);
+        e = pf_launch(m, w->encode, hi, split ? lo : nullptr, B, b_rows, p, true, epi);
     }
 };
 

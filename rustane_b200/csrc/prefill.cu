@@ -34,11 +34,10 @@ struct PrefillCtx {
     SampleGraphKey s_key;
     std::map<int, cudaGraphExec_t> s_graphs;  // captured multi-sample steps by number of occupied attention slices
     uint64_t s_graph_nodes = 0;
-    std::vector<CUtensorMap> w_qkv, w_o, w_13, w_2, k_pages, v_pages;  // per layer, built once
-    CUtensorMap w_head;
+    std::vector<CUtensorMap> k_pages, v_pages;  // per layer, built once
     std::vector<CUtensorMap> sk_qkv, sk_o, sk_13, sk_2;  // the same matrices in 128-row boxes (multi-sample decode)
     CUtensorMap sk_head;
-    // FP8 linears: one layer's four matrices widened to 16 bits before its GEMMs (the maps of every layer view these)
+    // FP8 linears: one layer's four matrices widened to 16 bits before its GEMMs
     void *f8_qkv = nullptr, *f8_o = nullptr, *f8_13 = nullptr, *f8_2 = nullptr;
     // multi-sample decode workspace (one arena, sized for s_cap samples)
     int s_cap = 0;
@@ -96,13 +95,12 @@ cudaError_t sk_launch(cd_model* m, bool split, const CUtensorMap& w, const CUten
 
 // weights, LM head and K pages: maps built once per model
 int ensure_weight_maps(cd_model* m, PrefillCtx* c, CUtensorMapDataType dt, CUtensorMapDataType kdt) {
-    if (!c->w_qkv.empty()) return CD_OK;
+    if (!c->k_pages.empty()) return CD_OK;
     const cd_config& cf = m->cfg;
     const int D = cf.dim, Q = cf.q_dim, KV = cf.kv_dim, H = cf.hidden;
-    c->w_qkv.resize(cf.nlayers); c->w_o.resize(cf.nlayers); c->w_13.resize(cf.nlayers); c->w_2.resize(cf.nlayers); c->k_pages.resize(cf.nlayers); c->v_pages.resize(cf.nlayers);
+    c->k_pages.resize(cf.nlayers); c->v_pages.resize(cf.nlayers);
     c->sk_qkv.resize(cf.nlayers); c->sk_o.resize(cf.nlayers); c->sk_13.resize(cf.nlayers); c->sk_2.resize(cf.nlayers);
-    bool ok = encode_2d(c->encode, &c->w_head, dt, m->lm_head, D, m->v_loc, (uint64_t)D * 2, 256) &&
-              encode_2d(c->encode, &c->sk_head, dt, m->lm_head, D, m->v_loc, (uint64_t)D * 2, 128);
+    bool ok = encode_2d(c->encode, &c->sk_head, dt, m->lm_head, D, m->v_loc, (uint64_t)D * 2, 128);
     auto pages = [&](int l) {
         return encode_pages(c, &c->k_pages[l], kdt, (const char*)m->layers[l].kv, 0, cf.hd, m->page_tokens, cf.kv_heads, m->num_pages) &&
                encode_pages(c, &c->v_pages[l], kdt, (const char*)m->layers[l].kv, 1, cf.hd, m->page_tokens, cf.kv_heads, m->num_pages);
@@ -111,17 +109,13 @@ int ensure_weight_maps(cd_model* m, PrefillCtx* c, CUtensorMapDataType dt, CUten
         const size_t n_qkv = (size_t)(Q + 2 * KV) * D, n_o = (size_t)D * Q, n_13 = (size_t)2 * H * D, n_2 = (size_t)D * H;
         if (cudaMalloc(&c->f8_qkv, n_qkv * 2) != cudaSuccess || cudaMalloc(&c->f8_o, n_o * 2) != cudaSuccess ||
             cudaMalloc(&c->f8_13, n_13 * 2) != cudaSuccess || cudaMalloc(&c->f8_2, n_2 * 2) != cudaSuccess) {
-            c->w_qkv.clear();
+            c->k_pages.clear();
             return fail(m, CD_ERR_CUDA, "prompt-pass buffers for the widened FP8 matrices");
         }
         for (int l = 0; l < cf.nlayers && ok; ++l) {
-            ok = ok && encode_2d(c->encode, &c->w_qkv[l], dt, c->f8_qkv, D, Q + 2 * KV, (uint64_t)D * 2, 256);
-            ok = ok && encode_2d(c->encode, &c->w_o[l], dt, c->f8_o, Q, D, (uint64_t)Q * 2, 256);
-            ok = ok && encode_2d(c->encode, &c->w_13[l], dt, c->f8_13, D, 2 * H, (uint64_t)D * 2, 256);
-            ok = ok && encode_2d(c->encode, &c->w_2[l], dt, c->f8_2, H, D, (uint64_t)H * 2, 256);
             ok = ok && pages(l);
         }
-        if (!ok) { c->w_qkv.clear(); return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for a weight matrix"); }
+        if (!ok) { c->k_pages.clear(); return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for a weight matrix"); }
         return CD_OK;
     }
     for (int l = 0; l < cf.nlayers && ok; ++l) {
@@ -130,13 +124,9 @@ int ensure_weight_maps(cd_model* m, PrefillCtx* c, CUtensorMapDataType dt, CUten
         ok = ok && encode_2d(c->encode, &c->sk_o[l], dt, L.wo, Q, D, (uint64_t)Q * 2, 128);
         ok = ok && encode_2d(c->encode, &c->sk_13[l], dt, L.w13, D, 2 * H, (uint64_t)D * 2, 128);
         ok = ok && encode_2d(c->encode, &c->sk_2[l], dt, L.w2, H, D, (uint64_t)H * 2, 128);
-        ok = ok && encode_2d(c->encode, &c->w_qkv[l], dt, L.wqkv, D, Q + 2 * KV, (uint64_t)D * 2, 256);
-        ok = ok && encode_2d(c->encode, &c->w_o[l], dt, L.wo, Q, D, (uint64_t)Q * 2, 256);
-        ok = ok && encode_2d(c->encode, &c->w_13[l], dt, L.w13, D, 2 * H, (uint64_t)D * 2, 256);
-        ok = ok && encode_2d(c->encode, &c->w_2[l], dt, L.w2, H, D, (uint64_t)H * 2, 256);
         ok = ok && pages(l);
     }
-    if (!ok) { c->w_qkv.clear(); return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for a weight matrix"); }
+    if (!ok) { c->k_pages.clear(); return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for a weight matrix"); }
     return CD_OK;
 }
 
@@ -198,12 +188,9 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
     T16* xn_lo = split ? xn + R * (size_t)std::max(D, Q) : nullptr;
     KT* q_lo = split ? qb + R * (size_t)Q : nullptr;
     T16* gate_lo = split ? gate + R * (size_t)H : nullptr;
-    CUtensorMap a_xn[2], a_attn[2], a_gate[2], a_q[2];
-    bool ok = true;
-    for (int h = 0; h < (split ? 2 : 1) && ok; ++h) {
-        ok = encode_2d(c->encode, &a_xn[h], dt, h ? xn_lo : xn, D, R, (uint64_t)D * 2, PF_BM) && encode_2d(c->encode, &a_attn[h], dt, h ? xn_lo : xn, Q, R, (uint64_t)Q * 2, PF_BM) &&
-             encode_2d(c->encode, &a_gate[h], dt, h ? gate_lo : gate, H, R, (uint64_t)H * 2, PF_BM) && encode_2d(c->encode, &a_q[h], kdt, h ? q_lo : qb, Q, R, (uint64_t)Q * 2, PF_BM);
-    }
+    CUtensorMap a_q[2];
+    const bool ok = encode_2d(c->encode, &a_q[0], kdt, qb, Q, R, (uint64_t)Q * 2, PF_BM) &&
+                    (!split || encode_2d(c->encode, &a_q[1], kdt, q_lo, Q, R, (uint64_t)Q * 2, PF_BM));
     if (!ok) return fail(m, CD_ERR_CUDA, "cuTensorMapEncodeTiled failed for an activation buffer");
 
     cudaError_t e;
@@ -249,7 +236,7 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
             PfGemm p = g; p.M = M; p.N = Q + 2 * KV; p.K = D;
             quantised(p, L.wqkv, D);
             PfEpiQKV<KT> epi{qb, q_lo, (KT*)L.kv, m->page_table, m->rope, Q, KV, hd, cf.kv_heads, m->page_tokens, pos0};
-            PF_TRY("qkv gemm", (pf_launch<256>(m, split, a_xn, c->w_qkv[l], p, bf16, epi)));
+            PF_TRY("qkv gemm", (pf_launch(m, c->encode, xn, xn_lo, fp8 ? c->f8_qkv : L.wqkv, Q + 2 * KV, p, bf16, epi)));
         }
         const PaOut<T16> attn_out{xn, xn_lo, Q, hd};
         if (hd == 128) PF_TRY("attention", (pa_launch<KT, 128, 128, false>(m, a_q, split, c->k_pages[l], c->v_pages[l], attn, cf.heads, attn_out)));
@@ -258,10 +245,10 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
             PfGemm p = g; p.M = M; p.N = D; p.K = Q;
             quantised(p, L.wo, Q);
             if (tpar) {
-                PF_TRY("wo gemm", (pf_launch<256>(m, split, a_attn, c->w_o[l], p, bf16, PfEpiPartial{tp_buf(), D})));
+                PF_TRY("wo gemm", (pf_launch(m, c->encode, xn, xn_lo, fp8 ? c->f8_o : L.wo, D, p, bf16, PfEpiPartial{tp_buf(), D})));
                 PF_TRY("wo all-reduce", tp_allreduce());
             } else {
-                PF_TRY("wo gemm", (pf_launch<256>(m, split, a_attn, c->w_o[l], p, bf16, PfEpiResidual{c->x, D, m->alpha})));
+                PF_TRY("wo gemm", (pf_launch(m, c->encode, xn, xn_lo, fp8 ? c->f8_o : L.wo, D, p, bf16, PfEpiResidual{c->x, D, m->alpha})));
             }
         }
         pf_rmsnorm_kernel<T16><<<M, 256, 0, m->stream>>>(c->x, L.gamma2, xn, xn_lo, D);
@@ -269,16 +256,16 @@ int run(cd_model* m, PrefillCtx* c, size_t n, bool split) {
         {   // gate = act(x2n W1) * (x2n W3)
             PfGemm p = g; p.M = M; p.N = 2 * H; p.K = D;
             quantised(p, L.w13, D);
-            PF_TRY("w13 gemm", (pf_launch<256>(m, split, a_xn, c->w_13[l], p, bf16, PfEpiGate<T16>{gate, gate_lo, H, m->opt.activation})));
+            PF_TRY("w13 gemm", (pf_launch(m, c->encode, xn, xn_lo, fp8 ? c->f8_13 : L.w13, 2 * H, p, bf16, PfEpiGate<T16>{gate, gate_lo, H, m->opt.activation})));
         }
         {   // x = x2 + alpha * (gate W2^T)
             PfGemm p = g; p.M = M; p.N = D; p.K = H;
             quantised(p, L.w2, H);
             if (tpar) {
-                PF_TRY("w2 gemm", (pf_launch<256>(m, split, a_gate, c->w_2[l], p, bf16, PfEpiPartial{tp_buf(), D})));
+                PF_TRY("w2 gemm", (pf_launch(m, c->encode, gate, gate_lo, fp8 ? c->f8_2 : L.w2, D, p, bf16, PfEpiPartial{tp_buf(), D})));
                 PF_TRY("w2 all-reduce", tp_allreduce());
             } else {
-                PF_TRY("w2 gemm", (pf_launch<256>(m, split, a_gate, c->w_2[l], p, bf16, PfEpiResidual{c->x, D, m->alpha})));
+                PF_TRY("w2 gemm", (pf_launch(m, c->encode, gate, gate_lo, fp8 ? c->f8_2 : L.w2, D, p, bf16, PfEpiResidual{c->x, D, m->alpha})));
             }
         }
     }

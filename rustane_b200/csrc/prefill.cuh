@@ -7,11 +7,19 @@
 // prompt pass in the reference's Metal decoder: it feeds prompt tokens one at a time
 // (inference.rs:650-670).
 //
-// One CTA = one 128 x BN output tile.  Warp 0: TMA producer (one thread).  Warp 1: owns the
-// tensor-memory allocation and issues the MMAs (one thread).  Warps 2-5: epilogue, each
-// reading the 32 accumulator lanes tcgen05.ld lets it see (lanes 32 * (warp % 4) ...).
-// Shared memory: a ring of NST stages, each a [128][64] A tile and a [BN][64] B tile of
-// 16-bit elements in the 128-byte-swizzled K-major layout TMA writes and the MMA reads.
+// A tile of the output is 128 CG rows x `bn` columns, CG = 1 or 2 CTAs.  As a pair (cta_group::2) each CTA stages its own 128
+// rows of A and half of the tile's rows of B, so B crosses L2 -> shared memory once for 256 rows; the even CTA issues the MMAs
+// of both.  CTAs are persistent (tiles in turn, row tiles fastest: neighbours share a weight tile in L2) and keep two
+// accumulators of 256 columns in tensor memory, so a tile's epilogue runs while the next tile is multiplied.
+// Warp 0: TMA producer (one thread).  Warp 1: owns the tensor-memory allocation and issues the MMAs (one thread).  Warps
+// 2-5: epilogue, each reading the 32 accumulator lanes tcgen05.ld lets it see (lanes 32 * (warp % 4) ...).
+// Shared memory: a ring of stages, each a [128][64] A tile (two under SPLIT) and a [bn / CG][64] B tile of 16-bit elements in
+// the 128-byte-swizzled K-major layout TMA writes and the MMA reads.
+// What bounds it: the tensor pipe (at hi + lo operands 256 columns take 1024 clocks of MMA for 48 KB a CTA).  One tile a CTA, one
+// accumulator and 256 columns a CTA of its own took 299, 173 and 96 us at 1024 rows x (22016, 12288 and, in the mean, 4096 features) of the 5B
+// model; this form 230, 130 and 88 us = 1600 TFLOP/s issued in the first.  At few rows the chain of a tile's MMAs
+// counts: with the loops of warps 0 and 1 in one thread each (their addresses not in uniform registers) a step of 64 along K took 890
+// clocks, as whole warps with one elected thread 624 (37 x 4096 x 4096: 36 and 27 us).
 // Every wait is bounded; on expiry the kernel records an error, skips its remaining
 // work, still meets the final barrier and frees its tensor memory.
 //
@@ -31,14 +39,13 @@ enum { DEV_ERR_PF_FULL = 8, DEV_ERR_PF_EMPTY = 9, DEV_ERR_PF_ACCUM = 10 };
 // SPLIT: the activation operand arrives as two 16-bit matrices hi + lo (lo = the rounding
 // error of hi, itself rounded), both multiplied with the same weight tile into the same
 // accumulator, so the product sees about 16 mantissa bits of the fp32 activation instead of 8.
-template <int BN, bool SPLIT> struct PfTile {
-    static constexpr uint32_t A_BYTES = PF_BM * PF_BK * 2, B_BYTES = BN * PF_BK * 2, STAGE = (SPLIT ? 2 : 1) * A_BYTES + B_BYTES;
-    static constexpr int NST = (192 * 1024) / STAGE > 6 ? 6 : (192 * 1024) / STAGE;
-    static constexpr size_t SMEM = (size_t)NST * STAGE + 1024 /* alignment slack */ + 256 /* barriers */;
-};
+constexpr uint32_t PF_A_BYTES = PF_BM * PF_BK * 2, PF_RING = 200 * 1024;
+constexpr int PF_MAX_STAGES = 8, PF_MAX_BN = 256;
+constexpr size_t PF_SMEM = PF_RING + 1024 /* alignment slack */ + 256 /* barriers */;
 
 struct PfGemm {
     int M, N, K;
+    int bn;  // columns of a tile: a multiple of 32, PF_MAX_BN at most
     int* err;
     // FP8 linears: B holds the e4m3 values widened to 16 bits; output column n is multiplied by the
     // row scale stored behind row n of the quantised matrix (Wfmt<Fp8Row>), nullptr otherwise
@@ -55,22 +62,72 @@ __device__ inline void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0,
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
-__device__ inline void tmem_alloc(uint32_t slot_smem, uint32_t ncols) {  // whole warp
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// one CTA of a pair: both of the pair's CTAs load into their own shared memory and count on the even CTA's barrier (no multicast)
+__device__ inline void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t leader_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(leader_bar), "r"(c0), "r"(c1) : "memory");
 }
-__device__ inline void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  // whole warp
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+template <int CG = 1> __device__ inline void tmem_alloc(uint32_t slot_smem, uint32_t ncols) {  // whole warp (of both CTAs of a pair)
+    if constexpr (CG == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+}
+template <int CG = 1> __device__ inline void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  // whole warp (of both CTAs of a pair)
+    if constexpr (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ inline void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ inline void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ inline void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+template <int CG = 1> __device__ inline void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (CG == 1)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ inline void umma_commit(uint32_t bar) {  // arrives on bar once every MMA issued so far has finished
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+// arrives on bar (CG = 2: on the barrier at this offset of both CTAs) once every MMA issued so far has finished
+template <int CG = 1> __device__ inline void umma_commit(uint32_t bar) {
+    if constexpr (CG == 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ inline bool elect_one() {  // true in one thread of a converged warp
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ inline uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ inline uint32_t cluster_addr(uint32_t addr, uint32_t rank) {  // the same shared-memory offset in CTA `rank` of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ inline void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ inline void mbar_arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// mbar_wait for a barrier that threads of the other CTA arrive on
+__device__ inline bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int limit = MBAR_WAIT_LIMIT) {
+    for (int i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
 }
 __device__ inline void tmem_ld32(uint32_t taddr, float (&v)[32]) {  // this lane's 32 consecutive accumulator columns
     uint32_t r[32];
@@ -127,7 +184,7 @@ struct PfEpiResidual {  // x += alpha * y on the fp32 residual stream
         float4* p = reinterpret_cast<float4*>(x + (size_t)row * ld + col);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            float4 t = p[i];
+            float4 t = __ldcg(p + i);
             t.x += alpha * v[4 * i]; t.y += alpha * v[4 * i + 1]; t.z += alpha * v[4 * i + 2]; t.w += alpha * v[4 * i + 3];
             p[i] = t;
         }
@@ -224,114 +281,166 @@ template <typename T16> struct PfEpiQKV {
 };
 
 // ------------------------------------------------------------------ the GEMM
-template <int BN, bool SPLIT, class Epi>
+template <int CG, bool SPLIT, class Epi>
 __global__ void __launch_bounds__(PF_THREADS, 1)
 pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_a_lo, const __grid_constant__ CUtensorMap tma_b,
                PfGemm p, uint32_t idesc, Epi epi) {
-    using TL = PfTile<BN, SPLIT>;
-    constexpr uint32_t B_OFF = (SPLIT ? 2 : 1) * TL::A_BYTES;  // stage = A hi | A lo (SPLIT) | B
-    constexpr int NST = TL::NST;
+    constexpr uint32_t B_OFF = (SPLIT ? 2 : 1) * PF_A_BYTES;  // stage = A hi | A lo (SPLIT) | B
     extern __shared__ unsigned char pf_raw[];
-    const int m0 = blockIdx.y * PF_BM, n0 = blockIdx.x * BN;
-    int b_row0 = n0;
-    if (p.tile_group != nullptr) {
-        const int g = p.tile_group[blockIdx.y];
-        if (g < 0) return;
-        b_row0 += g * p.group_rows;
-    }
+    const uint32_t rank = CG == 2 ? cluster_rank() : 0u;
+    const uint32_t stage = B_OFF + (uint32_t)(p.bn / CG) * PF_BK * 2;
+    const int nst = min(PF_MAX_STAGES, (int)(PF_RING / stage));
     const int nkb = (p.K + PF_BK - 1) / PF_BK;
+    const int tiles_m = (p.M + CG * PF_BM - 1) / (CG * PF_BM), tiles = tiles_m * ((p.N + p.bn - 1) / p.bn);
 
-    const uint32_t tiles = (smem_addr(pf_raw) + 1023u) & ~1023u;
-    const uint32_t bars = tiles + NST * TL::STAGE;
-    const uint32_t full0 = bars, empty0 = bars + 8u * NST, accum = bars + 16u * NST, slot = accum + 8u;
+    const uint32_t ring = (smem_addr(pf_raw) + 1023u) & ~1023u;
+    const uint32_t bars = ring + PF_RING;
+    const uint32_t full0 = bars, empty0 = full0 + 8u * PF_MAX_STAGES, accum0 = empty0 + 8u * PF_MAX_STAGES, drained0 = accum0 + 16u, slot = drained0 + 16u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NST; ++s) {
+        for (int s = 0; s < nst; ++s) {
             mbar_init(full0 + 8u * s, 1);
             mbar_init(empty0 + 8u * s, 1);
         }
-        mbar_init(accum, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(accum0 + 8u * b, 1);
+            mbar_init(drained0 + 8u * b, 4 * CG);  // one arrival per epilogue warp, those of both CTAs at the even one's
+        }
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(slot, BN);
+    if (warp == 1) tmem_alloc<CG>(slot, 2 * PF_MAX_BN);
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    if constexpr (CG == 2) cluster_sync();
+    else __syncthreads();
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(slot));
+    pdl_wait();  // under programmatic dependent launch: the operands and what the epilogue updates are the previous kernels'
+    pdl_launch_dependents();
     bool failed = false;
+    // whole warps wait and loop, one elected thread issues: addresses and descriptors stay in uniform registers
+    auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+        const bool ok = __all_sync(0xffffffffu, CG == 2 ? mbar_wait_cluster(bar, parity) : mbar_wait(bar, parity));
+        if (!ok) {
+            atomicExch(p.err, code);
+            failed = true;
+        }
+        return ok;
+    };
+    // the walk over this unit's tiles, the same in every role: first row (of the unit), first column, first row of B
+    auto at_tile = [&](int t, int& m0, int& n0, int& b0) {
+        const int mt = t % tiles_m;
+        m0 = mt * CG * PF_BM;
+        n0 = b0 = t / tiles_m * p.bn;
+        if (p.tile_group == nullptr) return true;
+        const int g = __ldcg(p.tile_group + mt);
+        b0 += g * p.group_rows;
+        return g >= 0;
+    };
+    const int unit = blockIdx.x / CG, units = gridDim.x / CG;
 
-    if (warp == 0) {
-        if (lane == 0) {  // ---- TMA producer
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int s = kb % NST;
-                if (kb >= NST && !mbar_wait(empty0 + 8u * s, ((kb / NST) - 1) & 1)) {
-                    atomicExch(p.err, DEV_ERR_PF_EMPTY);
-                    failed = true;
-                    break;
+    int s = 0, m0, n0, b0;
+    uint32_t ph = 0;  // ring position and its turn
+    auto next_stage = [&] {
+        if (++s == nst) { s = 0; ph ^= 1u; }
+    };
+    if (warp == 0) {  // ---- TMA producer
+        for (int t = unit; t < tiles && !failed; t += units) {
+            if (!at_tile(t, m0, n0, b0)) continue;
+            const int row = m0 + (int)rank * PF_BM, b_row = b0 + (int)rank * (p.bn / CG);
+            for (int kb = 0; kb < nkb; ++kb, next_stage()) {
+                if (!wait(empty0 + 8u * s, ph ^ 1u, DEV_ERR_PF_EMPTY)) break;
+                if (elect_one()) {
+                    const uint32_t a_dst = ring + s * stage, full = full0 + 8u * s;
+                    if (rank == 0) mbar_arrive_expect_tx(full, CG * stage);
+                    if constexpr (CG == 2) {
+                        const uint32_t bar = cluster_addr(full, 0);
+                        tma_load_2d_pair(a_dst, &tma_a, kb * PF_BK, row, bar);
+                        if (SPLIT) tma_load_2d_pair(a_dst + PF_A_BYTES, &tma_a_lo, kb * PF_BK, row, bar);
+                        tma_load_2d_pair(a_dst + B_OFF, &tma_b, kb * PF_BK, b_row, bar);
+                    } else {
+                        tma_load_2d(a_dst, &tma_a, kb * PF_BK, row, full);
+                        if (SPLIT) tma_load_2d(a_dst + PF_A_BYTES, &tma_a_lo, kb * PF_BK, row, full);
+                        tma_load_2d(a_dst + B_OFF, &tma_b, kb * PF_BK, b_row, full);
+                    }
                 }
-                const uint32_t a_dst = tiles + s * TL::STAGE, b_dst = a_dst + B_OFF;
-                mbar_arrive_expect_tx(full0 + 8u * s, TL::STAGE);
-                tma_load_2d(a_dst, &tma_a, kb * PF_BK, m0, full0 + 8u * s);
-                if (SPLIT) tma_load_2d(a_dst + TL::A_BYTES, &tma_a_lo, kb * PF_BK, m0, full0 + 8u * s);
-                tma_load_2d(b_dst, &tma_b, kb * PF_BK, b_row0, full0 + 8u * s);
+                __syncwarp();
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0) {  // ---- MMA issuer
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int s = kb % NST;
-                if (!mbar_wait(full0 + 8u * s, (kb / NST) & 1)) {
-                    atomicExch(p.err, DEV_ERR_PF_FULL);
-                    failed = true;
-                    break;
-                }
+        // the last stages are read before this CTA leaves: nothing arrives on its barriers afterwards
+        for (int k = 0; k < nst && !failed; ++k, next_stage()) wait(empty0 + 8u * s, ph ^ 1u, DEV_ERR_PF_EMPTY);
+    } else if (warp == 1) {  // ---- MMA issuer
+        int j = 0;
+        for (int t = unit; rank == 0 && t < tiles && !failed && nkb > 0; t += units) {
+            if (!at_tile(t, m0, n0, b0)) continue;
+            const uint32_t buf = j & 1, acc = tmem_base + buf * PF_MAX_BN;
+            if (!wait(drained0 + 8u * buf, ((j >> 1) & 1) ^ 1u, DEV_ERR_PF_ACCUM)) break;
+            tc_fence_after();
+            for (int kb = 0; kb < nkb; ++kb, next_stage()) {
+                if (!wait(full0 + 8u * s, ph, DEV_ERR_PF_FULL)) break;
                 tc_fence_after();
-                const uint64_t adesc = umma_desc(tiles + s * TL::STAGE), bdesc = umma_desc(tiles + s * TL::STAGE + B_OFF);
-                const uint64_t ldesc = umma_desc(tiles + s * TL::STAGE + TL::A_BYTES);
+                if (elect_one()) {
+                    const uint32_t base = ring + s * stage;
+                    const uint64_t adesc = umma_desc(base), ldesc = umma_desc(base + PF_A_BYTES), bdesc = umma_desc(base + B_OFF);
 #pragma unroll
-                for (int k = 0; k < PF_BK / 16; ++k) {  // 16 elements = 32 bytes further along K inside the swizzle span
-                    umma_f16(tmem_base, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0);
-                    if (SPLIT) umma_f16(tmem_base, ldesc + 2u * k, bdesc + 2u * k, idesc, 1u);
+                    for (int k = 0; k < PF_BK / 16; ++k) {  // 16 elements = 32 bytes further along K inside the swizzle span
+                        umma_f16<CG>(acc, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0);
+                        if (SPLIT) umma_f16<CG>(acc, ldesc + 2u * k, bdesc + 2u * k, idesc, 1u);
+                    }
+                    umma_commit<CG>(empty0 + 8u * s);  // the stage may be refilled once these MMAs have read it
+                    if (kb == nkb - 1) umma_commit<CG>(accum0 + 8u * buf);
                 }
-                umma_commit(empty0 + 8u * s);  // the stage may be refilled once these MMAs have read it
+                __syncwarp();
             }
-            if (!failed) umma_commit(accum);
+            ++j;
         }
     } else {  // ---- epilogue warps
         const int lane_base = (warp & 3) * 32;
-        const int row = m0 + lane_base + lane;
-        if (nkb > 0 && !mbar_wait(accum, 0)) {
-            atomicExch(p.err, DEV_ERR_PF_ACCUM);
-            failed = true;
-        }
-        if (!failed) {
+        int j = 0;
+        for (int t = unit; t < tiles && !failed; t += units) {
+            if (!at_tile(t, m0, n0, b0)) continue;
+            const uint32_t buf = j & 1, acc = tmem_base + buf * PF_MAX_BN + ((uint32_t)lane_base << 16);
+            const int row = m0 + (int)rank * PF_BM + lane_base + lane;
+            if (nkb > 0 && !wait(accum0 + 8u * buf, (j >> 1) & 1, DEV_ERR_PF_ACCUM)) break;
             tc_fence_after();
+            const int chunks = min(p.bn, p.N - n0 + 31) / 32;
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
+            for (int c = 0; c < chunks; ++c) {
                 float v[32];
                 if (nkb > 0) {
-                    tmem_ld32(tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)c * 32u, v);
+                    tmem_ld32(acc + (uint32_t)c * 32u, v);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = 0.0f;
                 }
-                if (p.qrows != nullptr && n0 + c * 32 < p.N) {
+                if (c == chunks - 1) {  // the accumulator may be overwritten
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if constexpr (CG == 2) mbar_arrive_cluster(cluster_addr(drained0 + 8u * buf, 0));
+                        else mbar_arrive(drained0 + 8u * buf);
+                    }
+                }
+                if (p.qrows != nullptr) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
                         v[i] *= *reinterpret_cast<const float*>(p.qrows + (size_t)(n0 + c * 32 + i) * p.qstride + p.qscale_off);
                 }
-                if (row < p.M && n0 + c * 32 < p.N) epi(row, n0 + c * 32, v);
+                if (row < p.M) epi(row, n0 + c * 32, v);
             }
+            ++j;
         }
     }
     if (__any_sync(0xffffffffu, failed)) {  // give copies that may still be in flight time to land before the CTA leaves
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
     }
     tc_fence_before();
-    __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, BN);
+    if constexpr (CG == 2) cluster_sync();
+    else __syncthreads();
+    if (warp == 1) tmem_dealloc<CG>(tmem_base, 2 * PF_MAX_BN);
+    if constexpr (CG == 2) cluster_sync();
 }
 
 // ------------------------------------------------------------------ the GEMM for a handful of rows

@@ -152,3 +152,15 @@ def test_attention_at_the_edges_of_its_tiles(R, oracle, hd, kv_heads, page, cach
     if cached:
         gm.prefill(prompt[:cached], want_logits=False)
     assert float(np.abs(gm.prefill(prompt[cached:]) - ref).max()) < SPLIT_TOL
+
+
+@pytest.mark.parametrize("mode", ["split", "fast"])
+@pytest.mark.parametrize("n,hidden", [(40, 48), (128, 9616), (129, 9616), (300, 11008), (1030, 9616)])
+def test_tiles_of_the_linears(R, oracle, n, hidden, mode):
+    """Tiles of one CTA and of a pair, several of them in turn on one unit (both accumulators used again), with a last row tile
+    of one row or of one of the pair's halves, and columns that end inside a tile."""
+    oc, om, gm = _models(R, oracle, (160, hidden, 2, 64, 1100, 1, 300), "bf16", {})
+    prompt = oracle.synth_prompt(11, oc.vocab, n)
+    _, ref = _oracle_prefill(oracle, om, prompt)
+    os.environ["CD_PREFILL"] = mode
+    assert float(np.abs(gm.prefill(prompt) - ref).max()) < (SPLIT_TOL if mode == "split" else LOGIT_TOL)
