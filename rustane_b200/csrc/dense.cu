@@ -48,14 +48,11 @@ cudaError_t enqueue_step_t(cd_model* m, const cd_step& p) {
         next_prompt_kernel<<<1, 1, 0, m->stream>>>(m->st, m->prompt_dev);
         count_launch(m);
     }
-    constexpr bool has_mega = !std::is_same<LT, Int4G32>::value;
-    bool use_mega = has_mega && p.one_kernel && m->mega;
-    if constexpr (has_mega) {
-        if (use_mega) {
-            e = launch_mega<WT, LT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0);
-            if (e == cudaErrorNotSupported) m->mega = use_mega = false;  // its buffers do not fit this model's shared memory: nothing was launched
-            else if (e != cudaSuccess) return e;
-        }
+    bool use_mega = p.one_kernel && m->mega;
+    if (use_mega) {
+        e = launch_mega<WT, LT, KT>(m, p.input >= 1 ? 1 : 0, p.head != HEAD_NONE ? 1 : 0);
+        if (e == cudaErrorNotSupported) m->mega = use_mega = false;  // its buffers do not fit this model's shared memory: nothing was launched
+        else if (e != cudaSuccess) return e;
     }
     if (!use_mega && p.input >= 1) {
         embed_kernel<WT><<<std::max(1, c.dim / 256), 256, 0, m->stream>>>((const WT*)m->embed, m->st, m->x_a, c.dim, m->full_cfg.vocab);
@@ -142,7 +139,7 @@ static int validate(const cd_config& c, int dtype) {
 // which walk their tiles of it one after the other: 0.5 us a tile, 1 to 1.2 with 2 or 4 q heads per kv head, 1.9 with 8.  The kernel
 // per operator spreads q heads times up to 32 slices.  Over 270 shapes (dim 512 to 4096; f32, 16 bits, FP8; 1 to 8 q heads per
 // kv head; 40 to 3500 positions) the tiles at which the two meet grow with the bytes of a layer's weights, as below; the choice
-// is within 0.2 % of the better form in the mean.  Us a token of 8 layers, persistent and per operator: dim 1024 in bf16, 8 q heads
+// is within 0.2 % of the better form in the mean, 0.7 % over 76 cells of INT4.  Us a token of 8 layers, persistent and per operator: dim 1024 in bf16, 8 q heads
 // on one kv head, 64 positions 200 and 219, 1000 positions 256 and 222 (limit 490); dim 2048, 16 on 4, 1000 positions 279 and 317
 // (limit 5600).  Grouped heads of small layers: 0.90 to 1.05 of the other's speed at any length.
 static size_t persistent_positions(const cd_model* m, size_t layer_bytes) {
@@ -153,7 +150,7 @@ static size_t persistent_positions(const cd_model* m, size_t layer_bytes) {
     if (mb < line.none_below_mb) return 0;
     const int dt = m->opt.weight_dtype;
     const size_t head_row = (size_t)c.dim * (dt == CD_DTYPE_F32 ? 4 : 2), cached_row = (size_t)c.hd * (m->kv_dtype == CD_DTYPE_F32 ? 4 : 2);
-    const size_t stage = mega_stage_bytes(m->mega_nd, m->mega_nh, is_quant(dt), lin_row_bytes(dt, std::max(c.dim, c.q_dim)), lin_row_bytes(dt, c.hidden), head_row);
+    const size_t stage = mega_stage_bytes(m->mega_nd, m->mega_nh, dt == CD_DTYPE_INT4_G32 ? MEGA_INT4 : dt == CD_DTYPE_FP8_E4M3 ? MEGA_FP8 : MEGA_PLAIN, lin_row_bytes(dt, std::max(c.dim, c.q_dim)), lin_row_bytes(dt, c.hidden), head_row);
     const double ctas_per_head = c.kv_heads <= m->sm_count ? std::min(m->sm_count / c.kv_heads, MEGA_CPH_CAP) : 1.0 / ((c.kv_heads + m->sm_count - 1) / m->sm_count);
     return (size_t)((line.tiles + line.per_mb * mb) * mega_tile_tokens(m->page_tokens, cached_row, stage) * ctas_per_head);
 }
@@ -229,15 +226,15 @@ int dense_alloc(const cd_config* cfg, const cd_options* opts_in, int untied, cd_
         }
         CKB(cudaMemcpyAsync(m->mega_layers, ml.data(), ml.size() * sizeof(MegaLayer), cudaMemcpyHostToDevice, m->stream));
         CKB(cudaStreamSynchronize(m->stream));
-        const int epc = dt == CD_DTYPE_F32 ? 4 : dt == CD_DTYPE_FP8_E4M3 ? 16 : 8;
+        const int epc = dt == CD_DTYPE_F32 ? 4 : is_quant(dt) ? 16 : 8;
         const int nd = (std::max(c.dim, c.q_dim) / epc + 255) / 256, nh = (c.hidden / epc + 255) / 256, g = c.gqa_ratio;
         // (c is this rank's shard under tensor parallelism: hidden and q_dim shrink, dim does not)
         const bool combo = tpw > 1 ? ((nd == 1 && (nh == 1 || nh == 2)) || (nd == 2 && nh >= 3 && nh <= 6)) && c.q_dim <= c.dim && g <= 2
-                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= (dt == CD_DTYPE_FP8_E4M3 ? 4 : 8))) && (g == 1 || g == 2 || ((g == 4 || g == MEGA_MAX_GQA) && m->kv_dtype == CD_DTYPE_F16));
-        if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 && dt != CD_DTYPE_FP8_E4M3 ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
+                                   : ((nd == 1 && nh <= 4) || (nd == 2 && nh <= (is_quant(dt) ? 4 : 8))) && (g == 1 || g == 2 || ((g == 4 || g == MEGA_MAX_GQA) && m->kv_dtype == CD_DTYPE_F16));
+        if (combo) { m->mega_nd = nd; m->mega_nh = nd == 1 ? (nh == 3 && !is_quant(dt) ? 4 : nh) : nh <= 4 ? 4 : nh <= 6 ? 6 : 8; }
         // tensor parallel: measured on the 5B model, the persistent kernel wins at 2 ranks (601 against 569 tokens/s) and
         // loses at 8 (841 against 896), where a layer's data are 8 us and its fixed per-phase times dominate either way
-        const bool mega_ok = dt != CD_DTYPE_INT4_G32 && (tpw == 1 || (tpw == 2 && dt != CD_DTYPE_F32 && !is_quant(dt)));
+        const bool mega_ok = tpw == 1 || (tpw == 2 && dt != CD_DTYPE_F32 && !is_quant(dt));
         // one persistent kernel per token where its tiling covers the shape; test_flags bit 1 keeps one kernel per operator, bit 4
         // takes the persistent one whatever the length
         m->mega = (opts.test_flags & 2) == 0 && mega_ok && m->mega_nd > 0;

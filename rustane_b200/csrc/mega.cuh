@@ -324,14 +324,35 @@ __device__ __noinline__ void stage_first_input(const MegaParams& p, float* xs) {
     mega_bar();
 }
 
+template <typename LT> struct RowChunks {  // this thread's 16-byte chunks of a stage's rows
+    uint32_t base, row_bytes;
+    int nchunks;
+    __device__ uint4 operator()(int j, int i) const {
+        const int c = (threadIdx.x & 255) + i * GEMV_CONSUMERS;
+        return c < nchunks ? lds128(base + (uint32_t)j * row_bytes + (uint32_t)c * 16u) : make_uint4(0, 0, 0, 0);
+    }
+};
+// a pair of fp32 values as fp16 hi + lo
+__device__ inline void fp16_pair(uint32_t& h, uint32_t& l, float a, float b) {
+    const __half2 p = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(p);
+    const __half2 q = __floats2half2_rn(isfinite(f.x) ? a - f.x : 0.0f, isfinite(f.y) ? b - f.y : 0.0f);
+    h = *reinterpret_cast<const uint32_t*>(&p);
+    l = *reinterpret_cast<const uint32_t*>(&q);
+}
+__device__ inline void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 // ---- the input slice a thread holds (chunks tid, tid + 256, ... of the vector, the same in both groups), and the rows of
 // a stage times it
 template <typename LT, int NITER> struct Slices {
     static constexpr int EPC = Wfmt<LT>::EPC;
     float x[NITER][EPC];
     __device__ void set(int i, int e, float4 v) { x[i][e] = v.x; x[i][e + 1] = v.y; x[i][e + 2] = v.z; x[i][e + 3] = v.w; }
-    // load(j, i): chunk i of row j; all of them are in registers when release() hands the stage back
-    template <int R, class Load, class Release> __device__ void rows(const Load& load, const Release& release, float (&acc)[R]) const {
+    // chunk i of row j of the stage at `base`; all of them are in registers when release() hands the stage back
+    template <int R, class Release> __device__ void rows(uint32_t base, uint32_t row_bytes, int K, const Release& release, float (&acc)[R]) const {
+        const RowChunks<LT> load{base, row_bytes, K / EPC};
         uint4 w[R][NITER];
 #pragma unroll
         for (int j = 0; j < R; ++j)
@@ -347,59 +368,165 @@ template <typename LT, int NITER> struct Slices {
         }
     }
 };
-__device__ inline void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// FP8 rows: the bytes widen to fp16 pairs exactly, and mma.m16n8k16 does what an fp32 FMA per weight did (with its
-// conversions two instructions per weight: the decoder was bound by issue slots, not by HBM).  Chunks stay where they are:
-// lane (g, t) = lane / 4, lane % 4 puts its own weights of two rows into rows g and g + 8 of A and its own inputs into
-// column g of B, so the diagonal elements (g, g) and (g + 8, g) are the sums over the four lanes of quad g; the others are
-// not used.  The inputs are fp16 pairs hi + lo, rounded to nearest, of x times a power of two that brings the largest of
+// Quantised rows on the tensor cores (mma.m16n8k16; with an fp32 FMA per weight the decoder was bound by issue slots).  Weights
+// widen to fp16 exactly; inputs are fp16 pairs hi + lo, rounded to nearest, of x times a power of two that brings the largest of
 // the vector to 2^14: off by at most 2^-23 of x (three of four fp32 values are exact), or by 2^-39 of the largest where that is
-// more.  Products are exact, sums fp32.  (5B model, one token: 1.60 ms, 1.85 ms with fp32 FMAs in a kernel per operator; error
-// against 64 bits 3.6e-4 both: the cache's rounding.)
-template <int NITER> struct Slices<Fp8Row, NITER> {
-    static constexpr int EPC = 16;
-    uint32_t hi[NITER][8], lo[NITER][8];
-    __device__ void set(int i, int e, float4 v) {
-        pair(hi[i][e / 2], lo[i][e / 2], v.x, v.y);
-        pair(hi[i][e / 2 + 1], lo[i][e / 2 + 1], v.z, v.w);
+// more.  Products are exact, sums fp32.  Chunks stay where they are in the row: lane (g, t) = lane / 4, lane % 4 puts its own
+// weights of two matrix rows into rows g and g + 8 of A: quad g holds chunk g % 4 of rows j + g / 4 and j + 2 + g / 4.  Column
+// 2 c of B is the hi, 2 c + 1 the lo part of chunk c's inputs, so that element (g, 2 (g % 4)) + (g, 2 (g % 4) + 1), which lane
+// t = g % 4 holds, is the sum over quad g's chunk; the others are not used.  256 weights per MMA; two MMAs for hi and lo over
+// eight chunks of two rows (128 weights each) took 15.4 us for the 90 MB of the 5B model's W1|W3 in FP8, HBM 14 us.
+struct QuantLane {
+    static __device__ int warp() { return (threadIdx.x & 255) >> 5; }
+    static __device__ int g() { return (threadIdx.x & 31) >> 2; }
+    static __device__ int t() { return threadIdx.x & 3; }
+    // the quad's sums of an MMA's result d, rows j .. j + 3 (or two of them), into acc: lanes that hold none add zero
+    template <int R> static __device__ void take(int j, float lower, float upper, float (&acc)[R]) {
+        const bool mine = t() == (g() & 3), second = g() >= 4;
+        acc[j] = mine && !second ? lower : 0.0f;
+        acc[j + 1] = mine && second ? lower : 0.0f;
+        if (R > 2) {
+            acc[R > 2 ? j + 2 : 0] = mine && !second ? upper : 0.0f;
+            acc[R > 2 ? j + 3 : 0] = mine && second ? upper : 0.0f;
+        }
     }
-    __device__ static void pair(uint32_t& h, uint32_t& l, float a, float b) {
-        const __half2 p = __floats2half2_rn(a, b);
-        const float2 f = __half22float2(p);
-        const __half2 q = __floats2half2_rn(isfinite(f.x) ? a - f.x : 0.0f, isfinite(f.y) ? b - f.y : 0.0f);
-        h = *reinterpret_cast<const uint32_t*>(&p);
-        l = *reinterpret_cast<const uint32_t*>(&q);
+    // the hi (even columns) or lo part of two inputs
+    static __device__ uint32_t part(float a, float b) {
+        uint32_t h, l;
+        fp16_pair(h, l, a, b);
+        return g() & 1 ? l : h;
+    }
+};
+// FP8: a chunk is 64 bytes, 16 a lane
+template <int NITER> struct Slices<Fp8Row, NITER> {
+    static constexpr int STEPS = 2 * NITER;
+    uint32_t x[STEPS][8];
+    __device__ static int lane_chunk(int i, int c) { return ((i * (GEMV_CONSUMERS / 32) + QuantLane::warp()) * 4 + c) * 4 + QuantLane::t(); }
+    __device__ void fill(const float* xs, float inv, float up, int K) {
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const int at = 16 * lane_chunk(i, QuantLane::g() >> 1);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 v = at < K ? *reinterpret_cast<const float4*>(xs + at + 4 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[i][2 * e] = QuantLane::part(v.x * inv * up, v.y * inv * up);
+                x[i][2 * e + 1] = QuantLane::part(v.z * inv * up, v.w * inv * up);
+            }
+        }
     }
     __device__ static uint32_t widen(uint32_t two) {
         const __half2 h(__nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)two, __NV_E4M3));
         return *reinterpret_cast<const uint32_t*>(&h);
     }
-    // (two chunks at a time: the inputs take the registers that holding a whole stage would need)
-    template <int R, class Load, class Release> __device__ void rows(const Load& load, const Release& release, float (&acc)[R]) const {
-        static_assert(R % 2 == 0, "rows come in pairs");
-        const int lane = threadIdx.x & 31, g = lane >> 2;
+    template <int R, class Release> __device__ void rows(uint32_t base, uint32_t row_bytes, int K, const Release& release, float (&acc)[R]) const {
+        static_assert(R == 2 || R == 4, "two or four rows");
+        float d[2][4] = {};
 #pragma unroll
-        for (int j = 0; j < R; j += 2) {
-            float dh[4] = {0.f, 0.f, 0.f, 0.f}, dl[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int i = 0; i < NITER; ++i) {
-                const uint4 w0 = load(j, i), w1 = load(j + 1, i);
-                const uint32_t u[4] = {w0.x, w0.y, w0.z, w0.w}, v[4] = {w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint32_t a0 = widen(u[k] & 0xffffu), a1 = widen(v[k] & 0xffffu), a2 = widen(u[k] >> 16), a3 = widen(v[k] >> 16);
-                    mma_f16(dh, a0, a1, a2, a3, hi[i][2 * k], hi[i][2 * k + 1]);
-                    mma_f16(dl, a0, a1, a2, a3, lo[i][2 * k], lo[i][2 * k + 1]);
-                }
+        for (int i = 0; i < STEPS; ++i) {
+            const int c = lane_chunk(i, QuantLane::g() & 3);
+            const uint32_t at = base + (uint32_t)(QuantLane::g() >> 2) * row_bytes + (uint32_t)c * 16u;
+            uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
+            if (16 * c < K) {
+                w0 = lds128(at);
+                if (R == 4) w1 = lds128(at + 2u * row_bytes);
             }
-            const bool diagonal = (lane & 3) == (g >> 1), odd = g & 1;
-            acc[j] = diagonal ? (odd ? dh[1] + dl[1] : dh[0] + dl[0]) : 0.0f;
-            acc[j + 1] = diagonal ? (odd ? dh[3] + dl[3] : dh[2] + dl[2]) : 0.0f;
+            const uint32_t u[4] = {w0.x, w0.y, w0.z, w0.w}, v[4] = {w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                mma_f16(d[k & 1], widen(u[k] & 0xffffu), R == 4 ? widen(v[k] & 0xffffu) : 0u, widen(u[k] >> 16), R == 4 ? widen(v[k] >> 16) : 0u, x[i][2 * k], x[i][2 * k + 1]);
         }
         release();
+        QuantLane::take<R>(0, (d[0][0] + d[0][1]) + (d[1][0] + d[1][1]), (d[0][2] + d[0][3]) + (d[1][2] + d[1][3]), acc);
+    }
+};
+// INT4 (groups of 32 with one fp16 scale): a chunk is a group, 4 bytes a lane; its sum times the group's scale in fp32.  A pair
+// of nibbles n = q + 8 masked out of its word is a pair of fp16 subnormals n 2^-24, exactly, or n 2^-20 where they lie four bits
+// up (their inputs carry the missing 2^-4); the sums start at -8 of the inputs', which two MMAs with a constant make for all rows
+// of the stage.  Bound by issue slots: with 1024 + n - 1032 for each pair, and a step's loads right ahead of their use, the 50
+// MB of the 5B model's W1|W3 took 18.0 us.
+template <int NITER> struct Slices<Int4G32, NITER> {
+    // Steps whose words are loaded ahead of the first one's product.  NEAR: a warp takes 16 groups at a time and quad c four
+    // neighbours, whose scales are one load, in an order of its own, so that the words of the four quads lie in different banks
+    // (W1|W3 14.8 us, 16.2 without).  Longer rows take groups one by one: W2's 11008 inputs are not a whole number of sixteens a
+    // warp, and the registers do not last (12.9 us against 10.5).
+    static constexpr int STEPS = 4 * NITER, BATCH = 4, NEAR = NITER == 1 ? 4 : 1;
+    uint32_t x[STEPS][4];
+    __device__ static int first_group(int i, int c) { return ((i / NEAR * (GEMV_CONSUMERS / 32) + QuantLane::warp()) * 4 + c) * NEAR; }
+    __device__ static int group_of(int i, int c) { return first_group(i, c) + ((i + c) & (NEAR - 1)); }
+    __device__ void fill(const float* xs, float inv, float up, int K) {
+        const float up4 = up * 0.0625f;
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const int at = group_of(i, QuantLane::g() >> 1) * 32 + 8 * QuantLane::t();
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            if (at < K) { a = *reinterpret_cast<const float4*>(xs + at); b = *reinterpret_cast<const float4*>(xs + at + 4); }
+            x[i][0] = QuantLane::part(a.x * inv * up, a.y * inv * up);
+            x[i][1] = QuantLane::part(a.z * inv * up4, a.w * inv * up4);
+            x[i][2] = QuantLane::part(b.x * inv * up, b.y * inv * up);
+            x[i][3] = QuantLane::part(b.z * inv * up4, b.w * inv * up4);
+        }
+    }
+    template <int R, class Release> __device__ void rows(uint32_t base, uint32_t row_bytes, int K, const Release& release, float (&acc)[R]) const {
+        static_assert(R == 2 || R % 4 == 0, "two rows, or fours");
+        constexpr int SETS = (R + 3) / 4, P = R == 2 ? 1 : 2;  // of four rows; lane's rows of a set
+        const int ngroups = K / 32, quad = QuantLane::g() & 3;
+        const uint32_t row = base + (uint32_t)(QuantLane::g() >> 2) * row_bytes, scale = row + Wfmt<Int4G32>::scale_off(K);
+        float sum[SETS][2] = {};
+#pragma unroll
+        for (int i0 = 0; i0 < STEPS; i0 += BATCH) {
+            if (i0 > 0 && first_group(i0, 0) >= ngroups) break;  // the whole warp's groups lie behind the row
+            uint32_t w[BATCH][SETS][2] = {};
+            unsigned short s[BATCH][SETS][2] = {};
+            uint2 s4[SETS][2] = {};
+            if (NEAR == 4 && first_group(i0, quad) < ngroups) {
+#pragma unroll
+                for (int j = 0; j < SETS; ++j)
+#pragma unroll
+                    for (int k = 0; k < P; ++k)
+                        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(s4[j][k].x), "=r"(s4[j][k].y)
+                                     : "r"(scale + (uint32_t)(4 * j + 2 * k) * row_bytes + (uint32_t)first_group(i0, quad) * 2u));
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int group = group_of(i0 + i, quad);
+                if (group < ngroups) {
+#pragma unroll
+                    for (int j = 0; j < SETS; ++j)
+#pragma unroll
+                        for (int k = 0; k < P; ++k) {
+                            const uint32_t off = (uint32_t)(4 * j + 2 * k) * row_bytes;
+                            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i][j][k]) : "r"(row + off + (uint32_t)group * 16u + 4u * QuantLane::t()));
+                            if (NEAR == 1) asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s[i][j][k]) : "r"(scale + off + (uint32_t)group * 2u));
+                        }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const uint32_t(&b)[4] = x[i0 + i];
+                constexpr uint32_t LOW = 0x000F000Fu, HIGH = 0x00F000F0u, LOW8 = 0x80088008u, HIGH8 = 0x80808080u;  // -8 in either place
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_f16(c, LOW8, LOW8, HIGH8, HIGH8, b[0], b[1]);
+                mma_f16(c, LOW8, LOW8, HIGH8, HIGH8, b[2], b[3]);
+                const uint32_t pick = 0x0010u + 0x0022u * (uint32_t)((i + quad) & 3);  // NEAR: this step's half of the four
+                const bool in = group_of(i0 + i, quad) < ngroups;
+                auto scale_of = [&](int j, int k) {
+                    const uint32_t bits = NEAR == 1 ? s[i][j][k] : in ? __byte_perm(s4[j][k].x, s4[j][k].y, pick) : 0u;
+                    return __half2float(__ushort_as_half((unsigned short)bits));
+                };
+#pragma unroll
+                for (int j = 0; j < SETS; ++j) {
+                    float d[4] = {c[0], c[1], c[2], c[3]};
+                    const uint32_t u = w[i][j][0], v = P == 2 ? w[i][j][1] : 0u;
+                    mma_f16(d, u & LOW, v & LOW, u & HIGH, v & HIGH, b[0], b[1]);
+                    mma_f16(d, (u >> 8) & LOW, (v >> 8) & LOW, (u >> 8) & HIGH, (v >> 8) & HIGH, b[2], b[3]);
+                    sum[j][0] = fmaf(d[0] + d[1], scale_of(j, 0), sum[j][0]);
+                    if (P == 2) sum[j][1] = fmaf(d[2] + d[3], scale_of(j, 1), sum[j][1]);
+                }
+            }
+        }
+        release();
+#pragma unroll
+        for (int j = 0; j < SETS; ++j) QuantLane::take<R>(4 * j, sum[j][0] * 16777216.0f, sum[j][1] * 16777216.0f, acc);
     }
 };
 
@@ -411,7 +538,6 @@ __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, f
     float* partial = reinterpret_cast<float*>(mega_dyn() + p.off_partial);
     constexpr int NW = GEMV_CONSUMERS / 32;
     const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255, lane = tid & 31, warp = tid >> 5;
-    const int nchunks = K / F::EPC;
     const uint32_t row_bytes = F::row_stride(K);
     const int ngroups = (r1 - r0 + R - 1) / R;
 
@@ -439,10 +565,7 @@ __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, f
         }
         float acc[R];
         x.template rows<R>(
-            [&](int j, int i) {
-                const int c = tid + i * GEMV_CONSUMERS;
-                return c < nchunks ? lds128(base + (uint32_t)j * row_bytes + (uint32_t)c * 16u) : make_uint4(0, 0, 0, 0);
-            },
+            base, row_bytes, K,
             [&]() {
                 __syncwarp();
                 if (lane == 0) mbar_arrive_n(ring.empty0 + 8u * s, 2);  // a stage expects 16 arrivals: eight warps of one group, twice each
@@ -451,6 +574,9 @@ __device__ inline void stream_partials(Ring& ring, const Slices<LT, NITER>& x, f
         if (F::ROW_SCALE) {
 #pragma unroll
             for (int j = 0; j < R; ++j) acc[j] = acc[j] * scale[j] * unscale;
+        } else if (F::QUANT) {
+#pragma unroll
+            for (int j = 0; j < R; ++j) acc[j] *= unscale;
         }
         int rr;
         const float tot = warp_reduce_rows<R>(acc, lane, rr);
@@ -649,21 +775,24 @@ enum { PH_QKV = 0, PH_WO = 1, PH_W13 = 2, PH_W2 = 3, PH_HEAD = 4 };
 // rows (one after the other: their product overflows where the vector is zero or tiny); the rows' results times unscale
 template <typename LT, int NITER, int R>
 __device__ inline void tagged_rows(Ring& ring, const MegaParams& p, float inv, float up, float unscale, float* norm_out, const int2& rows, int K) {
-    constexpr int EPC = Wfmt<LT>::EPC;
     const float* xs = reinterpret_cast<const float*>(mega_dyn() + p.off_xs);
-    const int tid = threadIdx.x & 255, nchunks = K / EPC;
     Slices<LT, NITER> x;
+    if constexpr (Wfmt<LT>::QUANT) {
+        x.fill(xs, inv, up, K);
+    } else {
+        constexpr int EPC = Wfmt<LT>::EPC;
+        const int tid = threadIdx.x & 255, nchunks = K / EPC;
 #pragma unroll
-    for (int i = 0; i < NITER; ++i) {
-        const int c = tid + i * GEMV_CONSUMERS;
+        for (int i = 0; i < NITER; ++i) {
+            const int c = tid + i * GEMV_CONSUMERS;
 #pragma unroll
-        for (int e = 0; e < EPC; e += 4) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (c < nchunks) v = *reinterpret_cast<const float4*>(xs + (size_t)c * EPC + e);
-            v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
-            if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x < 256 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
-            if (Wfmt<LT>::QUANT) { v.x *= up; v.y *= up; v.z *= up; v.w *= up; }
-            x.set(i, e, v);
+            for (int e = 0; e < EPC; e += 4) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c < nchunks) v = *reinterpret_cast<const float4*>(xs + (size_t)c * EPC + e);
+                v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+                if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x < 256 && c < nchunks) *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) = v;
+                x.set(i, e, v);
+            }
         }
     }
     stream_partials<LT, NITER, R>(ring, x, unscale, rows.x, rows.y, K, p);
@@ -822,8 +951,8 @@ __device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int at
             const int d = (4 * (s >> 1) + t) * 8 + 4 * (s & 1);
             const bool live = g < p.gqa && d < HD;
             const float4 v = live ? *reinterpret_cast<const float4*>(sh.q + g * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-            Slices<Fp8Row, 1>::pair(qa[s][0], qa[s][1], v.x * up, v.y * up);
-            Slices<Fp8Row, 1>::pair(qa[s][2], qa[s][3], v.z * up, v.w * up);
+            fp16_pair(qa[s][0], qa[s][1], v.x * up, v.y * up);
+            fp16_pair(qa[s][2], qa[s][3], v.z * up, v.w * up);
         }
         float acc[NH][8], m = NEG, lsum = 0.0f;  // m, lsum: of head h0 + g (lsum of this lane's positions), meaningful for g < NH
 #pragma unroll

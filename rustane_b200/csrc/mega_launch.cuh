@@ -14,9 +14,9 @@ using namespace cd;
 // ------------------------------------------------------------------ persistent kernel launch
 template <typename WT, typename LT, typename KT, int ND, int NH, bool TPAR, bool GROUPED>
 cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
-    constexpr bool Q = Wfmt<LT>::QUANT;
+    constexpr MegaRows Q = std::is_same<LT, Int4G32>::value ? MEGA_INT4 : std::is_same<LT, Fp8Row>::value ? MEGA_FP8 : MEGA_PLAIN;
     constexpr int RD = mega_stage_rows(ND, Q), RH = mega_stage_rows(NH, Q), RO = mega_head_rows(ND, Q);
-    constexpr int NO = Q ? 2 * ND : ND;  // an FP8 chunk is twice as many elements as one of the head's
+    constexpr int NO = Q != MEGA_PLAIN ? 2 * ND : ND;  // a quantised chunk is twice as many elements as one of the head's
     const cd_config& c = m->cfg;
     auto kern = decode_mega_kernel<WT, LT, KT, ND, RD, NH, RH, NO, RO, TPAR, GROUPED>;
     // every CTA owns rows of every matrix: what tells a CTA that another one is done with a vector is that one's next rows

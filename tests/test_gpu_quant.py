@@ -202,3 +202,30 @@ def test_fp8_chunks_per_thread(R, dim, hidden, vocab):
         x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
         assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
     assert (a.kernel_launches() - before == 6) == (vocab < 60000)
+
+
+@pytest.mark.parametrize("dim,hidden,heads,kv_heads,hd,value", [
+    (256, 640, 4, 4, 64, 0.0),              # one octet of groups, fewer than the warps
+    (1024, 2848, 8, 8, 128, 1e-20),         # a ragged last octet
+    (4096, 4128, 32, 32, 128, 1e-36),       # two chunks of W2's rows
+    (512, 8224, 4, 1, 128, None),           # three, grouped heads
+    (512, 12320, 4, 4, 128, None),          # four
+    (4224, 15360, 33, 33, 128, None),       # two of the others' rows
+    (1056, 2112, 8, 1, 64, None),           # eight q heads on one kv head
+])
+def test_int4_persistent_kernel_matches_the_kernel_per_operator(R, dim, hidden, heads, kv_heads, hd, value):
+    """INT4 rows through the tensor cores (exact fp16 weights, inputs as hi + lo pairs, a group's sum times its scale in fp32)
+    against the same rows through fp32 FMAs.  Inputs differ by at most 2^-23 relative and sums by their order: a few 1e-6 of logits
+    of order one over two layers; an fp16 cache entry may round to its neighbour.  A zero or tiny input must stay finite."""
+    cfg = R.Config(dim, hidden, heads, hd, 64, 2, 1500, kv_heads=kv_heads)
+    a, b = (R.Model.synthetic(cfg, 3, dtype="int4", mega=mega) for mega in (True, False))
+    before = a.kernel_launches()
+    for t in (7, 1499, 3):
+        x, y = a.decode_token_logits_from_id(t), b.decode_token_logits_from_id(t)
+        assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
+    assert a.kernel_launches() - before == 6
+    if value is not None:
+        x, y = a.decode_token(np.full(dim, value)), b.decode_token(np.full(dim, value))
+        assert np.isfinite(y).all() and np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
+        x, y = a.decode_token_logits_from_id(900), b.decode_token_logits_from_id(900)
+        assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
