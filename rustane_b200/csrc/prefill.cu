@@ -13,8 +13,9 @@
 #include <string>
 #include <vector>
 
-#include "kernels.cuh"
 #include "model.h"
+#include "sample_attn.cuh"
+#include "step.cuh"
 
 namespace cd {
 namespace {
@@ -32,7 +33,7 @@ struct SampleGraphKey {
 struct PrefillCtx {
     EncodeTiledFn encode = nullptr;
     SampleGraphKey s_key;
-    std::map<int, cudaGraphExec_t> s_graphs;  // captured multi-sample steps by number of occupied attention slices
+    std::map<int, cudaGraphExec_t> s_graphs;  // captured multi-sample steps by their attention's slices (SaSplit::id)
     uint64_t s_graph_nodes = 0;
     std::vector<CUtensorMap> k_pages, v_pages;  // per layer, built once
     std::vector<CUtensorMap> sk_qkv, sk_o, sk_13, sk_2;  // the same matrices in 128-row boxes (multi-sample decode)
@@ -42,7 +43,7 @@ struct PrefillCtx {
     // multi-sample decode workspace (one arena, sized for s_cap samples)
     int s_cap = 0;
     char* s_arena = nullptr;
-    float *sx = nullptr, *sq = nullptr, *sattn = nullptr, *slogits = nullptr, *spart_acc = nullptr, *spart_ml = nullptr;
+    float *sx = nullptr, *sq = nullptr, *slogits = nullptr, *spart_acc = nullptr, *spart_ml = nullptr;
     float* sksum = nullptr;  // [8 K slices][16][dim] partial sums of the linears that are cut along K
     float *sblock_vals = nullptr, *stopk_vals = nullptr, *smaxes = nullptr, *ssums = nullptr;
     uint32_t *sblock_idxs = nullptr, *stopk_idxs = nullptr, *sout_token = nullptr, *sring = nullptr;
@@ -70,14 +71,15 @@ cudaError_t sk_launch_t(cd_model* m, const CUtensorMap& w, const CUtensorMap& x,
     auto kern = pf_skinny_kernel<NB, Epi>;
     static bool attr_set = false;  // per instantiation
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkTile<NB>::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SkTile<NB>::smem(SkTile<NB>::STAGES_ALONE));
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((N + 127) / 128, kslices);
+    const int nst = (int)(lc.gridDim.x * lc.gridDim.y) <= m->sm_count ? SkTile<NB>::STAGES_ALONE : SkTile<NB>::STAGES_SHARED;
     lc.blockDim = dim3(PF_THREADS);
-    lc.dynamicSmemBytes = SkTile<NB>::SMEM;
+    lc.dynamicSmemBytes = SkTile<NB>::smem(nst);
     lc.stream = m->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernel fetches weights before it waits for its predecessor
@@ -85,7 +87,7 @@ cudaError_t sk_launch_t(cd_model* m, const CUtensorMap& w, const CUtensorMap& x,
     lc.attrs = at;
     lc.numAttrs = m->pdl ? 1 : 0;
     m->launches++;
-    return cudaLaunchKernelEx(&lc, kern, w, x, N, K, ns, make_idesc(NB, bf16), &m->st->error, epi);
+    return cudaLaunchKernelEx(&lc, kern, w, x, N, K, ns, nst, make_idesc(NB, bf16), &m->st->error, epi);
 }
 template <class Epi>
 cudaError_t sk_launch(cd_model* m, bool split, const CUtensorMap& w, const CUtensorMap& x, int N, int K, int ns, bool bf16,
@@ -302,7 +304,7 @@ int run_samples(cd_model* m, PrefillCtx* c, const uint32_t* first, int ns, size_
         const size_t S = SK_ROWS, W = (size_t)std::max(D, Q);  // blocks of 16 rows: hi parts, then lo parts
         size_t off = 0;
         auto carve = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 255) / 256 * 256; return o; };
-        const size_t o_x = carve(S * D * 4), o_q = carve(S * Q * 4), o_attn = carve(S * Q * 4), o_logits = carve(S * Vp * 4);
+        const size_t o_x = carve(S * D * 4), o_q = carve(S * Q * 4), o_logits = carve(S * Vp * 4);
         const size_t o_pacc = carve(S * cf.heads * m->nsplit * hd * 4), o_pml = carve(S * cf.heads * m->nsplit * 2 * 4);
         const size_t o_cnt = carve(S * cf.heads * 4), o_hcnt = carve(S * 4);
         const size_t o_bv = carve(S * NB * 4), o_bi = carve(S * NB * 4), o_tv = carve(S * NB * CD_MAX_GPU_TOPK * 4), o_ti = carve(S * NB * CD_MAX_GPU_TOPK * 4);
@@ -312,7 +314,7 @@ int run_samples(cd_model* m, PrefillCtx* c, const uint32_t* first, int ns, size_
         PF_TRY("sample workspace", cudaMalloc((void**)&c->s_arena, off));
         PF_TRY("sample workspace", cudaMemsetAsync(c->s_arena, 0, off, m->stream));
         char* b = c->s_arena;
-        c->sx = (float*)(b + o_x); c->sq = (float*)(b + o_q); c->sattn = (float*)(b + o_attn); c->slogits = (float*)(b + o_logits);
+        c->sx = (float*)(b + o_x); c->sq = (float*)(b + o_q); c->slogits = (float*)(b + o_logits);
         c->spart_acc = (float*)(b + o_pacc); c->spart_ml = (float*)(b + o_pml); c->scounters = (unsigned int*)(b + o_cnt);
         c->shead_counters = (unsigned int*)(b + o_hcnt); c->sblock_vals = (float*)(b + o_bv); c->sblock_idxs = (uint32_t*)(b + o_bi);
         c->stopk_vals = (float*)(b + o_tv); c->stopk_idxs = (uint32_t*)(b + o_ti); c->smaxes = (float*)(b + o_mx); c->ssums = (float*)(b + o_sm);
@@ -357,44 +359,42 @@ int run_samples(cd_model* m, PrefillCtx* c, const uint32_t* first, int ns, size_
 
     const float scale = 1.0f / std::sqrt((float)hd);
     const float inv_t = 1.0f / std::max(t, 1.17549435e-38f);  // decode.rs:174
-    const int split_blocks = (int)std::min<size_t>(256, ((size_t)ns * Q + 255) / 256);
+    const int shared_tokens = len0 / pt * pt;
+    const SaBlocks blocks{cf.gqa_ratio, ns};
     // one step of all samples; everything that changes from step to step is read on the device, except the
-    // number of attention slices that hold keys (`nsp`), which selects the captured graph
-    auto enqueue_step = [&](int nsp) -> int {
+    // attention's slices, which select the captured graph
+    auto enqueue_step = [&](const SaSplit& cut) -> int {
         pf_embed_samples_kernel<T16><<<ns, 256, 0, m->stream>>>((const T16*)m->embed, c->sst, c->sx, D, m->full_cfg.vocab);
         m->launches++;
         // Wo and W2 have few output rows: they are cut along K into `ks` slices and the following
         // RMSNorm kernel adds the slices' partial sums (in slice order) into the residual stream
         const int ks = std::max(1, std::min(8, m->sm_count / ((D + 127) / 128)));
         const int nthreads = std::min(1024, std::max(256, D / 4 / 32 * 32));
+        auto fold = [&](const float* gamma) {
+            return launch_chain(m, pf_reduce_rmsnorm_kernel<T16>, dim3(ns), dim3(nthreads), 0, c->sx, (const float*)c->sksum, ks, m->alpha, gamma, xn, xn_lo, D);
+        };
         for (int l = 0; l < cf.nlayers; ++l) {
             const cd_layer_dev& L = m->layers[l];
-            if (l == 0) pf_rmsnorm_kernel<T16><<<ns, 256, 0, m->stream>>>(c->sx, L.gamma1, xn, xn_lo, D);
-            else pf_reduce_rmsnorm_kernel<T16><<<ns, nthreads, 0, m->stream>>>(c->sx, c->sksum, ks, m->alpha, L.gamma1, xn, xn_lo, D);
+            if (l == 0) {
+                pf_rmsnorm_kernel<T16><<<ns, 256, 0, m->stream>>>(c->sx, L.gamma1, xn, xn_lo, D);
+                m->launches++;
+            } else {
+                PF_TRY("norm", fold(L.gamma1));
+            }
             {
                 SkEpiQKV<KT> epi{c->sq, (KT*)L.kv, m->page_table, m->rope, c->sst, Q, KV, hd, cf.kv_heads, pt, pps};
                 PF_TRY("qkv gemm", sk_launch(m, split, c->sk_qkv[l], a_xn, Q + 2 * KV, D, ns, bf16, epi));
             }
-            // two samples per attention CTA share each K/V tile of the prompt pages (measured best of 1, 2, 4, 8)
-            const dim3 agrid(cf.heads, nsp, (ns + 1) / 2);
-            const int shared_tokens = len0 / pt * pt;
-            if (hd == 128)
-                attn_decode_group_kernel<KT, 128, 2><<<agrid, 128, 0, m->stream>>>(c->sq, (const KT*)L.kv, m->page_table, c->sst, c->spart_acc, c->spart_ml,
-                                                                                    c->scounters, c->sattn, cf.kv_heads, cf.gqa_ratio, pt, nsp, scale, pps, ns,
-                                                                                    shared_tokens);
-            else
-                attn_decode_group_kernel<KT, 64, 2><<<agrid, 128, 0, m->stream>>>(c->sq, (const KT*)L.kv, m->page_table, c->sst, c->spart_acc, c->spart_ml,
-                                                                                   c->scounters, c->sattn, cf.kv_heads, cf.gqa_ratio, pt, nsp, scale, pps, ns,
-                                                                                   shared_tokens);
-            pf_split_kernel<T16><<<split_blocks, 256, 0, m->stream>>>(c->sattn, xn, attn_lo, (size_t)ns * Q);
+            const SampleAttn at{c->sq, m->page_table, c->sst, c->spart_acc, c->spart_ml, c->scounters, cf.kv_heads, pt, pps, m->nsplit, shared_tokens, blocks, cut, scale};
+            const dim3 agrid(cf.kv_heads, cut.shared + cut.own, blocks.count());
+            PF_TRY("attention", hd == 128 ? launch_chain(m, sample_attn_kernel<KT, T16, 128>, agrid, dim3(SA_THREADS), 0, at, (const KT*)L.kv, xn, attn_lo)
+                                          : launch_chain(m, sample_attn_kernel<KT, T16, 64>, agrid, dim3(SA_THREADS), 0, at, (const KT*)L.kv, xn, attn_lo));
             PF_TRY("wo gemm", sk_launch(m, split, c->sk_o[l], a_attn, D, Q, ns, bf16, SkEpiPartial{c->sksum, D}, ks));
-            pf_reduce_rmsnorm_kernel<T16><<<ns, nthreads, 0, m->stream>>>(c->sx, c->sksum, ks, m->alpha, L.gamma2, xn, xn_lo, D);
+            PF_TRY("norm", fold(L.gamma2));
             PF_TRY("w13 gemm", sk_launch(m, split, c->sk_13[l], a_xn, 2 * H, D, ns, bf16, SkEpiGate<T16>{gate, gate_lo, H, m->opt.activation}));
             PF_TRY("w2 gemm", sk_launch(m, split, c->sk_2[l], a_gate, D, H, ns, bf16, SkEpiPartial{c->sksum, D}, ks));
-            m->launches += 4;
         }
-        pf_reduce_rmsnorm_kernel<T16><<<ns, nthreads, 0, m->stream>>>(c->sx, c->sksum, ks, m->alpha, m->gamma_final, xn, xn_lo, D);
-        m->launches++;
+        PF_TRY("norm", fold(m->gamma_final));
         PF_TRY("head gemm", sk_launch(m, split, c->sk_head, a_xn, V, D, ns, bf16, SkEpiStore{c->slogits, Vp}));
         // each sample's own reductions and draw, on its own state; one launch covers all samples
         if (mode == 0) {
@@ -415,7 +415,7 @@ int run_samples(cd_model* m, PrefillCtx* c, const uint32_t* first, int ns, size_
         PF_TRY("step launch", cudaGetLastError());
         return CD_OK;
     };
-    // graphs of a step are kept per `nsp` for as long as the request parameters stay the same
+    // graphs of a step are kept per cut of the attention for as long as the request parameters stay the same
     const SampleGraphKey key{ns, mode, top_k, t, softcap, split ? 1 : 0, len0};
     if (!(key == c->s_key)) {
         for (auto& kv : c->s_graphs) cudaGraphExecDestroy(kv.second);
@@ -424,17 +424,17 @@ int run_samples(cd_model* m, PrefillCtx* c, const uint32_t* first, int ns, size_
     }
     for (size_t step = 0; step < nsteps; ++step) {
         const int attn_len = len0 + (int)step + 1;
-        const int nsp = std::max(1, std::min(m->nsplit, (attn_len + pt - 1) / pt));  // slices that hold keys at this position
+        const SaSplit cut = sa_split(shared_tokens, attn_len, blocks, cf.kv_heads, m->nsplit, m->sm_count);
         if (!m->opt.use_graph) {
-            if ((rc = enqueue_step(nsp))) return rc;
+            if ((rc = enqueue_step(cut))) return rc;
             continue;
         }
-        auto it = c->s_graphs.find(nsp);
+        auto it = c->s_graphs.find(cut.id());
         if (it == c->s_graphs.end()) {
             cudaGraph_t graph = nullptr;
             const uint64_t before = m->launches;
             PF_TRY("graph capture", cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-            rc = enqueue_step(nsp);
+            rc = enqueue_step(cut);
             const cudaError_t e2 = cudaStreamEndCapture(m->stream, &graph);
             if (rc || e2 != cudaSuccess) {
                 if (graph) cudaGraphDestroy(graph);
@@ -446,7 +446,7 @@ int run_samples(cd_model* m, PrefillCtx* c, const uint32_t* first, int ns, size_
             if (e != cudaSuccess) return cuda_fail("graph instantiate", e);
             c->s_graph_nodes = m->launches - before;
             m->launches = before;
-            it = c->s_graphs.emplace(nsp, exec).first;
+            it = c->s_graphs.emplace(cut.id(), exec).first;
         }
         PF_TRY("graph launch", cudaGraphLaunch(it->second, m->stream));
         m->launches += c->s_graph_nodes;

@@ -449,12 +449,16 @@ pf_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 // activations are the N side, [NB rows][64] with rows 0-15 the hi parts and rows 16-31 the lo
 // parts of the samples (NB = 16 without the lo parts).  D[feature lane][row column] in tensor
 // memory; an epilogue thread owns one feature and adds column j + 16 to column j.  One CTA per
-// 128 features, nine 20 KB stages: the kernel is a weight stream, bound by HBM.
+// 128 features and K slice.  The kernel is a weight stream; what bounds it is what a CTA has in flight, and its start and
+// end: eight 20 KB stages where every CTA has an SM of its own, five where two share one (a step of eight samples of
+// the 5B model 2.96 ms with five everywhere, 2.80 ms so).  Requesting 24-96 MB of the next matrix into L2 behind a kernel's own
+// loads made the step 5-8 % slower, four accumulators for a step's four MMAs changed nothing, and neither did
+// cutting K among the CTAs of a cluster (192 CTAs instead of 96 for q|k|v) or into twice as many slices.
 constexpr int SK_ROWS = 16;  // samples per call at most
 template <int NB> struct SkTile {
     static constexpr uint32_t A_BYTES = 128 * PF_BK * 2, B_BYTES = NB * PF_BK * 2, STAGE = A_BYTES + 2048 * ((B_BYTES + 2047) / 2048);
-    static constexpr int NST = 5;  // two CTAs per SM: one streams while its neighbour starts up or drains
-    static constexpr size_t SMEM = (size_t)NST * STAGE + 1024 + 256;
+    static constexpr int STAGES_ALONE = 8, STAGES_SHARED = 5;
+    static constexpr size_t smem(int nst) { return (size_t)nst * STAGE + 1024 + 256; }
 };
 
 struct SkEpiPartial {  // this K slice's partial sums: part[slice][s][f] = y[s]
@@ -534,9 +538,9 @@ template <typename T16> struct SkEpiQKV {  // RoPE pairs sit in neighbouring lan
 
 template <int NB, class Epi>
 __global__ void __launch_bounds__(PF_THREADS, 2)
-pf_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, int N, int K, int ns, uint32_t idesc, int* err, Epi epi) {
+pf_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, int N, int K, int ns, int nst, uint32_t idesc, int* err,
+                 Epi epi) {
     using TL = SkTile<NB>;
-    constexpr int NST = TL::NST;
     extern __shared__ unsigned char pf_raw[];
     const int n0 = blockIdx.x * 128;
     // blockIdx.y: which slice of K this CTA multiplies (a matrix with few rows is cut along K so that
@@ -544,11 +548,11 @@ pf_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constan
     const int nkb_all = (K + PF_BK - 1) / PF_BK, per = (nkb_all + (int)gridDim.y - 1) / (int)gridDim.y;
     const int kb_first = blockIdx.y * per, nkb = max(0, min(nkb_all, kb_first + per) - kb_first);
     const uint32_t tiles = (smem_addr(pf_raw) + 1023u) & ~1023u;
-    const uint32_t bars = tiles + NST * TL::STAGE;
-    const uint32_t full0 = bars, empty0 = bars + 8u * NST, accum = bars + 16u * NST, slot = accum + 8u;
+    const uint32_t bars = tiles + nst * TL::STAGE;
+    const uint32_t full0 = bars, empty0 = bars + 8u * nst, accum = bars + 16u * nst, slot = accum + 8u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NST; ++s) {
+        for (int s = 0; s < nst; ++s) {
             mbar_init(full0 + 8u * s, 1);
             mbar_init(empty0 + 8u * s, 1);
         }
@@ -562,47 +566,59 @@ pf_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constan
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(slot));
     bool failed = false;
+    // whole warps wait and loop, one elected thread issues: with the loops in one thread a step took 890 clocks (see above), 16 KB a
+    // CTA, which bound the kernel and not HBM (3.17 ms a step; 2.96)
+    auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+        if (!ok) {
+            atomicExch(err, code);
+            failed = true;
+        }
+        return ok;
+    };
     if (warp == 0) {
-        if (lane == 0) {
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int s = kb % NST;
-                if (kb >= NST && !mbar_wait(empty0 + 8u * s, ((kb / NST) - 1) & 1)) {
-                    atomicExch(err, DEV_ERR_PF_EMPTY);
-                    failed = true;
-                    break;
-                }
+        // Under programmatic dependent launch the first ring of weight tiles is requested before the previous kernel has
+        // finished; the activations it produces are requested only after the wait.
+        const int ahead = min(nst, nkb);
+        if (elect_one()) {
+            for (int kb = 0; kb < ahead; ++kb) {
+                mbar_arrive_expect_tx(full0 + 8u * kb, TL::A_BYTES + TL::B_BYTES);
+                tma_load_2d(tiles + kb * TL::STAGE, &tma_w, (kb_first + kb) * PF_BK, n0, full0 + 8u * kb);
+            }
+        }
+        __syncwarp();
+        pdl_wait();
+        pdl_launch_dependents();
+        if (elect_one()) {
+            for (int kb = 0; kb < ahead; ++kb) tma_load_2d(tiles + kb * TL::STAGE + TL::A_BYTES, &tma_x, (kb_first + kb) * PF_BK, 0, full0 + 8u * kb);
+        }
+        __syncwarp();
+        int s = 0, turn = 0;
+        for (int kb = nst; kb < nkb; ++kb) {
+            if (!wait(empty0 + 8u * s, turn, DEV_ERR_PF_EMPTY)) break;
+            if (elect_one()) {
                 const uint32_t a_dst = tiles + s * TL::STAGE;
                 mbar_arrive_expect_tx(full0 + 8u * s, TL::A_BYTES + TL::B_BYTES);
                 tma_load_2d(a_dst, &tma_w, (kb_first + kb) * PF_BK, n0, full0 + 8u * s);
-                // Under programmatic dependent launch the first ring of weight tiles is requested before the
-                // previous kernel has finished; the activations it produces are requested only after the wait.
-                if (kb == min(NST, nkb) - 1) {
-                    pdl_wait();
-                    pdl_launch_dependents();
-                    for (int k2 = 0; k2 <= kb; ++k2)
-                        tma_load_2d(tiles + (k2 % NST) * TL::STAGE + TL::A_BYTES, &tma_x, (kb_first + k2) * PF_BK, 0, full0 + 8u * (k2 % NST));
-                } else if (kb >= NST) {
-                    tma_load_2d(a_dst + TL::A_BYTES, &tma_x, (kb_first + kb) * PF_BK, 0, full0 + 8u * s);
-                }
+                tma_load_2d(a_dst + TL::A_BYTES, &tma_x, (kb_first + kb) * PF_BK, 0, full0 + 8u * s);
             }
-            if (nkb == 0) { pdl_wait(); pdl_launch_dependents(); }
+            __syncwarp();
+            if (++s == nst) { s = 0; turn ^= 1; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int s = kb % NST;
-                if (!mbar_wait(full0 + 8u * s, (kb / NST) & 1)) {
-                    atomicExch(err, DEV_ERR_PF_FULL);
-                    failed = true;
-                    break;
-                }
-                tc_fence_after();
+        int s = 0, turn = 0;
+        for (int kb = 0; kb < nkb; ++kb) {
+            if (!wait(full0 + 8u * s, turn, DEV_ERR_PF_FULL)) break;
+            tc_fence_after();
+            if (elect_one()) {
                 const uint64_t adesc = umma_desc(tiles + s * TL::STAGE), bdesc = umma_desc(tiles + s * TL::STAGE + TL::A_BYTES);
 #pragma unroll
                 for (int k = 0; k < PF_BK / 16; ++k) umma_f16(tmem_base, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0);
                 umma_commit(empty0 + 8u * s);
+                if (kb == nkb - 1) umma_commit(accum);
             }
-            if (!failed) umma_commit(accum);
+            __syncwarp();
+            if (++s == nst) { s = 0; turn ^= 1; }
         }
     } else {
         const int lane_base = (warp & 3) * 32;
@@ -667,13 +683,6 @@ __global__ void pf_embed_samples_kernel(const WT* __restrict__ embed, DevState* 
     for (int i = threadIdx.x; i < D; i += blockDim.x) x[(size_t)blockIdx.x * D + i] = Elem<WT>::to_f32(row[i]);
 }
 
-// fp32 values as a 16-bit hi (+ lo) GEMM operand
-template <typename T16>
-__global__ void pf_split_kernel(const float* __restrict__ in, T16* __restrict__ hi, T16* __restrict__ lo, size_t n) {
-    pdl_launch_dependents();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) pf_store(hi, lo, i, in[i]);
-}
-
 // x * rsqrt(mean(x^2) + eps) * gamma per row (cpu/rmsnorm.rs:149-183), written as 16-bit GEMM input
 template <typename T16>
 __global__ void __launch_bounds__(256) pf_rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ gamma, T16* __restrict__ out,
@@ -688,23 +697,45 @@ __global__ void __launch_bounds__(256) pf_rmsnorm_kernel(const float* __restrict
 }
 
 // The same after folding in a linear that was cut along K: x += alpha * (sum of the slices' partial
-// sums, in slice order), written back, then normalised.  One CTA of up to 1024 threads per row.
+// sums, in slice order), written back, then normalised.  One CTA of up to 1024 threads per row, four neighbouring entries a
+// thread and turn, all slices' loads of a turn in flight: the kernel is one memory latency and two block-wide sums long.
 template <typename T16>
 __global__ void __launch_bounds__(1024) pf_reduce_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ part, int nslices, float alpha,
                                                                  const float* __restrict__ gamma, T16* __restrict__ out, T16* __restrict__ out_lo, int D) {
     __shared__ float red[32];
+    constexpr int S = 8;  // slices at most
+    pdl_wait();
     pdl_launch_dependents();
-    float* row = x + (size_t)blockIdx.x * D;
+    float4* row = reinterpret_cast<float4*>(x + (size_t)blockIdx.x * D);
+    const float4* p4 = reinterpret_cast<const float4*>(part + (size_t)blockIdx.x * D);
+    const size_t slice = (size_t)SK_ROWS * D / 4;
     float ss = 0.0f;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        float acc = 0.0f;
-        for (int k = 0; k < nslices; ++k) acc += part[((size_t)k * SK_ROWS + blockIdx.x) * D + i];
-        const float v = row[i] + alpha * acc;
+    for (int i = threadIdx.x; i < D / 4; i += blockDim.x) {
+        float4 v = __ldcg(row + i), p[S];
+#pragma unroll
+        for (int k = 0; k < S; ++k) p[k] = k < nslices ? __ldcg(p4 + k * slice + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < S; ++k) { a.x += p[k].x; a.y += p[k].y; a.z += p[k].z; a.w += p[k].w; }
+        v.x += alpha * a.x; v.y += alpha * a.y; v.z += alpha * a.z; v.w += alpha * a.w;
         row[i] = v;
-        ss += v * v;
+        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
     const float inv = 1.0f / sqrtf(block_sum(ss, red) * (1.0f / (float)D) + RMS_EPS);
-    for (int i = threadIdx.x; i < D; i += blockDim.x) pf_store(out, out_lo, (size_t)blockIdx.x * D + i, row[i] * inv * gamma[i]);
+    for (int i = threadIdx.x; i < D / 4; i += blockDim.x) {  // (the entries this thread wrote)
+        const float4 v = row[i], g = reinterpret_cast<const float4*>(gamma)[i];
+        const float y[4] = {v.x * inv * g.x, v.y * inv * g.y, v.z * inv * g.z, v.w * inv * g.w};
+        uint2 hi, lo;
+        T16* h = reinterpret_cast<T16*>(&hi);
+        T16* l = reinterpret_cast<T16*>(&lo);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            h[k] = pf_cast<T16>(y[k]);
+            l[k] = pf_cast<T16>(y[k] - Elem<T16>::to_f32(h[k]));
+        }
+        reinterpret_cast<uint2*>(out + (size_t)blockIdx.x * D)[i] = hi;
+        if (out_lo != nullptr) reinterpret_cast<uint2*>(out_lo + (size_t)blockIdx.x * D)[i] = lo;
+    }
 }
 
 // ---------------------------------------------------------------------- tensor parallel: all-reduce of a [rows, dim] partial product

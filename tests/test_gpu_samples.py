@@ -19,13 +19,18 @@ CASES = [
     ((512, 1536, 8, 64, 256, 3, 8192), "bf16", dict(untied=1), 37, 64),     # prompt ends inside a page: copy-on-write
     ((256, 640, 2, 128, 256, 2, 1500), "f16", {}, 128, 64),                 # prompt ends on a page boundary, ragged vocab
     ((256, 512, 4, 64, 200, 2, 512), "bf16", dict(kv_heads=2), 50, 16),     # GQA, small pages
+    ((1024, 1536, 16, 64, 300, 2, 700), "f16", dict(kv_heads=1), 200, 32),   # sixteen q heads a kv head: two blocks a sample
+    ((2048, 2112, 24, 128, 320, 2, 1000), "bf16", dict(kv_heads=8), 170, 64), # three heads a kv head: blocks of two samples, the last of one
+    ((512, 1536, 8, 64, 256, 2, 1000), "bf16", dict(kv="bf16"), 200, 64),    # bf16 cache: three parts of q; few slices: several turns a warp
 ]
 
 
 def _model(R, O, dims, dtype, kw, page_tokens, max_samples, use_graph=False):
+    kw = dict(kw)
+    kv = kw.pop("kv", "auto")
     oc = oracle_cfg(O, *dims, dtype=dtype, **kw)
     return oc, R.Model.synthetic(gpu_cfg(R, oc), 11, untied_head=bool(oc.untied), dtype=dtype, page_tokens=page_tokens,
-                                 max_samples=max_samples, use_graph=use_graph)
+                                 max_samples=max_samples, use_graph=use_graph, kv_dtype=kv)
 
 
 @pytest.mark.parametrize("dims,dtype,kw,nprompt,page_tokens", CASES)
