@@ -114,6 +114,52 @@ struct EpiGateMoe {
     }
 };
 
+// Residual stream and, of the vector that becomes x2, what the router behind it needs: this CTA's share of every expert's
+// logit ahead of the norm's factor, route_part[CTA][e] = sum over its rows i of x2[i] gamma[i] W_r[e][i].  The kernel of the
+// experts adds the CTAs' shares up (moe_gate_kernel): a router kernel of its own cost its launch, a round of loads and an arrival counter.
+template <typename WT> struct EpiResidualRoute {
+    const float* res;
+    float* out;
+    float alpha;
+    const float* gamma;
+    const WT* wr;  // [experts][dim]
+    float* route_part;
+    int dim, experts;
+    // thread t takes expert t / 4 (and every 64th behind it) and every fourth of the CTA's rows; its first weights are
+    // requested ahead of the stream
+    static constexpr int PRE = 4;
+    struct Ahead { float w[PRE]; };
+    __device__ Ahead ahead(int t, int u0, int nu) const {
+        Ahead a;
+#pragma unroll
+        for (int k = 0; k < PRE; ++k) a.w[k] = t / 4 < experts && t % 4 + 4 * k < nu ? Elem<WT>::to_f32(wr[(size_t)(t / 4) * dim + u0 + t % 4 + 4 * k]) : 0.0f;
+        return a;
+    }
+    __device__ float operator()(int unit, const float (&y)[1]) const {  // returns what the shares are formed of
+        const float v = __ldcg(res + unit) + alpha * y[0];
+        out[unit] = v;
+        return v * gamma[unit];
+    }
+    // v: the CTA's nu values, `stride` floats apart in shared memory
+    __device__ void shares(const Ahead& a, int t, const float* v, int stride, int u0, int nu) const {
+        for (int e0 = 0; e0 < experts; e0 += 64) {  // (uniform: shuffles inside)
+            const int e = e0 + t / 4;
+            float s = 0.0f;
+            if (e < experts) {
+                for (int i = t % 4, k = 0; i < nu; i += 4, ++k) {
+                    const float w = e0 == 0 && k < PRE ? (k == 0 ? a.w[0] : k == 1 ? a.w[1] : k == 2 ? a.w[2] : a.w[3]) : Elem<WT>::to_f32(wr[(size_t)e * dim + u0 + i]);
+                    s = fmaf(v[(size_t)i * stride], w, s);
+                }
+            }
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (e < experts && t % 4 == 0) route_part[(size_t)blockIdx.x * experts + e] = s;
+        }
+    }
+};
+template <class Epi> struct EpiRoutes { static constexpr bool value = false; };
+template <typename WT> struct EpiRoutes<EpiResidualRoute<WT>> { static constexpr bool value = true; };
+
 // ---------------------------------------------------------------------- where the rows of a GEMV come from
 // SrcPlain: one matrix, row r at W + r * row_bytes.  The two expert sources assemble a virtual matrix from
 // the experts the router chose for this token (a device-side list, so the kernel reads its shape after
@@ -139,7 +185,7 @@ struct SrcExpertRows {
     int seg_rows, tail_rows;
     __device__ int rows(int, int nl) const { return nl * seg_rows + tail_rows; }
     __device__ int cols(int K, int) const { return K; }
-    __device__ void copy(uint32_t dst, const char* W, int row0, int nrows, uint32_t row_bytes, uint32_t bar, uint64_t policy, const int* list, int nl) const {
+    __device__ void copy(uint32_t dst, const char* W, int row0, int nrows, uint32_t row_bytes, uint32_t bar, uint64_t policy, const int* list, int nl, int lane) const {
         auto addr = [&](int v) -> const char* {
             const int sg = v / seg_rows;
             return sg < nl ? W + ((size_t)list[sg] * seg_rows + (size_t)(v - sg * seg_rows)) * row_bytes
@@ -147,9 +193,9 @@ struct SrcExpertRows {
         };
         const int last = row0 + nrows - 1;
         if (row0 >= nl * seg_rows || row0 / seg_rows == last / seg_rows) {
-            bulk_g2s_stream(dst, addr(row0), (uint32_t)nrows * row_bytes, bar, policy);
-        } else {
-            for (int j = 0; j < nrows; ++j) bulk_g2s_stream(dst + (uint32_t)j * row_bytes, addr(row0 + j), row_bytes, bar, policy);
+            if (lane == 0) bulk_g2s_stream(dst, addr(row0), (uint32_t)nrows * row_bytes, bar, policy);
+        } else if (lane < nrows) {
+            bulk_g2s_stream(dst + (uint32_t)lane * row_bytes, addr(row0 + lane), row_bytes, bar, policy);
         }
     }
 };
@@ -164,12 +210,13 @@ struct SrcExpertCols {
     uint32_t seg_bytes, tail_bytes;
     __device__ int rows(int N, int) const { return N; }
     __device__ int cols(int, int nl) const { return nl * seg_cols + tail_cols; }
-    __device__ void copy(uint32_t dst, const char* W, int row0, int nrows, uint32_t row_bytes, uint32_t bar, uint64_t policy, const int* list, int nl) const {
-        for (int j = 0; j < nrows; ++j) {
-            const uint32_t d = dst + (uint32_t)j * row_bytes;
-            for (int sg = 0; sg < nl; ++sg)
-                bulk_g2s_stream(d + (uint32_t)sg * seg_bytes, W + ((size_t)list[sg] * mat_rows + (size_t)(row0 + j)) * seg_bytes, seg_bytes, bar, policy);
-            if (tail_bytes) bulk_g2s_stream(d + (uint32_t)nl * seg_bytes, reinterpret_cast<const char*>(tail) + (size_t)(row0 + j) * tail_bytes, tail_bytes, bar, policy);
+    // a lane per piece: one lane for all of them took as long per row as the row's bytes
+    __device__ void copy(uint32_t dst, const char* W, int row0, int nrows, uint32_t row_bytes, uint32_t bar, uint64_t policy, const int* list, int nl, int lane) const {
+        for (int i = lane; i < nrows * (nl + 1); i += 32) {
+            const int j = i / (nl + 1), sg = i - j * (nl + 1);
+            const uint32_t d = dst + (uint32_t)j * row_bytes + (uint32_t)sg * seg_bytes;
+            if (sg < nl) bulk_g2s_stream(d, W + ((size_t)list[sg] * mat_rows + (size_t)(row0 + j)) * seg_bytes, seg_bytes, bar, policy);
+            else if (tail_bytes) bulk_g2s_stream(d, reinterpret_cast<const char*>(tail) + (size_t)(row0 + j) * tail_bytes, tail_bytes, bar, policy);
         }
     }
 };
@@ -272,7 +319,7 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
     __syncthreads();
 
     if (producer) {  // ---- producer: weights do not depend on the previous kernel
-        if (lane == 0) {
+        if (lane == 0 || Src::DYNAMIC) {  // a gathered stage's copies are shared out among the lanes
             const char* Wb = reinterpret_cast<const char*>(W) + (size_t)r0 * row_bytes;
             const uint64_t policy = l2_evict_first_policy();
             for (int g = 0; g < ngroups; ++g) {
@@ -284,11 +331,13 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
                 }
                 const int rows = min(R, (r1 - r0) - g * R);
                 const uint32_t bytes = (uint32_t)rows * row_bytes;
-                mbar_arrive_expect_tx(full0 + 8u * s, bytes);
-                if constexpr (Src::DYNAMIC) src.copy(ring + (uint32_t)s * stage_bytes, reinterpret_cast<const char*>(W), r0 + g * R, rows, row_bytes, full0 + 8u * s, policy, src_list, src_n);
-                else bulk_g2s_stream(ring + (uint32_t)s * stage_bytes, Wb + (size_t)g * stage_bytes, bytes, full0 + 8u * s, policy);
+                if (lane == 0) mbar_arrive_expect_tx(full0 + 8u * s, bytes);
+                if constexpr (Src::DYNAMIC) {
+                    __syncwarp();
+                    src.copy(ring + (uint32_t)s * stage_bytes, reinterpret_cast<const char*>(W), r0 + g * R, rows, row_bytes, full0 + 8u * s, policy, src_list, src_n, lane);
+                } else bulk_g2s_stream(ring + (uint32_t)s * stage_bytes, Wb + (size_t)g * stage_bytes, bytes, full0 + 8u * s, policy);
             }
-            if (next.w != nullptr) {  // queue the next kernel's first bytes behind our own last loads
+            if (lane == 0 && next.w != nullptr) {  // queue the next kernel's first bytes behind our own last loads
                 const long long nu0 = (long long)blockIdx.x * next.nunits / gridDim.x;
                 const long long nu1 = (long long)(blockIdx.x + 1) * next.nunits / gridDim.x;
                 const char* nb = reinterpret_cast<const char*>(next.w) + (size_t)nu0 * next.unit * next.row_bytes;
@@ -301,6 +350,19 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
     }
 
     // ---- consumers
+    auto route_ahead = [&]() {
+        if constexpr (EpiRoutes<Epi>::value) return epi.ahead(tid, u0, u1 - u0);
+        else return 0;
+    }();
+    // gamma is older than the kernel ahead (wider inputs: the registers do not last)
+    constexpr bool GAMMA_AHEAD = NORM && !In::CUSTOM && NITER * EPC <= 16;
+    float gm[GAMMA_AHEAD ? NITER : 1][GAMMA_AHEAD ? EPC : 4];
+    if constexpr (GAMMA_AHEAD) {
+#pragma unroll
+        for (int i = 0; i < NITER; ++i)
+#pragma unroll
+            for (int e = 0; e < EPC; ++e) gm[i][e] = tid + i * GEMV_CONSUMERS < nchunks ? gamma[(size_t)(tid + i * GEMV_CONSUMERS) * EPC + e] : 0.0f;
+    }
     pdl_wait();
     pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
     float xr[NITER][EPC];
@@ -349,7 +411,9 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
             if (c < nchunks) {
 #pragma unroll
                 for (int e = 0; e < EPC; e += 4) {
-                    const float4 g = *reinterpret_cast<const float4*>(gamma + (size_t)c * EPC + e);
+                    float4 g;
+                    if constexpr (GAMMA_AHEAD) g = make_float4(gm[i][e], gm[i][e + 1], gm[i][e + 2], gm[i][e + 3]);
+                    else g = *reinterpret_cast<const float4*>(gamma + (size_t)c * EPC + e);
                     xr[i][e] = xr[i][e] * inv * g.x;
                     xr[i][e + 1] = xr[i][e + 1] * inv * g.y;
                     xr[i][e + 2] = xr[i][e + 2] * inv * g.z;
@@ -428,7 +492,13 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
             for (int wi = 0; wi < NW; ++wi) sacc += partial[(u * UNIT + k) * NW + wi];
             y[k] = ngroups > 0 ? sacc : 0.0f;
         }
-        epi(unit0 + u0 + u, y);
+        if constexpr (EpiRoutes<Epi>::value) partial[u * NW] = epi(unit0 + u0 + u, y);
+        else epi(unit0 + u0 + u, y);
+    }
+    if constexpr (EpiRoutes<Epi>::value) {
+        static_assert(G == 1 && UNIT == 1, "one consumer group, single rows");
+        all_consumers_bar(GEMV_CONSUMERS);
+        epi.shares(route_ahead, tid, partial, NW, u0, u1 - u0);
     }
 }
 

@@ -53,7 +53,7 @@ cudaError_t launch_mla(cd_model* m, const MlaStep& p) {
         TRY(launch_chain(m, mla_attn_kernel<KT>, dim3(p.nsplit, d.head_blocks(), d.col_blocks()), dim3(256), smem, (const float*)p.qabs, (const KT*)p.pool,
                          (const int*)m->page_table, (const DevState*)m->st, p.part_acc, p.part_ml, d, p.nsplit, p.scale));
     }
-    return launch_chain(m, mla_out_kernel<WT>, dim3(d.heads, (d.vdim + 31) / 32), dim3(256), (d.latent + p.nsplit) * sizeof(float), (const float*)p.part_acc,
+    return launch_chain(m, mla_out_kernel<WT>, dim3(d.heads, (d.vdim + 31) / 32), dim3(256), (d.latent + 2 * p.nsplit) * sizeof(float), (const float*)p.part_acc,
                         (const float*)p.part_ml, (const WT*)p.wuv, p.out, (const DevState*)m->st, d, p.nsplit, mma ? MLA_MMA_TILE : MLA_TILE);
 #undef TRY
 }

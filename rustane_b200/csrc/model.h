@@ -104,6 +104,7 @@ struct cd_moe_state {
     unsigned int* router_counter = nullptr;
     int *loc_ids = nullptr, *n_loc = nullptr;
     void* qsplit = nullptr;         // [2][16][latent + rope] in the cache's type: the absorbed query as a 16-bit head and a 16-bit remainder
+    float* route_part = nullptr;    // [CTAs of the Wo GEMV][experts]: their shares of the logits (EpiResidualRoute)
     bool stream_ffn = false;        // the experts' rows go through the streamed GEMV (else: the plain-load kernels)
 };
 

@@ -83,6 +83,31 @@ void moe_release(cd_model* m) {
     m->moe = nullptr;
 }
 
+// How moe_gate_kernel takes a model's rows (eight rows a stage, fewer where a thread holds several chunks of x: with four, 16 KB, one thread could not issue copies as fast as HBM answers); nstages 0: it does not.
+struct GateShape {
+    int niter, rows_cap, nstages;
+    size_t smem;
+};
+template <typename WT>
+GateShape gate_shape(const cd_model* m) {
+    const cd_moe_state& S = *m->moe;
+    GateShape g{(m->cfg.dim / Elem<WT>::EPC + 255) / 256, 2 * (S.shared_cols / m->sm_count + 1 + S.mc.top_k * m->cfg.hidden / m->sm_count + 1), 0, 0};
+    const size_t stage = (size_t)(g.niter == 1 ? 8 : g.niter == 2 ? 4 : 2) * m->cfg.dim * sizeof(WT), fixed = moe_gate_fixed_bytes(g.rows_cap);
+    const size_t budget = (size_t)m->ring_kb * 1024;
+    if (g.niter > 4 || S.mc.n_experts > MOE_GATE_MAX_EXPERTS || fixed + 2 * stage > budget) return g;
+    g.nstages = (int)std::min<size_t>(8, (budget - fixed) / stage);
+    g.smem = std::max(g.nstages * stage + fixed, (size_t)116 * 1024);  // (at least half an SM's, as every streamed GEMV)
+    return g;
+}
+template <typename WT>
+cudaError_t launch_gate(cd_model* m, const MoeGate& p, const GateShape& g) {
+    auto go = [&](auto kern) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
+        return e != cudaSuccess ? e : launch_chain(m, kern, dim3(m->sm_count), dim3(GEMV_TMA_THREADS), g.smem, p);
+    };
+    return g.niter == 1 ? go(moe_gate_kernel<WT, 1, 8>) : g.niter == 2 ? go(moe_gate_kernel<WT, 2, 4>) : go(moe_gate_kernel<WT, 4, 2>);
+}
+
 // One token through the MoE + MLA decoder (moe.cuh).  WT: storage of all weights; KT: storage of the latent cache.
 template <typename WT, typename KT>
 cudaError_t enqueue_step_moe_t(cd_model* m, const cd_step& p) {
@@ -114,16 +139,43 @@ cudaError_t enqueue_step_moe_t(cd_model* m, const cd_step& p) {
         w2_set = (size_t)units * 4;
     }
     const uint32_t es = (uint32_t)sizeof(WT);
+    // the next GEMV's first rows, pulled into L2 behind a GEMV's own last loads
+    auto hint = [&](const void* w, int K, int N, int unit) {
+        m->next_stream = NextStream{m->prefetch_kb > 0 ? w : nullptr, Wfmt<WT>::row_stride(K), N / unit, unit, (uint32_t)m->prefetch_kb * 1024u};
+    };
+    // one GPU: the router's work goes into the kernels around it
+    const GateShape gate = gate_shape<WT>(m);
+    const bool fused_route = !ep && S.stream_ffn && gate.nstages > 0;
     for (int l = 0; l < c.nlayers; ++l) {
         const cd_moe_layer_dev& L = S.layers[l];
         int* sel = S.sel_ids + (size_t)l * mc.top_k;
         m->cur_cls = CLS_QKV;
+        hint(L.wo, c.heads * mc.v_dim, c.dim, 1);
         if (ep && l > 0) { m->tp_in.in_reduce = l; m->tp_in.res = m->x_b; m->tp_in.x_out = m->x_a; }  // x = x2 + alpha * sum(ranks' FFN partials)
         TRY((launch_gemv<WT, 1, true>(m, L.wqa, m->x_a, L.gamma1, nullptr, QA, c.dim, EpiStore{S.qa})));
         m->cur_cls = CLS_ATTN;
         TRY((launch_mla<WT, KT>(m, MlaStep{md, S.qa, L.wuk_t, L.wuv_t, L.gamma_kv, Rotation{m->rope, nullptr, mc.rope_dim}, m->layers[l].kv, S.qabs, S.qsplit,
                                            S.part_acc, S.part_ml, m->attn, S.nsplit, scale})));
         m->cur_cls = CLS_WO;
+        const SrcExpertCols s2{S.loc_ids, S.n_loc, L.ws2, c.hidden, S.shared_cols, c.dim, (uint32_t)c.hidden * es, (uint32_t)S.shared_cols * es};
+        auto hint_next = [&]() {
+            if (l + 1 < c.nlayers) hint(S.layers[l + 1].wqa, c.dim, QA, 1);
+            else if (p.head != HEAD_NONE) hint(m->lm_head, c.dim, m->v_loc, 1);
+        };
+        if (fused_route) {
+            const int wo_ctas = std::min(c.dim, m->sm_count);
+            const size_t row = (size_t)units * es;
+            const MoeGate g{L.w13, L.ws13, m->x_b, L.gamma2, S.route_part, wo_ctas, c.dim, c.hidden, S.shared_cols, RouteRule{mc.n_experts, mc.top_k, 1, 1}, sel, S.sel_w,
+                      S.loc_ids, S.n_loc, S.gate, gate.nstages, gate.rows_cap, &m->st->error, L.w2, L.ws2, (int)((size_t)m->prefetch_kb * 1024 / row)};
+            TRY((launch_gemv<WT, 1, false>(m, L.wo, m->attn, nullptr, nullptr, c.dim, c.heads * mc.v_dim,
+                                           EpiResidualRoute<WT>{m->x_a, m->x_b, m->alpha, L.gamma2, (const WT*)L.wr, S.route_part, c.dim, mc.n_experts})));
+            m->cur_cls = CLS_W13;
+            TRY(launch_gate<WT>(m, g, gate));
+            m->cur_cls = CLS_W2;
+            hint_next();
+            TRY((launch_gemv<WT, 1, false>(m, L.w2, S.gate, nullptr, nullptr, c.dim, units, EpiResidual{m->x_b, m->x_a, m->alpha}, s2)));
+            continue;
+        }
         TRY((launch_gemv<WT, 1, false>(m, L.wo, m->attn, nullptr, nullptr, c.dim, c.heads * mc.v_dim, EpiResidual{m->x_a, m->x_b, m->alpha})));
         m->cur_cls = CLS_W13;
         TRY(launch_chain(m, moe_router_kernel<WT, RouterRmsIn>, dim3((mc.n_experts + 3) / 4), dim3(128), std::max(c.dim, mc.n_experts + 1) * sizeof(float),
@@ -136,7 +188,7 @@ cudaError_t enqueue_step_moe_t(cd_model* m, const cd_step& p) {
             const SrcExpertRows s13{S.loc_ids, S.n_loc, L.ws13, 2 * c.hidden, 2 * S.shared_cols};
             TRY((launch_gemv<WT, 2, false>(m, L.w13, S.xn2, nullptr, nullptr, 2 * units, c.dim, EpiGateMoe{S.gate, S.loc_w, S.n_loc, c.hidden}, s13)));
             m->cur_cls = CLS_W2;
-            const SrcExpertCols s2{S.loc_ids, S.n_loc, L.ws2, c.hidden, S.shared_cols, c.dim, (uint32_t)c.hidden * es, (uint32_t)S.shared_cols * es};
+            hint_next();
             if (ep) TRY((launch_gemv<WT, 1, false>(m, L.w2, S.gate, nullptr, nullptr, c.dim, units, EpiPush{tp}, s2)));
             else TRY((launch_gemv<WT, 1, false>(m, L.w2, S.gate, nullptr, nullptr, c.dim, units, EpiResidual{m->x_b, m->x_a, m->alpha}, s2)));
         } else {
@@ -253,7 +305,7 @@ extern "C" int cd_moe_model_create_synthetic(const cd_config* cfg, const cd_moe_
     const size_t o_qa = carve((H * QH + C + R) * 4), o_qabs = carve(H * (C + R) * 4), o_pacc = carve((size_t)S->nsplit * H * C * 4);
     const size_t o_pml = carve((size_t)S->nsplit * H * 2 * 4), o_xn = carve(D * 4), o_sel = carve((size_t)c.nlayers * moe->top_k * 4), o_selw = carve(moe->top_k * 4);
     const size_t o_gate = carve(units * 4);
-    const size_t o_rl = carve((size_t)moe->n_experts * 4), o_rc = carve(4), o_lid = carve(SRC_MAX_LIST * 4), o_lw = carve(SRC_MAX_LIST * 4), o_nl = carve(4), o_qs = carve(32 * (C + R) * 2);
+    const size_t o_rl = carve((size_t)moe->n_experts * 4), o_rc = carve(4), o_lid = carve(SRC_MAX_LIST * 4), o_lw = carve(SRC_MAX_LIST * 4), o_nl = carve(4), o_qs = carve(32 * (C + R) * 2), o_rp = carve((size_t)m->sm_count * moe->n_experts * 4);
     e = cudaMalloc(&S->ws, off);
     if (e == cudaSuccess) e = cudaMemsetAsync(S->ws, 0, off, m->stream);
     if (e != cudaSuccess) { fail(m, CD_ERR_CUDA, std::string("MoE scratch: ") + cudaGetErrorString(e)); return bail(CD_ERR_CUDA); }
@@ -261,7 +313,7 @@ extern "C" int cd_moe_model_create_synthetic(const cd_config* cfg, const cd_moe_
     S->qa = (float*)(ws + o_qa); S->qabs = (float*)(ws + o_qabs); S->part_acc = (float*)(ws + o_pacc); S->part_ml = (float*)(ws + o_pml);
     S->xn2 = (float*)(ws + o_xn); S->sel_ids = (int*)(ws + o_sel); S->sel_w = (float*)(ws + o_selw); S->gate = (float*)(ws + o_gate);
     S->router_logits = (float*)(ws + o_rl); S->router_counter = (unsigned int*)(ws + o_rc); S->loc_ids = (int*)(ws + o_lid);
-    S->loc_w = (float*)(ws + o_lw); S->n_loc = (int*)(ws + o_nl); S->qsplit = ws + o_qs;
+    S->loc_w = (float*)(ws + o_lw); S->n_loc = (int*)(ws + o_nl); S->qsplit = ws + o_qs; S->route_part = (float*)(ws + o_rp);
     {
         // the streamed GEMV takes the expert matrices when a thread's share of the widest row fits its registers
         // (at most eight 16-byte chunks of x per thread) and every piece of a gathered row is a whole number of 16 bytes

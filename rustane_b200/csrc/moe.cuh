@@ -20,7 +20,7 @@
 //                        sum is pushed to every rank's inbox instead (the dense model's all-reduce)
 // All of them are HBM-bound streams of weight rows (or cache rows) with fp32 accumulation.
 #pragma once
-#include "common.cuh"
+#include "kernels.cuh"
 
 namespace cd {
 
@@ -195,16 +195,16 @@ mla_post_kernel(const float* __restrict__ qa, const WT* __restrict__ wuk_t, cons
         put(h, r % C, acc);
         return;
     }
-    pdl_wait();
-    pdl_launch_dependents();
-    const int pos = __ldcg(&st->pos);
+    const int pos = __ldcg(&st->pos);  // (older than the kernel ahead, and so are the rotations, the page and gamma)
     if (blockIdx.x + 1 < gridDim.x) {  // rotation of q's part of it
         const int i = 2 * (((int)blockIdx.x - n_absorb) * (int)blockDim.x + tid), h = i / R, k = i % R;
+        const float2 cs = i < H * R && k < rot.dims ? rot.at(pos, k >> 1) : make_float2(1.0f, 0.0f);
+        pdl_wait();
+        pdl_launch_dependents();
         if (i >= H * R) return;
         const float* q = qa + (size_t)h * QH + d.nope_n;
         float u = k < d.rope_n ? __ldcg(q + k) : 0.0f, v = k + 1 < d.rope_n ? __ldcg(q + k + 1) : 0.0f;
         if (k < rot.dims) {
-            const float2 cs = rot.at(pos, k >> 1);
             const float t = u * cs.x - v * cs.y;
             v = v * cs.x + u * cs.y;
             u = t;
@@ -217,23 +217,42 @@ mla_post_kernel(const float* __restrict__ qa, const WT* __restrict__ wuk_t, cons
     const float* craw = qa + (size_t)H * QH;
     float2* cs = reinterpret_cast<float2*>(sm + ((C + 1) & ~1));  // [dims / 2]
     auto cs_of = [&](int k) { return cs[k]; };
-    float ss = 0.0f;
-#pragma unroll 8
-    for (int i = tid; i < d.latent_n; i += blockDim.x) {
-        const float v = __ldcg(craw + i);
-        sm[i] = v;
-        ss += v * v;
-    }
     rot.fill(cs, pos);
-    const float tot = block_sum(ss, red);
-    const float inv = 1.0f / sqrtf(tot * (1.0f / (float)d.latent_n) + d.eps);
     const int page = page_table[pos / d.page_tokens], off = pos % d.page_tokens;
     KT* row = lat_pool + ((size_t)page * d.page_tokens + off) * (C + R);
-    for (int i = tid; i < C; i += blockDim.x) row[i] = Elem<KT>::from_f32(i < d.latent_n ? sm[i] * inv * gamma_kv[i] : 0.0f);
+    constexpr int B = 4;  // entries of a thread in flight
+    float gm[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) gm[b] = tid + 128 * b < d.latent_n ? gamma_kv[tid + 128 * b] : 0.0f;
+    pdl_wait();
+    pdl_launch_dependents();
+    float ss = 0.0f;
+    const float key = tid < d.rope_n ? __ldcg(craw + d.latent_n + tid) : 0.0f;
+    for (int i0 = tid; i0 < d.latent_n; i0 += 128 * B) {
+        float v[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) v[b] = i0 + 128 * b < d.latent_n ? __ldcg(craw + i0 + 128 * b) : 0.0f;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            if (i0 + 128 * b < d.latent_n) sm[i0 + 128 * b] = v[b];
+            ss += v[b] * v[b];
+        }
+    }
+    float* keys = reinterpret_cast<float*>(cs + (rot.dims + 1) / 2);  // [min(rope_n, 128)]
+    if (tid < d.rope_n) keys[tid] = key;
+    const float tot = block_sum(ss, red);
+    const float inv = 1.0f / sqrtf(tot * (1.0f / (float)d.latent_n) + d.eps);
+    for (int i0 = tid; i0 < C; i0 += 128 * B) {
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int i = i0 + 128 * b;
+            if (i < C) row[i] = Elem<KT>::from_f32(i < d.latent_n ? sm[i] * inv * (i0 == tid ? gm[b] : gamma_kv[i]) : 0.0f);
+        }
+    }
     for (int i = tid; i < R; i += blockDim.x)
-        row[C + i] = Elem<KT>::from_f32(i < d.rope_n ? rot.entry(i, cs_of, [&](int j) { return __ldcg(craw + d.latent_n + j); }) : 0.0f);
+        row[C + i] = Elem<KT>::from_f32(i < d.rope_n ? rot.entry(i, cs_of, [&](int j) { return j < 128 ? keys[j] : __ldcg(craw + d.latent_n + j); }) : 0.0f);
 }
-__host__ __device__ inline size_t mla_post_smem_floats(const MlaDims& d) { return max((128 / d.latent + 2) * d.nope, d.latent + 2 + d.rope); }
+__host__ __device__ inline size_t mla_post_smem_floats(const MlaDims& d) { return max((128 / d.latent + 2) * d.nope, d.latent + 4 + d.rope + min(d.rope_n, 128)); }
 __host__ __device__ inline int mla_post_ctas(const MlaDims& d) { return (d.heads * d.latent + 127) / 128 + (d.heads * d.rope + 255) / 256 + 1; }
 
 // ---------------------------------------------------------------------- latent attention, one slice of cached positions per CTA
@@ -347,56 +366,104 @@ template <typename WT>
 __global__ void __launch_bounds__(256)
 mla_out_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, const WT* __restrict__ wuv_t, float* __restrict__ attn_out,
                const DevState* st, MlaDims d, int nsplit_max, int tile) {
-    extern __shared__ float sm[];  // [C] the head's latent-space output, then [nsplit] slice weights
+    extern __shared__ float sm[];  // [C] the head's latent-space output, then [nsplit] slice weights and [nsplit] weighted sums
     constexpr float NEG = -3.402823466e+38f;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;  // eight warps
     const int H = d.heads, C = d.latent, V = d.vdim, h = blockIdx.x;
     float* lat = sm;
-    float* wsl = sm + C;
+    float *wsl = sm + C, *lsl = wsl + nsplit_max;
     __shared__ float s_inv;
+    // this CTA's 32 output rows of the head: four rows per warp, requested before the kernel ahead has ended
+    constexpr int EPC = Elem<WT>::EPC, PRE = 2;
+    const int dv0 = blockIdx.y * 32 + warp * 4, nchunks = C / EPC;
+    const bool early = dv0 + 4 <= V && nchunks <= 32 * PRE;
+    uint4 w[4][PRE];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < PRE; ++i)
+            w[r][i] = early && lane + 32 * i < nchunks ? ldg_stream(reinterpret_cast<const char*>(wuv_t + ((size_t)h * V + dv0 + r) * C) + (size_t)(lane + 32 * i) * 16)
+                                                       : make_uint4(0, 0, 0, 0);
     pdl_wait();
     pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
     // the attention kernel's split of this context: slices of `per` positions, the first `nsplit` of them hold any
     const int pos = __ldcg(&st->pos), per = d.slice(pos, nsplit_max, tile);
     const int nsplit = (pos - d.first_seen(pos)) / per + 1;
+    // the first entries of the head's column in every slice are requested together with the slices' maxima and sums
+    constexpr int B = 8;  // slices in flight
+    const float* pa = part_acc + (size_t)h * C;
+    auto load = [&](int s0, int c, float2 (&v)[B]) {
+#pragma unroll
+        for (int b = 0; b < B; ++b) v[b] = s0 + b < nsplit ? __ldcg(reinterpret_cast<const float2*>(pa + (size_t)(s0 + b) * H * C + c)) : make_float2(0.f, 0.f);
+    };
+    float2 first[B];
+    if (2 * tid < C) load(0, 2 * tid, first);
     if (warp == 0) {
         float M = NEG;
         for (int s = lane; s < nsplit; s += 32) {
             const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml) + (size_t)s * H + h);
-            if (ml.y > 0.0f) M = fmaxf(M, ml.x);
+            wsl[s] = ml.y > 0.0f ? ml.x : NEG;
+            lsl[s] = ml.y;
+            M = fmaxf(M, wsl[s]);
         }
         M = warp_max(M);
         for (int s = lane; s < nsplit; s += 32) {
-            const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml) + (size_t)s * H + h);
-            wsl[s] = ml.y > 0.0f ? expf(ml.x - M) : 0.0f;
+            wsl[s] = lsl[s] > 0.0f ? expf(wsl[s] - M) : 0.0f;
+            lsl[s] *= wsl[s];
         }
         // the slices' sums are added in slice order by one lane, so the result does not depend on the lane count
         __syncwarp();
         if (lane == 0) {
             float tot = 0.0f;
-            for (int s = 0; s < nsplit; ++s) {
-                const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml) + (size_t)s * H + h);
-                tot += ml.y * wsl[s];
-            }
+            for (int s = 0; s < nsplit; ++s) tot += lsl[s];
             s_inv = tot > 0.0f ? 1.0f / tot : 0.0f;
         }
     }
     __syncthreads();
     for (int c = 2 * tid; c < C; c += 2 * blockDim.x) {  // C is even
         float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll 16
-        for (int s = 0; s < nsplit; ++s) {  // slice order
-            const float2 v = __ldcg(reinterpret_cast<const float2*>(part_acc + ((size_t)s * H + h) * C + c));
-            a0 = fmaf(v.x, wsl[s], a0);
-            a1 = fmaf(v.y, wsl[s], a1);
+        for (int s0 = 0; s0 < nsplit; s0 += B) {  // slice order
+            float2 v[B];
+            if (s0 == 0 && c == 2 * tid) {
+#pragma unroll
+                for (int b = 0; b < B; ++b) v[b] = first[b];
+            } else {
+                load(s0, c, v);
+            }
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                if (s0 + b < nsplit) {
+                    a0 = fmaf(v[b].x, wsl[s0 + b], a0);
+                    a1 = fmaf(v[b].y, wsl[s0 + b], a1);
+                }
+            }
         }
         lat[c] = a0 * s_inv;
         lat[c + 1] = a1 * s_inv;
     }
     __syncthreads();
-    // this CTA's 32 output rows of the head: four rows per warp, their loads in flight together
-    const int dv0 = blockIdx.y * 32 + warp * 4;
-    if (dv0 + 4 <= V) {
+    if (early) {
+        float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < PRE; ++i) {
+            const int c = lane + 32 * i;
+            if (c < nchunks) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    float f[EPC];
+                    Elem<WT>::unpack(w[r][i], f);
+#pragma unroll
+                    for (int e = 0; e < EPC; e += 4) {
+                        const float4 x4 = *reinterpret_cast<const float4*>(lat + c * EPC + e);
+                        y[r] = fmaf(f[e], x4.x, y[r]); y[r] = fmaf(f[e + 1], x4.y, y[r]); y[r] = fmaf(f[e + 2], x4.z, y[r]); y[r] = fmaf(f[e + 3], x4.w, y[r]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) y[r] = warp_sum(y[r]);
+        if (lane < 4) attn_out[(size_t)h * V + dv0 + lane] = lane == 0 ? y[0] : lane == 1 ? y[1] : lane == 2 ? y[2] : y[3];
+    } else if (dv0 + 4 <= V) {  // their loads in flight together
         float y[4];
         warp_rows_dot<WT, 4>(wuv_t + ((size_t)h * V + dv0) * C, (size_t)C, lat, C, lane, y);
         if (lane < 4) attn_out[(size_t)h * V + dv0 + lane] = lane == 0 ? y[0] : lane == 1 ? y[1] : lane == 2 ? y[2] : y[3];
@@ -471,29 +538,44 @@ mla_attn_mma_kernel(const KT* __restrict__ qsplit, const KT* __restrict__ lat_po
     const uint32_t rows = smem_addr(rows_p), qh = smem_addr(qh_p), ql = smem_addr(ql_p), bar = smem_addr(bar_p);
     const uint32_t pha = smem_addr(ph), pla = smem_addr(pl);
 
-    pdl_wait();
-    pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
+    // the position and the cached rows but the newest are older than the kernel ahead (which works out q and that row): the first
+    // tile's are requested before it has ended
     const int pos = __ldcg(&st->pos), per = d.slice(pos, nsplit, T);
     const int t0 = d.first_seen(pos) + s * per, t1 = min(pos + 1, t0 + per);
-    if (t0 >= t1) return;  // a slice past the context: mla_out_kernel merges the slices that hold positions only
+    if (t0 >= t1) {  // a slice past the context: mla_out_kernel merges the slices that hold positions only
+        pdl_wait();
+        return;
+    }
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_fence_init();
     }
     if (tid < 16) { mrun[tid] = NEG; lrun[tid] = 0.0f; corr[tid] = 0.0f; }
     __syncthreads();
-    auto fetch = [&](int tb, bool with_q) {  // warp 0: one bulk copy per cached row of the tile (and per row of q)
-        const int nt = min(T, t1 - tb);
-        if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(nt + (with_q ? 32 : 0)) * (uint32_t)W * 2u);
-        __syncwarp();
-        // q as mla_post_kernel left it: 16 rows of 16-bit heads, 16 rows of remainders (rows of heads that do not exist are zero)
-        if (with_q) bulk_g2s(qh + (uint32_t)lane * LDB, qsplit + (size_t)lane * W, (uint32_t)W * 2u, bar);
-        for (int j = lane; j < nt; j += 32) {
-            const int t = tb + j, page = page_table[t / d.page_tokens], off = t % d.page_tokens;
-            bulk_g2s(rows + (uint32_t)j * LDB, lat_pool + ((size_t)page * d.page_tokens + off) * W, (uint32_t)W * 2u, bar);
-        }
+    auto fetch_row = [&](int tb, int j) {
+        const int t = tb + j, page = page_table[t / d.page_tokens], off = t % d.page_tokens;
+        bulk_g2s(rows + (uint32_t)j * LDB, lat_pool + ((size_t)page * d.page_tokens + off) * W, (uint32_t)W * 2u, bar);
     };
-    if (warp == 0) fetch(t0, true);
+    if (warp == 0) {  // one bulk copy per cached row of the tile (and per row of q)
+        const int nt = min(T, t1 - t0);
+        if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(nt + 32) * (uint32_t)W * 2u);
+        __syncwarp();
+        for (int j = lane; j < nt; j += 32)
+            if (t0 + j < pos) fetch_row(t0, j);
+    }
+    pdl_wait();
+    pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
+    if (warp == 0) {
+        // q as mla_post_kernel left it: 16 rows of 16-bit heads, 16 rows of remainders (rows of heads that do not exist are zero)
+        bulk_g2s(qh + (uint32_t)lane * LDB, qsplit + (size_t)lane * W, (uint32_t)W * 2u, bar);
+        if (lane == 0 && pos >= t0 && pos < t0 + T && pos < t1) fetch_row(t0, pos - t0);
+    }
+    auto fetch = [&](int tb) {  // warp 0
+        const int nt = min(T, t1 - tb);
+        if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)nt * (uint32_t)W * 2u);
+        __syncwarp();
+        for (int j = lane; j < nt; j += 32) fetch_row(tb, j);
+    };
     float acc[CW / 8][4];  // columns col0 + 8 nb + 2 (lane % 4) + {0, 1} of heads lane / 4 and lane / 4 + 8
 #pragma unroll
     for (int nb = 0; nb < CW / 8; ++nb) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.0f;
@@ -509,7 +591,7 @@ mla_attn_mma_kernel(const KT* __restrict__ qsplit, const KT* __restrict__ lat_po
         __syncthreads();  // the zero rows are in place
         // ---- scores of positions 16 warp .. 16 warp + 15
         const int j0 = 16 * warp;
-        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+        float c0[4] = {}, c1[4] = {}, d0[4] = {}, d1[4] = {};  // (the parts' sums apart: half the chain of dependent MMAs)
         if (j0 < nt) {
             const uint32_t a_off = (uint32_t)(lane & 15) * LDB + (uint32_t)(lane >> 4) * 16u;
             const uint32_t b_off = (uint32_t)(j0 + (lane & 7) + 8 * (lane >> 4)) * LDB + (uint32_t)((lane >> 3) & 1) * 16u;
@@ -520,11 +602,13 @@ mla_attn_mma_kernel(const KT* __restrict__ qsplit, const KT* __restrict__ lat_po
                 ldsm_x4(al, ql + a_off + (uint32_t)ks * 32u);
                 ldsm_x4(b, rows + b_off + (uint32_t)ks * 32u);
                 Mma16<KT>::mma(c0, ah, b[0], b[1]);
-                Mma16<KT>::mma(c0, al, b[0], b[1]);
+                Mma16<KT>::mma(d0, al, b[0], b[1]);
                 Mma16<KT>::mma(c1, ah, b[2], b[3]);
-                Mma16<KT>::mma(c1, al, b[2], b[3]);
+                Mma16<KT>::mma(d1, al, b[2], b[3]);
             }
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { c0[i] += d0[i]; c1[i] += d1[i]; }
         {
             const int ja = j0 + 2 * tq, jb = j0 + 8 + 2 * tq;
             sc[g * LDS + ja] = c0[0] * scale;       sc[g * LDS + ja + 1] = c0[1] * scale;
@@ -592,7 +676,7 @@ mla_attn_mma_kernel(const KT* __restrict__ qsplit, const KT* __restrict__ lat_po
             }
         }
         __syncthreads();  // every warp is done with the tile's rows
-        if (warp == 0 && tb + T < t1) fetch(tb + T, false);
+        if (warp == 0 && tb + T < t1) fetch(tb + T);
     }
 #pragma unroll
     for (int nb = 0; nb < CW / 8; ++nb) {
@@ -841,6 +925,223 @@ moe_w13_kernel(const float* __restrict__ xn, const WT* __restrict__ w13, const W
         float y[2];
         warp_rows_dot<WT, 2>(rows, (size_t)d.dim, xs, d.dim, lane, y);
         if (lane == 0) gate[u] = (y[0] / (1.0f + expf(-y[0]))) * y[1] * weight;
+    }
+}
+
+// ---------------------------------------------------------------------- router's choice and the experts' gate in one kernel
+// For a GPU that holds all experts: gate[u] as above, the weights streamed as in gemv_tma_kernel (kernels.cuh: one CTA per SM,
+// a producer that keeps a ring of stages of R rows full, eight consumer warps).  A CTA takes its share of the shared FFN's
+// rows first - they do not depend on the choice and are requested before the kernel ahead has ended - and of the chosen experts'
+// behind them.  The consumers form the normed input and add the CTAs' shares of the logits up (EpiResidualRoute); the
+// producer's warp then applies the routing rule while they work on the shared rows.  Every CTA makes the same choice from the
+// same sums; CTA 0 leaves it in memory.
+// What bounds it: HBM (92 MB a layer of configuration 5) behind the chain wait - shares - choice - first expert rows.
+struct MoeGate {
+    const void *w13, *ws13;       // [experts][2 hidden][dim], [2 shared_cols][dim]
+    const float *x, *gamma;       // the residual stream and its norm
+    const float* route_part;      // [nparts][experts]
+    int nparts, dim, hidden, shared_cols;
+    RouteRule rule;
+    int* sel_ids;                 // what CTA 0 leaves: the choice and its scores, and the same as the list that the W2 GEMV walks
+    float* sel_w;
+    int *loc_ids, *n_loc;
+    float* gate;
+    int nstages, rows_cap, *err;
+    // W2's rows, of which every CTA requests its first `ahead_rows` into L2 behind its own last loads
+    const void *w2, *ws2;
+    int ahead_rows;
+};
+constexpr int MOE_GATE_MAX_EXPERTS = 256, MOE_GATE_MAX_TOP = 16;
+__host__ __device__ inline size_t moe_gate_fixed_bytes(int rows_cap) {
+    return ((size_t)rows_cap * (GEMV_CONSUMERS / 32) + 256 + MOE_GATE_MAX_EXPERTS + 1 + 31) * sizeof(float) + 2 * 8 * 8 + 128;
+}
+
+template <typename WT, int NITER, int R>
+__global__ void __launch_bounds__(GEMV_TMA_THREADS, 1) moe_gate_kernel(const __grid_constant__ MoeGate p) {
+    constexpr int EPC = Elem<WT>::EPC, NW = GEMV_CONSUMERS / 32;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    __shared__ int list[MOE_GATE_MAX_TOP];
+    __shared__ float weight[MOE_GATE_MAX_TOP], red[32], s_inv;
+    const uint32_t row_bytes = (uint32_t)p.dim * (uint32_t)sizeof(WT), stage_bytes = R * row_bytes;
+    const int E = p.rule.experts, parts = 256 / E;  // threads that add up one expert's shares
+    float* partial = reinterpret_cast<float*>(smraw + (size_t)p.nstages * stage_bytes);  // [rows_cap][NW]
+    float* sums = partial + (size_t)p.rows_cap * NW;                                     // [parts][E]
+    float* scores = sums + 256;                                                          // [E], one group behind them
+    uint64_t* bars = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(scores + MOE_GATE_MAX_EXPERTS + 1) + 15) & ~(uintptr_t)15);
+    const uint32_t ring = smem_addr(smraw), full0 = smem_addr(bars), empty0 = full0 + 8u * p.nstages;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bid = blockIdx.x, nblk = gridDim.x;
+    const int nunits = p.rule.top * p.hidden;
+    const int su0 = (int)((long long)bid * p.shared_cols / nblk), su1 = (int)((long long)(bid + 1) * p.shared_cols / nblk);
+    const int eu0 = (int)((long long)bid * nunits / nblk), eu1 = (int)((long long)(bid + 1) * nunits / nblk);
+    const int ns = 2 * (su1 - su0), ne = 2 * (eu1 - eu0);  // rows
+    const int gs = (ns + R - 1) / R, ngroups = gs + (ne + R - 1) / R;
+    if (tid == 0) {
+        for (int s = 0; s < p.nstages; ++s) {
+            mbar_init(full0 + 8u * s, 1);
+            mbar_init(empty0 + 8u * s, NW);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    auto both_bar = [](int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(GEMV_TMA_THREADS) : "memory"); };
+
+    if (warp == NW) {  // ---- producer
+        const uint64_t policy = l2_evict_first_policy();
+        auto put = [&](int g) {  // one lane
+            const uint32_t dst = ring + (uint32_t)(g % p.nstages) * stage_bytes, full = full0 + 8u * (g % p.nstages);
+            const bool shared = g < gs;
+            const int row0 = (shared ? g : g - gs) * R, rows = min(R, (shared ? ns : ne) - row0);
+            mbar_arrive_expect_tx(full, (uint32_t)rows * row_bytes);
+            if (shared) {
+                bulk_g2s_stream(dst, reinterpret_cast<const char*>(p.ws13) + (size_t)(2 * su0 + row0) * row_bytes, (uint32_t)rows * row_bytes, full, policy);
+                return;
+            }
+            const int seg = 2 * p.hidden, v0 = 2 * eu0 + row0;
+            auto addr = [&](int v) { return reinterpret_cast<const char*>(p.w13) + ((size_t)list[v / seg] * seg + (size_t)(v % seg)) * row_bytes; };
+            if (v0 / seg == (v0 + rows - 1) / seg) {
+                bulk_g2s_stream(dst, addr(v0), (uint32_t)rows * row_bytes, full, policy);
+            } else {
+                for (int j = 0; j < rows; ++j) bulk_g2s_stream(dst + (uint32_t)j * row_bytes, addr(v0 + j), row_bytes, full, policy);
+            }
+        };
+        const int early = min(gs, p.nstages);
+        if (lane == 0)
+            for (int g = 0; g < early; ++g) put(g);
+        __syncwarp();
+        pdl_wait();
+        both_bar(9);  // the logits' sums and the norm's factor are there
+        for (int e = lane; e < E; e += 32) {
+            float t = 0.0f;
+            for (int k = 0; k < parts; ++k) t += sums[k * E + e];
+            scores[e] = t * s_inv;
+        }
+        __syncwarp();
+        route_pick(scores, scores + E, p.rule, lane, [&](int k, int bi, float bv) {
+            if (lane == 0) {
+                list[k] = bi;
+                weight[k] = bv;
+                if (bid == 0) { p.sel_ids[k] = bi; p.sel_w[k] = bv; p.loc_ids[k] = bi; }
+            }
+        });
+        if (bid == 0 && lane == 0) *p.n_loc = p.rule.top;
+        __syncwarp();
+        asm volatile("bar.arrive 10, %0;" ::"r"(GEMV_TMA_THREADS) : "memory");
+        if (lane == 0) {
+            for (int g = early; g < ngroups; ++g) {
+                if (g >= p.nstages && !mbar_wait(empty0 + 8u * (g % p.nstages), ((g / p.nstages) - 1) & 1)) {
+                    atomicExch(p.err, DEV_ERR_EMPTY_WAIT);
+                    break;
+                }
+                put(g);
+            }
+        }
+        __syncwarp();
+        const int r0 = (int)((long long)bid * p.dim / nblk), n = min((int)((long long)(bid + 1) * p.dim / nblk) - r0, p.ahead_rows);
+        const uint32_t piece = (uint32_t)p.hidden * (uint32_t)sizeof(WT), tail = (uint32_t)p.shared_cols * (uint32_t)sizeof(WT);
+        for (int i = lane; i < n * (p.rule.top + 1); i += 32) {
+            const int r = r0 + i / (p.rule.top + 1), k = i % (p.rule.top + 1);
+            if (k < p.rule.top) bulk_prefetch_l2(reinterpret_cast<const char*>(p.w2) + ((size_t)list[k] * p.dim + r) * piece, piece);
+            else if (tail) bulk_prefetch_l2(reinterpret_cast<const char*>(p.ws2) + (size_t)r * tail, tail);
+        }
+        return;
+    }
+
+    // ---- consumers
+    const int nchunks = p.dim / EPC;
+    float xr[NITER][EPC], gm[NITER][EPC];
+#pragma unroll
+    for (int i = 0; i < NITER; ++i) {
+        const int c = tid + i * GEMV_CONSUMERS;
+#pragma unroll
+        for (int e = 0; e < EPC; e += 4) {
+            const float4 g = c < nchunks ? *reinterpret_cast<const float4*>(p.gamma + (size_t)c * EPC + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            gm[i][e] = g.x; gm[i][e + 1] = g.y; gm[i][e + 2] = g.z; gm[i][e + 3] = g.w;
+        }
+    }
+    pdl_wait();
+    pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NITER; ++i) {
+        const int c = tid + i * GEMV_CONSUMERS;
+#pragma unroll
+        for (int e = 0; e < EPC; e += 4) {
+            const float4 v = c < nchunks ? __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)c * EPC + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
+        }
+    }
+    if (tid < parts * E) {
+        const float* at = p.route_part + tid % E;
+        float t = 0.0f;
+        constexpr int B = 40;  // in flight: all of them at 64 experts and 148 CTAs (as a loop of 20 and its remainder one by one: 10 us)
+        for (int k0 = tid / E; k0 < p.nparts; k0 += B * parts) {
+            float v[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) v[b] = k0 + b * parts < p.nparts ? __ldcg(at + (size_t)(k0 + b * parts) * E) : 0.0f;
+#pragma unroll
+            for (int b = 0; b < B; ++b) t += v[b];
+        }
+        sums[tid] = t;
+    }
+#pragma unroll
+    for (int i = 0; i < NITER; ++i)
+#pragma unroll
+        for (int e = 0; e < EPC; e += 4) ss += xr[i][e] * xr[i][e] + xr[i][e + 1] * xr[i][e + 1] + xr[i][e + 2] * xr[i][e + 2] + xr[i][e + 3] * xr[i][e + 3];
+    const float inv = 1.0f / sqrtf(consumer_sum(ss, red) * (1.0f / (float)p.dim) + RMS_EPS);
+    if (tid == 0) s_inv = inv;
+    both_bar(9);
+#pragma unroll
+    for (int i = 0; i < NITER; ++i)
+#pragma unroll
+        for (int e = 0; e < EPC; ++e) xr[i][e] = xr[i][e] * inv * gm[i][e];
+
+    bool ok = true;
+    for (int g = 0; g < ngroups; ++g) {
+        const int s = g % p.nstages;
+        if (!mbar_wait(full0 + 8u * s, (g / p.nstages) & 1)) {
+            atomicExch(p.err, DEV_ERR_FULL_WAIT);
+            ok = false;
+            break;
+        }
+        const uint32_t base = ring + (uint32_t)s * stage_bytes;
+        uint4 w[R][NITER];
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+#pragma unroll
+            for (int i = 0; i < NITER; ++i) {
+                const int c = tid + i * GEMV_CONSUMERS;
+                w[j][i] = c < nchunks ? lds128(base + (uint32_t)j * row_bytes + (uint32_t)c * 16u) : make_uint4(0, 0, 0, 0);
+            }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8u * s);  // this warp holds its slice in registers: stage may be refilled
+        float acc[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            float a = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NITER; ++i) a = Wfmt<WT>::dot(w[j][i], 0u, xr[i], a);
+            acc[j] = a;
+        }
+        int rr;
+        const float tot = warp_reduce_rows<R>(acc, lane, rr);
+        const int row = g < gs ? g * R + rr : ns + (g - gs) * R + rr;  // rows past a part's end were never copied: their sums are dropped
+        if ((lane & (32 / R - 1)) == 0 && row < (g < gs ? ns : ns + ne)) partial[row * NW + warp] = tot;
+    }
+    if (!ok) {
+        // leave only once the copies that may still be in flight have landed (bounded)
+        for (int s = 0; s < p.nstages; ++s) mbar_wait(full0 + 8u * s, 0);
+    }
+    both_bar(10);
+    if (!ok) return;
+    for (int u = tid; u < (ns + ne) / 2; u += GEMV_CONSUMERS) {
+        float y[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int wi = 0; wi < NW; ++wi) y[k] += partial[(2 * u + k) * NW + wi];
+        const int v = eu0 + u - ns / 2;  // a chosen expert's unit
+        const bool shared = u < ns / 2;
+        p.gate[shared ? nunits + su0 + u : v] = (y[0] / (1.0f + expf(-y[0]))) * y[1] * (shared ? 1.0f : weight[v / p.hidden]);
     }
 }
 
