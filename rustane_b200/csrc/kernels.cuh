@@ -251,10 +251,25 @@ __device__ inline float consumer_sum(float v, float* red, int group = 0) {  // r
     return t;
 }
 
+// two sums at once (one consumer group; red: 16 floats)
+__device__ inline float2 consumer_sum2(float a, float b, float* red) {
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 7;
+    a = warp_sum(a);
+    b = warp_sum(b);
+    gemv_group_bar(0);
+    if (lane == 0) { red[warp] = a; red[8 + warp] = b; }
+    gemv_group_bar(0);
+    float2 t = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < GEMV_CONSUMERS / 32; ++i) { t.x += red[i]; t.y += red[8 + i]; }
+    return t;
+}
+
 // How the input vector comes about.  GemvIn: the vector x, under NORM divided by its root mean square and times gamma,
 // or under tensor parallelism res + alpha * (sum of the ranks' partial vectors).  Other input types (CUSTOM) fill the
-// consumers' registers themselves: load(registers, thread, chunks, 8 floats of shared memory, group, whether the CTA
-// works on the second matrix of a pair, whether this thread's copy is the one to publish).
+// consumers' registers themselves: load(registers, thread, chunks, 16 floats of shared memory, the wait for the kernel ahead -
+// called once, behind the requests for what is older than that kernel -, whether the CTA works on the second matrix of a
+// pair, whether this thread's copy is the one to publish).
 struct GemvIn {
     static constexpr bool CUSTOM = false;
 };
@@ -363,12 +378,16 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
 #pragma unroll
             for (int e = 0; e < EPC; ++e) gm[i][e] = tid + i * GEMV_CONSUMERS < nchunks ? gamma[(size_t)(tid + i * GEMV_CONSUMERS) * EPC + e] : 0.0f;
     }
-    pdl_wait();
-    pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
+    auto begin = [] {
+        pdl_wait();
+        pdl_launch_dependents();  // after the wait: at most this kernel and the next one overlap
+    };
     float xr[NITER][EPC];
     if constexpr (In::CUSTOM) {
-        in.load(xr, tid, nchunks, red + 8 * group, group, Src::PAIR && unit0 > 0, bid == 0 && unit0 == 0 && group == 0);
+        static_assert(G == 1, "one consumer group");
+        in.load(xr, tid, nchunks, red, begin, Src::PAIR && unit0 > 0, bid == 0 && unit0 == 0);
     } else {
+    begin();
     float ss = 0.0f;
     const float* inbox = nullptr;  // tensor parallel: the input is res + alpha * (sum of the peers' partial vectors)
     if (tp.world > 1 && tp.in_reduce) {

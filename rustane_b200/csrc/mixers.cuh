@@ -90,7 +90,7 @@ struct InResidual {
     int n;
     // mean and reciprocal deviation of the vector spread over the consumers' registers
     template <int NITER, int EPC>
-    __device__ void moments(const float (&v)[NITER][EPC], int kind, int tid, int nchunks, float* red, int group, float& mean, float& r) const {
+    __device__ void moments(const float (&v)[NITER][EPC], int kind, int tid, int nchunks, float* red, float& mean, float& r) const {
         const float inv_n = 1.0f / (float)n;
         mean = 0.0f;
         if (kind == VecNorm::LAYER) {
@@ -99,7 +99,7 @@ struct InResidual {
             for (int i = 0; i < NITER; ++i)
 #pragma unroll
                 for (int e = 0; e < EPC; ++e) s += v[i][e];  // zero past the end
-            mean = consumer_sum(s, red, group) * inv_n;
+            mean = consumer_sum(s, red) * inv_n;
         }
         float ss = 0.0f;
 #pragma unroll
@@ -112,31 +112,50 @@ struct InResidual {
                 }
             }
         }
-        r = 1.0f / sqrtf(consumer_sum(ss, red, group) * inv_n + eps);
+        r = 1.0f / sqrtf(consumer_sum(ss, red) * inv_n + eps);
     }
     __device__ static float4 vec4(const float* p, size_t at) { return p != nullptr ? *reinterpret_cast<const float4*>(p + at) : make_float4(0.f, 0.f, 0.f, 0.f); }
-    template <int NITER, int EPC>
-    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, int group, bool, bool writer) const {
-        constexpr bool EARLY = NITER * EPC <= 32;  // the residual stream is requested together with y where registers allow
+    template <int NITER, int EPC, class Begin>
+    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, const Begin& begin, bool, bool writer) const {
+        constexpr bool EARLY = NITER * EPC <= 32;   // the residual stream is requested together with y where registers allow
+        constexpr bool AHEAD = NITER * EPC <= 16;   // and the weights ahead of the wait (3.1 us from the wait to the input with each requested at its use)
+        const bool normed = y != nullptr && post.kind != VecNorm::NONE;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+        float4 pw[AHEAD ? NITER : 1][EPC / 4], pb[AHEAD ? NITER : 1][EPC / 4], qw[AHEAD ? NITER : 1][EPC / 4], qb[AHEAD ? NITER : 1][EPC / 4];
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int i = 0; i < NITER; ++i)
+#pragma unroll
+                for (int e = 0; e < EPC / 4; ++e) {
+                    const size_t at = (size_t)(tid + i * GEMV_CONSUMERS) * EPC + 4 * e;
+                    const bool in = tid + i * GEMV_CONSUMERS < nchunks;
+                    pw[i][e] = normed && in ? vec4(post.w, at) : one;
+                    pb[i][e] = normed && in ? vec4(post.b, at) : zero;
+                    qw[i][e] = pre.kind != VecNorm::NONE && in ? vec4(pre.w, at) : zero;
+                    qb[i][e] = pre.kind != VecNorm::NONE && in ? vec4(pre.b, at) : zero;
+                }
+        }
+        begin();
         float xe[EARLY ? NITER : 1][EARLY ? EPC : 1];
+        float4 ad[AHEAD ? NITER : 1][EPC / 4];
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 v = zero;
                 if (c < nchunks && y != nullptr) v = __ldcg(reinterpret_cast<const float4*>(y + (size_t)c * EPC + e));
                 xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
                 if constexpr (EARLY) {
-                    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                    float4 b = zero;
                     if (c < nchunks) b = __ldcg(reinterpret_cast<const float4*>(x + (size_t)c * EPC + e));
                     xe[i][e] = b.x; xe[i][e + 1] = b.y; xe[i][e + 2] = b.z; xe[i][e + 3] = b.w;
                 }
+                if constexpr (AHEAD) ad[i][e / 4] = c < nchunks ? vec4(add, (size_t)c * EPC + e) : zero;
             }
         }
         float mean = 0.0f, r = 1.0f;
-        if (y != nullptr && post.kind != VecNorm::NONE) moments(xr, post.kind, tid, nchunks, red, group, mean, r);
-        const bool normed = y != nullptr && post.kind != VecNorm::NONE;
+        if (normed) moments(xr, post.kind, tid, nchunks, red, mean, r);
         r *= mult;
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
@@ -145,11 +164,14 @@ struct InResidual {
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
                 const size_t at = (size_t)c * EPC + e;
-                float4 b;
+                float4 b, w, o, a;
                 if constexpr (EARLY) b = make_float4(xe[i][e], xe[i][e + 1], xe[i][e + 2], xe[i][e + 3]);
                 else b = __ldcg(reinterpret_cast<const float4*>(x + at));
-                const float4 w = normed ? vec4(post.w, at) : make_float4(1.f, 1.f, 1.f, 1.f), o = normed ? vec4(post.b, at) : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 a = vec4(add, at);
+                if constexpr (AHEAD) {
+                    w = pw[i][e / 4]; o = pb[i][e / 4]; a = ad[i][e / 4];
+                } else {
+                    w = normed ? vec4(post.w, at) : one; o = normed ? vec4(post.b, at) : zero; a = vec4(add, at);
+                }
                 xr[i][e] = b.x + ((xr[i][e] - mean) * r * w.x + mult * o.x) + a.x;
                 xr[i][e + 1] = b.y + ((xr[i][e + 1] - mean) * r * w.y + mult * o.y) + a.y;
                 xr[i][e + 2] = b.z + ((xr[i][e + 2] - mean) * r * w.z + mult * o.z) + a.z;
@@ -158,7 +180,7 @@ struct InResidual {
             }
         }
         if (pre.kind == VecNorm::NONE) return;
-        moments(xr, pre.kind, tid, nchunks, red, group, mean, r);
+        moments(xr, pre.kind, tid, nchunks, red, mean, r);
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
@@ -166,7 +188,12 @@ struct InResidual {
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
                 const size_t at = (size_t)c * EPC + e;
-                const float4 w = vec4(pre.w, at), o = vec4(pre.b, at);
+                float4 w, o;
+                if constexpr (AHEAD) {
+                    w = qw[i][e / 4]; o = qb[i][e / 4];
+                } else {
+                    w = vec4(pre.w, at); o = vec4(pre.b, at);
+                }
                 xr[i][e] = (xr[i][e] - mean) * r * w.x + o.x;
                 xr[i][e + 1] = (xr[i][e + 1] - mean) * r * w.y + o.y;
                 xr[i][e + 2] = (xr[i][e + 2] - mean) * r * w.z + o.z;
@@ -183,41 +210,57 @@ struct InParallelMix {
     float* x_out;
     float mult, eps;
     int n;
-    template <int NITER, int EPC>
-    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, int group, bool, bool writer) const {
+    template <int NITER, int EPC, class Begin>
+    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, const Begin& begin, bool, bool writer) const {
+        constexpr bool AHEAD = NITER * EPC <= 16;  // the weights ahead of the wait, the vectors once, where registers allow
+        constexpr int NA = AHEAD ? NITER : 1;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 wp[NA][EPC / 4], wq[NA][EPC / 4], wg[NA][EPC / 4], va[NA][EPC / 4], vb[NA][EPC / 4], vx[NA][EPC / 4];
+        auto weight = [&](const float* p, int c, int e) { return c < nchunks ? *reinterpret_cast<const float4*>(p + (size_t)c * EPC + e) : zero; };
+        auto vec = [&](const float* p, int c, int e) { return c < nchunks ? __ldcg(reinterpret_cast<const float4*>(p + (size_t)c * EPC + e)) : zero; };
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int i = 0; i < NITER; ++i)
+#pragma unroll
+                for (int e = 0; e < EPC / 4; ++e) {
+                    const int c = tid + i * GEMV_CONSUMERS;
+                    wp[i][e] = weight(wl, c, 4 * e); wq[i][e] = weight(wr, c, 4 * e); wg[i][e] = weight(gain, c, 4 * e);
+                }
+        }
+        begin();
         float sl = 0.0f, sr = 0.0f;
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
-                if (c < nchunks) {
-                    const float4 a = __ldcg(reinterpret_cast<const float4*>(yl + (size_t)c * EPC + e)), b = __ldcg(reinterpret_cast<const float4*>(yr + (size_t)c * EPC + e));
-                    sl += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
-                    sr += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
-                }
+                const float4 a = vec(yl, c, e), b = vec(yr, c, e);
+                if constexpr (AHEAD) { va[i][e / 4] = a; vb[i][e / 4] = b; vx[i][e / 4] = vec(x, c, e); }
+                sl += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+                sr += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
             }
         }
-        const float rl = 0.5f / sqrtf(consumer_sum(sl, red, group) * (1.0f / (float)n) + eps);
-        const float rr = 0.5f / sqrtf(consumer_sum(sr, red, group) * (1.0f / (float)n) + eps);
+        const float2 both = consumer_sum2(sl, sr, red);
+        const float rl = 0.5f / sqrtf(both.x * (1.0f / (float)n) + eps);
+        const float rr = 0.5f / sqrtf(both.y * (1.0f / (float)n) + eps);
         float ss = 0.0f;
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
-                float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (c < nchunks) {
-                    const size_t at = (size_t)c * EPC + e;
-                    const float4 a = __ldcg(reinterpret_cast<const float4*>(yl + at)), b = __ldcg(reinterpret_cast<const float4*>(yr + at));
-                    const float4 p = *reinterpret_cast<const float4*>(wl + at), q = *reinterpret_cast<const float4*>(wr + at);
-                    z = make_float4(a.x * rl * p.x + b.x * rr * q.x, a.y * rl * p.y + b.y * rr * q.y, a.z * rl * p.z + b.z * rr * q.z, a.w * rl * p.w + b.w * rr * q.w);
+                float4 a, b, p, q;
+                if constexpr (AHEAD) {
+                    a = va[i][e / 4]; b = vb[i][e / 4]; p = wp[i][e / 4]; q = wq[i][e / 4];
+                } else {
+                    a = vec(yl, c, e); b = vec(yr, c, e); p = weight(wl, c, e); q = weight(wr, c, e);
                 }
+                const float4 z = make_float4(a.x * rl * p.x + b.x * rr * q.x, a.y * rl * p.y + b.y * rr * q.y, a.z * rl * p.z + b.z * rr * q.z, a.w * rl * p.w + b.w * rr * q.w);
                 xr[i][e] = z.x; xr[i][e + 1] = z.y; xr[i][e + 2] = z.z; xr[i][e + 3] = z.w;
                 ss += z.x * z.x + z.y * z.y + z.z * z.z + z.w * z.w;
             }
         }
-        const float r = mult / sqrtf(consumer_sum(ss, red, group) * (1.0f / (float)n) + eps);
+        const float r = mult / sqrtf(consumer_sum(ss, red) * (1.0f / (float)n) + eps);
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
@@ -225,7 +268,9 @@ struct InParallelMix {
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
                 const size_t at = (size_t)c * EPC + e;
-                const float4 b = __ldcg(reinterpret_cast<const float4*>(x + at)), g = *reinterpret_cast<const float4*>(gain + at);
+                float4 b, g;
+                if constexpr (AHEAD) { b = vx[i][e / 4]; g = wg[i][e / 4]; }
+                else { b = vec(x, c, e); g = weight(gain, c, e); }
                 xr[i][e] = b.x + xr[i][e] * r * g.x; xr[i][e + 1] = b.y + xr[i][e + 1] * r * g.y;
                 xr[i][e + 2] = b.z + xr[i][e + 2] * r * g.z; xr[i][e + 3] = b.w + xr[i][e + 3] * r * g.w;
                 if (writer) *reinterpret_cast<float4*>(x_out + at) = make_float4(xr[i][e], xr[i][e + 1], xr[i][e + 2], xr[i][e + 3]);
@@ -242,13 +287,34 @@ struct InMixerOutputs {
     const float *attn, *mem, *ssq, *norm, *gate;
     int n, vdim, nslice;
     float eps;
-    template <int NITER, int EPC>
-    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float*, int, bool second, bool) const {
+    template <int NITER, int EPC, class Begin>
+    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float*, const Begin& begin, bool second, bool) const {
+        begin();
         int hcur = -1;
         float rstd = 0.0f;
+        // a head's slices are summed in order, their loads in flight together (one after the other the second matrix's CTAs ended
+        // 5 us behind the first one's)
+        auto head_rstd = [&](int h) {
+            float s = 0.0f;
+            for (int k0 = 0; k0 < nslice; k0 += 8) {
+                float t[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) t[k] = k0 + k < nslice ? __ldcg(ssq + h * nslice + k0 + k) : 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) s += t[k];
+            }
+            return 1.0f / sqrtf(s / (float)vdim + eps);
+        };
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
+            float g[EPC], w[EPC];
+#pragma unroll
+            for (int e = 0; e < EPC; ++e) {
+                const bool in = second && c < nchunks && c * EPC + e < n;
+                g[e] = in ? __ldcg(gate + c * EPC + e) : 0.0f;
+                w[e] = in ? norm[c * EPC + e] : 0.0f;
+            }
 #pragma unroll
             for (int e = 0; e < EPC; e += 4) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -262,12 +328,10 @@ struct InMixerOutputs {
                     if (j < n) {
                         const int h = j / vdim;
                         if (h != hcur) {
-                            float s = 0.0f;
-                            for (int k = 0; k < nslice; ++k) s += __ldcg(ssq + h * nslice + k);
-                            rstd = 1.0f / sqrtf(s / (float)vdim + eps);
+                            rstd = head_rstd(h);
                             hcur = h;
                         }
-                        xr[i][e] = xr[i][e] * rstd * norm[j] * sigmoid(__ldcg(gate + j));
+                        xr[i][e] = xr[i][e] * rstd * w[e] * sigmoid(g[e]);
                     }
                 }
             }
@@ -281,8 +345,20 @@ struct InGatedNorm {
     const float *mem, *norm, *gate;
     int n;
     float eps;
-    template <int NITER, int EPC>
-    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, int group, bool, bool) const {
+    template <int NITER, int EPC, class Begin>
+    __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, const Begin& begin, bool, bool) const {
+        constexpr bool EARLY = NITER * EPC <= 16;  // weights ahead of the wait, gates together with the read-outs
+        float g[EARLY ? NITER : 1][EPC], w[EARLY ? NITER : 1][EPC];
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int i = 0; i < NITER; ++i)
+#pragma unroll
+                for (int e = 0; e < EPC; ++e) {
+                    const int c = tid + i * GEMV_CONSUMERS, j = c * EPC + e;
+                    w[i][e] = c < nchunks && j < n ? norm[j] : 0.0f;
+                }
+        }
+        begin();
         float ss = 0.0f;
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
@@ -292,12 +368,18 @@ struct InGatedNorm {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (c < nchunks) v = __ldcg(reinterpret_cast<const float4*>(mem + (size_t)c * EPC + e));
                 xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
+                if constexpr (EARLY) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (c * EPC + e + k < n) ss = fmaf(xr[i][e + k], xr[i][e + k], ss);  // another layer's values may lie behind the last head
+                    for (int k = e; k < e + 4; ++k) g[i][k] = c < nchunks && c * EPC + k < n ? __ldcg(gate + c * EPC + k) : 0.0f;
+                }
             }
         }
-        const float r = 1.0f / sqrtf(consumer_sum(ss, red, group) / (float)n + eps);
+#pragma unroll
+        for (int i = 0; i < NITER; ++i)
+#pragma unroll
+            for (int e = 0; e < EPC; ++e)
+                if ((tid + i * GEMV_CONSUMERS) * EPC + e < n) ss = fmaf(xr[i][e], xr[i][e], ss);  // another layer's values may lie behind the last head
+        const float r = 1.0f / sqrtf(consumer_sum(ss, red) / (float)n + eps);
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
@@ -305,7 +387,10 @@ struct InGatedNorm {
 #pragma unroll
             for (int e = 0; e < EPC; ++e) {
                 const int j = c * EPC + e;
-                xr[i][e] = j < n ? xr[i][e] * r * norm[j] * sigmoid(__ldcg(gate + j)) : 0.0f;
+                float ge, we;
+                if constexpr (EARLY) { ge = g[i][e]; we = w[i][e]; }
+                else { ge = j < n ? __ldcg(gate + j) : 0.0f; we = j < n ? norm[j] : 0.0f; }
+                xr[i][e] = j < n ? xr[i][e] * r * we * sigmoid(ge) : 0.0f;
             }
         }
     }
@@ -327,14 +412,16 @@ template <typename WT> struct EpiTokenGate {
 template <class In>
 __global__ void __launch_bounds__(GEMV_CONSUMERS) vector_input_kernel(In in, int n) {
     __shared__ float red[32];
-    pdl_wait();
-    pdl_launch_dependents();
+    auto begin = [] {
+        pdl_wait();
+        pdl_launch_dependents();
+    };
     if (n <= 4 * 4 * GEMV_CONSUMERS) {
         float xr[4][4];
-        in.load(xr, threadIdx.x, n / 4, red, 0, false, true);
+        in.load(xr, threadIdx.x, n / 4, red, begin, false, true);
     } else {
         float xr[16][4];
-        in.load(xr, threadIdx.x, n / 4, red, 0, false, true);
+        in.load(xr, threadIdx.x, n / 4, red, begin, false, true);
     }
 }
 
@@ -365,10 +452,13 @@ __device__ inline float sum_of_squares(const float* v, int n) {
     float s = 0.0f;
     if ((n & 3) == 0 && (reinterpret_cast<size_t>(v) & 15) == 0) {
         const float4* v4 = reinterpret_cast<const float4*>(v);
-#pragma unroll 8
-        for (int i = threadIdx.x; i < n / 4; i += MIX_THREADS) {
-            const float4 t = __ldcg(v4 + i);
-            s += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
+        constexpr int B = 8;  // in flight (as an unrolled loop the last, incomplete turn waited for one load after another)
+        for (int i0 = threadIdx.x; i0 < n / 4; i0 += B * MIX_THREADS) {
+            float4 t[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) t[b] = i0 + b * MIX_THREADS < n / 4 ? __ldcg(v4 + i0 + b * MIX_THREADS) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int b = 0; b < B; ++b) s += t[b].x * t[b].x + t[b].y * t[b].y + t[b].z * t[b].z + t[b].w * t[b].w;
         }
     } else {
 #pragma unroll 8
@@ -395,18 +485,23 @@ __device__ inline void mem_step(const MixerStep& p, int idx, float* sm, float* r
         const int r = rg + 16 * j;
         s[j] = live && r < d.dim ? __ldcg(reinterpret_cast<const float4*>(S + (size_t)r * d.vs)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    const bool linear = d.linear();
+    const float n0 = !linear && tid < d.dim ? __ldcg(nvec + tid) : 0.0f, m0 = linear ? 0.0f : __ldcg(mrun);
+    const float b_i = linear ? 0.0f : p.ib[h], b_f = linear ? 0.0f : p.fb[h], decay = linear ? d.decay[h] : 0.0f;
     pdl_wait();
     pdl_launch_dependents();
+    float v[4], acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = col + e < d.vdim ? __ldcg(p.proj + p.pl.rv + h * d.vdim + col + e) : 0.0f;
     float* qs = sm;
     float* ks = sm + d.dim;
     float* acc_s = sm + 2 * d.dim;  // [4 warps][MEM_SLICE]
-    const bool linear = d.linear();
     float mt = 0.0f, fa, ia = 1.0f, qscale = 1.0f;
     if (linear) {
-        fa = d.decay[h];
+        fa = decay;
     } else {
-        const float zi = __ldcg(p.proj + p.pl.ri + h) + p.ib[h], zf = __ldcg(p.proj + p.pl.rf + h) + p.fb[h];
-        const float gi = soft_cap(zi, d.cap), gf = log_sigmoid(soft_cap(zf, d.cap)), m0 = __ldcg(mrun);
+        const float zi = __ldcg(p.proj + p.pl.ri + h) + b_i, zf = __ldcg(p.proj + p.pl.rf + h) + b_f;
+        const float gi = soft_cap(zi, d.cap), gf = log_sigmoid(soft_cap(zf, d.cap));
         mt = fmaxf(gf + m0, gi);
         fa = expf(gf + m0 - mt);
         ia = expf(gi - mt);
@@ -420,16 +515,15 @@ __device__ inline void mem_step(const MixerStep& p, int idx, float* sm, float* r
         qs[i] = q;
         ks[i] = k;
         if (linear) continue;
-        const float nn = fa * __ldcg(nvec + i) + ia * k;
+        const float nn = fa * (i == tid ? n0 : __ldcg(nvec + i)) + ia * k;
         nvec[i] = nn;
         nq = fmaf(nn, q, nq);
     }
     nq = block_sum(nq, red);  // (its barriers publish qs and ks)
     if (tid == 0 && !linear) *mrun = mt;
-    float v[4], acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        v[e] = col + e < d.vdim ? ia * __ldcg(p.proj + p.pl.rv + h * d.vdim + col + e) : 0.0f;
+        v[e] = ia * v[e];
         if (linear) v[e] = silu(v[e]);  // silu(0) = 0
     }
     for (int r0 = rg; r0 < d.dim; r0 += 16 * PRE) {
@@ -488,9 +582,7 @@ __device__ inline void attn_step(const MixerStep& p, KT* __restrict__ pool, int 
     float* vc = kc + kr;                  // [vp]
     float* accs = vc + a.vp;              // [128 threads][8]
     float* ps = accs + MIX_THREADS * 8;   // [MAPS][MIX_TILE]
-    pdl_wait();
-    pdl_launch_dependents();
-    const int pos = __ldcg(&p.st->pos);
+    const int pos = __ldcg(&p.st->pos);  // older than the kernel ahead, and so are all cached rows but this position's
     const int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0, len = pos + 1 - lo;
     int per = (len + p.nsplit - 1) / p.nsplit;
     per = (per + MIX_TILE - 1) / MIX_TILE * MIX_TILE;
@@ -507,7 +599,21 @@ __device__ inline void attn_step(const MixerStep& p, KT* __restrict__ pool, int 
     int lv = 1;
     while (lv < nvc) lv <<= 1;            // lanes that share a row of values
     const int vch = tid % lv, vgrp = tid / lv, vgroups = MIX_THREADS / lv;
-    if (t0 < t1) {
+    // the value rows of a tile: requested before its scores are worked out, the first tile's before the kernel ahead has ended
+    constexpr int PRE = 4;
+    uint4 vw[PRE];
+    auto fetch_v = [&](int tb, int nt) {
+#pragma unroll
+        for (int u = 0; u < PRE; ++u) {
+            const int j = vgrp + u * vgroups;
+            vw[u] = make_uint4(0, 0, 0, 0);
+            if (vch < nvc && j < nt && tb + j != pos) vw[u] = ldg_stream_coherent(pool + v_off[j] + (size_t)vch * EPC);
+        }
+    };
+    if (t0 >= t1) {
+        pdl_wait();
+        pdl_launch_dependents();
+    } else {
         const bool newest = t1 == pos + 1;  // this slice holds the current position
         auto locate = [&](int tb) {
             if (tid < MIX_TILE) {
@@ -517,6 +623,10 @@ __device__ inline void attn_step(const MixerStep& p, KT* __restrict__ pool, int 
             }
         };
         locate(t0);
+        __syncthreads();
+        fetch_v(t0, min(MIX_TILE, t1 - t0));
+        pdl_wait();
+        pdl_launch_dependents();
         float rq = a.temperature(pos) * a.scale, rk = 1.0f;
         if (p.q_norm != nullptr) {
             const float sq = sum_of_squares(p.proj + p.pl.lq, a.H * MAPS * a.dim), sk = newest ? sum_of_squares(p.proj + p.pl.lk, a.G * MAPS * a.dim) : 0.0f;
@@ -552,15 +662,7 @@ __device__ inline void attn_step(const MixerStep& p, KT* __restrict__ pool, int 
         const float slope = p.slopes != nullptr ? p.slopes[h] : 0.0f;
         for (int tb = t0; tb < t1; tb += MIX_TILE) {
             const int nt = min(MIX_TILE, t1 - tb);
-            // the tile's value rows are requested before its scores are worked out
-            constexpr int PRE = 4;
-            uint4 vw[PRE];
-#pragma unroll
-            for (int u = 0; u < PRE; ++u) {
-                const int j = vgrp + u * vgroups;
-                vw[u] = make_uint4(0, 0, 0, 0);
-                if (vch < nvc && j < nt && tb + j != pos) vw[u] = ldg_stream_coherent(pool + v_off[j] + (size_t)vch * EPC);
-            }
+            if (tb > t0) fetch_v(tb, nt);
             // scores: warp w takes positions tb + 8 w .. + 7
             for (int j0 = 0; j0 < 8; j0 += 4 * side) {
                 float d[4][MAPS];
@@ -682,17 +784,27 @@ __device__ inline void attn_step(const MixerStep& p, KT* __restrict__ pool, int 
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    // the slices' maxima and sums, the head's gate and the first entries of all slices are requested together
+    const int used = (len + per - 1) / per;  // slices that hold positions
+    constexpr int B = 16;                    // of them in flight
+    float2 ml[MAPS];
+    float first[MAPS][B], t[MAPS][B];
+    auto load = [&](float (&v)[MAPS][B], int s0, int i) {
+#pragma unroll
+        for (int q = 0; q < MAPS; ++q)
+#pragma unroll
+            for (int s = 0; s < B; ++s) v[q][s] = s0 + s < used && i < a.vdim ? __ldcg(p.part_acc + ((size_t)(h * MAPS + q) * p.nsplit + s0 + s) * a.vp + i) : 0.0f;
+    };
+#pragma unroll
+    for (int q = 0; q < MAPS; ++q)  // nsplit <= 32: one slice per lane, the same in every warp
+        ml[q] = lane < p.nsplit ? __ldcg(reinterpret_cast<const float2*>(p.part_ml + (size_t)(h * MAPS + q) * p.nsplit * 2 + lane * 2)) : make_float2(NEG, 0.0f);
+    load(first, 0, tid);
+    const float gate = a.gate == 1 ? __ldcg(p.proj + p.pl.lg + h) : a.gate == 2 && tid < a.vdim ? __ldcg(p.proj + p.pl.lg + h * a.vdim + tid) : 0.0f;
+    const float sink = p.sink != nullptr ? p.sink[h] : NEG;
     float inv[MAPS];
 #pragma unroll
     for (int q = 0; q < MAPS; ++q) {
-        const float* pml = p.part_ml + (size_t)(h * MAPS + q) * p.nsplit * 2;
-        float ms = NEG, ls = 0.0f;  // nsplit <= 32: one slice per lane, the same in every warp
-        if (lane < p.nsplit) {
-            const float2 ml = __ldcg(reinterpret_cast<const float2*>(pml + lane * 2));
-            ms = ml.x;
-            ls = ml.y;
-        }
-        const float sink = p.sink != nullptr ? p.sink[h] : NEG;
+        const float ms = ml[q].x, ls = ml[q].y;
         const float M = fmaxf(warp_max(ls > 0.0f ? ms : NEG), sink);
         const float w = ls > 0.0f ? expf(ms - M) : 0.0f;
         inv[q] = 1.0f / (warp_sum(ls * w) + (p.sink != nullptr ? expf(sink - M) : 0.0f));
@@ -700,31 +812,35 @@ __device__ inline void attn_step(const MixerStep& p, KT* __restrict__ pool, int 
     }
     if (MAPS > 1) inv[MAPS - 1] *= -a.lambda;
     __syncthreads();
-    const int used = (len + per - 1) / per;  // slices that hold positions
     float ss = 0.0f;
     for (int i = tid; i < a.vdim; i += MIX_THREADS) {
-        float r = 0.0f;
+        float o[MAPS], r = 0.0f;
 #pragma unroll
-        for (int q = 0; q < MAPS; ++q) {
-            const float* pa = p.part_acc + (size_t)(h * MAPS + q) * p.nsplit * a.vp + i;
-            float o = 0.0f;
-            for (int s0 = 0; s0 < used; s0 += 16) {  // sixteen slices in flight together
-                float t[16];
+        for (int q = 0; q < MAPS; ++q) o[q] = 0.0f;
+        for (int s0 = 0; s0 < used; s0 += B) {
+            if (s0 == 0 && i == tid) {
 #pragma unroll
-                for (int s = 0; s < 16; ++s) t[s] = s0 + s < used ? __ldcg(pa + (size_t)(s0 + s) * a.vp) : 0.0f;
+                for (int q = 0; q < MAPS; ++q)
 #pragma unroll
-                for (int s = 0; s < 16; ++s)
-                    if (s0 + s < used) o = fmaf(t[s], ps[q * MIX_TILE + s0 + s], o);
+                    for (int s = 0; s < B; ++s) t[q][s] = first[q][s];
+            } else {
+                load(t, s0, i);
             }
-            r = fmaf(o, inv[q], r);
+#pragma unroll
+            for (int q = 0; q < MAPS; ++q)
+#pragma unroll
+                for (int s = 0; s < B; ++s)
+                    if (s0 + s < used) o[q] = fmaf(t[q][s], ps[q * MIX_TILE + s0 + s], o[q]);
         }
+#pragma unroll
+        for (int q = 0; q < MAPS; ++q) r = fmaf(o[q], inv[q], r);
         vc[i] = r;  // each thread reads its own entries again
         ss = fmaf(r, r, ss);
     }
     float f = MAPS > 1 ? a.out_scale / sqrtf(block_sum(ss, red) / (float)a.vdim + a.eps) : 1.0f;
-    if (a.gate == 1) f *= sigmoid(__ldcg(p.proj + p.pl.lg + h));
+    if (a.gate == 1) f *= sigmoid(gate);
     for (int i = tid; i < a.vdim; i += MIX_THREADS)
-        p.attn[h * a.vdim + i] = vc[i] * f * (a.gate == 2 ? sigmoid(__ldcg(p.proj + p.pl.lg + h * a.vdim + i)) : 1.0f);
+        p.attn[h * a.vdim + i] = vc[i] * f * (a.gate == 2 ? sigmoid(i == tid ? gate : __ldcg(p.proj + p.pl.lg + h * a.vdim + i)) : 1.0f);
     if (tid == 0) p.counters[h] = 0u;
 }
 

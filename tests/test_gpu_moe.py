@@ -17,6 +17,11 @@ SMALL = dict(dim=256, hidden=128, heads=4, seq=128, nlayers=2, vocab=1500, n_exp
              kv_latent=64, rope_dim=16, nope_dim=32, v_dim=32)
 MID = dict(dim=1024, hidden=704, heads=16, seq=512, nlayers=2, vocab=8192, n_experts=16, top_k=6, n_shared=2,
            kv_latent=512, rope_dim=64, nope_dim=128, v_dim=128)
+# the fused routing at its edges: no shared rows and experts that do not fill the summing threads; two and four chunks a
+# thread, the longest choice, the most experts (and more of them: the router as a kernel of its own)
+NO_SHARED = dict(SMALL, dim=264, hidden=104, n_experts=96, top_k=5, n_shared=0)
+WIDE = dict(SMALL, dim=2056, hidden=72, n_experts=256, top_k=16, n_shared=3, vocab=700)
+MANY = dict(SMALL, n_experts=264, top_k=3, vocab=700)
 
 
 def _pair(R, O, dims, dtype, seed, untied=False, **opts):
@@ -32,6 +37,10 @@ def _pair(R, O, dims, dtype, seed, untied=False, **opts):
     (SMALL, "f32", False, {}, 40),
     (SMALL, "bf16", True, dict(page_tokens=16), 70),          # several attention tiles and pages, untied head
     (MID, "bf16", False, dict(use_graph=True), 90),           # configuration 5's attention widths, top-6 of 16 experts
+    (NO_SHARED, "bf16", False, dict(use_graph=True), 20),
+    (WIDE, "bf16", False, {}, 20),
+    (WIDE, "f32", False, {}, 20),
+    (MANY, "f32", False, {}, 20),
 ])
 def test_moe_mla_logits_experts_and_greedy_ids_match_the_oracle(R, oracle, dims, dtype, untied, opts, ntok):
     om, gm = _pair(R, oracle, dims, dtype, 41, untied, **opts)
