@@ -14,7 +14,9 @@
 //                        (the cache is shared by the heads), running softmax, partial latent sums
 //   mla_out_kernel       merges the slices (fixed order) and applies W_uv_h: the head's output
 //   gemv_tma_kernel      Wo + scaled residual
-//   moe_router_kernel    RMSNorm, router logits, softmax over all experts, top-k (ties: lower index)
+//                        (one GPU: and each CTA's share of the router's logits)
+//   moe_gate_kernel      one GPU: RMSNorm, softmax over all experts, top-k (ties: lower index), and the gate below, streamed
+//   moe_router_kernel    several GPUs, or shapes it does not take: the choice as a kernel of its own, then
 //   moe_w13_kernel       gate = silu(xn W1) * (xn W3) * p for the chosen experts and the shared ones
 //   moe_w2_kernel        x = x2 + alpha * sum over experts of W2 gate; expert parallel: the rank's partial
 //                        sum is pushed to every rank's inbox instead (the dense model's all-reduce)
