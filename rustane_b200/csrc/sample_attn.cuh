@@ -199,7 +199,7 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
     const float dn = down[g];
     for (int i = 0; more;) {  // (uniform in the warp)
         const bool seen = g < rows && (!own || g / nh == z);  // a sample's own positions are its rows' only
-        const int at = w0;
+        const int at = w0, zt = z;
         {
             float c[2][4] = {}, d[2][4] = {};
 #pragma unroll
@@ -242,6 +242,9 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
                 }
             m = mnew;
             __syncwarp();
+            // the rows these positions belong to: all of the block's, or one sample's.  A probability of zero does not keep another
+            // sample's rows clean: an fp16 cache stores what overflows as infinity, and 0 * inf is NaN
+            const uint32_t mine = own ? ((1u << nh) - 1u) << (zt * nh) : (1u << SA_ROWS) - 1u;
             if (i > 1) {
 #pragma unroll
                 for (int r = 0; r < SA_ROWS; ++r) {
@@ -258,9 +261,12 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
                 float x[8];
                 Elem<KT>::unpack(vw[k], x);
 #pragma unroll
-                for (int r = 0; r < SA_ROWS; ++r)
+                for (int r = 0; r < SA_ROWS; ++r) {
+                    if (mine >> r & 1u) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(e[r], x[i], acc[r][i]);
+                        for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(e[r], x[i], acc[r][i]);
+                    }
+                }
             }
             if (more) fetch_v();
         }

@@ -145,3 +145,43 @@ def test_captured_step_graphs_follow_the_prompt_length(R, oracle):
         assert [g[:12] for g in got.tolist()] == [w[:12] for w in want], len(prompt)
         same = sum(int(a == b) for g, w in zip(got.tolist(), want) for a, b in zip(g, w))
         assert same >= 0.9 * 4 * nsteps, (len(prompt), same)
+
+
+@pytest.mark.parametrize("kv_heads,ns,nprompt,page_tokens,bad_at", [
+    (4, 8, 40, 16, 1),     # warps with two samples each
+    (4, 5, 40, 16, 4),     # one with two, the others with one
+    (2, 7, 100, 64, 5),    # two q heads a kv head, a block of three samples, several turns a warp
+    (1, 3, 40, 16, 1),     # a warp keeps to its sample
+])
+def test_a_sample_whose_cache_overflows_leaves_the_others_alone(R, kv_heads, ns, nprompt, page_tokens, bad_at):
+    """An fp16 cache stores a value past 65504 as infinity.  One sample's first token has such a value row: that sample's
+    output is not finite, and every other one takes the step that it takes alone."""
+    dim, heads, hd, vocab, bad = 256, 4, 64, 600, 599
+    rng = np.random.default_rng(3)
+    mat = lambda *s: (0.05 * rng.standard_normal(s)).astype(np.float32)  # noqa: E731
+    layers = []
+    for _ in range(2):
+        L = dict(wq=mat(dim, heads * hd), wk=mat(dim, kv_heads * hd), wv=mat(dim, kv_heads * hd), wo=mat(heads * hd, dim), w1=mat(dim, 512), w3=mat(dim, 512),
+                 w2=mat(dim, 512), gamma1=np.ones(dim, np.float32), gamma2=np.ones(dim, np.float32))
+        layers.append(L)
+    layers[0]["wv"][0] = 30000.0
+    embed = mat(vocab, dim)
+    embed[:, 0] = 0.0
+    embed[bad, 0] = 10.0
+    cfg = R.Config(dim, 512, heads, hd, 128, 2, vocab, kv_heads=kv_heads)
+    gm = R.Model.new(cfg, layers, dict(gamma_final=np.ones(dim, np.float32), embed=embed), dtype="f16", page_tokens=page_tokens, max_samples=ns)
+    prompt = (np.arange(nprompt) * 7 % 500).astype(np.uint32)
+    gm.prefill(prompt)
+    first = [500 + s for s in range(ns)]
+    first[bad_at] = bad
+    want = []
+    for s in range(ns):
+        gm.set_len(nprompt)
+        if s == bad_at:
+            assert not np.isfinite(gm.decode_token_from_id(bad)).all()
+        want.append(gm.decode_steps_greedy(first[s], 1).tolist() if s != bad_at else None)
+    gm.set_len(nprompt)
+    got, _ = gm.decode_steps_samples(first, 1, mode="greedy")
+    for s in range(ns):
+        if s != bad_at:
+            assert got[s].tolist() == want[s], s
