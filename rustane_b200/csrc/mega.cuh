@@ -440,31 +440,43 @@ template <int NITER> struct Slices<Fp8Row, NITER> {
     }
 };
 // INT4 (groups of 32 with one fp16 scale): a chunk is a group, 4 bytes a lane; its sum times the group's scale in fp32.  A pair
-// of nibbles n = q + 8 masked out of its word is a pair of fp16 subnormals n 2^-24, exactly, or n 2^-20 where they lie four bits
-// up (their inputs carry the missing 2^-4); the sums start at -8 of the inputs', which two MMAs with a constant make for all rows
-// of the stage.  Bound by issue slots: with 1024 + n - 1032 for each pair, and a step's loads right ahead of their use, the 50
-// MB of the 5B model's W1|W3 took 18.0 us.
+// of nibbles n = q + 8 is masked out of its word into the mantissas of a pair of fp16 1024.0 (1024 + n, or 1024 + 16 n where it
+// lies four bits up) and becomes q, exactly, with one more operation.  As the pair of subnormals that the mask alone gives (and the
+// offset off the sums) that operation is saved, but an MMA aligns its products by their operands' exponents, and a subnormal's
+// leading zeros count as digits: the FFN of one layer was off by 5e-6 to 1.2e-5 of its norm where fp32 FMAs leave 2.5e-6 to 8e-6
+// (dims 256 to 1024, even and heavy-tailed inputs); with q the two are equal to 0.4 %.  Bound by issue slots: the 50 MB
+// of the 5B model's W1|W3 take 16.4 us (14.6 as subnormals; 18.0 with a step's loads right ahead of their use), W2 10.6.
 template <int NITER> struct Slices<Int4G32, NITER> {
     // Steps whose words are loaded ahead of the first one's product.  NEAR: a warp takes 16 groups at a time and quad c four
     // neighbours, whose scales are one load, in an order of its own, so that the words of the four quads lie in different banks
-    // (W1|W3 14.8 us, 16.2 without).  Longer rows take groups one by one: W2's 11008 inputs are not a whole number of sixteens a
-    // warp, and the registers do not last (12.9 us against 10.5).
+    // (W1|W3, with subnormals, 14.8 us, 16.2 without).  Longer rows take groups one by one: W2's 11008 inputs are not a whole
+    // number of sixteens a warp, and the registers do not last (12.9 us against 10.5).
     static constexpr int STEPS = 4 * NITER, BATCH = 4, NEAR = NITER == 1 ? 4 : 1;
     uint32_t x[STEPS][4];
     __device__ static int first_group(int i, int c) { return ((i / NEAR * (GEMV_CONSUMERS / 32) + QuantLane::warp()) * 4 + c) * NEAR; }
     __device__ static int group_of(int i, int c) { return first_group(i, c) + ((i + c) & (NEAR - 1)); }
     __device__ void fill(const float* xs, float inv, float up, int K) {
-        const float up4 = up * 0.0625f;
 #pragma unroll
         for (int i = 0; i < STEPS; ++i) {
             const int at = group_of(i, QuantLane::g() >> 1) * 32 + 8 * QuantLane::t();
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
             if (at < K) { a = *reinterpret_cast<const float4*>(xs + at); b = *reinterpret_cast<const float4*>(xs + at + 4); }
             x[i][0] = QuantLane::part(a.x * inv * up, a.y * inv * up);
-            x[i][1] = QuantLane::part(a.z * inv * up4, a.w * inv * up4);
+            x[i][1] = QuantLane::part(a.z * inv * up, a.w * inv * up);
             x[i][2] = QuantLane::part(b.x * inv * up, b.y * inv * up);
-            x[i][3] = QuantLane::part(b.z * inv * up4, b.w * inv * up4);
+            x[i][3] = QuantLane::part(b.z * inv * up, b.w * inv * up);
         }
+    }
+    // the pair of nibbles in bits 0-3 or 4-7 of the halves of a word: as fp16 1024 + n or 1024 + 16 n, and from there n - 8, exactly
+    __device__ static uint32_t low(uint32_t w) {
+        const uint32_t b = (w & 0x000F000Fu) | 0x64006400u;
+        const __half2 q = __hsub2(*reinterpret_cast<const __half2*>(&b), __float2half2_rn(1032.0f));
+        return *reinterpret_cast<const uint32_t*>(&q);
+    }
+    __device__ static uint32_t high(uint32_t w) {
+        const uint32_t b = (w & 0x00F000F0u) | 0x64006400u;
+        const __half2 q = __hfma2(*reinterpret_cast<const __half2*>(&b), __float2half2_rn(0.0625f), __float2half2_rn(-72.0f));
+        return *reinterpret_cast<const uint32_t*>(&q);
     }
     template <int R, class Release> __device__ void rows(uint32_t base, uint32_t row_bytes, int K, const Release& release, float (&acc)[R]) const {
         static_assert(R == 2 || R % 4 == 0, "two rows, or fours");
@@ -503,10 +515,6 @@ template <int NITER> struct Slices<Int4G32, NITER> {
 #pragma unroll
             for (int i = 0; i < BATCH; ++i) {
                 const uint32_t(&b)[4] = x[i0 + i];
-                constexpr uint32_t LOW = 0x000F000Fu, HIGH = 0x00F000F0u, LOW8 = 0x80088008u, HIGH8 = 0x80808080u;  // -8 in either place
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_f16(c, LOW8, LOW8, HIGH8, HIGH8, b[0], b[1]);
-                mma_f16(c, LOW8, LOW8, HIGH8, HIGH8, b[2], b[3]);
                 const uint32_t pick = 0x0010u + 0x0022u * (uint32_t)((i + quad) & 3);  // NEAR: this step's half of the four
                 const bool in = group_of(i0 + i, quad) < ngroups;
                 auto scale_of = [&](int j, int k) {
@@ -515,10 +523,10 @@ template <int NITER> struct Slices<Int4G32, NITER> {
                 };
 #pragma unroll
                 for (int j = 0; j < SETS; ++j) {
-                    float d[4] = {c[0], c[1], c[2], c[3]};
+                    float d[4] = {0.f, 0.f, 0.f, 0.f};
                     const uint32_t u = w[i][j][0], v = P == 2 ? w[i][j][1] : 0u;
-                    mma_f16(d, u & LOW, v & LOW, u & HIGH, v & HIGH, b[0], b[1]);
-                    mma_f16(d, (u >> 8) & LOW, (v >> 8) & LOW, (u >> 8) & HIGH, (v >> 8) & HIGH, b[2], b[3]);
+                    mma_f16(d, low(u), P == 2 ? low(v) : 0u, high(u), P == 2 ? high(v) : 0u, b[0], b[1]);
+                    mma_f16(d, low(u >> 8), P == 2 ? low(v >> 8) : 0u, high(u >> 8), P == 2 ? high(v >> 8) : 0u, b[2], b[3]);
                     sum[j][0] = fmaf(d[0] + d[1], scale_of(j, 0), sum[j][0]);
                     if (P == 2) sum[j][1] = fmaf(d[2] + d[3], scale_of(j, 1), sum[j][1]);
                 }
@@ -526,7 +534,7 @@ template <int NITER> struct Slices<Int4G32, NITER> {
         }
         release();
 #pragma unroll
-        for (int j = 0; j < SETS; ++j) QuantLane::take<R>(4 * j, sum[j][0] * 16777216.0f, sum[j][1] * 16777216.0f, acc);
+        for (int j = 0; j < SETS; ++j) QuantLane::take<R>(4 * j, sum[j][0], sum[j][1], acc);
     }
 };
 

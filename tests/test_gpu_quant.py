@@ -229,3 +229,32 @@ def test_int4_persistent_kernel_matches_the_kernel_per_operator(R, dim, hidden, 
         assert np.isfinite(y).all() and np.abs(x - y).max() <= 2e-4 * np.abs(y).max()
         x, y = a.decode_token_logits_from_id(900), b.decode_token_logits_from_id(900)
         assert np.abs(x - y).max() < 2e-4 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("dtype,limit", [("int4", 3e-6), ("fp8", 3e-6)])
+@pytest.mark.parametrize("dim,hidden", [(256, 640), (512, 1536), (1024, 2848), (512, 12320)])
+def test_quantised_rows_on_the_tensor_cores_keep_the_inputs_23_bits(R, dim, hidden, dtype, limit):
+    """One layer's FFN alone (W_v = 0: no rounded cache entry on the way), rows through the tensor cores and through fp32 FMAs, on
+    inputs whose largest is some hundred times the typical one.  Input pairs are off by 2^-23 and sums of K products round at 2^-24 of
+    their terms: below 1e-6 of the output's norm.  Nibbles as fp16 subnormals had 3e-5 (an MMA aligns its products as if the leading
+    zeros of a subnormal were digits), inputs without their lo parts 1e-4."""
+    rng = np.random.default_rng(dim + hidden)
+    mat = lambda *s: (rng.standard_normal(s) / 25.0).astype(np.float32)  # noqa: E731
+    heads, hd = dim // 64, 64
+    L = dict(wq=mat(dim, dim), wk=mat(dim, dim), wv=np.zeros((dim, dim), np.float32), wo=mat(dim, dim), w1=mat(dim, hidden), w3=mat(dim, hidden), w2=mat(dim, hidden),
+             gamma1=np.ones(dim, np.float32), gamma2=np.ones(dim, np.float32))
+    head = dict(gamma_final=np.ones(dim, np.float32), embed=mat(300, dim))
+    cfg = R.Config(dim, hidden, heads, hd, 64, 1, 300)
+    a, b = (R.Model.new(cfg, [L], head, dtype=dtype, mega=mega) for mega in (True, False))
+    worst = 0.0
+    for _ in range(6):
+        x = (rng.standard_normal(dim) * np.exp(1.5 * rng.standard_normal(dim))).astype(np.float32)
+        outs = []
+        for m in (a, b):
+            m.set_len(0)
+            before = m.kernel_launches()
+            outs.append(m.decode_token(x).astype(np.float64) - x)
+            if m is a:
+                assert m.kernel_launches() - before <= 2  # the persistent kernel
+        worst = max(worst, np.linalg.norm(outs[0] - outs[1]) / np.linalg.norm(outs[1]))
+    assert worst < limit, worst
