@@ -89,7 +89,7 @@ cudaError_t hybrid_step_t(cd_model* m, const cd_step& p) {
             const size_t smem = std::max(mixer_attn_smem_floats(L.ad.kr(), L.ad.vp, L.ad.maps), mixer_mem_smem_floats(L.md.dim)) * sizeof(float);
             auto go = [&](auto kern) {
                 if (smem > 48 * 1024) {
-                    const cudaError_t r_ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                    const cudaError_t r_ = allow_shared_memory((const void*)kern);
                     if (r_ != cudaSuccess) return r_;
                 }
                 return launch_chain(m, kern, dim3(L.md.H * L.md.nslice + L.ad.H * L.nsplit), dim3(MIX_THREADS), smem, q, (KT*)kv);

@@ -91,7 +91,7 @@ cudaError_t launch_attn_window(cd_model* m, const AttnWindow& p, const KT* q_hi,
     const size_t smem = attn_window_smem(p.a.kp, p.a.vp);
     const dim3 grid((p.rows + AW_TILE - 1) / AW_TILE, p.a.H * p.a.maps);
     auto go = [&](auto kern) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_shared_memory((const void*)kern);
         if (e != cudaSuccess) return e;
         kern<<<grid, 128, smem, m->stream>>>(p, q_hi, q_lo, pool, hi, lo);
         m->launches++;

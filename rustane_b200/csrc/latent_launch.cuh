@@ -37,7 +37,7 @@ cudaError_t launch_mla(cd_model* m, const MlaStep& p) {
         if (mma) {
             const size_t smem = mla_mma_smem_bytes(d.row());
             auto go = [&](auto kern, int cols) {
-                cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                const cudaError_t r = allow_shared_memory((const void*)kern);
                 if (r != cudaSuccess) return r;
                 return launch_chain(m, kern, dim3(p.nsplit, d.head_blocks(), (d.latent + cols - 1) / cols), dim3(MLA_MMA_THREADS), smem, (const KT*)p.qsplit, (const KT*)p.pool,
                                     (const int*)m->page_table, (const DevState*)m->st, p.part_acc, p.part_ml, d, p.nsplit, p.scale, &m->st->error);
@@ -49,7 +49,7 @@ cudaError_t launch_mla(cd_model* m, const MlaStep& p) {
     }
     if (!mma) {
         const size_t smem = mla_attn_smem_floats(d) * sizeof(float);
-        TRY(cudaFuncSetAttribute(mla_attn_kernel<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        TRY(allow_shared_memory((const void*)mla_attn_kernel<KT>));
         TRY(launch_chain(m, mla_attn_kernel<KT>, dim3(p.nsplit, d.head_blocks(), d.col_blocks()), dim3(256), smem, (const float*)p.qabs, (const KT*)p.pool,
                          (const int*)m->page_table, (const DevState*)m->st, p.part_acc, p.part_ml, d, p.nsplit, p.scale));
     }

@@ -45,12 +45,8 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     if (fixed + off + (TPAR ? 2 : 4) * stage_cap > budget) return cudaErrorNotSupported;
     const int nstages = (int)std::min<size_t>(16, (budget - fixed - off) / stage_cap) & ~1;  // even: slots alternate between the two consumer groups
     const size_t ring = (size_t)nstages * stage_cap, smem = ring + off;
-    static size_t smem_set = 0;
-    if (smem > smem_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        smem_set = smem;
-    }
+    cudaError_t e = allow_shared_memory((const void*)kern);
+    if (e != cudaSuccess) return e;
     MegaParams p;
     p.layers = (const MegaLayer*)m->mega_layers;
     p.embed = m->embed; p.lm_head = m->lm_head; p.gamma_final = m->gamma_final;
@@ -83,7 +79,7 @@ cudaError_t launch_mega_t(cd_model* m, int input_embed, int want_logits) {
     at[0].val.cooperative = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&lc, kern, p);
+    e = cudaLaunchKernelEx(&lc, kern, p);
     count_launch(m);
     return e;
 }

@@ -4,6 +4,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <set>
+#include <utility>
 
 #include "step.cuh"
 
@@ -87,6 +90,22 @@ void advance(cd_model* m, size_t n) {
 }  // namespace
 
 namespace cd {
+cudaError_t allow_shared_memory(const void* kernel) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;  // (device, kernel)
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const std::lock_guard<std::mutex> lock(mu);
+    if (done.count({dev, kernel})) return cudaSuccess;
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+    if (e == cudaSuccess) done.insert({dev, kernel});
+    return e;
+}
+
 // Counts a launch; in profiling mode also drops an event behind it so the time since
 // the previous event can be charged to the launch's class.
 void count_launch(cd_model* m) {

@@ -236,6 +236,9 @@ int model_finish(cd_model* m);
 int check_room(cd_model* m, size_t need);
 int set_state(cd_model* m, uint32_t token);
 void count_launch(cd_model* m);
+// Lets launches of a kernel take what shared memory a block may have.  The limit belongs to the kernel and is the last one set: a
+// model's own need in its place, set ahead of each launch, is lowered by a smaller model on another thread before the launch.
+cudaError_t allow_shared_memory(const void* kernel);
 // the dense family's batched prompt pass (prefill.cu): on CD_OK the cache holds positions len .. len+n-1 of the prompt in
 // m->prompt_dev and m->x_a holds the last position's hidden state; CD_ERR_UNSUPPORTED: use the per-token path
 int prefill_batched(cd_model* m, size_t n);

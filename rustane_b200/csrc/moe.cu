@@ -102,7 +102,7 @@ GateShape gate_shape(const cd_model* m) {
 template <typename WT>
 cudaError_t launch_gate(cd_model* m, const MoeGate& p, const GateShape& g) {
     auto go = [&](auto kern) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
+        const cudaError_t e = allow_shared_memory((const void*)kern);
         return e != cudaSuccess ? e : launch_chain(m, kern, dim3(m->sm_count), dim3(GEMV_TMA_THREADS), g.smem, p);
     };
     return g.niter == 1 ? go(moe_gate_kernel<WT, 1, 8>) : g.niter == 2 ? go(moe_gate_kernel<WT, 2, 4>) : go(moe_gate_kernel<WT, 4, 2>);
@@ -133,11 +133,7 @@ cudaError_t enqueue_step_moe_t(cd_model* m, const cd_step& p) {
     const int W = mc.kv_latent + mc.rope_dim, QA = c.q_dim + W, units = mc.top_k * c.hidden + S.shared_cols;
     const bool ep = m->tp_world > 1;
     const float scale = 1.0f / std::sqrt((float)c.hd);
-    static size_t w2_set = 0;  // per instantiation
-    if (!S.stream_ffn && (size_t)units * 4 > w2_set) {
-        TRY(cudaFuncSetAttribute(moe_w2_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, units * 4));
-        w2_set = (size_t)units * 4;
-    }
+    if (!S.stream_ffn) TRY(allow_shared_memory((const void*)moe_w2_kernel<WT>));
     const uint32_t es = (uint32_t)sizeof(WT);
     // the next GEMV's first rows, pulled into L2 behind a GEMV's own last loads
     auto hint = [&](const void* w, int K, int N, int unit) {

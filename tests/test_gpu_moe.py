@@ -93,3 +93,30 @@ def test_moe_mla_prompt_session_and_sampling_paths(R, oracle):
     assert greedy == want
     with pytest.raises(R.CudaDecodeError):
         gm.decode_steps_samples([1, 2], 4)
+
+
+def test_two_mixtures_of_different_widths_on_two_threads(R):
+    """The limit of a kernel's shared memory is one for all models of the process: the wide model's kernels have to launch
+    whatever the narrow one's last needed."""
+    import threading
+    narrow, wide = dict(SMALL, seq=400), dict(SMALL, dim=2048, hidden=704, seq=400, vocab=700)
+    models = [R.Model.moe_synthetic(R.MoeConfig(**d), 5, dtype="bf16") for d in (narrow, wide)]
+    alone = [m.decode_token_logits_from_id(7) for m in models]
+    got, failed = [[], []], []
+
+    def go(i):
+        try:
+            for _ in range(300):
+                models[i].set_len(0)
+                got[i].append(models[i].decode_token_logits_from_id(7))
+        except Exception as e:
+            failed.append(e)
+
+    threads = [threading.Thread(target=go, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed[0]
+    for i in range(2):
+        assert all(np.array_equal(g, alone[i]) for g in got[i])
