@@ -2,9 +2,8 @@
 // prompt's full pages are common, later pages a sample's own.
 //
 // Scores against the shared positions are a product with M = (sample, q head) pairs that look at one kv head: mma.m16n8k16,
-// eight pairs a block, their q split into 16-bit parts in rows 0-7 and 8-15, so one instruction gives both parts of eight
-// positions' scores and no shuffle adds them up.  fp16 caches: two parts of q times a power of two (within 2^-23 of q, as in
-// mega.cuh); bf16 caches: three parts, 24 bits.  Probabilities and their products with V stay fp32 FMAs.
+// eight pairs a block, their q split into three 16-bit parts in rows 0-7 and 8-15, so one instruction gives two parts of eight
+// positions' scores and no shuffle adds them up.  Probabilities and their products with V stay fp32 FMAs.
 //
 // grid = (kv heads, slices, blocks of pairs).  The first slices cut the shared positions; the slices behind them cut the samples' own
 // positions, each the same positions of all samples of the block.  A CTA has four warps; a warp takes sixteen positions (of one
@@ -64,17 +63,17 @@ struct SampleAttn {
     float scale;
 };
 
-// the 16-bit parts of a pair of values: hi in rows 0-7, the next in rows 8-15 of one product; a third part in a product of its own
+// The 16-bit parts of a pair of values: hi in rows 0-7 of a product, the next in rows 8-15; the third joins the second's sum.
+// Together they hold all 24 bits (fp16: of a value within 2^-15 of the row's largest, which is scaled to 2^14).
 template <typename KT> struct SaParts;
 template <> struct SaParts<__half> {
-    static constexpr bool THIRD = false, SCALED = true;
-    __device__ static void split(float a, float b, uint32_t (&w)[3]) {
+    static constexpr bool SCALED = true;
+    __device__ static uint32_t next(float& a, float& b) {
         const __half2 p = __floats2half2_rn(a, b);
         const float2 f = __half22float2(p);
-        const __half2 r = __floats2half2_rn(isfinite(f.x) ? a - f.x : 0.0f, isfinite(f.y) ? b - f.y : 0.0f);
-        w[0] = *reinterpret_cast<const uint32_t*>(&p);
-        w[1] = *reinterpret_cast<const uint32_t*>(&r);
-        w[2] = 0u;
+        a = isfinite(f.x) ? a - f.x : 0.0f;
+        b = isfinite(f.y) ? b - f.y : 0.0f;
+        return *reinterpret_cast<const uint32_t*>(&p);
     }
     __device__ static void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
         asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -82,16 +81,13 @@ template <> struct SaParts<__half> {
     }
 };
 template <> struct SaParts<__nv_bfloat16> {
-    static constexpr bool THIRD = true, SCALED = false;
-    __device__ static void split(float a, float b, uint32_t (&w)[3]) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
-            const float2 f = __bfloat1622float2(p);
-            w[i] = *reinterpret_cast<const uint32_t*>(&p);
-            a = isfinite(f.x) ? a - f.x : 0.0f;
-            b = isfinite(f.y) ? b - f.y : 0.0f;
-        }
+    static constexpr bool SCALED = false;
+    __device__ static uint32_t next(float& a, float& b) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+        const float2 f = __bfloat1622float2(p);
+        a = isfinite(f.x) ? a - f.x : 0.0f;
+        b = isfinite(f.y) ? b - f.y : 0.0f;
+        return *reinterpret_cast<const uint32_t*>(&p);
     }
     __device__ static void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
         asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -101,7 +97,7 @@ template <> struct SaParts<__nv_bfloat16> {
 
 // T16: the following GEMM's operand; out[sample][heads * hd] its hi part, out_lo (or nullptr) the remainder
 template <typename KT, typename T16, int HD>
-__global__ void __launch_bounds__(SA_THREADS, SaParts<KT>::THIRD && HD == 128 ? 2 : SA_PER_SM)
+__global__ void __launch_bounds__(SA_THREADS, SA_PER_SM)
 sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ kv_pool, T16* __restrict__ out, T16* __restrict__ out_lo) {
     using Parts = SaParts<KT>;
     constexpr float NEG = -3.402823466e+38f;
@@ -201,32 +197,46 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
         const bool seen = g < rows && (!own || g / nh == z);  // a sample's own positions are its rows' only
         const int at = w0, zt = z;
         {
-            float c[2][4] = {}, d[2][4] = {};
+            // A step's product starts at zero and is added in fp32: an MMA truncates where it adds to its accumulator, and the chain of
+            // them through a head's 128 elements left 2.1 times the error of fp32 FMAs in the output (7.1e-7 and 3.4e-7 behind 1024
+            // positions).  So, with q's 24 bits and one rounding less ahead of the exponential, it is 0.83 to 1.11 times
+            // theirs (heads of 64 and 128, 12 to 1044 positions, even and heavy-tailed q; 16 seeds each); the 5B model's eight
+            // samples take 47.7 ms a call instead of 47.3.
+            float c[2][4] = {}, even[2][4];
 #pragma unroll
             for (int s = 0; s < HD / 16; ++s) {  // step s: elements 4 b .. 4 b + 3, b = s % 2, of chunk 4 (s / 2) + t
-                const float4 v = *reinterpret_cast<const float4*>(qs + g * LDQ + (4 * (s >> 1) + t) * 8 + 4 * (s & 1));
+                float4 v = *reinterpret_cast<const float4*>(qs + g * LDQ + (4 * (s >> 1) + t) * 8 + 4 * (s & 1));
                 uint32_t a[3], b[3];
-                Parts::split(v.x, v.y, a);
-                Parts::split(v.z, v.w, b);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    a[k] = Parts::next(v.x, v.y);
+                    b[k] = Parts::next(v.z, v.w);
+                }
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const uint32_t k0 = (s & 1) ? kw[j][s >> 1].z : kw[j][s >> 1].x, k1 = (s & 1) ? kw[j][s >> 1].w : kw[j][s >> 1].y;
-                    Parts::mma(c[j], a[0], a[1], b[0], b[1], k0, k1);
-                    if (Parts::THIRD) Parts::mma(d[j], a[2], 0u, b[2], 0u, k0, k1);
+                    float part[4] = {};
+                    Parts::mma(part, 0u, a[2], 0u, b[2], k0, k1);
+                    Parts::mma(part, a[0], a[1], b[0], b[1], k0, k1);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (s & 1) c[j][i] += even[j][i] + part[i];
+                        else even[j][i] = part[i];
+                    }
                 }
             }
-            float sc[2][2], top = NEG;  // row g, positions w0 + 8 j + 2 t + {0, 1}
+            float sc[2][2], top = NEG;  // row g, positions w0 + 8 j + 2 t + {0, 1}, ahead of the factor `dn`
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const bool live = seen && at + 8 * j + 2 * t + i < end;
-                    sc[j][i] = live ? (c[j][i] + (c[j][i + 2] + d[j][i])) * dn : NEG;
+                    sc[j][i] = live ? c[j][i] + c[j][i + 2] : NEG;
                     top = fmaxf(top, sc[j][i]);
                 }
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-            const float mnew = fmaxf(m, top), corr = expf(m - mnew);
+            const float mnew = top > NEG ? fmaxf(m, top * dn) : m, corr = expf(m - mnew);
             more = turn(++i);
             if (more) fetch_k();  // (the products with the last ones are done)
             __syncwarp();
@@ -236,7 +246,7 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const bool live = seen && at + 8 * j + 2 * t + i < end;
-                    const float e = live ? expf(sc[j][i] - mnew) : 0.0f;
+                    const float e = live ? expf(fmaf(sc[j][i], dn, -mnew)) : 0.0f;
                     lsum += e;
                     probs[(8 * j + 2 * t + i) * SA_ROWS + g] = e;
                 }
