@@ -223,6 +223,37 @@ template <> struct Elem<__half> {
     __device__ static inline float to_f32(__half v) { return __half2float(v); }
 };
 
+// ------------------------------------------------------------------ mma.sync on 16-bit operands
+// d += A B, fp32 sums (m16n8k16).  All 32 lanes of a warp take part: volatile keeps the instruction ahead of divergent code behind it.
+// part: the next 16-bit part of a pair of fp32 values, which become the remainders (zero where a part is not finite).
+template <typename T> struct Mma16;
+template <> struct Mma16<__half> {
+    __device__ static inline void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+    __device__ static inline uint32_t part(float& a, float& b) {
+        const __half2 p = __floats2half2_rn(a, b);
+        const float2 f = __half22float2(p);
+        a = isfinite(f.x) ? a - f.x : 0.0f;
+        b = isfinite(f.y) ? b - f.y : 0.0f;
+        return *reinterpret_cast<const uint32_t*>(&p);
+    }
+};
+template <> struct Mma16<__nv_bfloat16> {
+    __device__ static inline void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+    __device__ static inline uint32_t part(float& a, float& b) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+        const float2 f = __bfloat1622float2(p);
+        a = isfinite(f.x) ? a - f.x : 0.0f;
+        b = isfinite(f.y) ? b - f.y : 0.0f;
+        return *reinterpret_cast<const uint32_t*>(&p);
+    }
+};
+
 // ------------------------------------------------------------------ weight-row formats of the GEMV
 // How one matrix row is laid out in HBM and how a 16-byte chunk of it meets the
 // thread's slice of x.  Plain element types: K elements, nothing else.  The two

@@ -332,18 +332,6 @@ template <typename LT> struct RowChunks {  // this thread's 16-byte chunks of a 
         return c < nchunks ? lds128(base + (uint32_t)j * row_bytes + (uint32_t)c * 16u) : make_uint4(0, 0, 0, 0);
     }
 };
-// a pair of fp32 values as fp16 hi + lo
-__device__ inline void fp16_pair(uint32_t& h, uint32_t& l, float a, float b) {
-    const __half2 p = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(p);
-    const __half2 q = __floats2half2_rn(isfinite(f.x) ? a - f.x : 0.0f, isfinite(f.y) ? b - f.y : 0.0f);
-    h = *reinterpret_cast<const uint32_t*>(&p);
-    l = *reinterpret_cast<const uint32_t*>(&q);
-}
-__device__ inline void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 // ---- the input slice a thread holds (chunks tid, tid + 256, ... of the vector, the same in both groups), and the rows of
 // a stage times it
 template <typename LT, int NITER> struct Slices {
@@ -392,9 +380,8 @@ struct QuantLane {
     }
     // the hi (even columns) or lo part of two inputs
     static __device__ uint32_t part(float a, float b) {
-        uint32_t h, l;
-        fp16_pair(h, l, a, b);
-        return g() & 1 ? l : h;
+        const uint32_t hi = Mma16<__half>::part(a, b), lo = Mma16<__half>::part(a, b);
+        return g() & 1 ? lo : hi;
     }
 };
 // FP8: a chunk is 64 bytes, 16 a lane
@@ -433,7 +420,8 @@ template <int NITER> struct Slices<Fp8Row, NITER> {
             const uint32_t u[4] = {w0.x, w0.y, w0.z, w0.w}, v[4] = {w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                mma_f16(d[k & 1], widen(u[k] & 0xffffu), R == 4 ? widen(v[k] & 0xffffu) : 0u, widen(u[k] >> 16), R == 4 ? widen(v[k] >> 16) : 0u, x[i][2 * k], x[i][2 * k + 1]);
+                Mma16<__half>::mma(d[k & 1], {widen(u[k] & 0xffffu), R == 4 ? widen(v[k] & 0xffffu) : 0u, widen(u[k] >> 16), R == 4 ? widen(v[k] >> 16) : 0u}, x[i][2 * k],
+                                   x[i][2 * k + 1]);
         }
         release();
         QuantLane::take<R>(0, (d[0][0] + d[0][1]) + (d[1][0] + d[1][1]), (d[0][2] + d[0][3]) + (d[1][2] + d[1][3]), acc);
@@ -525,8 +513,8 @@ template <int NITER> struct Slices<Int4G32, NITER> {
                 for (int j = 0; j < SETS; ++j) {
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
                     const uint32_t u = w[i][j][0], v = P == 2 ? w[i][j][1] : 0u;
-                    mma_f16(d, low(u), P == 2 ? low(v) : 0u, high(u), P == 2 ? high(v) : 0u, b[0], b[1]);
-                    mma_f16(d, low(u >> 8), P == 2 ? low(v >> 8) : 0u, high(u >> 8), P == 2 ? high(v >> 8) : 0u, b[2], b[3]);
+                    Mma16<__half>::mma(d, {low(u), P == 2 ? low(v) : 0u, high(u), P == 2 ? high(v) : 0u}, b[0], b[1]);
+                    Mma16<__half>::mma(d, {low(u >> 8), P == 2 ? low(v >> 8) : 0u, high(u >> 8), P == 2 ? high(v >> 8) : 0u}, b[2], b[3]);
                     sum[j][0] = fmaf(d[0] + d[1], scale_of(j, 0), sum[j][0]);
                     if (P == 2) sum[j][1] = fmaf(d[2] + d[3], scale_of(j, 1), sum[j][1]);
                 }
@@ -958,9 +946,13 @@ __device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int at
         for (int s = 0; s < 8; ++s) {
             const int d = (4 * (s >> 1) + t) * 8 + 4 * (s & 1);
             const bool live = g < p.gqa && d < HD;
-            const float4 v = live ? *reinterpret_cast<const float4*>(sh.q + g * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-            fp16_pair(qa[s][0], qa[s][1], v.x * up, v.y * up);
-            fp16_pair(qa[s][2], qa[s][3], v.z * up, v.w * up);
+            float4 v = live ? *reinterpret_cast<const float4*>(sh.q + g * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v.x *= up; v.y *= up; v.z *= up; v.w *= up;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {  // hi, lo
+                qa[s][k] = Mma16<__half>::part(v.x, v.y);
+                qa[s][2 + k] = Mma16<__half>::part(v.z, v.w);
+            }
         }
         float acc[NH][8], m = NEG, lsum = 0.0f;  // m, lsum: of head h0 + g (lsum of this lane's positions), meaningful for g < NH
 #pragma unroll
@@ -995,8 +987,8 @@ __device__ inline bool attention_grouped(Ring& ring, const MegaParams& p, int at
                         const int ch = 4 * j + t;
                         uint4 k = make_uint4(0, 0, 0, 0);
                         if (klive) k = kpos == pos ? sh.row[ch] : lds128(kbase + (uint32_t)(w0 + g) * row_bytes + (uint32_t)ch * 16u);
-                        mma_f16(c, qa[2 * j][0], qa[2 * j][1], qa[2 * j][2], qa[2 * j][3], k.x, k.y);
-                        mma_f16(c2, qa[2 * j + 1][0], qa[2 * j + 1][1], qa[2 * j + 1][2], qa[2 * j + 1][3], k.z, k.w);
+                        Mma16<__half>::mma(c, qa[2 * j], k.x, k.y);
+                        Mma16<__half>::mma(c2, qa[2 * j + 1], k.z, k.w);
                     }
                 }
                 // scores of head g at positions 2 t and 2 t + 1; this warp's heads move to g = 0 .. NH - 1

@@ -16,6 +16,7 @@
 // samples, with five shuffles per position, head and sample, took 33 us of the layer; a conversion kernel followed.
 #pragma once
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -63,43 +64,12 @@ struct SampleAttn {
     float scale;
 };
 
-// The 16-bit parts of a pair of values: hi in rows 0-7 of a product, the next in rows 8-15; the third joins the second's sum.
-// Together they hold all 24 bits (fp16: of a value within 2^-15 of the row's largest, which is scaled to 2^14).
-template <typename KT> struct SaParts;
-template <> struct SaParts<__half> {
-    static constexpr bool SCALED = true;
-    __device__ static uint32_t next(float& a, float& b) {
-        const __half2 p = __floats2half2_rn(a, b);
-        const float2 f = __half22float2(p);
-        a = isfinite(f.x) ? a - f.x : 0.0f;
-        b = isfinite(f.y) ? b - f.y : 0.0f;
-        return *reinterpret_cast<const uint32_t*>(&p);
-    }
-    __device__ static void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-};
-template <> struct SaParts<__nv_bfloat16> {
-    static constexpr bool SCALED = false;
-    __device__ static uint32_t next(float& a, float& b) {
-        const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
-        const float2 f = __bfloat1622float2(p);
-        a = isfinite(f.x) ? a - f.x : 0.0f;
-        b = isfinite(f.y) ? b - f.y : 0.0f;
-        return *reinterpret_cast<const uint32_t*>(&p);
-    }
-    __device__ static void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-};
-
 // T16: the following GEMM's operand; out[sample][heads * hd] its hi part, out_lo (or nullptr) the remainder
 template <typename KT, typename T16, int HD>
 __global__ void __launch_bounds__(SA_THREADS, SA_PER_SM)
 sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ kv_pool, T16* __restrict__ out, T16* __restrict__ out_lo) {
-    using Parts = SaParts<KT>;
+    using X = Mma16<KT>;
+    constexpr bool SCALED = std::is_same<KT, __half>::value;
     constexpr float NEG = -3.402823466e+38f;
     constexpr int CH = HD / 8, SIDES = 32 / CH, NV = 16 / SIDES, NK = CH / 4;  // 16-byte chunks of a row; V rows side by side, and in turn; K chunks a lane
     constexpr int LDQ = HD + 4;                                                 // (rows of q on different banks)
@@ -172,7 +142,7 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
             mx = fmaxf(fmaxf(fmaxf(mx, fabsf(v[i].x)), fmaxf(fabsf(v[i].y), fabsf(v[i].z))), fabsf(v[i].w));
         }
         float up = 1.0f, dn = 1.0f;
-        if (Parts::SCALED) {
+        if (SCALED) {
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             const int e = (int)(__float_as_uint(mx) >> 23), f = e == 255 ? 127 : min(253, max(1, 268 - e));
@@ -206,18 +176,20 @@ sample_attn_kernel(const __grid_constant__ SampleAttn p, const KT* __restrict__ 
 #pragma unroll
             for (int s = 0; s < HD / 16; ++s) {  // step s: elements 4 b .. 4 b + 3, b = s % 2, of chunk 4 (s / 2) + t
                 float4 v = *reinterpret_cast<const float4*>(qs + g * LDQ + (4 * (s >> 1) + t) * 8 + 4 * (s & 1));
+                // hi parts in rows 0-7, the next in rows 8-15; the third joins the second's sum.  Together they hold all 24 bits (fp16: of
+                // a value within 2^-15 of the row's largest)
                 uint32_t a[3], b[3];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    a[k] = Parts::next(v.x, v.y);
-                    b[k] = Parts::next(v.z, v.w);
+                    a[k] = X::part(v.x, v.y);
+                    b[k] = X::part(v.z, v.w);
                 }
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const uint32_t k0 = (s & 1) ? kw[j][s >> 1].z : kw[j][s >> 1].x, k1 = (s & 1) ? kw[j][s >> 1].w : kw[j][s >> 1].y;
                     float part[4] = {};
-                    Parts::mma(part, 0u, a[2], 0u, b[2], k0, k1);
-                    Parts::mma(part, a[0], a[1], b[0], b[1], k0, k1);
+                    X::mma(part, {0u, a[2], 0u, b[2]}, k0, k1);
+                    X::mma(part, {a[0], a[1], b[0], b[1]}, k0, k1);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         if (s & 1) c[j][i] += even[j][i] + part[i];
