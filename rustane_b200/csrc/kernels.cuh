@@ -340,7 +340,9 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
             for (int g = 0; g < ngroups; ++g) {
                 if (next.test_drop && blockIdx.x == 0 && g == ngroups - 1) break;  // test hook: this stage never arrives
                 const int s = g % nstages;
-                if (g >= nstages && !mbar_wait(empty0 + 8u * s, ((g / nstages) - 1) & 1)) {
+                bool ok = g < nstages || mbar_wait(empty0 + 8u * s, ((g / nstages) - 1) & 1);
+                if constexpr (Src::DYNAMIC) ok = __all_sync(0xffffffffu, ok);  // all lanes copy on, or none: their bounded waits may end apart
+                if (!ok) {
                     atomicExch(err, DEV_ERR_EMPTY_WAIT);
                     break;
                 }
