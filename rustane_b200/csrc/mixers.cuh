@@ -213,6 +213,8 @@ struct InParallelMix {
     template <int NITER, int EPC, class Begin>
     __device__ void load(float (&xr)[NITER][EPC], int tid, int nchunks, float* red, const Begin& begin, bool, bool writer) const {
         constexpr bool AHEAD = NITER * EPC <= 16;  // the weights ahead of the wait, the vectors once, where registers allow
+        // (a sum of squares with its roundings written out: which products the compiler fuses otherwise follows the code around it)
+        auto squares = [](const float4& v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.x, v.x, v.y * v.y))); };
         constexpr int NA = AHEAD ? NITER : 1;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         float4 wp[NA][EPC / 4], wq[NA][EPC / 4], wg[NA][EPC / 4], va[NA][EPC / 4], vb[NA][EPC / 4], vx[NA][EPC / 4];
@@ -236,8 +238,8 @@ struct InParallelMix {
             for (int e = 0; e < EPC; e += 4) {
                 const float4 a = vec(yl, c, e), b = vec(yr, c, e);
                 if constexpr (AHEAD) { va[i][e / 4] = a; vb[i][e / 4] = b; vx[i][e / 4] = vec(x, c, e); }
-                sl += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
-                sr += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+                sl += squares(a);
+                sr += squares(b);
             }
         }
         const float2 both = consumer_sum2(sl, sr, red);
@@ -257,7 +259,7 @@ struct InParallelMix {
                 }
                 const float4 z = make_float4(a.x * rl * p.x + b.x * rr * q.x, a.y * rl * p.y + b.y * rr * q.y, a.z * rl * p.z + b.z * rr * q.z, a.w * rl * p.w + b.w * rr * q.w);
                 xr[i][e] = z.x; xr[i][e + 1] = z.y; xr[i][e + 2] = z.z; xr[i][e + 3] = z.w;
-                ss += z.x * z.x + z.y * z.y + z.z * z.z + z.w * z.w;
+                ss += squares(z);
             }
         }
         const float r = mult / sqrtf(consumer_sum(ss, red) * (1.0f / (float)n) + eps);
