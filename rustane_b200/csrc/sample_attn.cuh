@@ -15,42 +15,12 @@
 // the bytes (16.8 MB a layer of the 5B model at 1024 positions) are there before q is.  One CUDA-core CTA per q head, slice and two
 // samples, with five shuffles per position, head and sample, took 33 us of the layer; a conversion kernel followed.
 #pragma once
-#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
+#include "sample_split.h"
 
 namespace cd {
-
-constexpr int SA_ROWS = 8, SA_TILE = 64, SA_WARP_TILE = 16, SA_THREADS = 128, SA_PER_SM = 3;
-
-// How `heads / kv_heads` q heads of `samples` samples make blocks of at most SA_ROWS pairs: several samples with all their heads
-// of the group, or some heads of one sample.
-struct SaBlocks {
-    int gqa, samples;
-    __host__ __device__ int heads() const { return gqa < SA_ROWS ? gqa : SA_ROWS; }            // q heads of a sample in a block
-    __host__ __device__ int head_blocks() const { return (gqa + SA_ROWS - 1) / SA_ROWS; }
-    __host__ __device__ int per_block() const { return SA_ROWS / heads(); }                    // samples in a block (1 where the heads fill it)
-    __host__ __device__ int count() const { return head_blocks() * ((samples + per_block() - 1) / per_block()); }
-};
-
-// Slices of a step at this length: every CTA takes at most `rounds` turns of sixteen positions a warp (a slice of own positions:
-// `spans` times sixteen positions of each sample), as few as the partials' buffers and one wave of CTAs allow.  (A second wave costs
-// as much as the first: its positions are requested only when it starts.)
-struct SaSplit {
-    int rounds, spans, shared, own;
-    int id() const { return (rounds * 64 + shared) * 64 + own; }
-};
-inline SaSplit sa_split(int shared_tokens, int attn_len, const SaBlocks& blocks, int kv_heads, int max_slices, int sms) {
-    auto up = [](int a, int b) { return (a + b - 1) / b; };
-    const int ts = up(shared_tokens, SA_TILE), to = up(attn_len - shared_tokens, SA_WARP_TILE);
-    const int most = std::min(max_slices, std::max(sms * SA_PER_SM / (kv_heads * blocks.count()), ts > 0 ? 2 : 1));
-    for (int r = 1;; ++r) {
-        const SaSplit s{r, std::max(1, 4 * r / std::min(blocks.per_block(), blocks.samples)), up(ts, r), 0};
-        const int own = up(to, s.spans);
-        if (s.shared + own <= most || r >= ts + to * SA_ROWS) return SaSplit{r, s.spans, s.shared, own};
-    }
-}
 
 struct SampleAttn {
     const float* q;          // [samples][heads][hd]
