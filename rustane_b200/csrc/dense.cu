@@ -139,9 +139,9 @@ static int validate(const cd_config& c, int dtype) {
 // which walk their tiles of it one after the other: 0.5 us a tile, 1 to 1.2 with 2 or 4 q heads per kv head, 1.9 with 8.  The kernel
 // per operator spreads q heads times up to 32 slices.  Over 270 shapes (dim 512 to 4096; f32, 16 bits, FP8; 1 to 8 q heads per
 // kv head; 40 to 3500 positions) the tiles at which the two meet grow with the bytes of a layer's weights, as below; the choice
-// is within 0.2 % of the better form in the mean, 0.7 % over 76 cells of INT4.  Us a token of 8 layers, persistent and per operator: dim 1024 in bf16, 8 q heads
-// on one kv head, 64 positions 200 and 219, 1000 positions 256 and 222 (limit 490); dim 2048, 16 on 4, 1000 positions 279 and 317
-// (limit 5600).  Grouped heads of small layers: 0.90 to 1.05 of the other's speed at any length.
+// is within 0.2 % of the better form in the mean, 0.5 % over 88 cells of INT4 (10 % off at dim 4096, 8 q heads per kv head, 3500
+// positions).  Us a token of 8 layers, persistent and per operator: dim 1024 in bf16, 8 q heads on one kv head, 64 positions 200 and
+// 219, 1000 positions 256 and 222 (limit 490); dim 2048, 16 on 4, 1000 positions 279 and 317 (limit 5600).  Grouped heads of small layers: 0.90 to 1.05 of the other's speed at any length.
 static size_t persistent_positions(const cd_model* m, size_t layer_bytes) {
     struct Line { double tiles, per_mb, none_below_mb; };
     const cd_config& c = m->cfg;

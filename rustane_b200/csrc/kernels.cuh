@@ -389,63 +389,63 @@ gemv_tma_kernel(const WT* __restrict__ W, const float* __restrict__ x, const flo
         static_assert(G == 1, "one consumer group");
         in.load(xr, tid, nchunks, red, begin, Src::PAIR && unit0 > 0, bid == 0 && unit0 == 0);
     } else {
-    begin();
-    float ss = 0.0f;
-    const float* inbox = nullptr;  // tensor parallel: the input is res + alpha * (sum of the peers' partial vectors)
-    if (tp.world > 1 && tp.in_reduce) {
-        const unsigned int seq = __ldcg(&tp.st->ar_base) + (unsigned int)tp.in_reduce;
-        float* base = reinterpret_cast<float*>(tp.peers[tp.rank]);
-        inbox = base + (size_t)(seq % 3u) * tp.world * tp.dim;
-        // re-arm the slot two all-reduces ahead (nobody reads or writes it now), split over the CTAs
-        uint4* rearm = reinterpret_cast<uint4*>(base + (size_t)((seq + 2u) % 3u) * tp.world * tp.dim);
-        const int n4 = group == 0 ? tp.world * tp.dim / 4 : 0;
-        for (int j = blockIdx.x * GEMV_CONSUMERS + tid; j < n4; j += gridDim.x * GEMV_CONSUMERS)
-            rearm[j] = make_uint4(TP_SENTINEL, TP_SENTINEL, TP_SENTINEL, TP_SENTINEL);
-    }
-#pragma unroll
-    for (int i = 0; i < NITER; ++i) {
-        const int c = tid + i * GEMV_CONSUMERS;
-#pragma unroll
-        for (int e = 0; e < EPC; e += 4) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (c < nchunks) {
-                if (inbox != nullptr) {
-                    float4 a;  // summed in fixed rank order: identical on every rank
-                    if (!tp_gather4(inbox, tp.world, tp.dim, (size_t)c * EPC + e, a, tp.st, tp.wait_ns)) atomicCAS(err, 0, DEV_ERR_TP_WAIT);
-                    const float4 r4 = __ldcg(reinterpret_cast<const float4*>(tp.res + (size_t)c * EPC + e));
-                    v = make_float4(r4.x + tp.alpha * a.x, r4.y + tp.alpha * a.y, r4.z + tp.alpha * a.z, r4.w + tp.alpha * a.w);
-                    if (blockIdx.x == 0 && group == 0) *reinterpret_cast<float4*>(tp.x_out + (size_t)c * EPC + e) = v;
-                } else {
-                    v = __ldcg(reinterpret_cast<const float4*>(x + (size_t)c * EPC + e));
-                }
-            }
-            xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
-            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        begin();
+        float ss = 0.0f;
+        const float* inbox = nullptr;  // tensor parallel: the input is res + alpha * (sum of the peers' partial vectors)
+        if (tp.world > 1 && tp.in_reduce) {
+            const unsigned int seq = __ldcg(&tp.st->ar_base) + (unsigned int)tp.in_reduce;
+            float* base = reinterpret_cast<float*>(tp.peers[tp.rank]);
+            inbox = base + (size_t)(seq % 3u) * tp.world * tp.dim;
+            // re-arm the slot two all-reduces ahead (nobody reads or writes it now), split over the CTAs
+            uint4* rearm = reinterpret_cast<uint4*>(base + (size_t)((seq + 2u) % 3u) * tp.world * tp.dim);
+            const int n4 = group == 0 ? tp.world * tp.dim / 4 : 0;
+            for (int j = blockIdx.x * GEMV_CONSUMERS + tid; j < n4; j += gridDim.x * GEMV_CONSUMERS)
+                rearm[j] = make_uint4(TP_SENTINEL, TP_SENTINEL, TP_SENTINEL, TP_SENTINEL);
         }
-    }
-    if (NORM) {
-        const float tot = consumer_sum(ss, red + 8 * group, group);
-        const float inv = 1.0f / sqrtf(tot * (1.0f / (float)K) + eps);
 #pragma unroll
         for (int i = 0; i < NITER; ++i) {
             const int c = tid + i * GEMV_CONSUMERS;
-            if (c < nchunks) {
 #pragma unroll
-                for (int e = 0; e < EPC; e += 4) {
-                    float4 g;
-                    if constexpr (GAMMA_AHEAD) g = make_float4(gm[i][e], gm[i][e + 1], gm[i][e + 2], gm[i][e + 3]);
-                    else g = *reinterpret_cast<const float4*>(gamma + (size_t)c * EPC + e);
-                    xr[i][e] = xr[i][e] * inv * g.x;
-                    xr[i][e + 1] = xr[i][e + 1] * inv * g.y;
-                    xr[i][e + 2] = xr[i][e + 2] * inv * g.z;
-                    xr[i][e + 3] = xr[i][e + 3] * inv * g.w;
-                    if (norm_out != nullptr && blockIdx.x == 0 && group == 0)
-                        *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) =
-                            make_float4(xr[i][e], xr[i][e + 1], xr[i][e + 2], xr[i][e + 3]);
+            for (int e = 0; e < EPC; e += 4) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c < nchunks) {
+                    if (inbox != nullptr) {
+                        float4 a;  // summed in fixed rank order: identical on every rank
+                        if (!tp_gather4(inbox, tp.world, tp.dim, (size_t)c * EPC + e, a, tp.st, tp.wait_ns)) atomicCAS(err, 0, DEV_ERR_TP_WAIT);
+                        const float4 r4 = __ldcg(reinterpret_cast<const float4*>(tp.res + (size_t)c * EPC + e));
+                        v = make_float4(r4.x + tp.alpha * a.x, r4.y + tp.alpha * a.y, r4.z + tp.alpha * a.z, r4.w + tp.alpha * a.w);
+                        if (blockIdx.x == 0 && group == 0) *reinterpret_cast<float4*>(tp.x_out + (size_t)c * EPC + e) = v;
+                    } else {
+                        v = __ldcg(reinterpret_cast<const float4*>(x + (size_t)c * EPC + e));
+                    }
+                }
+                xr[i][e] = v.x; xr[i][e + 1] = v.y; xr[i][e + 2] = v.z; xr[i][e + 3] = v.w;
+                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            }
+        }
+        if (NORM) {
+            const float tot = consumer_sum(ss, red + 8 * group, group);
+            const float inv = 1.0f / sqrtf(tot * (1.0f / (float)K) + eps);
+#pragma unroll
+            for (int i = 0; i < NITER; ++i) {
+                const int c = tid + i * GEMV_CONSUMERS;
+                if (c < nchunks) {
+#pragma unroll
+                    for (int e = 0; e < EPC; e += 4) {
+                        float4 g;
+                        if constexpr (GAMMA_AHEAD) g = make_float4(gm[i][e], gm[i][e + 1], gm[i][e + 2], gm[i][e + 3]);
+                        else g = *reinterpret_cast<const float4*>(gamma + (size_t)c * EPC + e);
+                        xr[i][e] = xr[i][e] * inv * g.x;
+                        xr[i][e + 1] = xr[i][e + 1] * inv * g.y;
+                        xr[i][e + 2] = xr[i][e + 2] * inv * g.z;
+                        xr[i][e + 3] = xr[i][e + 3] * inv * g.w;
+                        if (norm_out != nullptr && blockIdx.x == 0 && group == 0)
+                            *reinterpret_cast<float4*>(norm_out + (size_t)c * EPC + e) =
+                                make_float4(xr[i][e], xr[i][e + 1], xr[i][e + 2], xr[i][e + 3]);
+                    }
                 }
             }
         }
-    }
     }
 
     bool ok = true;

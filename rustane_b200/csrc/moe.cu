@@ -83,7 +83,8 @@ void moe_release(cd_model* m) {
     m->moe = nullptr;
 }
 
-// How moe_gate_kernel takes a model's rows (eight rows a stage, fewer where a thread holds several chunks of x: with four, 16 KB, one thread could not issue copies as fast as HBM answers); nstages 0: it does not.
+// How moe_gate_kernel takes a model's rows (eight rows a stage, fewer where a thread holds several chunks of x: with four, 16 KB,
+// one thread could not issue copies as fast as HBM answers); nstages 0: it does not.
 struct GateShape {
     int niter, rows_cap, nstages;
     size_t smem;
@@ -161,8 +162,9 @@ cudaError_t enqueue_step_moe_t(cd_model* m, const cd_step& p) {
         if (fused_route) {
             const int wo_ctas = std::min(c.dim, m->sm_count);
             const size_t row = (size_t)units * es;
-            const MoeGate g{L.w13, L.ws13, m->x_b, L.gamma2, S.route_part, wo_ctas, c.dim, c.hidden, S.shared_cols, RouteRule{mc.n_experts, mc.top_k, 1, 1}, sel, S.sel_w,
-                      S.loc_ids, S.n_loc, S.gate, gate.nstages, gate.rows_cap, &m->st->error, L.w2, L.ws2, (int)((size_t)m->prefetch_kb * 1024 / row)};
+            const MoeGate g{L.w13, L.ws13, m->x_b, L.gamma2, S.route_part, wo_ctas, c.dim, c.hidden, S.shared_cols,
+                            RouteRule{mc.n_experts, mc.top_k, 1, 1}, sel, S.sel_w, S.loc_ids, S.n_loc, S.gate, gate.nstages, gate.rows_cap, &m->st->error,
+                            L.w2, L.ws2, (int)((size_t)m->prefetch_kb * 1024 / row)};
             TRY((launch_gemv<WT, 1, false>(m, L.wo, m->attn, nullptr, nullptr, c.dim, c.heads * mc.v_dim,
                                            EpiResidualRoute<WT>{m->x_a, m->x_b, m->alpha, L.gamma2, (const WT*)L.wr, S.route_part, c.dim, mc.n_experts})));
             m->cur_cls = CLS_W13;
